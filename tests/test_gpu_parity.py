@@ -286,3 +286,25 @@ def test_standard_vcycle(kind):
     f = m.F[:, 0]
     assert abs(its - itso) <= 1
     assert abs(f @ u - f @ uo) / abs(f @ uo) < 1e-8
+
+
+@pytest.mark.parametrize("shape", [(3, 3, 3), (8, 6, 5), (15, 71, 9), (31, 33, 17), (63, 16, 40), (130, 9, 11)])
+@pytest.mark.parametrize("holes", [False, True])
+def test_ku_tile_edges(shape, holes):
+    # K*u tiles: the smallest grid (one tile, one chunk), extents around a tile's height and width,
+    # z-chunks with a short last one, several y tiles; with holes the tiles come from the domain's list
+    from top3d_xl_b200 import Context
+    vox = np.ones(shape, bool)
+    if holes:
+        vox[:, 1:-1, :] = np.random.default_rng(3).random((shape[0], shape[1] - 2, shape[2])) < 0.7
+    m = O.build_model(vox)
+    x = np.random.default_rng(1).uniform(0.05, 1.0, m.levels[0].numElements)
+    S = m.S
+    E = S.modulusMin + x ** S.SIMPpenalty * (S.modulus - S.modulusMin)
+    sol = O.Solver(m)
+    sol.assemble(E)
+    u = np.random.default_rng(2).standard_normal(m.levels[0].numDOFs)
+    with Context("fp64") as ctx:
+        ctx.load_voxels(vox)
+        ctx.set_moduli(E)
+        assert _rel(ctx.ku(u), sol.ku(u)) < 1e-13

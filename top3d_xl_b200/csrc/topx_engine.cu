@@ -21,7 +21,7 @@ Engine::Engine(Model& model, int precision, int device, bool coarse_coop) : M(mo
   // other host threads (and their synchronous set-up copies) never stall or break this one's
   // graph captures; every host-side copy below waits for this stream first
   TOPX_CUDA_OK(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
-  prepare_fem_kernels();
+  prepare_ku_kernels();
   prepare_nd_kernels();
   nl = M.numLevels;
   if (nl < 3 || int(M.levels.size()) != nl) throw std::runtime_error("model hierarchy not built");
@@ -108,6 +108,7 @@ Engine::Engine(Model& model, int precision, int device, bool coarse_coop) : M(mo
   }
   // ---- element matrices ---------------------------------------------------------
   upload_ke(M.Ke.data());
+  kumodes = ku_modes(M.Ke.data());
   {
     std::vector<double> T2 = galerkin_templates(M.Ke, M.levels[1].span);
     const std::vector<double> P4 = child_prolongators(M.levels[1].span);
@@ -185,22 +186,19 @@ Engine::Engine(Model& model, int precision, int device, bool coarse_coop) : M(mo
   {
     std::vector<uint8_t> pn(size_t(G[0].nnodes()), 0);
     for (auto k : M.levels[0].nodMapBack) pn[k - 1] = 1;
+    kush = ku_shape(G[0]);
     std::vector<uint32_t> zr;
-    const std::vector<uint32_t> act = ku_active_tiles(G[0], pn, &zr);
+    const std::vector<uint32_t> act = ku_active_tiles(G[0], kush, pn, &zr);
     const std::vector<uint8_t> all(pn.size(), 1);
-    const size_t full = ku_active_tiles(G[0], all).size();
+    const size_t full = size_t(kush.grid.x) * kush.grid.y * kush.grid.z;
     if (!act.empty() && act.size() < full * 9 / 10) {
       kuTiles.upload(act.data(), act.size());
-      // an empty row list (no present node on the row y = ny) launches no last-row kernel
-      const std::vector<uint32_t> rows = ku_active_row_tiles(G[0], pn);
-      if (!rows.empty()) kuRows.upload(rows.data(), rows.size());
       kuZr.upload(zr.data(), zr.size());
-      kut = KuTiles{kuTiles.p, int(act.size()), rows.empty() ? kuTiles.p : kuRows.p, int(rows.size()), kuZr.p};
     }
     const std::vector<uint32_t> fact = filter_active_tiles(G[0], pn);
     if (!fact.empty() && fact.size() < filter_active_tiles(G[0], all).size() * 9 / 10) {
       filterTiles.upload(fact.data(), fact.size());
-      fut = KuTiles{filterTiles.p, int(fact.size())};
+      fut = FilterTiles{filterTiles.p, int(fact.size())};
     }
     // elementwise level-1 passes skip the 32-node chunks without a present node
     const size_t nchunk = (pn.size() + 31) / 32;
@@ -568,7 +566,7 @@ void Engine::vcycle_standard(bool init, PcgScalars* sc) {
   const double om = M.S.weightFactorJacobi;
   sec_begin(SEC_RESTRICT);
   launch_jacobi_pre<double, double, double>(st, G[0], kw.r.p, v.d1.p, present[0].p, kw.z.p, om, sc);
-  launch_ku<double>(st, KU_PLAIN, G[0], kw.z.p, nullptr, nullptr, kw.q.p, E64.p, fixbits.p, cfix64.p, sc, rs1, kut);
+  ku(KU_PLAIN, kw.z.p, nullptr, nullptr, kw.q.p, sc, nullptr);
   launch_residual_inplace<double, double>(st, G[0], kw.r.p, kw.q.p, sc);
   launch_restrict<double, double>(st, M.levels[1].span, kw.q.p, G[0], v.tmp1.p, v.tmp2.p, v.rl[1].p, G[1], cols1);
   for (int l = 1; l < nl - 1; ++l) {
@@ -592,7 +590,7 @@ void Engine::vcycle_standard(bool init, PcgScalars* sc) {
   }
   launch_prolong_add<double, double, double>(st, M.levels[1].span, v.xl[1].p, G[1], kw.r.p, v.d1.p, present[0].p,
                                              kw.z.p, G[0], om, sc);
-  launch_ku<double>(st, KU_PLAIN, G[0], kw.z.p, nullptr, nullptr, kw.q.p, E64.p, fixbits.p, cfix64.p, sc, rs1, kut);
+  ku(KU_PLAIN, kw.z.p, nullptr, nullptr, kw.q.p, sc, nullptr);
   launch_jacobi_correct<double, double, double>(st, G[0], kw.r.p, kw.q.p, v.d1.p, present[0].p, kw.z.p, om, true,
                                                 init, sc, rs1);
   sec_end();
@@ -607,6 +605,28 @@ void Engine::vcycle(bool init, PcgScalars* sc) {
     vcycle_t<float>(v32, init, sc);
 }
 
+void Engine::ku(KuMode mode, const double* in, const double* pin, double* pout, double* out, PcgScalars* sc,
+                double* y) {
+  KuArgs a{};
+  a.g = G[0];
+  a.sh = kush;
+  a.K = kumodes;
+  a.in = in;
+  a.z = in;
+  a.pin = pin;
+  a.pout = pout;
+  a.out = out;
+  a.E = E64.p;
+  a.flags = fixbits.p;
+  a.cfix = cfix64.p;
+  a.sc = sc;
+  a.rs = rs1;
+  a.active = kuTiles.p;
+  a.zr = kuZr.p;
+  a.yacc = y;
+  launch_ku(st, mode, a, int(kuTiles.n));
+}
+
 // ---------------------------------------------------------------------------
 // Solving_PCG (TOP3D_XL.m:600-639) on device-resident scalars
 // ---------------------------------------------------------------------------
@@ -617,7 +637,7 @@ int Engine::pcg(const double* b, double* y, bool warm, double tol, int maxIT) {
   std::snprintf(key, sizeof(key), "pcg_init:%p:%p:%d:%.17g:%d", (const void*)b, (const void*)y, int(warm), tol, maxIT);
   run_graph(key, [&]() {
     if (warm)
-      launch_ku<double>(st, KU_PLAIN, g, y, nullptr, nullptr, kw.q.p, E64.p, fixbits.p, cfix64.p, sc, rs1, kut);
+      ku(KU_PLAIN, y, nullptr, nullptr, kw.q.p, sc, nullptr);
     else
       TOPX_CUDA_OK(cudaMemsetAsync(kw.q.p, 0, kw.q.bytes(), st));
     launch_residual_init<double>(st, g, b, kw.q.p, kw.r.p, sc, rs1, tol, maxIT);
@@ -634,7 +654,7 @@ int Engine::pcg(const double* b, double* y, bool warm, double tol, int maxIT) {
         for (int c = 0; c < CH; ++c) {  // CH is even: every chunk starts from p
           double* pin = (c & 1) ? kw.p2.p : kw.p.p;
           double* pnew = (c & 1) ? kw.p.p : kw.p2.p;
-          launch_ku<double>(st, KU_P_UPDATE, g, pin, kw.z.p, pnew, kw.q.p, E64.p, fixbits.p, cfix64.p, sc, rs1, kut, y);
+          ku(KU_P_UPDATE, kw.z.p, pin, pnew, kw.q.p, sc, y);
           launch_pcg_update<double, double>(st, g, y, nullptr, pnew, kw.r.p, kw.q.p, sc, rs1, act1);
           vcycle(false, sc);
         }
@@ -648,7 +668,7 @@ int Engine::pcg(const double* b, double* y, bool warm, double tol, int maxIT) {
       if (prof_) TOPX_CUDA_OK(cudaEventRecord(pev[2 * c], st));
       double* pin = (launched & 1) ? kw.p2.p : kw.p.p;
       double* pnew = (launched & 1) ? kw.p.p : kw.p2.p;
-      launch_ku<double>(st, KU_P_UPDATE, g, pin, kw.z.p, pnew, kw.q.p, E64.p, fixbits.p, cfix64.p, sc, rs1, kut, y);
+      ku(KU_P_UPDATE, kw.z.p, pin, pnew, kw.q.p, sc, y);
       if (prof_) TOPX_CUDA_OK(cudaEventRecord(pev[2 * c + 1], st));
       sec_begin(SEC_UPDATE);
       launch_pcg_update<double, double>(st, g, y, nullptr, pnew, kw.r.p, kw.q.p, sc, rs1, act1);
@@ -758,7 +778,7 @@ void Engine::apply_K(const double* h_u, double* h_y) {
   du.alloc(size_t(G[0].stride) * 3);
   dy.alloc(size_t(G[0].stride) * 3);
   launch_compact_to_grid_nodes<double>(st, cu.p, du.p, G[0], nodMapBack0.p, Nn);
-  launch_ku<double>(st, KU_PLAIN, G[0], du.p, nullptr, nullptr, dy.p, E64.p, fixbits.p, cfix64.p, nullptr, rs1);
+  ku(KU_PLAIN, du.p, nullptr, nullptr, dy.p, nullptr, nullptr);
   launch_grid_to_compact_nodes<double>(st, dy.p, cu.p, G[0], nodMapBack0.p, Nn);
   TOPX_CUDA_OK(cudaStreamSynchronize(st));
   copy_sync(h_y, cu.p, sizeof(double) * Nn * 3, cudaMemcpyDeviceToHost);

@@ -214,11 +214,13 @@ class Engine {
   DevBuf<double> fl_F;
   int nflag = 0;
   DevBuf<uint32_t> kuTiles;  // level-1 K*u tiles that own a node of the domain
-  DevBuf<uint32_t> kuRows;   // and the last-row kernel's tiles that hold one of the row y = ny
   DevBuf<uint32_t> kuZr;     // per listed tile, its planes that hold a present node
-  KuTiles kut;               // their list (null: the whole grid)
+  KuShape kush{};
+  KuModes kumodes{};
+  // u or z, the directions, the result, and the solution to step; PLAIN: in -> out
+  void ku(KuMode mode, const double* in, const double* pin, double* pout, double* out, PcgScalars* sc, double* y);
   DevBuf<uint32_t> filterTiles;  // the same for the filter's K*u (its own z-chunks)
-  KuTiles fut;
+  FilterTiles fut;
   DevBuf<uint32_t> act1Mask;     // level-1 chunk mask (chunk_active) of an irregular domain
   const uint32_t* act1 = nullptr;  // null: every chunk holds a present node
   DevBuf<uint32_t> cols1Mask;      // level-1 (x, z) columns that hold a present node

@@ -1,78 +1,17 @@
-// Level-1 elasticity kernels of the TOP3D_XL B200 path: matrix-free K*u,
-// Jacobi diagonal, PCG vector algebra, trilinear multigrid transfers, SIMP,
+// Level-1 elasticity kernels of the TOP3D_XL B200 path (the operator is in topx_ku.cu): Jacobi diagonal, PCG vector algebra, trilinear multigrid transfers, SIMP,
 // unit compliance.  FP64 (plain path) and FP32 (mixed path) instantiations.
 #include <cmath>
-#include <mutex>
 #include <stdexcept>
 #include <type_traits>
-#include <vector>
 
-#include "topx_ke_classes.h"
 #include "topx_kernels.cuh"
 
 namespace topx {
 
 __constant__ double c_Ke64[576];
-__constant__ float c_Ke32[576];
-
-template <typename T>
-__device__ __forceinline__ T ke(int i);
-template <>
-__device__ __forceinline__ double ke<double>(int i) {
-  return c_Ke64[i];
-}
-template <>
-__device__ __forceinline__ float ke<float>(int i) {
-  return c_Ke32[i];
-}
-
-// The ten values of Ke (topx_ke_classes.h): the level-1 operator addresses these instead of
-// 576 constants, so they stay in uniform registers for the whole launch.
-__constant__ double c_Kc64[kKeClasses];
-__constant__ float c_Kc32[kKeClasses];
-
-template <typename T>
-__device__ __forceinline__ T kcls(int c);
-template <>
-__device__ __forceinline__ double kcls<double>(int c) {
-  return c_Kc64[c];
-}
-template <>
-__device__ __forceinline__ float kcls<float>(int c) {
-  return c_Kc32[c];
-}
-// entry idx of Ke from its class (idx is a compile-time constant once the loops are unrolled)
-template <typename T>
-__device__ __forceinline__ T kcl(int idx) {
-  const int code = ke_class_code(idx);
-  return code > 0 ? kcls<T>(code - 1) : -kcls<T>(-code - 1);
-}
 
 void upload_ke(const double* Ke576) {
-  float f[576];
-  for (int i = 0; i < 576; ++i) f[i] = float(Ke576[i]);
   TOPX_CUDA_OK(cudaMemcpyToSymbol(c_Ke64, Ke576, sizeof(double) * 576));
-  TOPX_CUDA_OK(cudaMemcpyToSymbol(c_Ke32, f, sizeof(float) * 576));
-  // class values from the first entry of each class; every other entry must agree to rounding
-  double v[kKeClasses];
-  bool seen[kKeClasses] = {};
-  for (int i = 0; i < 576; ++i) {
-    const int code = ke_class_code(i), c = (code > 0 ? code : -code) - 1;
-    if (!seen[c]) {
-      v[c] = code > 0 ? Ke576[i] : -Ke576[i];
-      seen[c] = true;
-    }
-  }
-  for (int i = 0; i < 576; ++i) {
-    const int code = ke_class_code(i), c = (code > 0 ? code : -code) - 1;
-    const double e = code > 0 ? v[c] : -v[c];
-    if (!(std::fabs(Ke576[i] - e) <= 1e-13 * std::fabs(v[c])))
-      throw std::runtime_error("element stiffness does not have the hex8 value classes");
-  }
-  float vf[kKeClasses];
-  for (int c = 0; c < kKeClasses; ++c) vf[c] = float(v[c]);
-  TOPX_CUDA_OK(cudaMemcpyToSymbol(c_Kc64, v, sizeof(v)));
-  TOPX_CUDA_OK(cudaMemcpyToSymbol(c_Kc32, vf, sizeof(vf)));
 }
 
 static inline unsigned grid1d(int64_t n, int threads, int cap = 148 * 16) {
@@ -80,574 +19,6 @@ static inline unsigned grid1d(int64_t n, int threads, int cap = 148 * 16) {
   if (b < 1) b = 1;
   if (b > cap) b = cap;
   return unsigned(b);
-}
-
-// ---------------------------------------------------------------------------
-// K*u, level 1 (Solving_KbyU_MatrixFree, TOP3D_XL.m:684-725).
-//
-// Node-centric gather: one thread per grid node owns its 3 DOFs.  A CTA of
-// 32x8 nodes marches 16 node planes along z, keeping a ring of three
-// (32+2)x(8+2) planes of u (masked by the free-DOF mask) and two planes of
-// element moduli in shared memory, and sums, for each of the 8 surrounding
-// hexes, the node's 3 rows of E_e*Ke times the hex's 24 DOFs (Ke addressed through
-// its ten value classes, held in uniform registers).  No atomics: the result is deterministic.  The reference's per-element BC
-// matrices (uniqueKesFree_/uniqueKesFixed_) reduce exactly to
-//     y = m .* K_E (m .* u) + (1-m) .* cfix .* u
-// with m the free-DOF mask and cfix(node) = sum over its hexes of 1/nAdj.
-// The PCG mode forms the direction p = z (+ beta*p) on the fly (the update
-// kernel stores it) and reduces p'q.
-// ---------------------------------------------------------------------------
-constexpr int KY = 32, KX = 8, KZC = 16;  // CTA = KY x KX nodes, marching KZC node planes along z
-constexpr int KNT = KY * KX;
-
-// Node value seen by the operator: u (plain) or the PCG direction p = z (+ beta p_old).
-template <typename T, int MODE>
-__device__ __forceinline__ void ku_fetch(const T* __restrict__ in, const T* __restrict__ zin, int64_t n, int64_t S,
-                                         bool first, T beta, T& v0, T& v1, T& v2) {
-  if (MODE == KU_PLAIN) {
-    v0 = in[n];
-    v1 = in[n + S];
-    v2 = in[n + 2 * S];
-  } else if (first) {
-    v0 = zin[n];
-    v1 = zin[n + S];
-    v2 = zin[n + 2 * S];
-  } else {
-    v0 = zin[n] + beta * in[n];
-    v1 = zin[n + S] + beta * in[n + S];
-    v2 = zin[n + 2 * S] + beta * in[n + 2 * S];
-  }
-}
-
-// Accumulate, for the four hexes on one side of the node plane (upper: oz = 0,
-// lower: oz = -1), the node's 3 rows of Ke times the hex's 24 DOFs, then add
-// E_e * acc to y in the reference's local-node order.  PL(dz, c, dx, dy) is the (masked)
-// value of component c of the neighbour at offset (dy, dx, dz); EL(oz, ox, oy) the modulus of
-// the hex whose lowest corner is at offset (oy, ox, oz).
-template <typename T, int OZ, typename FPL, typename FEL>
-__device__ __forceinline__ void ku_half(FPL&& PL, FEL&& EL, T (&y)[3]) {
-  T acc[4][3];
-#pragma unroll
-  for (int e = 0; e < 4; ++e) acc[e][0] = acc[e][1] = acc[e][2] = T(0);
-#pragma unroll
-  for (int dz = OZ; dz <= OZ + 1; ++dz)
-#pragma unroll
-    for (int dx = -1; dx <= 1; ++dx)
-#pragma unroll
-      for (int dy = -1; dy <= 1; ++dy) {
-        const T u0 = PL(dz, 0, dx, dy);
-        const T u1 = PL(dz, 1, dx, dy);
-        const T u2 = PL(dz, 2, dx, dy);
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const int oy = (e & 1) ? 0 : -1, ox = (e & 2) ? 0 : -1;
-          const int ly = dy - oy, lx = dx - ox, lz = dz - OZ;
-          if (ly < 0 || ly > 1 || lx < 0 || lx > 1 || lz < 0 || lz > 1) continue;
-          const int a = hex_local(-oy, -ox, -OZ), b = hex_local(ly, lx, lz);
-#pragma unroll
-          for (int i = 0; i < 3; ++i) {
-            T s = acc[e][i];
-            s = fma(kcl<T>((3 * a + i) * 24 + 3 * b + 0), u0, s);
-            s = fma(kcl<T>((3 * a + i) * 24 + 3 * b + 1), u1, s);
-            s = fma(kcl<T>((3 * a + i) * 24 + 3 * b + 2), u2, s);
-            acc[e][i] = s;
-          }
-        }
-      }
-#pragma unroll
-  for (int a = (OZ == 0 ? 0 : 4); a < (OZ == 0 ? 4 : 8); ++a) {
-    const int oy = -hex_ly(a), ox = -hex_lx(a);
-    const int e = (oy + 1) + 2 * (ox + 1);
-    const T Ee = EL(OZ, ox, oy);
-#pragma unroll
-    for (int i = 0; i < 3; ++i) y[i] = fma(Ee, acc[e][i], y[i]);
-  }
-}
-
-// Plane loads are asynchronous copies one plane ahead: the raw values of node plane z+2
-// (u, or z and p_old in PCG mode) land in a staging area and element plane z+1 in a third
-// element slot while plane z is computed; the next iteration forms the masked values of
-// the staged plane in the node ring.  Only the free-DOF bits ride in registers.
-constexpr int KU_NP = (KX + 2) * (KY + 2), KU_EP = (KX + 1) * (KY + 1);
-static_assert(KU_NP <= 2 * KNT && KU_EP <= 2 * KNT, "two staged positions per thread");
-
-template <int BYTES>
-__device__ __forceinline__ void cp_async_el(void* smem, const void* gmem, bool pred) {
-  static_assert(BYTES == 4 || BYTES == 8, "element copy size");
-  const unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(smem));
-  const int n = pred ? BYTES : 0;  // 0: fill with zeros, read nothing
-  asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"(s), "l"(gmem), "n"(BYTES), "r"(n) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
-
-// A tile of the launch: blockIdx, or entry blockIdx.x of a list of the tiles that own a node of
-// the domain (y-tile | x-tile << 10 | z-chunk << 20); tiles of void alone are not launched.
-__device__ __forceinline__ void ku_tile(const uint32_t* __restrict__ active, int& ty, int& tx, int& tz) {
-  if (active) {
-    const uint32_t t = active[blockIdx.x];
-    ty = int(t & 1023u);
-    tx = int((t >> 10) & 1023u);
-    tz = int(t >> 20);
-  } else {
-    ty = blockIdx.x;
-    tx = blockIdx.y;
-    tz = blockIdx.z;
-  }
-}
-
-// In PCG mode with yacc given, each node also takes the previous iteration's solution step
-// y += lam p_in (p_in: that iteration's direction; none on the first step).
-template <typename T>
-__device__ __forceinline__ void ku_solution_step(double* __restrict__ yacc, const T* __restrict__ in, int64_t n,
-                                                 int64_t S, double lam) {
-#pragma unroll
-  for (int c = 0; c < 3; ++c) yacc[n + c * S] = fma(lam, double(in[n + c * S]), yacc[n + c * S]);
-}
-
-// Shared memory of the tile kernel (dynamic: above the 48 KB of static shared memory in PCG mode)
-template <typename T, int MODE>
-struct KuSmem {
-  T su[3][3][KX + 2][KY + 2];  // ring of 3 node planes: [slot][comp][x][y], masked by the free mask
-  T se[3][KX + 1][KY + 1];     // ring of 3 element planes
-  T sa[3][KU_NP];              // staged raw plane: u (plain) or z (PCG mode)
-  T sb[MODE == KU_PLAIN ? 1 : 3][MODE == KU_PLAIN ? 1 : KU_NP];  // staged p_old (PCG mode)
-  // PCG mode with the solution step: y at the thread's own node of the staged plane, and the
-  // step length of the previous iteration (read where used: no register across the plane loop)
-  double sy[MODE == KU_PLAIN ? 1 : 3][MODE == KU_PLAIN ? 1 : KNT];
-  double s_lam;
-};
-
-template <typename T, int MODE>
-__global__ void __launch_bounds__(KNT, 3) k_ku_l1(Grid g, int zc, const T* __restrict__ in, const T* __restrict__ zin,
-                                                  T* __restrict__ pout, T* __restrict__ out, const T* __restrict__ E,
-                                                  const uint8_t* __restrict__ fixbits, const T* __restrict__ cfix,
-                                                  PcgScalars* sc, RedScratch rs, const uint32_t* __restrict__ active,
-                                                  double* __restrict__ yacc, const uint32_t* __restrict__ zr) {
-  if (MODE != KU_PLAIN && sc->done) return;
-  extern __shared__ __align__(16) unsigned char ku_dyn_smem[];
-  KuSmem<T, MODE>& sm = *reinterpret_cast<KuSmem<T, MODE>*>(ku_dyn_smem);
-  auto& su = sm.su;
-  auto& se = sm.se;
-  auto& sa = sm.sa;
-  auto& sb = sm.sb;
-  auto& sy = sm.sy;
-  double& s_lam = sm.s_lam;
-  const int nny = g.ny + 1, nnx = g.nx + 1, nnz = g.nz + 1;
-  const int64_t S = g.stride;
-  int tyi, txi, tzi;
-  ku_tile(active, tyi, txi, tzi);
-  const int y0 = tyi * KY, x0 = txi * KX;
-  int zc0 = tzi * zc, zend = min(zc0 + zc, nnz);
-  if (active && zr) {  // only the planes of the chunk that hold a present node
-    const uint32_t r = zr[blockIdx.x];
-    zc0 = int(r & 0xffffu);
-    zend = int(r >> 16);
-  }
-  const int ty = threadIdx.x, tx = threadIdx.y;
-  const int tid = ty + KY * tx;
-  const bool first = (MODE != KU_PLAIN) && sc->first;
-  const T beta = (MODE != KU_PLAIN) ? T(sc->beta) : T(0);
-  const T* const araw = MODE == KU_PLAIN ? in : zin;
-  uint8_t fbs[2];
-  const bool ystep = MODE != KU_PLAIN && yacc && !first;
-  const bool yown = y0 + ty < nny && x0 + tx < nnx;
-  if (ystep && tid == 0) s_lam = sc->lam;
-
-  // issue the copies of node plane zp into the staging area (and its free bits into fbs)
-  auto issue_nodes = [&](int zp) {
-#pragma unroll
-    for (int s = 0; s < 2; ++s) {
-      const int i = tid + s * KNT;
-      fbs[s] = 0;
-      if (i < KU_NP) {
-        const int sy = i % (KY + 2), sx = i / (KY + 2);
-        const int gy = y0 - 1 + sy, gx = x0 - 1 + sx;
-        const bool ok = zp >= 0 && zp < nnz && gy >= 0 && gy < nny && gx >= 0 && gx < nnx;
-        const int64_t n = ok ? gy + int64_t(nny) * (gx + int64_t(nnx) * zp) : 0;
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          cp_async_el<sizeof(T)>(&sa[c][i], araw + n + c * S, ok);
-          if (MODE != KU_PLAIN) cp_async_el<sizeof(T)>(&sb[c][i], in + n + c * S, ok && !first);
-        }
-        if (ok) fbs[s] = fixbits[n];
-      }
-    }
-  };
-  auto issue_elems = [&](int ez, int slot) {
-#pragma unroll
-    for (int s = 0; s < 2; ++s) {
-      const int i = tid + s * KNT;
-      if (i < KU_EP) {
-        const int sy = i % (KY + 1), sx = i / (KY + 1);
-        const int ey = y0 - 1 + sy, ex = x0 - 1 + sx;
-        const bool ok = ez >= 0 && ez < g.nz && ey >= 0 && ey < g.ny && ex >= 0 && ex < g.nx;
-        const int64_t e = ok ? ey + int64_t(g.ny) * (ex + int64_t(g.nx) * ez) : 0;
-        cp_async_el<sizeof(T)>(&se[slot][sx][sy], E + e, ok);
-      }
-    }
-  };
-  // The previous iteration's solution step y += lam p_in rides with the plane copies: y at the
-  // thread's own node of plane zp is copied beside the staged plane, and when that plane is
-  // formed the thread adds lam times the staged p_in there and stores y.
-  auto issue_y = [&](int zp) {
-    if (ystep && yown && zp >= zc0 && zp < zend) {
-      const int64_t n = (y0 + ty) + int64_t(nny) * ((x0 + tx) + int64_t(nnx) * zp);
-#pragma unroll
-      for (int c = 0; c < 3; ++c) cp_async_el<8>(&sy[c][tid], yacc + n + c * S, true);
-    }
-  };
-  auto step_y = [&](int zp) {
-    if (ystep && yown && zp >= zc0 && zp < zend) {
-      const int64_t n = (y0 + ty) + int64_t(nny) * ((x0 + tx) + int64_t(nnx) * zp);
-      const int io = (ty + 1) + (KY + 2) * (tx + 1);  // the own node's staging position
-      const double lam = s_lam;
-#pragma unroll
-      for (int c = 0; c < 3; ++c) yacc[n + c * S] = fma(lam, double(sb[c][io]), sy[c][tid]);
-    }
-  };
-  // masked values of the staged plane into node slot `slot`
-  auto form_nodes = [&](int slot) {
-#pragma unroll
-    for (int s = 0; s < 2; ++s) {
-      const int i = tid + s * KNT;
-      if (i < KU_NP) {
-        const int sy = i % (KY + 2), sx = i / (KY + 2);
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          T v = sa[c][i];
-          if (MODE != KU_PLAIN && !first) v = v + beta * sb[c][i];
-          su[slot][c][sx][sy] = ((fbs[s] >> c) & 1) ? T(0) : v;
-        }
-      }
-    }
-  };
-
-  // prologue: node planes zc0-1, zc0 formed; element planes zc0-1, zc0 and node plane zc0+1 in flight
-  issue_nodes(zc0 - 1);
-  cp_async_commit();
-  cp_async_wait_all();
-  __syncthreads();
-  form_nodes(0);
-  __syncthreads();
-  issue_nodes(zc0);
-  issue_y(zc0);
-  cp_async_commit();
-  cp_async_wait_all();
-  __syncthreads();
-  form_nodes(1);
-  step_y(zc0);
-  __syncthreads();
-  issue_elems(zc0 - 1, 0);
-  issue_elems(zc0, 1);
-  issue_nodes(zc0 + 1);
-  issue_y(zc0 + 1);
-  cp_async_commit();
-  const int gy = y0 + ty, gx = x0 + tx;
-  const bool own = gy < nny && gx < nnx;
-  double dot = 0.0;
-  for (int k = 0; zc0 + k < zend; ++k) {
-    const int z = zc0 + k;
-    cp_async_wait_all();
-    __syncthreads();
-    form_nodes((k + 2) % 3);
-    step_y(z + 1);
-    __syncthreads();
-    if (z + 1 < zend) {
-      issue_nodes(z + 2);
-      issue_y(z + 2);
-      issue_elems(z + 1, (k + 2) % 3);
-      cp_async_commit();
-    }
-    const int64_t n = gy + int64_t(nny) * (gx + int64_t(nnx) * z);
-    const uint8_t fbo = own ? fixbits[n] : uint8_t(0);
-    if (own) {
-      const T(*const pl[3])[KX + 2][KY + 2] = {su[k % 3], su[(k + 1) % 3], su[(k + 2) % 3]};
-      const T(*const el[2])[KY + 1] = {se[k % 3], se[(k + 1) % 3]};
-      T y[3] = {T(0), T(0), T(0)};
-      auto PL = [&](int dz, int c, int dx, int dy) { return pl[dz + 1][c][tx + 1 + dx][ty + 1 + dy]; };
-      auto EL = [&](int oz, int ox, int oy) { return el[oz + 1][tx + 1 + ox][ty + 1 + oy]; };
-      ku_half<T, 0>(PL, EL, y);   // hexes above the node: local nodes 1-4
-      ku_half<T, -1>(PL, EL, y);  // hexes below the node: local nodes 5-8
-      // the node's own value: masked copy in the ring for free DOFs, unmasked for fixed ones
-      T p[3] = {pl[1][0][tx + 1][ty + 1], pl[1][1][tx + 1][ty + 1], pl[1][2][tx + 1][ty + 1]};
-      if (fbo) {
-        T p0, p1, p2;
-        ku_fetch<T, MODE>(in, zin, n, S, first, beta, p0, p1, p2);
-        const T cf = cfix[n];
-        if (fbo & 1) {
-          p[0] = p0;
-          y[0] = cf * p0;
-        }
-        if (fbo & 2) {
-          p[1] = p1;
-          y[1] = cf * p1;
-        }
-        if (fbo & 4) {
-          p[2] = p2;
-          y[2] = cf * p2;
-        }
-      }
-      out[n] = y[0];
-      out[n + S] = y[1];
-      out[n + 2 * S] = y[2];
-      if (MODE != KU_PLAIN) {
-        if (pout) {  // the direction p = z (+ beta p_old) for the PCG update (another buffer than in)
-          pout[n] = p[0];
-          pout[n + S] = p[1];
-          pout[n + 2 * S] = p[2];
-        }
-        dot += double(p[0]) * double(y[0]) + double(p[1]) * double(y[1]) + double(p[2]) * double(y[2]);
-      }
-    }
-  }
-  cp_async_wait_all();
-  if (MODE != KU_PLAIN) {
-    double v[1] = {dot}, tot[1];
-    if (reduce_publish<1>(v, rs, tot) && tid == 0) sc->pq = tot[0];
-  }
-}
-
-// The last node row y = ny of the grid, when the tile kernel's y-tiles end exactly at it: with
-// ny a multiple of the tile height the tile kernel would otherwise run whole tiles for this one
-// row (node counts here are 2^k + 1).  A CTA takes 32 x 8 nodes of the row (x, z); its
-// threads first stage, together, the masked values of rows y = ny - 1 and ny over the tile and
-// a one-node halo, their free bits, and the moduli of element row ny - 1 in shared memory (with
-// y the fastest index every node of this row sits in its own DRAM sectors, so the loads are
-// issued all at once rather than one neighbour at a time), then each thread applies the same
-// operator, in the same FMA order, as the tile kernel to its node.  The p'q partial sum is
-// added to the tile kernel's.
-constexpr int KLX = 32, KLZ = 8;
-
-template <typename T, int MODE>
-__global__ void __launch_bounds__(KLX * KLZ) k_ku_l1_lastrow(Grid g, const T* __restrict__ in, const T* __restrict__ zin,
-                                                             T* __restrict__ pout, T* __restrict__ out,
-                                                             const T* __restrict__ E, const uint8_t* __restrict__ fixbits,
-                                                             const T* __restrict__ cfix, PcgScalars* sc, RedScratch rs,
-                                                             double* __restrict__ yacc, const uint32_t* __restrict__ rows) {
-  if (MODE != KU_PLAIN && sc->done) return;
-  __shared__ T sp[3][KLZ + 2][KLX + 2][2];  // masked values, [comp][z][x][row y = ny - 1, ny]
-  __shared__ T se[KLZ + 1][KLX + 1];        // moduli of element row ny - 1
-  __shared__ uint8_t sfb[KLZ + 2][KLX + 2][2];
-  const int nny = g.ny + 1, nnx = g.nx + 1, nnz = g.nz + 1;
-  const int64_t S = g.stride;
-  const bool first = (MODE != KU_PLAIN) && sc->first;
-  const T beta = (MODE != KU_PLAIN) ? T(sc->beta) : T(0);
-  const bool ystep = MODE != KU_PLAIN && yacc && !first;
-  const double lam = ystep ? sc->lam : 0.0;
-  const int Y = nny - 1;
-  int bx = blockIdx.x, bz = blockIdx.y;
-  if (rows) {  // entry blockIdx.x of the tiles that hold a present node of the row
-    bx = int(rows[blockIdx.x] & 0xffffu);
-    bz = int(rows[blockIdx.x] >> 16);
-  }
-  const int x0 = bx * KLX, z0 = bz * KLZ;
-  const int tid = threadIdx.x;
-  // stage: position i -> row (i & 1), halo x and z; the two rows of one (x, z) are adjacent in memory
-  constexpr int NPOS = 2 * (KLX + 2) * (KLZ + 2);
-  for (int i = tid; i < NPOS; i += KLX * KLZ) {
-    const int row = i & 1, rest = i >> 1;
-    const int sx = rest % (KLX + 2), sz = rest / (KLX + 2);
-    const int gx = x0 - 1 + sx, gz = z0 - 1 + sz;
-    const bool ok = gx >= 0 && gx < nnx && gz >= 0 && gz < nnz;
-    T v0 = T(0), v1 = T(0), v2 = T(0);
-    uint8_t fb = 0;
-    if (ok) {
-      const int64_t n = (Y - 1 + row) + int64_t(nny) * (gx + int64_t(nnx) * gz);
-      ku_fetch<T, MODE>(in, zin, n, S, first, beta, v0, v1, v2);
-      fb = fixbits[n];
-    }
-    sp[0][sz][sx][row] = (fb & 1) ? T(0) : v0;
-    sp[1][sz][sx][row] = (fb & 2) ? T(0) : v1;
-    sp[2][sz][sx][row] = (fb & 4) ? T(0) : v2;
-    sfb[sz][sx][row] = fb;
-  }
-  for (int i = tid; i < (KLX + 1) * (KLZ + 1); i += KLX * KLZ) {
-    const int sx = i % (KLX + 1), sz = i / (KLX + 1);
-    const int ex = x0 - 1 + sx, ez = z0 - 1 + sz;
-    const bool ok = ex >= 0 && ex < g.nx && ez >= 0 && ez < g.nz;
-    se[sz][sx] = ok ? E[(Y - 1) + int64_t(g.ny) * (ex + int64_t(g.nx) * ez)] : T(0);
-  }
-  __syncthreads();
-  const int lx = tid % KLX, lz = tid / KLX;
-  const int x = x0 + lx, z = z0 + lz;
-  double dot = 0.0;
-  if (x < nnx && z < nnz) {
-    // neighbours at y + 1 and hexes above the row lie outside the grid: zero
-    auto PL = [&](int dz, int c, int dx, int dy) { return dy > 0 ? T(0) : sp[c][lz + 1 + dz][lx + 1 + dx][dy + 1]; };
-    auto EL = [&](int oz, int ox, int oy) { return oy == 0 ? T(0) : se[lz + 1 + oz][lx + 1 + ox]; };
-    T y[3] = {T(0), T(0), T(0)};
-    ku_half<T, 0>(PL, EL, y);
-    ku_half<T, -1>(PL, EL, y);
-    const int64_t n = Y + int64_t(nny) * (x + int64_t(nnx) * z);
-    const uint8_t fbo = sfb[lz + 1][lx + 1][1];
-    T p[3] = {sp[0][lz + 1][lx + 1][1], sp[1][lz + 1][lx + 1][1], sp[2][lz + 1][lx + 1][1]};
-    if (fbo) {
-      T p0, p1, p2;
-      ku_fetch<T, MODE>(in, zin, n, S, first, beta, p0, p1, p2);
-      const T cf = cfix[n];
-      if (fbo & 1) {
-        p[0] = p0;
-        y[0] = cf * p0;
-      }
-      if (fbo & 2) {
-        p[1] = p1;
-        y[1] = cf * p1;
-      }
-      if (fbo & 4) {
-        p[2] = p2;
-        y[2] = cf * p2;
-      }
-    }
-    out[n] = y[0];
-    out[n + S] = y[1];
-    out[n + 2 * S] = y[2];
-    if (ystep) ku_solution_step(yacc, in, n, S, lam);
-    if (MODE != KU_PLAIN) {
-      if (pout) {
-        pout[n] = p[0];
-        pout[n + S] = p[1];
-        pout[n + 2 * S] = p[2];
-      }
-      dot += double(p[0]) * double(y[0]) + double(p[1]) * double(y[1]) + double(p[2]) * double(y[2]);
-    }
-  }
-  if (MODE != KU_PLAIN) {
-    double v[1] = {dot}, tot[1];
-    if (reduce_publish<1>(v, rs, tot) && threadIdx.x == 0) sc->pq += tot[0];
-  }
-}
-
-static int g_num_sms = 148;
-// once per device and process: engines on several host threads share the attributes
-void prepare_fem_kernels() {
-  static std::mutex mu;
-  static bool done[64] = {};
-  int dev = 0;
-  TOPX_CUDA_OK(cudaGetDevice(&dev));
-  std::lock_guard<std::mutex> lock(mu);
-  if (dev >= 0 && dev < 64 && done[dev]) return;
-  int n = 0;
-  TOPX_CUDA_OK(cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev));
-  if (n > 0) g_num_sms = n;
-  TOPX_CUDA_OK(cudaFuncSetAttribute(k_ku_l1<double, KU_PLAIN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    int(sizeof(KuSmem<double, KU_PLAIN>))));
-  TOPX_CUDA_OK(cudaFuncSetAttribute(k_ku_l1<double, KU_P_UPDATE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    int(sizeof(KuSmem<double, KU_P_UPDATE>))));
-  TOPX_CUDA_OK(cudaFuncSetAttribute(k_ku_l1<float, KU_PLAIN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    int(sizeof(KuSmem<float, KU_PLAIN>))));
-  TOPX_CUDA_OK(cudaFuncSetAttribute(k_ku_l1<float, KU_P_UPDATE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    int(sizeof(KuSmem<float, KU_P_UPDATE>))));
-  if (dev >= 0 && dev < 64) done[dev] = true;
-}
-
-// z-chunk length of the K*u launch: fewest (waves x halo-inclusive planes) for three CTAs per SM
-static int ku_z_chunk(int nny, int nnx, int nnz) {
-  const int64_t tiles = int64_t((nny + KY - 1) / KY) * ((nnx + KX - 1) / KX);
-  const int64_t slots = int64_t(g_num_sms) * 3;
-  int best = KZC;
-  int64_t bestCost = -1;
-  for (int zc = 1; zc <= 24; ++zc) {
-    const int64_t ctas = tiles * ((nnz + zc - 1) / zc);
-    const int64_t cost = ((ctas + slots - 1) / slots) * (zc + 2);
-    if (bestCost < 0 || cost < bestCost) {
-      bestCost = cost;
-      best = zc;
-    }
-  }
-  return best;
-}
-
-// Tile grid of the level-1 K*u launch: y-tiles (a last node row that would fill a tile on its own
-// goes to k_ku_l1_lastrow instead), x-tiles and z-chunks.
-struct KuGeometry {
-  bool lastrow;
-  int rows, zc;
-  dim3 grd;
-};
-static KuGeometry ku_geometry(Grid g) {
-  KuGeometry k;
-  k.lastrow = g.ny >= KY && g.ny % KY == 0;
-  k.rows = k.lastrow ? g.ny : g.nny();
-  k.zc = ku_z_chunk(k.rows, g.nnx(), g.nnz());
-  k.grd = dim3((k.rows + KY - 1) / KY, (g.nnx() + KX - 1) / KX, (g.nnz() + k.zc - 1) / k.zc);
-  return k;
-}
-
-std::vector<uint32_t> ku_active_tiles(Grid g, const std::vector<uint8_t>& present, std::vector<uint32_t>* zranges) {
-  const KuGeometry k = ku_geometry(g);
-  const int nny = g.nny(), nnx = g.nnx(), nnz = g.nnz();
-  if (k.grd.x > 1024 || k.grd.y > 1024 || k.grd.z > 4095 || nnz > 65535) return {};
-  std::vector<uint32_t> list;
-  if (zranges) zranges->clear();
-  for (unsigned tz = 0; tz < k.grd.z; ++tz)
-    for (unsigned tx = 0; tx < k.grd.y; ++tx)
-      for (unsigned ty = 0; ty < k.grd.x; ++ty) {
-        int lo = -1, hi = -1;
-        for (int z = int(tz) * k.zc; z < std::min(nnz, int(tz + 1) * k.zc); ++z) {
-          bool any = false;
-          for (int x = int(tx) * KX; x < std::min(nnx, int(tx + 1) * KX) && !any; ++x)
-            for (int y = int(ty) * KY; y < std::min(k.rows, int(ty + 1) * KY) && !any; ++y)
-              any = present[size_t(y + int64_t(nny) * (x + int64_t(nnx) * z))] != 0;
-          if (any) {
-            if (lo < 0) lo = z;
-            hi = z + 1;
-          }
-        }
-        if (lo >= 0) {
-          list.push_back(ty | (tx << 10) | (tz << 20));
-          if (zranges) zranges->push_back(uint32_t(lo) | (uint32_t(hi) << 16));
-        }
-      }
-  return list;
-}
-
-std::vector<uint32_t> ku_active_row_tiles(Grid g, const std::vector<uint8_t>& present) {
-  const KuGeometry k = ku_geometry(g);
-  std::vector<uint32_t> list;
-  if (!k.lastrow) return list;
-  const int nny = g.nny(), nnx = g.nnx(), nnz = g.nnz(), Y = nny - 1;
-  for (int bz = 0; bz < (nnz + KLZ - 1) / KLZ; ++bz)
-    for (int bx = 0; bx < (nnx + KLX - 1) / KLX; ++bx) {
-      bool any = false;
-      for (int z = bz * KLZ; z < std::min(nnz, (bz + 1) * KLZ) && !any; ++z)
-        for (int x = bx * KLX; x < std::min(nnx, (bx + 1) * KLX) && !any; ++x)
-          any = present[size_t(Y + int64_t(nny) * (x + int64_t(nnx) * z))] != 0;
-      if (any) list.push_back(uint32_t(bx) | (uint32_t(bz) << 16));
-    }
-  return list;
-}
-
-template <typename T>
-void launch_ku(cudaStream_t st, KuMode mode, Grid g, const T* in, const T* z, T* pout, T* out, const T* E,
-               const uint8_t* fixbits, const T* cfix, PcgScalars* sc, RedScratch rs, KuTiles tiles, double* yacc) {
-  if (mode == KU_PLAIN) yacc = nullptr;
-  const KuGeometry k = ku_geometry(g);
-  const bool lastrow = k.lastrow;
-  const int zc = k.zc;
-  dim3 blk(KY, KX, 1);
-  dim3 grd = tiles.list ? dim3(unsigned(tiles.n)) : k.grd;
-  if (tiles.list && tiles.n == 0) grd = dim3(0);
-  if (grd.x == 0) {
-  } else if (mode == KU_PLAIN)
-    (k_ku_l1<T, KU_PLAIN><<<grd, blk, sizeof(KuSmem<T, KU_PLAIN>), st>>>(g, zc, in, z, pout, out, E, fixbits, cfix,
-                                                                       sc, rs, tiles.list, yacc, tiles.zr),
-     topx::count_launch());
-  else
-    (k_ku_l1<T, KU_P_UPDATE><<<grd, blk, sizeof(KuSmem<T, KU_P_UPDATE>), st>>>(g, zc, in, z, pout, out, E, fixbits,
-                                                                             cfix, sc, rs, tiles.list, yacc, tiles.zr),
-     topx::count_launch());
-  if (lastrow && !(tiles.list && tiles.rows && tiles.nrows == 0)) {
-    const uint32_t* rows = tiles.list ? tiles.rows : nullptr;
-    const dim3 nb = rows ? dim3(unsigned(tiles.nrows)) : dim3((g.nnx() + KLX - 1) / KLX, (g.nnz() + KLZ - 1) / KLZ);
-    if (mode == KU_PLAIN)
-      (k_ku_l1_lastrow<T, KU_PLAIN><<<nb, KLX * KLZ, 0, st>>>(g, in, z, pout, out, E, fixbits, cfix, sc, rs, yacc, rows),
-       topx::count_launch());
-    else
-      (k_ku_l1_lastrow<T, KU_P_UPDATE><<<nb, KLX * KLZ, 0, st>>>(g, in, z, pout, out, E, fixbits, cfix, sc, rs, yacc, rows),
-       topx::count_launch());
-  }
-  TOPX_CUDA_OK(cudaGetLastError());
 }
 
 // ---------------------------------------------------------------------------
@@ -669,7 +40,7 @@ __global__ void k_diag_l1(Grid g, const TE* __restrict__ E, const uint8_t* __res
         const int ey = gy - hex_ly(a), ex = gx - hex_lx(a), ez = gz - hex_lz(a);
         if (ey < 0 || ey >= g.ny || ex < 0 || ex >= g.nx || ez < 0 || ez >= g.nz) continue;
         const double Ee = double(E[ey + int64_t(g.ny) * (ex + int64_t(g.nx) * ez)]);
-        for (int c = 0; c < 3; ++c) s[c] += double(ke<double>((3 * a + c) * 25)) * Ee;
+        for (int c = 0; c < 3; ++c) s[c] += c_Ke64[(3 * a + c) * 25] * Ee;
       }
       const uint8_t fb = fixbits[n];
       for (int c = 0; c < 3; ++c) v[c] = 1.0 / ((fb >> c) & 1 ? double(cfix[n]) : s[c]);
@@ -1346,8 +717,6 @@ void launch_unit_compliance(cudaStream_t st, Grid g, const double* U, const int3
 
 // explicit instantiations
 #define TOPX_INST(T)                                                                                             \
-  template void launch_ku<T>(cudaStream_t, KuMode, Grid, const T*, const T*, T*, T*, const T*, const uint8_t*,   \
-                             const T*, PcgScalars*, RedScratch, KuTiles, double*);                               \
   template void launch_diag_l1<T, T>(cudaStream_t, Grid, const T*, const uint8_t*, const T*, const uint8_t*, T*); \
   template void launch_residual_init<T>(cudaStream_t, Grid, const T*, const T*, T*, PcgScalars*, RedScratch,     \
                                         double, int);                                                            \

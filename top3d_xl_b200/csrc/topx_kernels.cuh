@@ -44,27 +44,41 @@ enum KuMode { KU_PLAIN = 0, KU_P_UPDATE = 2 };
 void upload_ke(const double* Ke576);
 
 // --- level-1 elasticity --------------------------------------------------
-// Tiles of the level-1 K*u launch that own a node of the domain (ku_active_tiles); a null list
-// launches the whole grid
-struct KuTiles {
-  const uint32_t* list = nullptr;
-  int n = 0;
-  // the last-row kernel's (x, z) tiles that hold a present node of the row y = ny (x | z << 16);
-  // used when list is given (non-null with nrows = 0: no last-row launch)
-  const uint32_t* rows = nullptr;
-  int nrows = 0;
-  // per listed tile, the planes [lo, hi) of its z-chunk that hold a present node (lo | hi << 16);
-  // the tile kernel marches only those (null: the whole chunk)
-  const uint32_t* zr = nullptr;
+// Ke in the basis of sums and differences along the three axes (topx_ku.cu): normal strains a - b on the
+// diagonal and b, shear g, bending p and q, torsion r - s and s, triple differences h
+struct KuModes {
+  double a_b, b, g, p, q, r_s, s, h;
 };
-// zranges (optional): the z-range entry of each listed tile
-std::vector<uint32_t> ku_active_tiles(Grid g, const std::vector<uint8_t>& present,
+KuModes ku_modes(const double* Ke576);
+// Tile of the level-1 K*u: TY x TX nodes written by PY x PX threads, zc planes per CTA
+struct KuShape {
+  int PY, PX, TY, TX, zc;
+  dim3 grid;
+};
+KuShape ku_shape(Grid g);
+struct KuArgs {
+  Grid g;
+  KuShape sh;
+  KuModes K;
+  const double* in;   // u (KU_PLAIN)
+  const double* z;    // KU_P_UPDATE
+  const double* pin;  // the previous direction
+  double* pout;       // takes the new one (another buffer)
+  double* out;
+  const double* E;
+  const uint8_t* flags;  // bits 0-2: fixed x, y, z
+  const double* cfix;
+  PcgScalars* sc;
+  RedScratch rs;
+  const uint32_t* active;  // the tiles that own a node of the domain (ku_active_tiles), or null for all
+  const uint32_t* zr;      // per listed tile, the planes [lo, hi) of its z-chunk that hold a present node (lo | hi << 16)
+  double* yacc;
+};
+// tiles of the launch that own a node of the domain; zranges (optional): the z-range entry of each
+std::vector<uint32_t> ku_active_tiles(Grid g, const KuShape& k, const std::vector<uint8_t>& present,
                                       std::vector<uint32_t>* zranges = nullptr);
-std::vector<uint32_t> ku_active_row_tiles(Grid g, const std::vector<uint8_t>& present);
-template <typename T>
-void launch_ku(cudaStream_t st, KuMode mode, Grid g, const T* in, const T* z, T* pout, T* out, const T* E,
-               const uint8_t* fixbits, const T* cfix, PcgScalars* sc, RedScratch rs, KuTiles tiles = KuTiles{},
-               double* yacc = nullptr);
+// ntiles: entries of args.active
+void launch_ku(cudaStream_t st, KuMode mode, const KuArgs& args, int ntiles);
 template <typename TE, typename T = TE>
 void launch_diag_l1(cudaStream_t st, Grid g, const TE* E, const uint8_t* fixbits, const TE* cfix,
                     const uint8_t* present, T* d);
@@ -134,8 +148,8 @@ void launch_galerkin_span2(cudaStream_t st, Grid gc, const double* Ksf, const ui
 template <typename T>
 void launch_diag_coarse(cudaStream_t st, Grid g, const double* Ks, const uint8_t* present, T* d);
 
-// caches the SM count used to shape the K*u launch (call once per device, outside capture)
-void prepare_fem_kernels();
+// shared-memory limits of the K*u launches (call once per device, outside capture)
+void prepare_ku_kernels();
 
 // Control words of the persistent coarse solve (zeroed before first use; err != 0 after a CTA
 // gave up waiting, and then the words, and the solve's counters, must be zeroed again).

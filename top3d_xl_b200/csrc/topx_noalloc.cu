@@ -64,8 +64,7 @@ void Engine::apply_K_device(const double* d_u, double* d_y, double* grid_u, doub
   // the scratch keeps the previous call's contents: grid nodes outside the domain must read 0
   TOPX_CUDA_OK(cudaMemsetAsync(grid_u, 0, sizeof(double) * size_t(g.stride) * 3, st));
   launch_compact_to_grid_nodes<double>(st, d_u, grid_u, g, nodMapBack0.p, Nn);
-  launch_ku<double>(st, KU_PLAIN, g, grid_u, nullptr, nullptr, grid_y, E64.p, fixbits.p, cfix64.p, nullptr,
-                    RedScratch{nullptr, nullptr});
+  ku(KU_PLAIN, grid_u, nullptr, nullptr, grid_y, nullptr, nullptr);
   launch_grid_to_compact_nodes<double>(st, grid_y, d_y, g, nodMapBack0.p, Nn);
   TOPX_CUDA_OK(cudaStreamSynchronize(st));
 }

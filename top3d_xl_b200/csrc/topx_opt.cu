@@ -219,7 +219,7 @@ std::vector<uint32_t> filter_active_tiles(Grid g, const std::vector<uint8_t>& pr
 
 template <typename T>
 void launch_filter_ku(cudaStream_t st, KuMode mode, Grid g, const FilterKe<T>& kf, const T* in, const T* z, T* pout, T* out,
-                      const uint8_t* solid, PcgScalars* sc, RedScratch rs, KuTiles tiles) {
+                      const uint8_t* solid, PcgScalars* sc, RedScratch rs, FilterTiles tiles) {
   (void)pout;
   const FilterGeometry f = filter_geometry(g);
   dim3 blk(FKY, FKX, 1);
@@ -563,9 +563,9 @@ template void launch_filter_e2n<float>(cudaStream_t, Grid, const float*, float*,
 template void launch_filter_diag<double>(cudaStream_t, Grid, const uint8_t*, const FilterKe<double>&, double*);
 template void launch_filter_diag<float>(cudaStream_t, Grid, const uint8_t*, const FilterKe<double>&, float*);
 template void launch_filter_ku<double>(cudaStream_t, KuMode, Grid, const FilterKe<double>&, const double*, const double*, double*, double*,
-                                       const uint8_t*, PcgScalars*, RedScratch, KuTiles);
+                                       const uint8_t*, PcgScalars*, RedScratch, FilterTiles);
 template void launch_filter_ku<float>(cudaStream_t, KuMode, Grid, const FilterKe<float>&, const float*, const float*, float*, float*,
-                                      const uint8_t*, PcgScalars*, RedScratch, KuTiles);
+                                      const uint8_t*, PcgScalars*, RedScratch, FilterTiles);
 template void launch_filter_residual_init<double>(cudaStream_t, Grid, const double*, const double*, double*, double*,
                                                   double*, PcgScalars*, RedScratch, double, int, const uint32_t*);
 template void launch_filter_residual_init<float>(cudaStream_t, Grid, const float*, const float*, float*, float*,

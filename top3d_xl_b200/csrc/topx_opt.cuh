@@ -31,9 +31,14 @@ template <typename T>
 void launch_filter_e2n(cudaStream_t st, Grid g, const T* srcE, T* node, const uint32_t* act = nullptr);
 template <typename T>
 void launch_filter_diag(cudaStream_t st, Grid g, const uint8_t* solid, const FilterKe<double>& kf, T* dp);
+// tiles of the filter operator's launch that own a node of the domain (a null list launches all)
+struct FilterTiles {
+  const uint32_t* list = nullptr;
+  int n = 0;
+};
 template <typename T>
 void launch_filter_ku(cudaStream_t st, KuMode mode, Grid g, const FilterKe<T>& kf, const T* in, const T* z, T* pout,
-                      T* out, const uint8_t* solid, PcgScalars* sc, RedScratch rs, KuTiles tiles = KuTiles{});
+                      T* out, const uint8_t* solid, PcgScalars* sc, RedScratch rs, FilterTiles tiles = FilterTiles{});
 // tiles of the filter's K*u launch that own a node of the domain (a null list launches them all)
 std::vector<uint32_t> filter_active_tiles(Grid g, const std::vector<uint8_t>& present);
 template <typename T>
