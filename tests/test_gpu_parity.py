@@ -308,3 +308,31 @@ def test_ku_tile_edges(shape, holes):
         ctx.load_voxels(vox)
         ctx.set_moduli(E)
         assert _rel(ctx.ku(u), sol.ku(u)) < 1e-13
+
+
+@pytest.mark.parametrize("shape", [(3, 3, 3), (9, 41, 7), (33, 20, 12), (14, 70, 30), (30, 9, 65)])
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_pcg_step_edges(shape, precision):
+    # the PCG step's fused passes (the direction formed inside K*u from the residual and the level-2
+    # correction, the residual's update with the y pass of its restriction): tiles, chunks and
+    # padded rows of odd extents; the bars are test_pcg's, its counts within one (a knife edge of the stop test)
+    from top3d_xl_b200 import Context
+    vox = np.ones(shape, bool)
+    m = O.build_model(vox)
+    x = np.random.default_rng(1).uniform(0.3, 1.0, m.levels[0].numElements)
+    S = m.S
+    E = S.modulusMin + x ** S.SIMPpenalty * (S.modulus - S.modulusMin)
+    sol = O.Solver(m)
+    sol.assemble(E)
+    uo, itso, _ = O.pcg(sol.ku, sol.vcycle, m.F[:, 0], m.S.tol, m.S.maxIT)
+    f = m.F[:, 0]
+    with Context(precision) as ctx:
+        ctx.load_voxels(vox)
+        ctx.set_moduli(E)
+        ctx.assemble()
+        r = np.random.default_rng(3).standard_normal(m.levels[0].numDOFs)
+        assert _rel(ctx.vcycle(r), sol.vcycle(r)) < (1e-11 if precision == "fp64" else 1e-5)
+        u, its = ctx.pcg()
+    assert abs(its - itso) <= 1
+    if its == itso:
+        assert abs(f @ u - f @ uo) / abs(f @ uo) < (1e-8 if precision == "fp64" else 1e-6)

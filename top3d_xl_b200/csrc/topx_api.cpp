@@ -421,19 +421,20 @@ topx_status topx_ku_noalloc(topx_ctx* ctx, const double* u_dev, double* y_dev, s
                   "call such as topx_set_moduli");
     topx::Engine& eng = *ctx->engine;
     if (!u_dev || !y_dev || ndof != size_t(eng.Nn) * 3) return fail(ctx, TOPX_ERR_ARG, "DOF size mismatch");
-    const size_t grid = size_t(eng.G[0].stride) * 3;
-    const size_t need = 2 * grid * sizeof(double);
+    // the limit counts the grid's nodes without the rows that pad its y extent
+    const size_t nodes = (size_t(eng.node_rows()) * eng.G[0].nnx() * eng.G[0].nnz() + 31) / 32 * 32;
+    const size_t need = 2 * 3 * nodes * sizeof(double);
     if (need > topx::noalloc_scratch_bytes())
       return fail(ctx, TOPX_ERR_ARG,
                   "topx_ku_noalloc: this model needs " + std::to_string(need) + " bytes of scratch (2 x 3 x " +
-                      std::to_string(eng.G[0].stride) + " padded grid nodes x 8 B); the fixed scratch holds " +
+                      std::to_string(nodes) + " padded grid nodes x 8 B); the fixed scratch holds " +
                       std::to_string(topx::noalloc_scratch_bytes()) + " bytes; use topx_ku for this model");
     DeviceScope scope(ctx->params.device);
     if (!on_device(u_dev, ctx->params.device) || !on_device(y_dev, ctx->params.device))
       return fail(ctx, TOPX_ERR_ARG, "topx_ku_noalloc: u and y must be device (or managed) memory of the "
                                      "context's GPU");
     double* s = topx::noalloc_scratch(ctx->params.device);
-    eng.apply_K_device(u_dev, y_dev, s, s + grid);
+    eng.apply_K_device(u_dev, y_dev, s);
     return TOPX_OK;
   });
 }

@@ -21,12 +21,12 @@ static inline unsigned grid1d(int64_t n, int threads, int cap = 148 * 16) {
 // ---------------------------------------------------------------------------
 constexpr int GL2_ELEMS = 16, GL2_THREADS = 192;
 
-__global__ void __launch_bounds__(GL2_THREADS) k_galerkin_l2(Grid gc, const double* __restrict__ Ef,
+__global__ void __launch_bounds__(GL2_THREADS) k_galerkin_l2(Grid gf, Grid gc, const double* __restrict__ Ef,
                                                              const double* __restrict__ Tm, double* __restrict__ Ks) {
   __shared__ double sE[GL2_ELEMS][64];
   const int64_t nce = gc.nelems();
   const int64_t j0 = int64_t(blockIdx.x) * GL2_ELEMS;
-  const int fny = 4 * gc.ny, fnx = 4 * gc.nx;
+  const int fny = gf.nny(), fnx = gf.nnx();
   for (int i = threadIdx.x; i < GL2_ELEMS * 64; i += GL2_THREADS) {
     const int jj = i / 64, c = i % 64;
     const int64_t j = j0 + jj;
@@ -77,9 +77,9 @@ __global__ void __launch_bounds__(GL2_THREADS) k_galerkin_l2(Grid gc, const doub
   }
 }
 
-void launch_galerkin_l2(cudaStream_t st, Grid gc, const double* Efine, const double* Tm, double* Ks) {
+void launch_galerkin_l2(cudaStream_t st, Grid gf, Grid gc, const double* Efine, const double* Tm, double* Ks) {
   const int64_t nb = (gc.nelems() + GL2_ELEMS - 1) / GL2_ELEMS;
-  (k_galerkin_l2<<<unsigned(nb), GL2_THREADS, 0, st>>>(gc, Efine, Tm, Ks), topx::count_launch());
+  (k_galerkin_l2<<<unsigned(nb), GL2_THREADS, 0, st>>>(gf, gc, Efine, Tm, Ks), topx::count_launch());
   TOPX_CUDA_OK(cudaGetLastError());
 }
 
@@ -87,7 +87,7 @@ void launch_galerkin_l2(cudaStream_t st, Grid gc, const double* Efine, const dou
 // Ks2_j = sum_c E_c T_sel(j,c) + F_j, where T_sel is the child's template or the
 // template of its BC-modified Ke (uniqueKesFree_), and F_j collects the
 // E-independent uniqueKesFixed_ parts.
-__global__ void __launch_bounds__(GL2_THREADS) k_galerkin_l2_flagged(Grid gc, const double* __restrict__ Ef,
+__global__ void __launch_bounds__(GL2_THREADS) k_galerkin_l2_flagged(Grid gf, Grid gc, const double* __restrict__ Ef,
                                                                      const int32_t* __restrict__ fl_elem,
                                                                      const int32_t* __restrict__ fl_tsel,
                                                                      const double* __restrict__ fl_F,
@@ -97,7 +97,7 @@ __global__ void __launch_bounds__(GL2_THREADS) k_galerkin_l2_flagged(Grid gc, co
   __shared__ int sT[64];
   const int f = blockIdx.x;
   const int64_t j = fl_elem[f];
-  const int fny = 4 * gc.ny, fnx = 4 * gc.nx;
+  const int fny = gf.nny(), fnx = gf.nnx();
   const int gy = int(j % gc.ny), gx = int((j / gc.ny) % gc.nx), gz = int(j / (int64_t(gc.ny) * gc.nx));
   for (int c = threadIdx.x; c < 64; c += GL2_THREADS) {
     const int cy = c & 3, cx = (c >> 2) & 3, cz = c >> 4;
@@ -112,10 +112,10 @@ __global__ void __launch_bounds__(GL2_THREADS) k_galerkin_l2_flagged(Grid gc, co
   }
 }
 
-void launch_galerkin_l2_flagged(cudaStream_t st, Grid gc, const double* Efine, int nflag, const int32_t* fl_elem,
+void launch_galerkin_l2_flagged(cudaStream_t st, Grid gf, Grid gc, const double* Efine, int nflag, const int32_t* fl_elem,
                                 const int32_t* fl_tsel, const double* fl_F, const double* Tall, double* Ks) {
   if (nflag <= 0) return;
-  (k_galerkin_l2_flagged<<<nflag, GL2_THREADS, 0, st>>>(gc, Efine, fl_elem, fl_tsel, fl_F, Tall, Ks), topx::count_launch());
+  (k_galerkin_l2_flagged<<<nflag, GL2_THREADS, 0, st>>>(gf, gc, Efine, fl_elem, fl_tsel, fl_F, Tall, Ks), topx::count_launch());
   TOPX_CUDA_OK(cudaGetLastError());
 }
 

@@ -24,6 +24,8 @@ Engine::Engine(Model& model, int precision, int device, bool coarse_coop) : M(mo
   prepare_ku_kernels();
   prepare_nd_kernels();
   nl = M.numLevels;
+  if (nl >= 3 && int(M.levels.size()) == nl && M.levels[1].span != KU_SPAN)
+    throw std::runtime_error("the first coarsening does not have span 4");
   if (nl < 3 || int(M.levels.size()) != nl) throw std::runtime_error("model hierarchy not built");
   for (int l = 0; l < nl; ++l) {
     const Level& L = M.levels[l];
@@ -31,10 +33,19 @@ Engine::Engine(Model& model, int precision, int device, bool coarse_coop) : M(mo
     g.ny = L.resY;
     g.nx = L.resX;
     g.nz = L.resZ;
+    // level-1 rows along y hold a multiple of four nodes (the last up to three are absent), so that every row
+    // starts on a 16-byte boundary in FP64 and FP32 (what TMA copies need)
+    if (l == 0) g.ny = int(round_up(L.resY + 1, 4)) - 1;
     g.stride = round_up(g.nnodes(), 32);
     G.push_back(g);
   }
   const Level& l1 = M.levels[0];
+  nodeRows = l1.resY + 1;
+  // a level-1 node (y, x, z), and the element whose lowest corner it is, share one index: y + nny (x + nnx z)
+  auto pad_node = [&](int64_t k) { return k % (l1.resY + 1) + G[0].nny() * (k / (l1.resY + 1)); };
+  auto pad_elem = [&](int64_t e) {
+    return e % l1.resY + G[0].nny() * ((e / l1.resY) % l1.resX + G[0].nnx() * (e / (int64_t(l1.resY) * l1.resX)));
+  };
   Ne = l1.numElements;
   Nn = l1.numNodes;
   // ---- presence masks per level -------------------------------------------
@@ -42,18 +53,25 @@ Engine::Engine(Model& model, int precision, int device, bool coarse_coop) : M(mo
   epresent.resize(nl);
   for (int l = 0; l < nl; ++l) {
     const Level& L = M.levels[l];
-    std::vector<uint8_t> pn(size_t(G[l].nnodes()), 0), pe(size_t(G[l].nelems()), 0);
-    for (auto k : L.nodMapBack) pn[k - 1] = 1;
-    for (auto k : L.eleMapBack) pe[k - 1] = 1;
+    std::vector<uint8_t> pn(size_t(G[l].nnodes()), 0), pe(size_t(l ? G[l].nelems() : G[l].nnodes()), 0);
+    for (auto k : L.nodMapBack) pn[l ? k - 1 : pad_node(k - 1)] = 1;
+    for (auto k : L.eleMapBack) pe[l ? k - 1 : pad_elem(k - 1)] = 1;
     present[l].upload(pn.data(), pn.size());
-    epresent[l].upload(pe.data(), pe.size());
-    if (l == 0) solid1.upload(pe.data(), pe.size());
+    if (l == 0)
+      solid1.upload(pe.data(), pe.size());
+    else
+      epresent[l].upload(pe.data(), pe.size());
   }
   std::vector<int32_t> emb(Ne), nmb(Nn);
-  for (int64_t e = 0; e < Ne; ++e) emb[e] = l1.eleMapBack[e] - 1;
-  for (int64_t k = 0; k < Nn; ++k) nmb[k] = l1.nodMapBack[k] - 1;
+  for (int64_t e = 0; e < Ne; ++e) emb[e] = int32_t(pad_elem(l1.eleMapBack[e] - 1));
+  for (int64_t k = 0; k < Nn; ++k) nmb[k] = int32_t(pad_node(l1.nodMapBack[k] - 1));
   eleMapBack0.upload(emb.data(), emb.size());
   nodMapBack0.upload(nmb.data(), nmb.size());
+  {
+    std::vector<int32_t> fwd(size_t(G[0].nnodes()), -1);
+    for (int64_t k = 0; k < Nn; ++k) fwd[size_t(nmb[k])] = int32_t(k);
+    nodMapFwd0.upload(fwd.data(), fwd.size());
+  }
   // ---- boundary conditions: global form of the per-element BC matrices -------
   // (TOP3D_XL.m:1338-1437).  Check that the element matrices reduce to
   // y = m.*K(m.*u) + (1-m).*cfix.*u before relying on it.
@@ -63,14 +81,14 @@ Engine::Engine(Model& model, int precision, int device, bool coarse_coop) : M(mo
     uint8_t b = 0;
     for (int c = 0; c < 3; ++c)
       if (M.fixedDOFs[size_t(k) * 3 + c]) b |= uint8_t(1u << c);
-    fb[nmb[k]] = b;
+    fb[nmb[k]] = b | 8u;  // present
   }
   std::vector<double> cacc(size_t(Nn) * 3, 0.0);
   for (int a = 0; a < 8; ++a)
     for (int64_t e = 0; e < Ne; ++e) {
       const int32_t sl = M.mapUniqueKes[e];
       const int32_t node = l1.eNodMat[size_t(e) * 8 + a];
-      const uint8_t nb = fb[nmb[node - 1]];
+      const uint8_t nb = fb[nmb[node - 1]] & 7u;
       if (sl == 0) {
         if (nb) throw std::runtime_error("unsupported boundary conditions: element without BC matrix at a fixed DOF");
         continue;
@@ -185,10 +203,10 @@ Engine::Engine(Model& model, int precision, int device, bool coarse_coop) : M(mo
   // ---- level-1 K*u: the tiles that own a node of the domain (when voids leave some out) -----
   {
     std::vector<uint8_t> pn(size_t(G[0].nnodes()), 0);
-    for (auto k : M.levels[0].nodMapBack) pn[k - 1] = 1;
-    kush = ku_shape(G[0]);
+    for (auto k : nmb) pn[size_t(k)] = 1;
+    kush = ku_shape(G[0], nodeRows);
     std::vector<uint32_t> zr;
-    const std::vector<uint32_t> act = ku_active_tiles(G[0], kush, pn, &zr);
+    const std::vector<uint32_t> act = ku_active_tiles(G[0], nodeRows, kush, pn, &zr);
     const std::vector<uint8_t> all(pn.size(), 1);
     const size_t full = size_t(kush.grid.x) * kush.grid.y * kush.grid.z;
     if (!act.empty() && act.size() < full * 9 / 10) {
@@ -215,22 +233,6 @@ Engine::Engine(Model& model, int precision, int device, bool coarse_coop) : M(mo
     if (nact < nchunk * 9 / 10) {
       act1Mask.upload(mask.data(), mask.size());
       act1 = act1Mask.p;
-    }
-    // the level-1 restriction's y pass skips (x, z) columns without a present node
-    const int64_t ncol = int64_t(G[0].nnx()) * G[0].nnz(), nny1 = G[0].nny();
-    std::vector<uint32_t> cm(size_t((ncol + 31) / 32), 0u);
-    int64_t ncact = 0;
-    for (int64_t q = 0; q < ncol; ++q) {
-      bool any = false;
-      for (int64_t y = 0; y < nny1 && !any; ++y) any = pn[size_t(y + nny1 * q)] != 0;
-      if (any) {
-        cm[size_t(q / 32)] |= 1u << (q % 32);
-        ++ncact;
-      }
-    }
-    if (ncact < ncol * 9 / 10) {
-      cols1Mask.upload(cm.data(), cm.size());
-      cols1 = cols1Mask.p;
     }
   }
   // ---- coarsest level: nested-dissection plan and factor storage -----------------
@@ -290,8 +292,12 @@ Engine::Engine(Model& model, int precision, int device, bool coarse_coop) : M(mo
   {
     const size_t S1 = size_t(G[0].stride) * 3;
     for (DevBuf<double>* b : {&kw.r, &kw.z, &kw.p, &kw.q, &kw.p2}) b->alloc(S1);
-    E64.alloc(size_t(G[0].nelems()));
+    d0.alloc(size_t(G[0].stride));
+    kw.ty.alloc(size_t(G[1].nny()) * G[0].nnx() * G[0].nnz() * 3);
+    E64.alloc(size_t(G[0].stride));
     cfix64.upload(cf.data(), cf.size());
+    for (double& v : cf) v = v != 0.0 ? 1.0 / v : 0.0;
+    icfix64.upload(cf.data(), cf.size());
     if (!pre32()) {
       alloc_vwork(v64);
       if (M.S.typeVcycle == 1) {
@@ -387,10 +393,10 @@ void Engine::alloc_vwork(VWork<TC>& v) {
     v.rl[l].alloc(Sl);
     v.xl[l].alloc(Sl);
     if (l < nl - 1) v.dl[l].alloc(Sl);
-    const Grid& gf = G[l - 1];
-    const Grid& gc = G[l];
-    tmax = std::max(tmax, size_t(gc.nny()) * gf.nnx() * gf.nnz());
+    if (l > 1 && G[l - 1].nnodes() > kRestrictOneLaunch)
+      tmax = std::max(tmax, size_t(G[l].nny()) * G[l - 1].nnx() * G[l - 1].nnz());
   }
+  if (!std::is_same<TC, double>::value) v.rc64.alloc(size_t(G[1].stride) * 3);
   v.tmp1.alloc(tmax * 3);
   v.tmp2.alloc(tmax * 3);
 }
@@ -399,21 +405,21 @@ template <typename TF>
 void Engine::alloc_fwork(FWork<TF>& f) {
   const size_t N1 = size_t(G[0].nnodes());
   for (DevBuf<TF>* b : {&f.fr, &f.fz, &f.fp, &f.fq, &f.fy, &f.fb}) b->alloc(N1);
-  f.fsrc.alloc(size_t(G[0].nelems()));
+  f.fsrc.alloc(N1);
   f.fdp[0].alloc(N1);
   f.fdp[1].alloc(N1);
 }
 
 void Engine::read_scalars(PcgScalars& h, const PcgScalars* d) const {
   TOPX_CUDA_OK(cudaMemcpyAsync(h_sc, d, sizeof(PcgScalars), cudaMemcpyDeviceToHost, st));
-  if (coopCtas) TOPX_CUDA_OK(cudaMemcpyAsync(h_ctl, coopCtl.p, sizeof(CoopControl), cudaMemcpyDeviceToHost, st));
+  TOPX_CUDA_OK(cudaMemcpyAsync(h_ctl, coopCtl.p, sizeof(CoopControl), cudaMemcpyDeviceToHost, st));
   TOPX_CUDA_OK(cudaStreamSynchronize(st));
   h = *h_sc;
   check_device_waits();
 }
 
 void Engine::check_coop_waits() {
-  if (coopCtas) TOPX_CUDA_OK(cudaMemcpyAsync(h_ctl, coopCtl.p, sizeof(CoopControl), cudaMemcpyDeviceToHost, st));
+  TOPX_CUDA_OK(cudaMemcpyAsync(h_ctl, coopCtl.p, sizeof(CoopControl), cudaMemcpyDeviceToHost, st));
   TOPX_CUDA_OK(cudaStreamSynchronize(st));
   check_device_waits();
 }
@@ -423,11 +429,11 @@ void Engine::copy_sync(void* dst, const void* src, size_t bytes, cudaMemcpyKind 
   TOPX_CUDA_OK(cudaStreamSynchronize(st));
 }
 
-// The persistent coarse solve's dependency waits set an error word instead of spinning on (they
-// are bounded); the word was copied into pinned memory before the caller's stream sync.  A word
+// The persistent coarse solve's dependency waits and the K*u's waits for its copies set an error word instead
+// of spinning on (they are bounded); the word was copied into pinned memory before the caller's stream sync.  A word
 // that is set is cleared (so the engine stays usable) and reported.
 void Engine::check_device_waits() const {
-  if (coopCtas && h_ctl->err) {
+  if (h_ctl->err) {
     const int err = h_ctl->err;
     h_ctl->err = 0;
     // a launch that gave up may leave chunk tickets and dependency counts behind
@@ -436,7 +442,8 @@ void Engine::check_device_waits() const {
     if (ndDone.p) TOPX_CUDA_OK(cudaMemsetAsync(ndDone.p, 0, sizeof(unsigned) * ndDone.n, st));
     TOPX_CUDA_OK(cudaStreamSynchronize(st));
     throw DeviceWaitError(err == kCoopErrWait ? "coarse solve: a dependency wait gave up (persistent launch not co-resident)"
-                                              : "coarse solve: unknown wait error");
+                          : err == kCoopErrCopy ? "K*u: a wait for copies into shared memory gave up"
+                                                : "unknown wait error");
   }
 }
 
@@ -500,13 +507,13 @@ void Engine::assemble() {
 void Engine::assemble_launches() {
   sec_begin(SEC_DIAG);
   if (!pre32())
-    launch_diag_l1<double>(st, G[0], E64.p, fixbits.p, cfix64.p, present[0].p, v64.d1.p);
+    launch_diag_l1<double>(st, G[0], E64.p, fixbits.p, cfix64.p, present[0].p, v64.d1.p, d0.p);
   else
-    launch_diag_l1<double, float>(st, G[0], E64.p, fixbits.p, cfix64.p, present[0].p, v32.d1.p);
+    launch_diag_l1<float>(st, G[0], E64.p, fixbits.p, cfix64.p, present[0].p, v32.d1.p, d0.p);
   sec_end();
   sec_begin(SEC_GALERKIN2);
-  launch_galerkin_l2(st, G[1], E64.p, Tall.p, Ks[1].p);
-  launch_galerkin_l2_flagged(st, G[1], E64.p, nflag, fl_elem.p, fl_tsel.p, fl_F.p, Tall.p, Ks[1].p);
+  launch_galerkin_l2(st, G[0], G[1], E64.p, Tall.p, Ks[1].p);
+  launch_galerkin_l2_flagged(st, G[0], G[1], E64.p, nflag, fl_elem.p, fl_tsel.p, fl_F.p, Tall.p, Ks[1].p);
   sec_end();
   sec_begin(SEC_GALERKIN3);
   for (int l = 2; l < nl; ++l) launch_galerkin_span2(st, G[l], Ks[l - 1].p, epresent[l].p, W8.p, Ks[l].p);
@@ -532,12 +539,31 @@ void Engine::factor_coarsest() {
 // ---------------------------------------------------------------------------
 // 'Adapted' V-cycle (TOP3D_XL.m:747-781)
 // ---------------------------------------------------------------------------
+void Engine::residual(ResidualMode mode, double* r, const double* b, PcgScalars* sc, double tol, int maxIT) {
+  ResidualArgs a{};
+  a.g = G[0];
+  a.r = r;
+  a.b = b;
+  a.q = kw.q.p;
+  a.D = d0.p;
+  a.pre32 = pre32();
+  a.flags = fixbits.p;
+  a.icfix = icfix64.p;
+  a.tmp = kw.ty.p;
+  a.act = act1;
+  a.sc = sc;
+  a.rs = rs1;
+  a.tol = tol;
+  a.maxIT = maxIT;
+  launch_residual(st, mode, a, G[1]);
+}
+
 template <typename TC>
-void Engine::vcycle_t(VWork<TC>& v, bool init, PcgScalars* sc) {
+void Engine::coarse_correction(VWork<TC>& v, bool dot, bool init, PcgScalars* sc) {
   sec_begin(SEC_RESTRICT);
-  launch_restrict<double, TC>(st, M.levels[1].span, kw.r.p, G[0], v.tmp1.p, v.tmp2.p, v.rl[1].p, G[1], cols1);
+  launch_restrict_xz<TC>(st, kw.ty.p, G[0], v.rl[1].p, v.rc64.p, G[1], sc);
   for (int l = 2; l < nl; ++l)
-    launch_restrict<TC, TC>(st, M.levels[l].span, v.rl[l - 1].p, G[l - 1], v.tmp1.p, v.tmp2.p, v.rl[l].p, G[l]);
+    launch_restrict<TC>(st, v.rl[l - 1].p, G[l - 1], v.tmp1.p, v.tmp2.p, v.rl[l].p, G[l], sc);
   sec_end();
   sec_begin(SEC_COARSE_SOLVE);
   {
@@ -546,12 +572,22 @@ void Engine::vcycle_t(VWork<TC>& v, bool init, PcgScalars* sc) {
   }
   sec_end();
   sec_begin(SEC_PROLONG);
-  const double om = M.S.weightFactorJacobi;
   for (int l = nl - 2; l >= 1; --l)
     launch_prolong_smooth<TC, TC, TC>(st, M.levels[l + 1].span, v.xl[l + 1].p, G[l + 1], v.rl[l].p, v.dl[l].p,
-                                      present[l].p, v.xl[l].p, G[l], om, false, false, sc, rs1);
+                                      present[l].p, v.xl[l].p, G[l], M.S.weightFactorJacobi,
+                                      dot && l == 1 ? v.rc() : nullptr, init, sc, rs1);
+  sec_end();
+}
+
+template <typename TC>
+void Engine::vcycle_t(VWork<TC>& v, PcgScalars* sc) {
+  sec_begin(SEC_RESTRICT);
+  residual(RES_KEEP, kw.r.p, nullptr, sc, 0.0, 0);
+  sec_end();
+  coarse_correction<TC>(v, false, false, sc);
+  sec_begin(SEC_PROLONG);
   launch_prolong_smooth<TC, double, TC>(st, M.levels[1].span, v.xl[1].p, G[1], kw.r.p, v.d1.p, present[0].p,
-                                        kw.z.p, G[0], om, true, init, sc, rs1, act1);
+                                        kw.z.p, G[0], M.S.weightFactorJacobi, nullptr, false, sc, rs1, act1);
   sec_end();
 }
 
@@ -568,13 +604,13 @@ void Engine::vcycle_standard(bool init, PcgScalars* sc) {
   launch_jacobi_pre<double, double, double>(st, G[0], kw.r.p, v.d1.p, present[0].p, kw.z.p, om, sc);
   ku(KU_PLAIN, kw.z.p, nullptr, nullptr, kw.q.p, sc, nullptr);
   launch_residual_inplace<double, double>(st, G[0], kw.r.p, kw.q.p, sc);
-  launch_restrict<double, double>(st, M.levels[1].span, kw.q.p, G[0], v.tmp1.p, v.tmp2.p, v.rl[1].p, G[1], cols1);
+  residual(RES_KEEP, kw.q.p, nullptr, sc, 0.0, 0);
+  launch_restrict_xz<double>(st, kw.ty.p, G[0], v.rl[1].p, nullptr, G[1], sc);
   for (int l = 1; l < nl - 1; ++l) {
     launch_jacobi_pre<double, double, double>(st, G[l], v.rl[l].p, v.dl[l].p, present[l].p, v.xl[l].p, om, sc);
     launch_ku_coarse(st, G[l], Ks[l].p, epresent[l].p, present[l].p, v.xl[l].p, vq[l].p, sc);
     launch_residual_inplace<double, double>(st, G[l], v.rl[l].p, vq[l].p, sc);
-    launch_restrict<double, double>(st, M.levels[l + 1].span, vq[l].p, G[l], v.tmp1.p, v.tmp2.p, v.rl[l + 1].p,
-                                    G[l + 1]);
+    launch_restrict<double>(st, vq[l].p, G[l], v.tmp1.p, v.tmp2.p, v.rl[l + 1].p, G[l + 1], sc);
   }
   sec_end();
   sec_begin(SEC_COARSE_SOLVE);
@@ -596,34 +632,41 @@ void Engine::vcycle_standard(bool init, PcgScalars* sc) {
   sec_end();
 }
 
-void Engine::vcycle(bool init, PcgScalars* sc) {
-  if (!pre32() && M.S.typeVcycle == 1)
+void Engine::precondition(bool init, PcgScalars* sc) {
+  if (standard())
     vcycle_standard(init, sc);
   else if (!pre32())
-    vcycle_t<double>(v64, init, sc);
+    coarse_correction<double>(v64, true, init, sc);
   else
-    vcycle_t<float>(v32, init, sc);
+    coarse_correction<float>(v32, true, init, sc);
 }
 
 void Engine::ku(KuMode mode, const double* in, const double* pin, double* pout, double* out, PcgScalars* sc,
-                double* y) {
+                double* y, const int32_t* compact) {
   KuArgs a{};
   a.g = G[0];
   a.sh = kush;
   a.K = kumodes;
+  a.gc = G[1];
   a.in = in;
-  a.z = in;
+  a.D = d0.p;
+  a.xc = pre32() ? static_cast<const void*>(v32.xl[1].p) : v64.xl[1].p;
+  a.pre32 = pre32();
+  a.omega2 = 2.0 * M.S.weightFactorJacobi;
   a.pin = pin;
   a.pout = pout;
   a.out = out;
   a.E = E64.p;
   a.flags = fixbits.p;
   a.cfix = cfix64.p;
+  a.icfix = icfix64.p;
   a.sc = sc;
   a.rs = rs1;
+  a.err = &coopCtl.p->err;
   a.active = kuTiles.p;
   a.zr = kuZr.p;
   a.yacc = y;
+  a.compact = compact;
   launch_ku(st, mode, a, int(kuTiles.n));
 }
 
@@ -640,9 +683,24 @@ int Engine::pcg(const double* b, double* y, bool warm, double tol, int maxIT) {
       ku(KU_PLAIN, y, nullptr, nullptr, kw.q.p, sc, nullptr);
     else
       TOPX_CUDA_OK(cudaMemsetAsync(kw.q.p, 0, kw.q.bytes(), st));
-    launch_residual_init<double>(st, g, b, kw.q.p, kw.r.p, sc, rs1, tol, maxIT);
-    vcycle(true, sc);
+    if (standard())
+      launch_residual_init(st, g, b, kw.q.p, kw.r.p, sc, rs1, tol, maxIT);
+    else
+      residual(RES_INIT, kw.r.p, b, sc, tol, maxIT);
+    precondition(true, sc);
   });
+  auto step_ku = [&](double* pin, double* pnew) {
+    if (standard())
+      ku(KU_P_UPDATE, kw.z.p, pin, pnew, kw.q.p, sc, y);
+    else
+      ku(KU_FUSED, kw.r.p, pin, pnew, kw.q.p, sc, y);
+  };
+  auto step_residual = [&]() {
+    if (standard())
+      launch_pcg_update(st, g, kw.r.p, kw.q.p, sc, rs1, act1);
+    else
+      residual(RES_UPDATE, kw.r.p, nullptr, sc, tol, maxIT);
+  };
   const int CH = 8;
   PcgScalars h{};
   int launched = 0;
@@ -654,9 +712,9 @@ int Engine::pcg(const double* b, double* y, bool warm, double tol, int maxIT) {
         for (int c = 0; c < CH; ++c) {  // CH is even: every chunk starts from p
           double* pin = (c & 1) ? kw.p2.p : kw.p.p;
           double* pnew = (c & 1) ? kw.p.p : kw.p2.p;
-          ku(KU_P_UPDATE, kw.z.p, pin, pnew, kw.q.p, sc, y);
-          launch_pcg_update<double, double>(st, g, y, nullptr, pnew, kw.r.p, kw.q.p, sc, rs1, act1);
-          vcycle(false, sc);
+          step_ku(pin, pnew);
+          step_residual();
+          precondition(false, sc);
         }
       });
       launched += CH;
@@ -668,12 +726,12 @@ int Engine::pcg(const double* b, double* y, bool warm, double tol, int maxIT) {
       if (prof_) TOPX_CUDA_OK(cudaEventRecord(pev[2 * c], st));
       double* pin = (launched & 1) ? kw.p2.p : kw.p.p;
       double* pnew = (launched & 1) ? kw.p.p : kw.p2.p;
-      ku(KU_P_UPDATE, kw.z.p, pin, pnew, kw.q.p, sc, y);
+      step_ku(pin, pnew);
       if (prof_) TOPX_CUDA_OK(cudaEventRecord(pev[2 * c + 1], st));
       sec_begin(SEC_UPDATE);
-      launch_pcg_update<double, double>(st, g, y, nullptr, pnew, kw.r.p, kw.q.p, sc, rs1, act1);
+      step_residual();
       sec_end();
-      vcycle(false, sc);
+      precondition(false, sc);
     }
     read_scalars(h, sc);
     if (prof_) {
@@ -773,13 +831,11 @@ int Engine::filter(int slot, const double* d_src, double* d_out) {
 // ---------------------------------------------------------------------------
 void Engine::apply_K(const double* h_u, double* h_y) {
   TOPX_CUDA_OK(cudaStreamSynchronize(st));
-  DevBuf<double> cu, du, dy;
+  DevBuf<double> cu, du;
   cu.upload(h_u, size_t(Nn) * 3);
   du.alloc(size_t(G[0].stride) * 3);
-  dy.alloc(size_t(G[0].stride) * 3);
   launch_compact_to_grid_nodes<double>(st, cu.p, du.p, G[0], nodMapBack0.p, Nn);
-  ku(KU_PLAIN, du.p, nullptr, nullptr, dy.p, nullptr, nullptr);
-  launch_grid_to_compact_nodes<double>(st, dy.p, cu.p, G[0], nodMapBack0.p, Nn);
+  ku(KU_PLAIN, du.p, nullptr, nullptr, cu.p, nullptr, nullptr, nodMapFwd0.p);
   TOPX_CUDA_OK(cudaStreamSynchronize(st));
   copy_sync(h_y, cu.p, sizeof(double) * Nn * 3, cudaMemcpyDeviceToHost);
 }
@@ -793,7 +849,12 @@ void Engine::apply_vcycle(const double* h_r, double* h_z) {
   copy_sync(scE.p, &z, sizeof(z), cudaMemcpyHostToDevice);
   TOPX_CUDA_OK(cudaMemsetAsync(kw.r.p, 0, kw.r.bytes(), st));
   launch_compact_to_grid_nodes<double>(st, cu.p, kw.r.p, G[0], nodMapBack0.p, Nn);
-  vcycle(true, scE.p);
+  if (standard())
+    vcycle_standard(true, scE.p);
+  else if (!pre32())
+    vcycle_t<double>(v64, scE.p);
+  else
+    vcycle_t<float>(v32, scE.p);
   launch_grid_to_compact_nodes<double>(st, kw.z.p, cu.p, G[0], nodMapBack0.p, Nn);
   check_coop_waits();
   copy_sync(h_z, cu.p, sizeof(double) * Nn * 3, cudaMemcpyDeviceToHost);
@@ -930,7 +991,10 @@ void Engine::get_diag(int level, double* h_d) const {
   }
   // the engine stores reciprocal diagonals
   for (int64_t k = 0; k < L.numNodes; ++k)
-    for (int c = 0; c < 3; ++c) h_d[3 * k + c] = 1.0 / dense[(L.nodMapBack[k] - 1) + c * g.stride];
+    for (int c = 0; c < 3; ++c) {
+      const int64_t id = L.nodMapBack[k] - 1, n = level == 1 ? id % nodeRows + g.nny() * (id / nodeRows) : id;
+      h_d[3 * k + c] = 1.0 / dense[n + c * g.stride];
+    }
 }
 
 // ---------------------------------------------------------------------------

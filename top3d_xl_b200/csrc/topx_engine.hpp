@@ -97,6 +97,7 @@ struct IterRecord {
 struct KrylovWork {
   DevBuf<double> r, z, p, q;
   DevBuf<double> p2;  // the direction alternates between p and p2 (K*u reads one, writes the other)
+  DevBuf<double> ty;  // y pass of the residual's restriction
 };
 
 // Multigrid preconditioner workspace in its storage precision TC (double for
@@ -106,7 +107,9 @@ template <typename TC>
 struct VWork {
   DevBuf<TC> d1;
   std::vector<DevBuf<TC>> rl, xl, dl;  // per level (index = level-1; level 1 uses the Krylov vectors)
-  DevBuf<TC> tmp1, tmp2;                // separable restriction passes
+  DevBuf<TC> tmp1, tmp2;               // separable restriction passes of large coarse levels
+  DevBuf<double> rc64;                 // FP64 copy of the level-2 residual (TC = float)
+  const double* rc() const { return rc64.p ? rc64.p : reinterpret_cast<const double*>(rl[1].p); }
 };
 
 // PDE-filter workspace (scalar node fields) in precision TF.
@@ -143,7 +146,7 @@ class Engine {
   // for tests: y = K u (FP64), z = M r (V-cycle in the engine precision)
   void apply_K(const double* h_u, double* h_y);
   // y = K u on device vectors (compact DOF order) with caller-provided grid scratch; topx_noalloc.cu
-  void apply_K_device(const double* d_u, double* d_y, double* grid_u, double* grid_y);
+  void apply_K_device(const double* d_u, double* d_y, double* grid_u);
   void apply_vcycle(const double* h_r, double* h_z);
   // runs one bounded device wait into its poll limit (test of the give-up path)
   void selftest_wait(int which);
@@ -154,6 +157,7 @@ class Engine {
   bool step(IterRecord& rec);  // false when the loop condition ends the run
   double cSolid() const { return cSolid_; }
   int loop() const { return loop_; }
+  int node_rows() const { return nodeRows; }  // level-1 node rows along y without padding
   const std::string& info() const { return info_; }
 
   // ---- measurement ----------------------------------------------------------
@@ -187,10 +191,15 @@ class Engine {
   void alloc_vwork(VWork<TC>& v);
   template <typename TF>
   void alloc_fwork(FWork<TF>& f);
+  // xl[1] from the level-1 residual whose y pass is in kw.ty; dot: completes z'r in sc
   template <typename TC>
-  void vcycle_t(VWork<TC>& v, bool init, PcgScalars* sc);
+  void coarse_correction(VWork<TC>& v, bool dot, bool init, PcgScalars* sc);
+  template <typename TC>
+  void vcycle_t(VWork<TC>& v, PcgScalars* sc);
   void vcycle_standard(bool init, PcgScalars* sc);
-  void vcycle(bool init, PcgScalars* sc);
+  bool standard() const { return !pre32() && M.S.typeVcycle == 1; }
+  void precondition(bool init, PcgScalars* sc);  // inside the PCG
+  void residual(ResidualMode mode, double* r, const double* b, PcgScalars* sc, double tol, int maxIT);
   int pcg(const double* b, double* y, bool warm, double tol, int maxIT);
   template <typename TF>
   int filter_t(FWork<TF>& f, int slot, const double* d_src, double* d_out);
@@ -204,8 +213,10 @@ class Engine {
   // level-1 static data
   DevBuf<uint8_t> fixbits, solid1;
   std::vector<DevBuf<uint8_t>> present, epresent;  // per level
-  DevBuf<int32_t> eleMapBack0, nodMapBack0;
-  DevBuf<double> E64, cfix64;        // dense moduli (elements) and fixed-DOF diagonal (nodes)
+  DevBuf<int32_t> eleMapBack0, nodMapBack0, nodMapFwd0;  // fwd: compact id of a grid node, or -1
+  int nodeRows = 0;   // node rows along y without the padding ones
+  DevBuf<double> d0;  // inverse diagonal of a node's free DOFs (rounded as the preconditioner's d1)
+  DevBuf<double> E64, cfix64, icfix64;  // dense moduli (elements, at their lowest node), fixed-DOF diagonal and its inverse (nodes)
   std::vector<DevBuf<double>> F, U;  // per load case, dense SoA FP64
   // coarse operators
   std::vector<DevBuf<double>> Ks;  // per level (index = level-1), dense elements x 576
@@ -217,14 +228,14 @@ class Engine {
   DevBuf<uint32_t> kuZr;     // per listed tile, its planes that hold a present node
   KuShape kush{};
   KuModes kumodes{};
-  // u or z, the directions, the result, and the solution to step; PLAIN: in -> out
-  void ku(KuMode mode, const double* in, const double* pin, double* pout, double* out, PcgScalars* sc, double* y);
+  // u, z or r, the directions, the result, and the solution to step; PLAIN: in -> out
+  // (compact: out takes the compact DOF order instead of the grid's)
+  void ku(KuMode mode, const double* in, const double* pin, double* pout, double* out, PcgScalars* sc, double* y,
+          const int32_t* compact = nullptr);
   DevBuf<uint32_t> filterTiles;  // the same for the filter's K*u (its own z-chunks)
   FilterTiles fut;
   DevBuf<uint32_t> act1Mask;     // level-1 chunk mask (chunk_active) of an irregular domain
   const uint32_t* act1 = nullptr;  // null: every chunk holds a present node
-  DevBuf<uint32_t> cols1Mask;      // level-1 (x, z) columns that hold a present node
-  const uint32_t* cols1 = nullptr;
   // coarsest level: nested-dissection plan, its device copy and the factor tiles
   NDPlan nd;
   NDDevice ndd;

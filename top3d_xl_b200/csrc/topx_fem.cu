@@ -1,8 +1,7 @@
 // Level-1 elasticity kernels of the TOP3D_XL B200 path (the operator is in topx_ku.cu): Jacobi diagonal, PCG vector algebra, trilinear multigrid transfers, SIMP,
 // unit compliance.  FP64 (plain path) and FP32 (mixed path) instantiations.
-#include <cmath>
+#include <algorithm>
 #include <stdexcept>
-#include <type_traits>
 
 #include "topx_kernels.cuh"
 
@@ -26,138 +25,239 @@ static inline unsigned grid1d(int64_t n, int threads, int cap = 148 * 16) {
 // hexes, in local-node order, of E_e * diag(Ke); fixed DOFs take cfix.  Stored
 // as its reciprocal (0 on absent nodes) so the smoother multiplies.
 // ---------------------------------------------------------------------------
-template <typename TE, typename T>
-__global__ void k_diag_l1(Grid g, const TE* __restrict__ E, const uint8_t* __restrict__ fixbits,
-                          const TE* __restrict__ cfix, const uint8_t* __restrict__ present, T* __restrict__ d) {
+template <typename T>
+__global__ void k_diag_l1(Grid g, const double* __restrict__ E, const uint8_t* __restrict__ fixbits,
+                          const double* __restrict__ cfix, const uint8_t* __restrict__ present, T* __restrict__ d,
+                          double* __restrict__ d0) {
   const int64_t N = g.nnodes();
   const int nny = g.ny + 1, nnx = g.nx + 1;
   for (int64_t n = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; n < N; n += int64_t(gridDim.x) * blockDim.x) {
-    double v[3] = {0.0, 0.0, 0.0};
+    double v[3] = {0.0, 0.0, 0.0}, v0 = 0.0;
     if (present[n]) {
       const int gy = int(n % nny), gx = int((n / nny) % nnx), gz = int(n / (int64_t(nny) * nnx));
       double s[3] = {0.0, 0.0, 0.0};
       for (int a = 0; a < 8; ++a) {
         const int ey = gy - hex_ly(a), ex = gx - hex_lx(a), ez = gz - hex_lz(a);
         if (ey < 0 || ey >= g.ny || ex < 0 || ex >= g.nx || ez < 0 || ez >= g.nz) continue;
-        const double Ee = double(E[ey + int64_t(g.ny) * (ex + int64_t(g.nx) * ez)]);
+        const double Ee = E[ey + int64_t(nny) * (ex + int64_t(nnx) * ez)];
         for (int c = 0; c < 3; ++c) s[c] += c_Ke64[(3 * a + c) * 25] * Ee;
       }
       const uint8_t fb = fixbits[n];
-      for (int c = 0; c < 3; ++c) v[c] = 1.0 / ((fb >> c) & 1 ? double(cfix[n]) : s[c]);
+      for (int c = 0; c < 3; ++c) v[c] = 1.0 / ((fb >> c) & 1 ? cfix[n] : s[c]);
+      v0 = 1.0 / s[0];
     }
     for (int c = 0; c < 3; ++c) d[n + c * g.stride] = T(v[c]);
+    d0[n] = double(T(v0));
   }
 }
 
-template <typename TE, typename T>
-void launch_diag_l1(cudaStream_t st, Grid g, const TE* E, const uint8_t* fixbits, const TE* cfix,
-                    const uint8_t* present, T* d) {
-  (k_diag_l1<TE, T><<<grid1d(g.nnodes(), 256), 256, 0, st>>>(g, E, fixbits, cfix, present, d), topx::count_launch());
+template <typename T>
+void launch_diag_l1(cudaStream_t st, Grid g, const double* E, const uint8_t* fixbits, const double* cfix,
+                    const uint8_t* present, T* d, double* d0) {
+  (k_diag_l1<T><<<grid1d(g.nnodes(), 256), 256, 0, st>>>(g, E, fixbits, cfix, present, d, d0), topx::count_launch());
   TOPX_CUDA_OK(cudaGetLastError());
 }
 
 // ---------------------------------------------------------------------------
 // PCG vector algebra (TOP3D_XL.m:613-622)
 // ---------------------------------------------------------------------------
-template <typename T>
-__global__ void k_residual_init(Grid g, const T* __restrict__ b, const T* __restrict__ Ay, T* __restrict__ r,
-                                PcgScalars* sc, RedScratch rs, double tol, int maxIT) {
+__device__ __forceinline__ void load4(const double* p, double (&v)[4]) {
+  const double2 a = *reinterpret_cast<const double2*>(p), b = *reinterpret_cast<const double2*>(p + 2);
+  v[0] = a.x;
+  v[1] = a.y;
+  v[2] = b.x;
+  v[3] = b.y;
+}
+__device__ __forceinline__ void pcg_start(PcgScalars* sc, double bb, double tol, int maxIT) {
+  sc->normB = sqrt(bb);
+  sc->tol = tol;
+  sc->maxIT = maxIT;
+  sc->its = 0;
+  sc->done = 0;
+  sc->first = 1;
+  sc->beta = 0.0;
+}
+__device__ __forceinline__ void pcg_stop_test(PcgScalars* sc, double lam, double rr) {
+  sc->lam = lam;
+  sc->rr = rr;
+  sc->resnorm = sqrt(rr) / sc->normB;
+  sc->its += 1;
+  sc->first = 0;
+  if (sc->resnorm < sc->tol)
+    sc->done = 1;
+  else if (sc->its >= sc->maxIT)
+    sc->done = 2;
+}
+
+// The first V-cycle of a solve and every iteration run one pass over the level-1 residual: the update
+// r -= lambda q (or r = b - q), the sums r'r and r'D r, and the y pass of the restriction from the new
+// values.  A lane takes four nodes along y (32 bytes of every field, and a coarse node's own cell: rows hold a
+// multiple of four nodes), sums their taps for the coarse node at its first one and for the next one, and hands
+// the latter to the next lane; a warp takes whole lines, 32 cells at a time, so that nothing but that
+// hand-over, from lane 31 to the next round's lane 0, crosses a round.  z'r needs no pass of its own:
+// r'z = omega2 r'D r + (P'r)'xc.
+template <int MODE, typename TC>
+__global__ void __launch_bounds__(256) k_residual(const __grid_constant__ ResidualArgs a, int lines, int cy, FastDiv dcy) {
+  if (MODE == RES_UPDATE && a.sc->done) return;
+  const int lane = threadIdx.x & 31;
+  const int64_t S = a.g.stride, nlines = int64_t(a.g.nx + 1) * (a.g.nz + 1), ts = nlines * cy;
+  double* __restrict__ const r = a.r;
+  const double* __restrict__ const src = MODE == RES_INIT ? a.b : a.r;
+  const double* __restrict__ const q = a.q;
+  const double* __restrict__ const D = a.D;
+  const double lam = MODE == RES_UPDATE ? a.sc->x1 / a.sc->pq : 0.0;
+  double s0 = 0.0, rd = 0.0;  // b'b or r'r, and r'D r
+  const int64_t line0 = (int64_t(blockIdx.x) * 8 + (threadIdx.x >> 5)) * lines;
+  const int cells = line0 < nlines ? int(min(int64_t(lines), nlines - line0)) * cy : 0;
+  double carry[3] = {0.0, 0.0, 0.0};  // lane 31's part of the next cell's node
+  for (int i0 = 0; i0 < cells; i0 += 32) {
+    const int i = i0 + lane;
+    const int64_t cell = line0 * cy + i, n = 4 * cell;
+    double v[3][4];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) v[c][0] = v[c][1] = v[c][2] = v[c][3] = 0.0;
+    if (i < cells && chunk_active(a.act, n)) {
+      double w[3][4], d[4];
+      unsigned f = 0;
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        load4(src + n + c * S, v[c]);
+        if (MODE != RES_KEEP) load4(q + n + c * S, w[c]);
+      }
+      if (MODE != RES_KEEP) {
+        load4(D + n, d);
+        f = *reinterpret_cast<const unsigned*>(a.flags + n) & 0x07070707u;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            if (MODE == RES_INIT) s0 = fma(v[c][k], v[c][k], s0);
+            v[c][k] = MODE == RES_INIT ? v[c][k] - w[c][k] : v[c][k] - lam * w[c][k];
+            if (MODE == RES_UPDATE) s0 = fma(v[c][k], v[c][k], s0);
+          }
+          *reinterpret_cast<double2*>(r + n + c * S) = make_double2(v[c][0], v[c][1]);
+          *reinterpret_cast<double2*>(r + n + c * S + 2) = make_double2(v[c][2], v[c][3]);
+        }
+        if (f) {  // fixed DOFs have their own diagonal
+          for (int k = 0; k < 4; ++k)
+            for (int c = 0; c < 3; ++c)
+              rd = fma(v[c][k] * v[c][k], f >> (8 * k + c) & 1u ? double(TC(a.icfix[n + k])) : d[k], rd);
+        } else {
+#pragma unroll
+          for (int k = 0; k < 4; ++k)
+            rd = fma(d[k], fma(v[2][k], v[2][k], fma(v[1][k], v[1][k], v[0][k] * v[0][k])), rd);
+        }
+      }
+    }
+    const bool begins = i - cy * int(dcy.div(uint32_t(i))) == 0;  // the line's first cell
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      const double own = fma(0.25, v[c][3], fma(0.5, v[c][2], fma(0.75, v[c][1], v[c][0])));
+      const double next = fma(0.25, v[c][1], fma(0.5, v[c][2], 0.75 * v[c][3]));
+      double prev = __shfl_up_sync(0xffffffffu, next, 1);
+      if (lane == 0) prev = carry[c];
+      carry[c] = __shfl_sync(0xffffffffu, next, 31);
+      if (i < cells) a.tmp[cell + c * ts] = begins ? own : own + prev;
+    }
+  }
+  if (MODE != RES_KEEP) {
+    double t[2] = {s0, rd}, tot[2];
+    if (reduce_publish<2>(t, a.rs, tot) && threadIdx.x == 0) {
+      a.sc->rdr = tot[1];
+      if (MODE == RES_INIT)
+        pcg_start(a.sc, tot[0], a.tol, a.maxIT);
+      else
+        pcg_stop_test(a.sc, lam, tot[0]);
+    }
+  }
+}
+// Lines of a warp: fewest rounds of 32 cells one after another, with 24 warps of an SM at a time; of those the fewest
+// lines (the reduction at a CTA's end costs about a round)
+static int residual_lines(int64_t nlines, int cy) {
+  const int64_t slots = 148 * 24;
+  int best = 1;
+  int64_t bestCost = -1;
+  for (int l = 1; l <= 64; ++l) {
+    const int64_t warps = (nlines + l - 1) / l, waves = (warps + slots - 1) / slots;
+    const int64_t cost = waves * ((int64_t(l) * cy + 31) / 32 + 1);
+    if (bestCost < 0 || cost < bestCost) {
+      bestCost = cost;
+      best = l;
+    }
+  }
+  return best;
+}
+void launch_residual(cudaStream_t st, ResidualMode mode, const ResidualArgs& args, Grid gc) {
+  const int cy = gc.nny();
+  if (args.g.nny() != 4 * cy) throw std::runtime_error("level-1 rows do not hold four nodes per coarse node");
+  const int64_t nlines = int64_t(args.g.nnx()) * args.g.nnz();
+  const int lines = residual_lines(nlines, cy);
+  const unsigned nb = unsigned((nlines + 8 * lines - 1) / (8 * lines));
+  const FastDiv dcy{uint32_t(cy)};
+  auto go = [&](auto kernel) { (kernel<<<nb, 256, 0, st>>>(args, lines, cy, dcy), topx::count_launch()); };
+  if (mode == RES_KEEP)
+    go(k_residual<RES_KEEP, double>);
+  else if (mode == RES_INIT && args.pre32)
+    go(k_residual<RES_INIT, float>);
+  else if (mode == RES_INIT)
+    go(k_residual<RES_INIT, double>);
+  else if (args.pre32)
+    go(k_residual<RES_UPDATE, float>);
+  else
+    go(k_residual<RES_UPDATE, double>);
+  TOPX_CUDA_OK(cudaGetLastError());
+}
+
+// The 'Standard' V-cycle's own residual start and update (it restricts another vector)
+__global__ void k_residual_init(Grid g, const double* __restrict__ b, const double* __restrict__ Ay,
+                                double* __restrict__ r, PcgScalars* sc, RedScratch rs, double tol, int maxIT) {
   const int64_t N = g.nnodes(), S = g.stride;
   double bb = 0.0;
   for (int64_t n = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; n < N; n += int64_t(gridDim.x) * blockDim.x) {
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-      const T bv = b[n + c * S];
+      const double bv = b[n + c * S];
       r[n + c * S] = bv - Ay[n + c * S];
-      bb += double(bv) * double(bv);
+      bb += bv * bv;
     }
   }
   double v[1] = {bb}, tot[1];
-  if (reduce_publish<1>(v, rs, tot) && threadIdx.x == 0) {
-    sc->normB = sqrt(tot[0]);
-    sc->tol = tol;
-    sc->maxIT = maxIT;
-    sc->its = 0;
-    sc->done = 0;
-    sc->first = 1;
-    sc->beta = 0.0;
-  }
+  if (reduce_publish<1>(v, rs, tot) && threadIdx.x == 0) pcg_start(sc, tot[0], tol, maxIT);
 }
 
-template <typename T>
-void launch_residual_init(cudaStream_t st, Grid g, const T* b, const T* Ay, T* r, PcgScalars* sc, RedScratch rs,
-                          double tol, int maxIT) {
-  (k_residual_init<T><<<grid1d(g.nnodes(), 256), 256, 0, st>>>(g, b, Ay, r, sc, rs, tol, maxIT), topx::count_launch());
+void launch_residual_init(cudaStream_t st, Grid g, const double* b, const double* Ay, double* r, PcgScalars* sc,
+                          RedScratch rs, double tol, int maxIT) {
+  (k_residual_init<<<grid1d(g.nnodes(), 256), 256, 0, st>>>(g, b, Ay, r, sc, rs, tol, maxIT), topx::count_launch());
   TOPX_CUDA_OK(cudaGetLastError());
 }
 
-template <typename T>
-struct Vec2;
-template <>
-struct Vec2<double> {
-  using type = double2;
-};
-template <>
-struct Vec2<float> {
-  using type = float2;
-};
-
-// PGIVEN: p already holds the new direction (written by K*u), z is not read and p not written,
-// and the solution step y += lambda p is left to the next K*u (which reads this p as its p_in) or
-// to launch_pcg_flush after the last iteration: lambda goes to sc->lam and y is not touched here
-template <typename T, typename TY, bool PGIVEN>
-__global__ void k_pcg_update(Grid g, TY* __restrict__ y, const T* __restrict__ z, T* __restrict__ p,
-                             T* __restrict__ r, const T* __restrict__ q, PcgScalars* sc, RedScratch rs,
-                             const uint32_t* __restrict__ act) {
+__global__ void k_pcg_update(Grid g, double* __restrict__ r, const double* __restrict__ q, PcgScalars* sc,
+                             RedScratch rs, const uint32_t* __restrict__ act) {
   if (sc->done) return;
-  const bool first = sc->first;
-  const T beta = T(sc->beta);
   const double lam = sc->x1 / sc->pq;
-  const T lamT = T(lam);
-  const TY lamY = TY(lam);
   const int64_t S = g.stride;  // a multiple of 32, so node pairs are aligned
   const int64_t npair = (g.nnodes() + 1) / 2;
   double rr = 0.0;
-  using V2 = typename Vec2<T>::type;
-  using Y2 = typename Vec2<TY>::type;
   for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < npair; i += int64_t(gridDim.x) * blockDim.x) {
     if (!chunk_active(act, 2 * i)) continue;  // both nodes of the pair lie in one chunk
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
       const int64_t k = 2 * i + c * S;
-      V2 pv = *reinterpret_cast<const V2*>(p + k);
-      if (!PGIVEN) {
-        const V2 zv = *reinterpret_cast<const V2*>(z + k);
-        pv.x = first ? zv.x : zv.x + beta * pv.x;
-        pv.y = first ? zv.y : zv.y + beta * pv.y;
-        *reinterpret_cast<V2*>(p + k) = pv;
-      }
-      if (!PGIVEN) {
-        Y2 yv = *reinterpret_cast<const Y2*>(y + k);
-        yv.x = fma(lamY, TY(pv.x), yv.x);
-        yv.y = fma(lamY, TY(pv.y), yv.y);
-        *reinterpret_cast<Y2*>(y + k) = yv;
-      }
-      const V2 qv = *reinterpret_cast<const V2*>(q + k);
-      V2 rv = *reinterpret_cast<const V2*>(r + k);
-      rv.x = rv.x - lamT * qv.x;
-      rv.y = rv.y - lamT * qv.y;
-      *reinterpret_cast<V2*>(r + k) = rv;
-      rr += double(rv.x) * double(rv.x) + double(rv.y) * double(rv.y);
+      const double2 qv = *reinterpret_cast<const double2*>(q + k);
+      double2 rv = *reinterpret_cast<const double2*>(r + k);
+      rv.x = rv.x - lam * qv.x;
+      rv.y = rv.y - lam * qv.y;
+      *reinterpret_cast<double2*>(r + k) = rv;
+      rr += rv.x * rv.x + rv.y * rv.y;
     }
   }
   double v[1] = {rr}, tot[1];
-  if (reduce_publish<1>(v, rs, tot) && threadIdx.x == 0) {
-    sc->lam = lam;
-    sc->rr = tot[0];
-    sc->resnorm = sqrt(tot[0]) / sc->normB;
-    sc->its += 1;
-    sc->first = 0;
-    if (sc->resnorm < sc->tol)
-      sc->done = 1;
-    else if (sc->its >= sc->maxIT)
-      sc->done = 2;
-  }
+  if (reduce_publish<1>(v, rs, tot) && threadIdx.x == 0) pcg_stop_test(sc, lam, tot[0]);
+}
+void launch_pcg_update(cudaStream_t st, Grid g, double* r, const double* q, PcgScalars* sc, RedScratch rs,
+                       const uint32_t* act) {
+  (k_pcg_update<<<grid1d(g.nnodes(), 256), 256, 0, st>>>(g, r, q, sc, rs, act), topx::count_launch());
+  TOPX_CUDA_OK(cudaGetLastError());
 }
 
 // y += sc->lam * p over every node: the solution step of the last PCG iteration (PGIVEN updates
@@ -187,39 +287,76 @@ void launch_pcg_flush(cudaStream_t st, Grid g, double* y, const double* p, const
   TOPX_CUDA_OK(cudaGetLastError());
 }
 
-template <typename T, typename TY>
-void launch_pcg_update(cudaStream_t st, Grid g, TY* y, const T* z, T* p, T* r, const T* q, PcgScalars* sc,
-                       RedScratch rs, const uint32_t* act) {
-  if (z)
-    (k_pcg_update<T, TY, false><<<grid1d(g.nnodes(), 256), 256, 0, st>>>(g, y, z, p, r, q, sc, rs, act),
-     topx::count_launch());
-  else
-    (k_pcg_update<T, TY, true><<<grid1d(g.nnodes(), 256), 256, 0, st>>>(g, y, z, p, r, q, sc, rs, act),
-     topx::count_launch());
-  TOPX_CUDA_OK(cudaGetLastError());
-}
-
 // ---------------------------------------------------------------------------
 // Trilinear restriction R = P^T (Solving_RestrictResidual, TOP3D_XL.m:783-798)
-// as three separable passes (y, x, z).  Weights (S-|d|)/S are exact in binary,
+// as separable passes (y, x, z).  Weights (S-|d|)/S are exact in binary,
 // equal to the reference's multiGridOperatorRI entries.
 // ---------------------------------------------------------------------------
-template <typename TI, typename T, int S, int AXIS>
-__global__ void k_restrict_axis(const TI* __restrict__ in, int64_t istr, int iny, int inx, int inz,
+// x and z passes of the level-1 restriction in one launch: 32 neighbouring (y, x) nodes of a coarse plane per
+// block, a warp per z tap; the x sums meet in shared memory.  tmp (6 B per level-1 node) comes from L2.
+template <typename T>
+__global__ void __launch_bounds__(32 * (2 * KU_SPAN - 1)) k_restrict_xz(const double* __restrict__ tmp, int inx, int inz,
+                                                                       T* __restrict__ out, double* __restrict__ out64,
+                                                                       int64_t ostr, int ony, int onx, FastDiv dy,
+                                                                       const PcgScalars* sc) {
+  if (sc && sc->done) return;
+  constexpr int W = 2 * KU_SPAN - 1;
+  __shared__ double sx[W][3][32];
+  const int lane = threadIdx.x, dz = threadIdx.y, oz = blockIdx.y;
+  const uint32_t m = blockIdx.x * 32 + lane, N = uint32_t(ony) * onx;
+  const int64_t ts = int64_t(ony) * inx * inz;
+  const int iz = KU_SPAN * oz + dz - (KU_SPAN - 1);
+  double t[3] = {0.0, 0.0, 0.0};
+  if (m < N && iz >= 0 && iz < inz) {
+    const int ox = int(dy.div(m)), oy = int(m) - ox * ony;
+#pragma unroll
+    for (int dx = -(KU_SPAN - 1); dx <= KU_SPAN - 1; ++dx) {
+      const int ix = KU_SPAN * ox + dx;
+      if (ix < 0 || ix >= inx) continue;
+      const double w = double(KU_SPAN - (dx < 0 ? -dx : dx)) / KU_SPAN;
+      const int64_t k = oy + int64_t(ony) * (ix + int64_t(inx) * iz);
+#pragma unroll
+      for (int c = 0; c < 3; ++c) t[c] = fma(w, tmp[k + c * ts], t[c]);
+    }
+  }
+#pragma unroll
+  for (int c = 0; c < 3; ++c) sx[dz][c][lane] = t[c];
+  __syncthreads();
+  if (dz < 3 && m < N) {
+    double s = 0.0;
+#pragma unroll
+    for (int k = 0; k < W; ++k) {
+      const int d = k - (KU_SPAN - 1);
+      s = fma(double(KU_SPAN - (d < 0 ? -d : d)) / KU_SPAN, sx[k][dz][lane], s);
+    }
+    const int64_t n = m + int64_t(N) * oz + dz * ostr;
+    out[n] = T(s);
+    if (out64) out64[n] = s;
+  }
+}
+template <typename T>
+void launch_restrict_xz(cudaStream_t st, const double* tmp, Grid gf, T* out, double* out64, Grid gc,
+                        const PcgScalars* sc) {
+  const int cy = gc.nny(), cx = gc.nnx();
+  const dim3 nb(unsigned((cy * cx + 31) / 32), unsigned(gc.nnz()));
+  (k_restrict_xz<T><<<nb, dim3(32, 2 * KU_SPAN - 1), 0, st>>>(tmp, gf.nnx(), gf.nnz(), out, out64, gc.stride, cy, cx,
+                                                              FastDiv{uint32_t(cy)}, sc),
+   topx::count_launch());
+  TOPX_CUDA_OK(cudaGetLastError());
+}
+template void launch_restrict_xz<double>(cudaStream_t, const double*, Grid, double*, double*, Grid, const PcgScalars*);
+template void launch_restrict_xz<float>(cudaStream_t, const double*, Grid, float*, double*, Grid, const PcgScalars*);
+
+template <typename T, int S, int AXIS>
+__global__ void k_restrict_axis(const T* __restrict__ in, int64_t istr, int iny, int inx, int inz,
                                 T* __restrict__ out, int64_t ostr, int ony, int onx, int onz, FastDiv fdy,
-                                FastDiv fdx, const uint32_t* __restrict__ cols) {
+                                FastDiv fdx, const PcgScalars* sc) {
+  if (sc && sc->done) return;
   const uint32_t N = uint32_t(ony) * onx * onz;
   for (uint32_t n = blockIdx.x * blockDim.x + threadIdx.x; n < N; n += gridDim.x * blockDim.x) {
     const uint32_t q = fdy.div(n), oz = fdx.div(q);
     const int oy = int(n - q * uint32_t(ony)), ox = int(q - oz * uint32_t(onx));
     T acc[3] = {T(0), T(0), T(0)};
-    // y pass with a column mask: an input (x, z) column without a present node is zero, and so
-    // is the output (written without reading the column)
-    if (AXIS == 0 && cols && ((__ldg(cols + (q >> 5)) >> (q & 31)) & 1u) == 0u) {
-#pragma unroll
-      for (int c = 0; c < 3; ++c) out[n + c * ostr] = T(0);
-      continue;
-    }
 #pragma unroll
     for (int d = -(S - 1); d <= S - 1; ++d) {
       int iy = oy, ix = ox, iz = int(oz);
@@ -246,25 +383,17 @@ __global__ void k_restrict_axis(const TI* __restrict__ in, int64_t istr, int iny
   }
 }
 
-// The restriction in one pass, for small grids (launch-latency bound): L threads per coarse node,
-// one per (x, z) column of its (2S-1)^3 fine taps.  Thread (dx, dz) forms the column's y sum as the
-// first axis pass does (a column without a present node is zero, unread), thread dz of the node
-// the x sum of its columns as the second pass does, and thread 0 the z sum as the third; each sum
-// keeps the pass's element type and tap order, so the result equals the three passes bit for bit.
-template <int S>
-struct RestrictCoop {
-  static constexpr int W = 2 * S - 1;           // taps per axis
-  static constexpr int L = S == 4 ? 64 : 16;    // threads per coarse node (>= W * W)
-  static constexpr int NODES = 256 / L;         // coarse nodes per block
-};
-template <int S, typename TI, typename T>
-__global__ void __launch_bounds__(256) k_restrict_coop(const TI* __restrict__ in, int64_t istr, int iny, int inx,
+// The restriction between coarse levels in one launch, for grids where launches count: 16 threads per coarse node, one
+// per (x, z) column of its 27 fine taps.  Thread (dx, dz) forms the column's y sum as the first axis
+// pass does, thread dz of the node the x sum of its columns as the second pass does, and thread 0
+// the z sum as the third; each sum keeps the pass's element type and tap order, so the result
+// equals the three passes bit for bit.
+template <typename T>
+__global__ void __launch_bounds__(256) k_restrict_coop(const T* __restrict__ in, int64_t istr, int iny, int inx,
                                                       int inz, T* __restrict__ out, int64_t ostr, int ony, int onx,
-                                                      int onz, FastDiv fdy, FastDiv fdx,
-                                                      const uint32_t* __restrict__ cols) {
-  using RC = RestrictCoop<S>;
-  constexpr int W = RC::W, L = RC::L, NODES = RC::NODES;
-  static_assert(W * W <= L, "a thread per tap column");
+                                                      int onz, FastDiv fdy, FastDiv fdx, const PcgScalars* sc) {
+  if (sc && sc->done) return;
+  constexpr int W = 3, L = 16, NODES = 256 / L;
   __shared__ T sy[NODES][W * W][3];  // y sums of the node's (dx, dz) columns
   __shared__ T sx[NODES][W][3];      // x sums per dz
   const int sub = threadIdx.x / L, lane = threadIdx.x % L;
@@ -275,20 +404,17 @@ __global__ void __launch_bounds__(256) k_restrict_coop(const TI* __restrict__ in
     const uint32_t q = valid ? fdy.div(n) : 0u, oz = valid ? fdx.div(q) : 0u;
     const int oy = int(n - q * uint32_t(ony)), ox = int(q - oz * uint32_t(onx));
     if (valid && lane < W * W) {
-      const int ix = S * ox + lane % W - (S - 1), iz = S * int(oz) + lane / W - (S - 1);
+      const int ix = 2 * ox + lane % W - 1, iz = 2 * int(oz) + lane / W - 1;
       T t[3] = {T(0), T(0), T(0)};
       if (ix >= 0 && ix < inx && iz >= 0 && iz < inz) {
-        const uint32_t col = uint32_t(ix) + uint32_t(inx) * uint32_t(iz);
-        if (!cols || ((__ldg(cols + (col >> 5)) >> (col & 31)) & 1u) != 0u) {
 #pragma unroll
-          for (int dy = -(S - 1); dy <= S - 1; ++dy) {
-            const int iy = S * oy + dy;
-            if (iy < 0 || iy >= iny) continue;
-            const T w = T(S - (dy < 0 ? -dy : dy)) / T(S);
-            const int64_t k = iy + int64_t(iny) * (ix + int64_t(inx) * iz);
+        for (int dy = -1; dy <= 1; ++dy) {
+          const int iy = 2 * oy + dy;
+          if (iy < 0 || iy >= iny) continue;
+          const T w = T(2 - (dy < 0 ? -dy : dy)) / T(2);
+          const int64_t k = iy + int64_t(iny) * (ix + int64_t(inx) * iz);
 #pragma unroll
-            for (int c = 0; c < 3; ++c) t[c] = fma(w, T(in[k + c * istr]), t[c]);
-          }
+          for (int c = 0; c < 3; ++c) t[c] = fma(w, in[k + c * istr], t[c]);
         }
       }
 #pragma unroll
@@ -298,12 +424,12 @@ __global__ void __launch_bounds__(256) k_restrict_coop(const TI* __restrict__ in
     if (valid && lane < W) {
       T t[3] = {T(0), T(0), T(0)};
 #pragma unroll
-      for (int dx = -(S - 1); dx <= S - 1; ++dx) {
-        const int ix = S * ox + dx;
+      for (int dx = -1; dx <= 1; ++dx) {
+        const int ix = 2 * ox + dx;
         if (ix < 0 || ix >= inx) continue;
-        const T w = T(S - (dx < 0 ? -dx : dx)) / T(S);
+        const T w = T(2 - (dx < 0 ? -dx : dx)) / T(2);
 #pragma unroll
-        for (int c = 0; c < 3; ++c) t[c] = fma(w, sy[sub][lane * W + dx + (S - 1)][c], t[c]);
+        for (int c = 0; c < 3; ++c) t[c] = fma(w, sy[sub][lane * W + dx + 1][c], t[c]);
       }
 #pragma unroll
       for (int c = 0; c < 3; ++c) sx[sub][lane][c] = t[c];
@@ -312,12 +438,12 @@ __global__ void __launch_bounds__(256) k_restrict_coop(const TI* __restrict__ in
     if (valid && lane == 0) {
       T acc[3] = {T(0), T(0), T(0)};
 #pragma unroll
-      for (int dz = -(S - 1); dz <= S - 1; ++dz) {
-        const int iz = S * int(oz) + dz;
+      for (int dz = -1; dz <= 1; ++dz) {
+        const int iz = 2 * int(oz) + dz;
         if (iz < 0 || iz >= inz) continue;
-        const T w = T(S - (dz < 0 ? -dz : dz)) / T(S);
+        const T w = T(2 - (dz < 0 ? -dz : dz)) / T(2);
 #pragma unroll
-        for (int c = 0; c < 3; ++c) acc[c] = fma(w, sx[sub][dz + (S - 1)][c], acc[c]);
+        for (int c = 0; c < 3; ++c) acc[c] = fma(w, sx[sub][dz + 1][c], acc[c]);
       }
 #pragma unroll
       for (int c = 0; c < 3; ++c) out[n + c * ostr] = acc[c];
@@ -326,34 +452,25 @@ __global__ void __launch_bounds__(256) k_restrict_coop(const TI* __restrict__ in
   }
 }
 
-template <typename TI, typename T>
-void launch_restrict(cudaStream_t st, int span, const TI* in, Grid gf, T* tmp1, T* tmp2, T* out, Grid gc,
-                     const uint32_t* cols) {
+template <typename T>
+void launch_restrict(cudaStream_t st, const T* in, Grid gf, T* tmp1, T* tmp2, T* out, Grid gc, const PcgScalars* sc) {
   const int fy = gf.nny(), fx = gf.nnx(), fz = gf.nnz();
   const int cy = gc.nny(), cx = gc.nnx(), cz = gc.nnz();
   const int64_t s1 = int64_t(cy) * fx * fz, s2 = int64_t(cy) * cx * fz;
   if (gf.nnodes() >= (int64_t(1) << 32)) throw std::runtime_error("grid too large for 32-bit node indices");
   const FastDiv dcy{uint32_t(cy)}, dfx{uint32_t(fx)}, dcx{uint32_t(cx)};
-  if (gf.nnodes() <= (int64_t(1) << 21) && (span == 2 || span == 4)) {
-    // small grids are launch-latency bound: one launch, a thread per tap column of a coarse node
-    if (span == 4)
-      (k_restrict_coop<4, TI, T><<<grid1d(gc.nnodes() * RestrictCoop<4>::L, 256), 256, 0, st>>>(
-           in, gf.stride, fy, fx, fz, out, gc.stride, cy, cx, cz, dcy, dcx, cols),
-       topx::count_launch());
-    else
-      (k_restrict_coop<2, TI, T><<<grid1d(gc.nnodes() * RestrictCoop<2>::L, 256), 256, 0, st>>>(
-           in, gf.stride, fy, fx, fz, out, gc.stride, cy, cx, cz, dcy, dcx, cols),
-       topx::count_launch());
-  } else if (span == 4) {
-    (k_restrict_axis<TI, T, 4, 0><<<grid1d(s1, 256), 256, 0, st>>>(in, gf.stride, fy, fx, fz, tmp1, s1, cy, fx, fz, dcy, dfx, cols), topx::count_launch());
-    (k_restrict_axis<T, T, 4, 1><<<grid1d(s2, 256), 256, 0, st>>>(tmp1, s1, cy, fx, fz, tmp2, s2, cy, cx, fz, dcy, dcx, nullptr), topx::count_launch());
-    (k_restrict_axis<T, T, 4, 2><<<grid1d(gc.nnodes(), 256), 256, 0, st>>>(tmp2, s2, cy, cx, fz, out, gc.stride, cy,
-                                                                             cx, cz, dcy, dcx, nullptr), topx::count_launch());
+  if (gf.nnodes() <= kRestrictOneLaunch) {
+    (k_restrict_coop<T><<<grid1d(gc.nnodes() * 16, 256), 256, 0, st>>>(in, gf.stride, fy, fx, fz, out, gc.stride, cy, cx,
+                                                                       cz, dcy, dcx, sc),
+     topx::count_launch());
   } else {
-    (k_restrict_axis<TI, T, 2, 0><<<grid1d(s1, 256), 256, 0, st>>>(in, gf.stride, fy, fx, fz, tmp1, s1, cy, fx, fz, dcy, dfx, cols), topx::count_launch());
-    (k_restrict_axis<T, T, 2, 1><<<grid1d(s2, 256), 256, 0, st>>>(tmp1, s1, cy, fx, fz, tmp2, s2, cy, cx, fz, dcy, dcx, nullptr), topx::count_launch());
-    (k_restrict_axis<T, T, 2, 2><<<grid1d(gc.nnodes(), 256), 256, 0, st>>>(tmp2, s2, cy, cx, fz, out, gc.stride, cy,
-                                                                             cx, cz, dcy, dcx, nullptr), topx::count_launch());
+    (k_restrict_axis<T, 2, 0><<<grid1d(s1, 256), 256, 0, st>>>(in, gf.stride, fy, fx, fz, tmp1, s1, cy, fx, fz, dcy, dfx, sc),
+     topx::count_launch());
+    (k_restrict_axis<T, 2, 1><<<grid1d(s2, 256), 256, 0, st>>>(tmp1, s1, cy, fx, fz, tmp2, s2, cy, cx, fz, dcy, dcx, sc),
+     topx::count_launch());
+    (k_restrict_axis<T, 2, 2><<<grid1d(gc.nnodes(), 256), 256, 0, st>>>(tmp2, s2, cy, cx, fz, out, gc.stride, cy, cx, cz,
+                                                                         dcy, dcx, sc),
+     topx::count_launch());
   }
   TOPX_CUDA_OK(cudaGetLastError());
 }
@@ -362,7 +479,8 @@ void launch_restrict(cudaStream_t st, int span, const TI* in, Grid gf, T* tmp1, 
 // Prolongation + Jacobi up-smoothing of the 'Adapted' V-cycle
 // (TOP3D_XL.m:757-778, Solving_InterpolationDeviation 800-814):
 //   x = omega*(r./d) + P*xc + (omega*r)./d   on present fine nodes.
-// The level-1 instance also reduces z'r and updates beta/x1 (TOP3D_XL.m:626-630).
+// Inside the PCG the level-2 instance completes z'r (see k_residual) and updates beta/x1
+// (TOP3D_XL.m:626-630); the level-1 prolongation itself is formed by the next K*u.
 // ---------------------------------------------------------------------------
 // SMOOTH = false (the 'Standard' V-cycle) stops after omega*(r/d) + P(xc); the Jacobi
 // correction against K x follows in k_jacobi_correct.
@@ -370,9 +488,10 @@ template <typename TX, typename T, typename TD, int S, bool DOT, bool SMOOTH = t
 __global__ void __launch_bounds__(256) k_prolong_smooth(const TX* __restrict__ xc, Grid gc, const T* __restrict__ r,
                                                         const TD* __restrict__ dinv,
                                                         const uint8_t* __restrict__ present, T* __restrict__ x,
-                                                        Grid gf, FastDiv dny, FastDiv dnx, T omega, PcgScalars* sc,
-                                                        RedScratch rs, int init, const uint32_t* __restrict__ act) {
-  if ((DOT || !SMOOTH) && sc->done) return;
+                                                        Grid gf, FastDiv dny, FastDiv dnx, T omega,
+                                                        const double* __restrict__ rc, PcgScalars* sc, RedScratch rs,
+                                                        int init, double omega2, const uint32_t* __restrict__ act) {
+  if (sc && sc->done) return;
   const uint32_t fny = uint32_t(gf.nny()), fnx = uint32_t(gf.nnx());
   const uint32_t nn = uint32_t(gf.nnodes());  // < 2^32 (checked at launch)
   const int cny = gc.nny(), cnx = gc.nnx();
@@ -416,7 +535,7 @@ __global__ void __launch_bounds__(256) k_prolong_smooth(const TX* __restrict__ x
         t = t + pc[c];
         if (SMOOTH) t = t + (omega * rv[c]) * di[c];
         v[c] = t;
-        if (DOT) zr += double(t) * double(rv[c]);
+        if (DOT) zr = fma(double(t), rc[n + c * gf.stride], zr);
       }
     }
 #pragma unroll
@@ -425,39 +544,30 @@ __global__ void __launch_bounds__(256) k_prolong_smooth(const TX* __restrict__ x
   if (DOT) {
     double vv[1] = {zr}, tot[1];
     if (reduce_publish<1>(vv, rs, tot) && threadIdx.x == 0) {
-      if (init) {
-        sc->x1 = tot[0];
-      } else {
-        sc->beta = tot[0] / sc->x1;
-        sc->x1 = tot[0];
-      }
+      const double x2 = fma(omega2, sc->rdr, tot[0]);
+      if (!init) sc->beta = x2 / sc->x1;
+      sc->x1 = x2;
     }
   }
 }
 
 template <typename TX, typename T, typename TD>
 void launch_prolong_smooth(cudaStream_t st, int span, const TX* xc, Grid gc, const T* r, const TD* d,
-                           const uint8_t* present, T* x, Grid gf, double omega, bool dot, bool init,
+                           const uint8_t* present, T* x, Grid gf, double omega, const double* rc, bool init,
                            PcgScalars* sc, RedScratch rs, const uint32_t* act) {
   if (gf.nnodes() >= (int64_t(1) << 32)) throw std::runtime_error("grid too large for 32-bit node indices");
   const unsigned nb = grid1d(gf.nnodes(), 256, 148 * 8);
-  const T w = T(omega);
   const FastDiv dny{uint32_t(gf.nny())}, dnx{uint32_t(gf.nnx())};
-  if (span == 4) {
-    if (dot)
-      (k_prolong_smooth<TX, T, TD, 4, true><<<nb, 256, 0, st>>>(xc, gc, r, d, present, x, gf, dny, dnx, w, sc, rs, init, act),
-       topx::count_launch());
-    else
-      (k_prolong_smooth<TX, T, TD, 4, false><<<nb, 256, 0, st>>>(xc, gc, r, d, present, x, gf, dny, dnx, w, sc, rs, init, act),
-       topx::count_launch());
-  } else {
-    if (dot)
-      (k_prolong_smooth<TX, T, TD, 2, true><<<nb, 256, 0, st>>>(xc, gc, r, d, present, x, gf, dny, dnx, w, sc, rs, init, act),
-       topx::count_launch());
-    else
-      (k_prolong_smooth<TX, T, TD, 2, false><<<nb, 256, 0, st>>>(xc, gc, r, d, present, x, gf, dny, dnx, w, sc, rs, init, act),
-       topx::count_launch());
-  }
+  auto go = [&](auto kernel) {
+    (kernel<<<nb, 256, 0, st>>>(xc, gc, r, d, present, x, gf, dny, dnx, T(omega), rc, sc, rs, init ? 1 : 0, 2.0 * omega, act),
+     topx::count_launch());
+  };
+  if (span == 4)
+    go(k_prolong_smooth<TX, T, TD, 4, false>);
+  else if (rc)
+    go(k_prolong_smooth<TX, T, TD, 2, true>);
+  else
+    go(k_prolong_smooth<TX, T, TD, 2, false>);
   TOPX_CUDA_OK(cudaGetLastError());
 }
 
@@ -465,18 +575,17 @@ template <typename TX, typename T, typename TD>
 void launch_prolong_add(cudaStream_t st, int span, const TX* xc, Grid gc, const T* r, const TD* d,
                         const uint8_t* present, T* x, Grid gf, double omega, PcgScalars* sc) {
   const unsigned nb = grid1d(gf.nnodes(), 256, 148 * 8);
-  const T w = T(omega);
   RedScratch none{nullptr, nullptr};
   if (gf.nnodes() >= (int64_t(1) << 32)) throw std::runtime_error("grid too large for 32-bit node indices");
   const FastDiv dny{uint32_t(gf.nny())}, dnx{uint32_t(gf.nnx())};
+  auto go = [&](auto kernel) {
+    (kernel<<<nb, 256, 0, st>>>(xc, gc, r, d, present, x, gf, dny, dnx, T(omega), nullptr, sc, none, 0, 0.0, nullptr),
+     topx::count_launch());
+  };
   if (span == 4)
-    (k_prolong_smooth<TX, T, TD, 4, false, false><<<nb, 256, 0, st>>>(xc, gc, r, d, present, x, gf, dny, dnx, w, sc,
-                                                                      none, 0, nullptr),
-     topx::count_launch());
+    go(k_prolong_smooth<TX, T, TD, 4, false, false>);
   else
-    (k_prolong_smooth<TX, T, TD, 2, false, false><<<nb, 256, 0, st>>>(xc, gc, r, d, present, x, gf, dny, dnx, w, sc,
-                                                                      none, 0, nullptr),
-     topx::count_launch());
+    go(k_prolong_smooth<TX, T, TD, 2, false, false>);
   TOPX_CUDA_OK(cudaGetLastError());
 }
 
@@ -682,16 +791,14 @@ void launch_simp_scatter(cudaStream_t st, const double* xPhys, const int32_t* el
 // TopOpti_ComputeUnitCompliance (TOP3D_XL.m:579-598): ce_e = u_e^T Ke u_e with the
 // unmodified Ke, one thread per element (compact order), FP64.
 __global__ void k_unit_compliance(Grid g, const double* __restrict__ U, const int32_t* __restrict__ emb0,
-                                  int64_t Ne, FastDiv dy, FastDiv dx, double w, int acc, double* __restrict__ ce) {
+                                  int64_t Ne, double w, int acc, double* __restrict__ ce) {
   const int nny = g.ny + 1, nnx = g.nx + 1;
   for (int64_t e = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; e < Ne; e += int64_t(gridDim.x) * blockDim.x) {
-    const uint32_t id = uint32_t(emb0[e]);  // element id on the full box, < 2^31
-    const uint32_t q = dy.div(id), ez = dx.div(q);
-    const int ey = int(id - q * uint32_t(g.ny)), ex = int(q - ez * uint32_t(g.nx));
+    const int64_t id = emb0[e];  // the index of its lowest node
     double u[24];
 #pragma unroll
     for (int a = 0; a < 8; ++a) {
-      const int64_t n = (ey + hex_ly(a)) + int64_t(nny) * ((ex + hex_lx(a)) + int64_t(nnx) * (ez + hex_lz(a)));
+      const int64_t n = id + hex_ly(a) + int64_t(nny) * (hex_lx(a) + int64_t(nnx) * hex_lz(a));
 #pragma unroll
       for (int c = 0; c < 3; ++c) u[3 * a + c] = U[n + c * g.stride];
     }
@@ -709,36 +816,26 @@ __global__ void k_unit_compliance(Grid g, const double* __restrict__ U, const in
 }
 void launch_unit_compliance(cudaStream_t st, Grid g, const double* U, const int32_t* eleMapBack0, int64_t Ne,
                             double weight, bool accumulate, double* ce) {
-  const FastDiv dy{uint32_t(g.ny)}, dx{uint32_t(g.nx)};
-  (k_unit_compliance<<<grid1d(Ne, 128), 128, 0, st>>>(g, U, eleMapBack0, Ne, dy, dx, weight, accumulate ? 1 : 0, ce),
+  (k_unit_compliance<<<grid1d(Ne, 128), 128, 0, st>>>(g, U, eleMapBack0, Ne, weight, accumulate ? 1 : 0, ce),
    topx::count_launch());
   TOPX_CUDA_OK(cudaGetLastError());
 }
 
 // explicit instantiations
 #define TOPX_INST(T)                                                                                             \
-  template void launch_diag_l1<T, T>(cudaStream_t, Grid, const T*, const uint8_t*, const T*, const uint8_t*, T*); \
-  template void launch_residual_init<T>(cudaStream_t, Grid, const T*, const T*, T*, PcgScalars*, RedScratch,     \
-                                        double, int);                                                            \
-  template void launch_restrict<T, T>(cudaStream_t, int, const T*, Grid, T*, T*, T*, Grid, const uint32_t*);     \
+  template void launch_diag_l1<T>(cudaStream_t, Grid, const double*, const uint8_t*, const double*,              \
+                                  const uint8_t*, T*, double*);                                                    \
+  template void launch_restrict<T>(cudaStream_t, const T*, Grid, T*, T*, T*, Grid, const PcgScalars*);           \
   template void launch_prolong_smooth<T, T, T>(cudaStream_t, int, const T*, Grid, const T*, const T*,            \
-                                               const uint8_t*, T*, Grid, double, bool, bool, PcgScalars*,        \
-                                               RedScratch, const uint32_t*);                                     \
-  template void launch_compact_to_grid_nodes<T>(cudaStream_t, const double*, T*, Grid, const int32_t*, int64_t); \
-  template void launch_grid_to_compact_nodes<T>(cudaStream_t, const T*, double*, Grid, const int32_t*, int64_t);
+                                               const uint8_t*, T*, Grid, double, const double*, bool,            \
+                                               PcgScalars*, RedScratch, const uint32_t*);
 TOPX_INST(double)
 TOPX_INST(float)
-template void launch_pcg_update<double, double>(cudaStream_t, Grid, double*, const double*, double*, double*,
-                                                const double*, PcgScalars*, RedScratch, const uint32_t*);
-template void launch_pcg_update<float, float>(cudaStream_t, Grid, float*, const float*, float*, float*, const float*,
-                                              PcgScalars*, RedScratch, const uint32_t*);
-template void launch_diag_l1<double, float>(cudaStream_t, Grid, const double*, const uint8_t*, const double*,
-                                           const uint8_t*, float*);
-template void launch_restrict<double, float>(cudaStream_t, int, const double*, Grid, float*, float*, float*, Grid,
-                                             const uint32_t*);
+template void launch_compact_to_grid_nodes<double>(cudaStream_t, const double*, double*, Grid, const int32_t*, int64_t);
+template void launch_grid_to_compact_nodes<double>(cudaStream_t, const double*, double*, Grid, const int32_t*, int64_t);
 template void launch_prolong_smooth<float, double, float>(cudaStream_t, int, const float*, Grid, const double*,
-                                                          const float*, const uint8_t*, double*, Grid, double, bool,
-                                                          bool, PcgScalars*, RedScratch, const uint32_t*);
+                                                          const float*, const uint8_t*, double*, Grid, double,
+                                                          const double*, bool, PcgScalars*, RedScratch, const uint32_t*);
 template void launch_prolong_add<double, double, double>(cudaStream_t, int, const double*, Grid, const double*,
                                                         const double*, const uint8_t*, double*, Grid, double,
                                                         PcgScalars*);

@@ -14,25 +14,28 @@
 // come first, so a smooth field cancels exactly at the start instead of at the end of long sums.
 //
 // Tiles.  A CTA of 256 threads marches a z-chunk of a PY x PX tile of node columns (y fastest), one
-// thread per column; the outer ring is halo.  A thread copies the values of its own node two
-// planes ahead, asynchronously, into slots that only it reads, forms the operator's input
+// thread per column; the outer ring is halo.  One thread copies the boxes of a plane's fields two planes ahead by
+// TMA (out-of-grid entries arrive as zeros); every thread forms the operator's input at its own node
 // there (masked u, or the PCG direction), and exchanges through shared memory twice per plane: its
 // value with the other corners of its face, and its face's forces with the nodes at those corners.  The
-// transformed face of the plane below and the forces from the layer below stay in registers.  A
-// node takes no separate launch for the last row of a grid.  No atomics: the result is deterministic.
+// transformed face of the plane below and the forces from the layer below stay in registers.  No
+// atomics: the result is deterministic.
 //
-// Measured on a B200, one PCG-mode launch (128x256x128, 64x128x64 and 50x100x50 elements): 185, 36
-// and 27 us, with Ke's 576 entries in a 32 x 8 tile and a launch for the last row 280, 54 and 32 us.
-// Bound by the shared-memory and load/store pipe (71 % of its wavefronts; the FP64 pipe 31 %,
-// DRAM 37 %): 8-byte accesses, since rows of an odd number of nodes start at odd addresses.  What was
-// slower there: three planes in flight (257 us: the slots take the L1 cache that serves the halo),
-// two planes per barrier (275), loads into registers one plane ahead (386), CTAs of 128 threads (203)
-// or 512 (190), three CTAs per SM with spills (319).
+// Measured on a B200, one PCG-mode launch (128x256x128, 64x128x64 and 50x100x50 elements), the direction formed
+// from the residual and the level-2 correction included: 188, 40 and 29 us.  With z read from memory 185, 36 and
+// 27 us, to which the prolongation that wrote z added 80, 25 and 21 us.  With Ke's 576 entries in a 32 x 8 tile and
+// a launch for the last row, z read: 280, 54 and 32 us.  What bounds it is the number of instructions an SM issues
+// (0.5 per cycle and scheduler with its 16 warps, a third of them FP64; DRAM 35 %), then the two barriers of a plane.  What was slower:
+// 8-byte asynchronous copies by every thread instead of TMA (300 us: they need L1 lines, of which little is left
+// beside the shared memory), a spilled register (local memory goes to L2 for the same reason: 240 to 320), two
+// planes per barrier, loads into registers one plane ahead, CTAs of 128 or 512 threads, three CTAs per SM.
 #include <algorithm>
 #include <cmath>
 #include <stdexcept>
 #include <type_traits>
 #include <vector>
+
+#include <cuda.h>
 
 #include "topx_ke_classes.h"
 #include "topx_kernels.cuh"
@@ -45,6 +48,7 @@ constexpr int KU_NT = 256;  // threads of a CTA
 constexpr int KU_CTAS = 2;  // CTAs of an SM
 constexpr int KU_PAD = 64;  // reach of a neighbour index (PY + 1)
 constexpr int KU_ROW = KU_NT + KU_PAD;
+constexpr int KU_COARSE = 64;  // coarse nodes of a tile per plane
 
 template <int BYTES>
 __device__ __forceinline__ void cp_async_el(void* smem, const void* gmem, bool pred) {
@@ -53,9 +57,38 @@ __device__ __forceinline__ void cp_async_el(void* smem, const void* gmem, bool p
   const int n = pred ? BYTES : 0;  // 0: fill with zeros, read nothing
   asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"(s), "l"(gmem), "n"(BYTES), "r"(n) : "memory");
 }
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait_all_but_one() { asm volatile("cp.async.wait_group 1;" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// One barrier per stage counts the bytes of its TMA copies.
+__device__ __forceinline__ unsigned smem_addr(const void* p) { return static_cast<unsigned>(__cvta_generic_to_shared(p)); }
+__device__ __forceinline__ void mbar_init(uint64_t* b) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(b)) : "memory");
+}
+__device__ __forceinline__ void mbar_expect(uint64_t* b, unsigned bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(b)), "r"(bytes) : "memory");
+}
+// waits for the phase of the given parity; bounded (about a second in all), false when it gave up
+__device__ __forceinline__ bool mbar_wait(uint64_t* b, unsigned parity) {
+  for (unsigned it = 0; it < (1u << 20); ++it) {
+    unsigned ok;
+    asm volatile(
+        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
+        : "=r"(ok)
+        : "r"(smem_addr(b)), "r"(parity)
+        : "memory");
+    if (ok) return true;
+  }
+  return false;
+}
+// box of a 4-dimensional map (y, x, z, component) at (y, x, z, 0): entries outside the array read as zero.  y is
+// even: a copy starts on a 16-byte boundary.
+__device__ __forceinline__ void tma_load(void* dst, const CUtensorMap* map, int y, int x, int z, uint64_t* bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.shared::cta.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];" ::"r"(
+          smem_addr(dst)),
+      "l"(map), "r"(y), "r"(x), "r"(z), "r"(0), "r"(smem_addr(bar))
+      : "memory");
+}
 
 // an array element at a 32-bit byte offset from a uniform base
 template <typename T>
@@ -64,12 +97,24 @@ __device__ __forceinline__ T* at(T* base, uint32_t bytes) {
   return reinterpret_cast<T*>(reinterpret_cast<C*>(base) + bytes);
 }
 
+// Maps of the arrays that a launch reads through TMA, and the places of their boxes in a stage
+struct KuMaps {
+  CUtensorMap a, E, p, y, D;  // u, z or r; (PCG) p_in, y; (fused) the Jacobi diagonal
+};
+// Offsets in doubles of a stage's boxes, and its length; boxes start on 128-byte boundaries
+struct KuStage {
+  int E, p, y, D, len;
+};
+
 template <int MODE>
 struct KuSmem {
-  static constexpr int NF = MODE == KU_PLAIN ? 4 : 10;
-  double stage[2][NF][KU_NT];  // of two planes: a[3], E, then (PCG) p_in[3], y[3]
-  double su[2][3][KU_ROW];     // a plane's masked values, and those of the plane below, read by their own threads
-  double cor[3][3][KU_ROW];    // face forces for the corners (y+1, x), (y, x+1), (y+1, x+1)
+  static constexpr bool FUSED = MODE == KU_FUSED;
+  double su[2][3][KU_ROW];   // a plane's masked values, and those of the plane below, read by their own threads
+  double cor[3][3][KU_ROW];  // face forces for the corners (y+1, x), (y, x+1), (y+1, x+1)
+  double xc[FUSED ? 3 : 1][FUSED ? 3 : 1][FUSED ? KU_COARSE : 1];  // ring of level-2 planes under the tile
+  int at[FUSED ? 3 : 1][FUSED ? KU_NT : 1];  // the thread's level-2 copy (element, slot) and its node's place in a cell
+  double zc[FUSED ? 2 : 1][FUSED ? 3 : 1][FUSED ? KU_NT : 1];  // xc at the node's (y, x) on the planes that end its cell
+  uint64_t bar[2];
 };
 
 // One element layer between two transformed faces: W0 (below) and W1 (above), faces [component x, y, z]
@@ -140,12 +185,16 @@ __device__ __forceinline__ void ku_layer(const KuModes& K, double E, double (&W0
 }
 
 // MODE KU_PLAIN: out = K in.  KU_P_UPDATE: p = z + beta p_in (p = z on the first step) for a given z.
-// It stores p, reduces p'q into sc->pq and applies the previous iteration's solution step y += lam p_in.
-template <int MODE>
-__global__ void __launch_bounds__(KU_NT, KU_CTAS) k_ku(const __grid_constant__ KuArgs a) {
+// KU_FUSED: z = omega2 (r D) + P xc is formed here from the residual r, the inverse diagonal D (one
+// value per node: the diagonal entries of its free DOFs are equal) and the level-2 correction xc, so no
+// pass over the level-1 grid writes or reads z.  TC: the preconditioner's type.
+// Both store p, reduce p'q into sc->pq and apply the previous iteration's solution step y += lam p_in.
+template <int MODE, typename TC>
+__global__ void __launch_bounds__(KU_NT, KU_CTAS)
+    k_ku(const __grid_constant__ KuArgs a, const __grid_constant__ KuMaps maps, const KuStage sg, const unsigned bytes) {
   constexpr bool PCG = MODE != KU_PLAIN;
-  extern __shared__ __align__(16) unsigned char ku_dyn_smem[];
-  KuSmem<MODE>& sm = *reinterpret_cast<KuSmem<MODE>*>(ku_dyn_smem);
+  extern __shared__ __align__(128) double ku_stages[];  // two planes' boxes, then the rest
+  KuSmem<MODE>& sm = *reinterpret_cast<KuSmem<MODE>*>(ku_stages + 2 * sg.len);
   const int t = threadIdx.x, PY = a.sh.PY;
   const int nny = a.g.ny + 1, nnx = a.g.nx + 1, nnz = a.g.nz + 1;
   const int64_t S = a.g.stride;
@@ -167,69 +216,150 @@ __global__ void __launch_bounds__(KU_NT, KU_CTAS) k_ku(const __grid_constant__ K
   const int gy = y0 - 1 + ly, gx = x0 - 1 + lx;      // this thread's node, and the lower corner of its face
   const bool in_tile = lx < a.sh.PX;
   const bool inb = in_tile && gy >= 0 && gy < nny && gx >= 0 && gx < nnx;
-  const bool einb = in_tile && gy >= 0 && gy < a.g.ny && gx >= 0 && gx < a.g.nx;
   const bool own = inb && ly >= 1 && ly <= a.sh.TY && lx >= 1 && lx <= a.sh.TX;
   // byte offsets of the node on plane 0 and of a plane (an array has less than 4 GB: checked at launch)
   const uint32_t n0 = inb ? 8u * uint32_t(gy + nny * gx) : 0u, np = 8u * uint32_t(nny) * uint32_t(nnx);
-  const uint32_t e0 = einb ? 8u * uint32_t(gy + a.g.ny * gx) : 0u, ep = 8u * uint32_t(a.g.ny) * uint32_t(a.g.nx);
-  const double* const araw = MODE == KU_P_UPDATE ? a.z : a.in;
+  // the node's place in a box of TY + 4 rows from y0 - 2, and (own nodes) in y's box of the tile itself
+  const int PB = a.sh.TY + 4, bx = PB * a.sh.PX, o = in_tile ? lx * PB + ly + 1 : 0;
+  const int oy = own ? (lx - 1) * a.sh.TY + ly - 1 : 0, by = a.sh.TY * a.sh.TX;
+  const TC* const xc = static_cast<const TC*>(a.xc);
 
-  auto issue = [&](int zp, int s) {
-    const bool ok = inb && zp >= 0 && zp < nnz && zp <= zend;
-    const uint32_t n = ok ? n0 + np * uint32_t(zp) : 0u;
-    const bool yok = PCG && own && zp >= zc0 && zp < zend;
+  // level-2 nodes under the tile (fused), copied by the threads t < 3 cn; kept in shared memory, since the loop
+  // needs every register
+  const int Zfirst = max(zc0 - 1, 0) / KU_SPAN;
+  if (MODE == KU_FUSED) {
+    const int Yc0 = max(y0 - 1, 0) / KU_SPAN, Xc0 = max(x0 - 1, 0) / KU_SPAN;
+    const int cny = min((y0 + a.sh.TY) / KU_SPAN + 1, a.gc.ny) - Yc0 + 1;
+    const int cn = cny * (min((x0 + a.sh.TX) / KU_SPAN + 1, a.gc.nx) - Xc0 + 1);
+    const int c = t / cn, r = t - c * cn, xx = r / cny, yy = r - xx * cny;
+    sm.at[0][t] = c < 3 ? int((Yc0 + yy) + (a.gc.ny + 1) * (Xc0 + xx) + c * a.gc.stride) : -1;
+    sm.at[1][t] = c * KU_COARSE + r;
+    const int Y = gy / KU_SPAN, X = gx / KU_SPAN;
 #pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      cp_async_el<8>(&sm.stage[s][c][t], at(araw + c * S, n), ok);
-      if (PCG) {
-        cp_async_el<8>(&sm.stage[s][4 + c][t], at(a.pin + c * S, n), ok);
-        cp_async_el<8>(&sm.stage[s][7 + c][t], at(a.yacc + c * S, yok ? n : 0u), yok);
-      }
+    for (int i = 0; i < 3; ++i) sm.zc[0][i][t] = sm.zc[1][i][t] = 0.0;  // stays so off the level-2 grid (weight 0)
+    sm.at[2][t] = inb && gy <= KU_SPAN * a.gc.ny ? (Y - Yc0) + cny * (X - Xc0) + (gy % KU_SPAN << 8) + (gx % KU_SPAN << 10) + (cny << 12) : -1;
+  }
+  auto issue_coarse = [&](int Z) {
+    const int e = sm.at[0][t];
+    if (e >= 0) {
+      const bool ok = Z <= a.gc.nz;
+      TC* dst = reinterpret_cast<TC*>(&sm.xc[Z % 3][0][0]) + sm.at[1][t];
+      cp_async_el<int(sizeof(TC))>(dst, xc + (ok ? int64_t(e) + int64_t(a.gc.ny + 1) * (a.gc.nx + 1) * Z : 0), ok);
     }
-    const bool eok = einb && zp >= zc0 && zp >= 1 && zp <= a.g.nz && zp <= zend;  // the layer between zp - 1 and zp
-    cp_async_el<8>(&sm.stage[s][3][t], at(a.E, eok ? e0 + ep * uint32_t(zp - 1) : 0u), eok);
   };
+  // one thread issues the copies of plane zp and of the layer below it
+  auto issue = [&](int zp, int s) {
+    if (t == 0) {
+      double* d = ku_stages + s * sg.len;
+      mbar_expect(&sm.bar[s], bytes);
+      tma_load(d, &maps.a, y0 - 2, x0 - 1, zp, &sm.bar[s]);
+      tma_load(d + sg.E, &maps.E, y0 - 2, x0 - 1, zp - 1, &sm.bar[s]);
+      if (PCG) {
+        tma_load(d + sg.p, &maps.p, y0 - 2, x0 - 1, zp, &sm.bar[s]);
+        tma_load(d + sg.y, &maps.y, y0, x0, zp, &sm.bar[s]);
+      }
+      if (MODE == KU_FUSED) tma_load(d + sg.D, &maps.D, y0 - 2, x0 - 1, zp, &sm.bar[s]);
+    }
+    // the far end of the cell that begins on plane zp, whose readers are past a barrier by then
+    if (MODE == KU_FUSED && zp % KU_SPAN == 0) issue_coarse(zp / KU_SPAN + 1);
+  };
+  if (t == 0) {
+    mbar_init(&sm.bar[0]);
+    mbar_init(&sm.bar[1]);
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
+  __syncthreads();
+  if (MODE == KU_FUSED) {
+    for (int Z = 0; Z < 3; ++Z) issue_coarse(Zfirst + Z);
+  }
   issue(zc0 - 1, 0);
-  cp_async_commit();
   issue(zc0, 1);
-  cp_async_commit();
   auto flags_at = [&](int zp) -> unsigned {
-    return inb && zp >= 0 && zp < nnz && zp <= zend ? unsigned(a.flags[(n0 + np * uint32_t(zp)) / 8u]) : 0u;
+    return inb && zp >= 0 && zp < nnz ? unsigned(a.flags[(n0 + np * uint32_t(zp)) / 8u]) : 0u;
   };
   unsigned f = flags_at(zc0 - 1), fo = 0;  // of the plane, and of the one below
   const bool first = PCG && a.sc->first;
   const double beta = PCG ? a.sc->beta : 0.0, lam = PCG ? a.sc->lam : 0.0;
-  if (PCG && a.sc->done) {
+  bool ok = true;  // no wait gave up
+  if (PCG && a.sc->done) {  // the same for the whole launch
     cp_async_wait_all();
+    ok = mbar_wait(&sm.bar[0], 0) && mbar_wait(&sm.bar[1], 0);
+    if (!ok && t == 0) atomicCAS(a.err, 0, kCoopErrCopy);
     return;
   }
+  // xc interpolated to the node's (y, x) on level-2 plane Z (fused)
+  auto coarse = [&](int Z) {
+    const int e = sm.at[2][t];
+    if (e < 0) return;
+    const int c0 = e & 255, wy = e >> 8 & 3, wx = e >> 10 & 3, dy = wy ? 1 : 0, dx = wx ? e >> 12 : 0;
+    const TC* p = reinterpret_cast<const TC*>(&sm.xc[Z % 3][0][0]) + c0;
+    const double fy = double(wy) / KU_SPAN, fx = double(wx) / KU_SPAN;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      const TC* q = p + c * KU_COARSE;
+      double s = (1.0 - fy) * (1.0 - fx) * double(q[0]);
+      s = fma(fy * (1.0 - fx), double(q[dy]), s);
+      s = fma((1.0 - fy) * fx, double(q[dx]), s);
+      sm.zc[Z & 1][c][t] = fma(fy * fx, double(q[dx + dy]), s);
+    }
+  };
   double dot = 0.0;
   // Plane zp in slot s, and the element layer below it (between the faces Wp and W): plane zp - 1 is then
   // complete.  G holds its forces in face modes, Bn takes the layer's part of plane zp's.
   auto step = [&](int zp, int s, double (&Wp)[3][4], double (&W)[3][4], double (&G)[3][4], double (&Bn)[3][4]) {
     const uint32_t n = n0 + np * uint32_t(zp);
     const bool mine = own && zp >= zc0 && zp < zend;
-    cp_async_wait_all_but_one();
-    const double E = sm.stage[s][3][t];
+    const double* st = ku_stages + s * sg.len;
+    if (ok) ok = mbar_wait(&sm.bar[s], unsigned(zp - zc0 + 1) >> 1 & 1u);
+    if (MODE == KU_FUSED) cp_async_wait_all();  // level-2 planes, a plane ahead of their use
+    const double E = st[sg.E + o];
     double v[3], y[3];
 #pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      v[c] = sm.stage[s][c][t];
-      if (PCG) {
-        const double po = sm.stage[s][4 + c][t];
-        if (!first) v[c] = fma(beta, po, v[c]);
-        if (mine) {
-          *at(a.pout + c * S, n) = v[c];
-          if (!first) *at(a.yacc + c * S, n) = fma(lam, po, sm.stage[s][7 + c][t]);
-        }
+    for (int c = 0; c < 3; ++c) v[c] = st[c * bx + o];
+    if (MODE == KU_FUSED) {
+      const int Z = zp / KU_SPAN, tz = zp & (KU_SPAN - 1);
+      if (zp < zc0) {
+        __syncthreads();  // the first level-2 planes, copied by other threads
+        coarse(Zfirst);
+        coarse(Zfirst + 1);
+      } else if (tz == 0 && zp > 0) {
+        coarse(Z + 1);
       }
-      if (f & (1u << c)) v[c] = 0.0;
-      sm.su[s][c][t] = v[c];
+      const double D = st[sg.D + o];
+      // z is zero off the domain: no correction there, and r is zero
+      const double wz = f & 8u ? tz * (1.0 / KU_SPAN) : 0.0, wa = f & 8u ? 1.0 - tz * (1.0 / KU_SPAN) : 0.0;
+      double d[3] = {D, D, D};
+      if (f & 7u)
+#pragma unroll
+        for (int c = 0; c < 3; ++c)
+          if (f & (1u << c)) d[c] = double(TC(*at(a.icfix, n)));  // a fixed DOF's diagonal
+#pragma unroll
+      for (int c = 0; c < 3; ++c)
+        v[c] = fma(a.omega2 * v[c], d[c], fma(wz, sm.zc[(Z + 1) & 1][c][t], wa * sm.zc[Z & 1][c][t]));
     }
-    if (zp + 2 <= zend) issue(zp + 2, s);
-    cp_async_commit();
+    if (PCG) {
+      if (!first) {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) v[c] = fma(beta, st[sg.p + c * bx + o], v[c]);
+      }
+      if (mine) {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) *at(a.pout + c * S, n) = v[c];
+        if (!first)
+#pragma unroll
+          for (int c = 0; c < 3; ++c)
+            *at(a.yacc + c * S, n) = fma(lam, st[sg.p + c * bx + o], st[sg.y + c * by + oy]);
+      }
+    }
+    if (f & 7u)
+#pragma unroll
+      for (int c = 0; c < 3; ++c)
+        if (f & (1u << c)) v[c] = 0.0;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) sm.su[s][c][t] = v[c];
     const unsigned fn = flags_at(zp + 1);
     __syncthreads();
+    if (zp + 2 <= zend) issue(zp + 2, s);  // every thread has read the stage
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
       const double* u = sm.su[s][c] + t;
@@ -255,18 +385,34 @@ __global__ void __launch_bounds__(KU_NT, KU_CTAS) k_ku(const __grid_constant__ K
         __syncthreads();
         if (own) {
           const uint32_t m = n - np;
+          double p[3];
 #pragma unroll
           for (int c = 0; c < 3; ++c) {
-            double yv = ((y[c] + sm.cor[0][c][KU_PAD + t - 1]) + sm.cor[1][c][KU_PAD + t - PY]) +
-                        sm.cor[2][c][KU_PAD + t - PY - 1];
-            double p = sm.su[s ^ 1][c][t];
-            if (fo & (1u << c)) {  // a fixed DOF: its own value, unmasked
-              p = PCG ? *at(a.pout + c * S, m) : *at(a.in + c * S, m);
-              yv = *at(a.cfix, m) * p;
-            }
-            *at(a.out + c * S, m) = yv;
-            if (PCG) dot = fma(p, yv, dot);
+            y[c] = (y[c] + sm.cor[1][c][KU_PAD + t - PY]) +
+                   (sm.cor[0][c][KU_PAD + t - 1] + sm.cor[2][c][KU_PAD + t - PY - 1]);
+            if (PCG) p[c] = sm.su[s ^ 1][c][t];
           }
+          if (fo & 7u) {  // a fixed DOF: its own value, unmasked
+            const double cf = *at(a.cfix, m);
+#pragma unroll
+            for (int c = 0; c < 3; ++c)
+              if (fo & (1u << c)) {
+                p[c] = PCG ? *at(a.pout + c * S, m) : *at(a.in + c * S, m);
+                y[c] = cf * p[c];
+              }
+          }
+          if (MODE == KU_PLAIN && a.compact) {
+            const int k = a.compact[m / 8u];
+            if (k >= 0)
+#pragma unroll
+              for (int c = 0; c < 3; ++c) a.out[3 * int64_t(k) + c] = y[c];
+          } else {
+#pragma unroll
+            for (int c = 0; c < 3; ++c) *at(a.out + c * S, m) = y[c];
+          }
+          if (PCG)
+#pragma unroll
+            for (int c = 0; c < 3; ++c) dot = fma(p[c], y[c], dot);
         }
       }
     }
@@ -295,16 +441,44 @@ __global__ void __launch_bounds__(KU_NT, KU_CTAS) k_ku(const __grid_constant__ K
       }
   }
   cp_async_wait_all();
+  if (!ok) atomicCAS(a.err, 0, kCoopErrCopy);
   if (PCG) {
     double r[1] = {dot}, tot[1];
     if (reduce_publish<1>(r, a.rs, tot) && t == 0) a.sc->pq = tot[0];
   }
 }
 
-template <int MODE>
+template <int MODE, typename TC>
 void ku_smem_attr() {
-  TOPX_CUDA_OK(cudaFuncSetAttribute(k_ku<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    int(sizeof(KuSmem<MODE>))));
+  TOPX_CUDA_OK(cudaFuncSetAttribute(k_ku<MODE, TC>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024 / KU_CTAS));
+}
+
+// cuTensorMapEncodeTiled through the runtime (the library does not link the driver)
+using EncodeTiled = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
+                                 const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
+                                 CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+EncodeTiled encode_tiled() {
+  static const EncodeTiled fn = [] {
+    void* p = nullptr;
+    cudaDriverEntryPointQueryResult q = cudaDriverEntryPointSymbolNotFound;
+    TOPX_CUDA_OK(cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &q));
+    if (!p || q != cudaDriverEntryPointSuccess) throw std::runtime_error("cuTensorMapEncodeTiled is not available");
+    return reinterpret_cast<EncodeTiled>(p);
+  }();
+  return fn;
+}
+
+// map of ncomp node fields of the grid, boxes of by x bx nodes of one plane
+CUtensorMap field_map(const double* p, const Grid& g, int ncomp, int by, int bx) {
+  CUtensorMap m;
+  const cuuint64_t dim[4] = {cuuint64_t(g.nny()), cuuint64_t(g.nnx()), cuuint64_t(g.nnz()), cuuint64_t(ncomp)};
+  const cuuint64_t stride[3] = {8 * dim[0], 8 * dim[0] * dim[1], 8 * cuuint64_t(g.stride)};
+  const cuuint32_t box[4] = {cuuint32_t(by), cuuint32_t(bx), 1, cuuint32_t(ncomp)}, one[4] = {1, 1, 1, 1};
+  if (encode_tiled()(&m, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 4, const_cast<double*>(p), dim, stride, box, one,
+                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+    throw std::runtime_error("cuTensorMapEncodeTiled failed");
+  return m;
 }
 
 int ku_num_sms() {
@@ -317,8 +491,10 @@ int ku_num_sms() {
 }  // namespace
 
 void prepare_ku_kernels() {
-  ku_smem_attr<KU_PLAIN>();
-  ku_smem_attr<KU_P_UPDATE>();
+  ku_smem_attr<KU_PLAIN, double>();
+  ku_smem_attr<KU_P_UPDATE, double>();
+  ku_smem_attr<KU_FUSED, double>();
+  ku_smem_attr<KU_FUSED, float>();
 }
 
 // Sign of corner a in mode (sy, sx, sz); the y difference runs from the upper to the lower row, along the y axis.
@@ -370,29 +546,30 @@ KuModes ku_modes(const double* Ke576) {
 }
 
 // Tile and z-chunk of the launch.  A CTA's time goes with its planes (zc + 2 formed for zc written, and
-// about two planes' worth of start and end), each plane's with its warps and with the
-// 32-byte sectors its unaligned rows of PY nodes touch.  Every tile height whose tiles come out
-// even, with the widest tile that then fits the CTA, and every chunk length are compared; past six
-// waves the last one's share is small.  In a sweep of tiles and chunks at the three sizes above no
-// other choice was more than 8 % faster than the one taken.
-KuShape ku_shape(Grid g) {
-  const int nny = g.nny(), nnx = g.nnx(), nnz = g.nnz();
+// about two planes' worth of start and end), each plane's with its warps and the sectors that its rows touch;
+// two CTAs fit an SM, a last wave that is nearly empty costs about half a wave, and long chunks drift apart
+// and lose the halo planes that neighbours share in L2.  Every even tile height whose tiles come out
+// even, with the widest tile that then fits the CTA, and every chunk length are compared.  Sweeps of tiles and
+// chunks at the sizes above found at most 5 % more.
+KuShape ku_shape(Grid g, int rows) {
+  const int nny = rows, nnx = g.nnx(), nnz = g.nnz();
   if (g.nnodes() >= (int64_t(1) << 29)) throw std::runtime_error("grid too large for 32-bit byte offsets");
   const double slots = double(KU_CTAS) * ku_num_sms();
   KuShape best{};
   double bestCost = -1;
   for (int nty = 1; nty <= nny; ++nty) {
-    const int TY = (nny + nty - 1) / nty, PY = TY + 2;
+    const int TY = (((nny + nty - 1) / nty) + 1) & ~1, PY = TY + 2;  // even: a box starts on a 16-byte boundary
     if (PY > KU_PAD - 2 || (nny + TY - 1) / TY != nty) continue;
     if (PY * 3 > KU_NT) continue;
     if (TY < 6 && nny >= 6) break;
     const int TXmax = std::min(KU_NT / PY - 2, nnx);
     const int ntx = (nnx + TXmax - 1) / TXmax, TX = (nnx + ntx - 1) / ntx, PX = TX + 2;
+    if (((PY + 2) / KU_SPAN + 2) * ((PX + 2) / KU_SPAN + 2) > KU_COARSE) continue;
     const double plane_cost = (PY * PX + 31) / 32 * (1.0 + 3.0 / PY) / 8.0 + 0.4;
     for (int zc = 1; zc <= 64 && zc <= nnz + 1; ++zc) {
       const double ctas = double(nty) * ntx * ((nnz + zc - 1) / zc);
-      const double waves = ctas / slots, w = waves > 6 ? waves + 0.5 : std::ceil(waves);
-      const double cost = w * (zc + 4) * plane_cost;
+      const double waves = ctas / slots, w = waves <= 1.0 ? 1.0 : 0.5 * (waves + std::ceil(waves));
+      const double cost = (w + 0.3) * (zc + 4) * (1.0 + 0.003 * zc) * plane_cost;
       if (bestCost < 0 || cost < bestCost) {
         bestCost = cost;
         best = KuShape{PY, PX, TY, TX, zc, dim3(unsigned(nty), unsigned(ntx), unsigned((nnz + zc - 1) / zc))};
@@ -403,7 +580,7 @@ KuShape ku_shape(Grid g) {
   return best;
 }
 
-std::vector<uint32_t> ku_active_tiles(Grid g, const KuShape& k, const std::vector<uint8_t>& present,
+std::vector<uint32_t> ku_active_tiles(Grid g, int rows, const KuShape& k, const std::vector<uint8_t>& present,
                                       std::vector<uint32_t>* zranges) {
   const int nny = g.nny(), nnx = g.nnx(), nnz = g.nnz();
   if (k.grid.x > 1024 || k.grid.y > 1024 || k.grid.z > 4095 || nnz > 65535) return {};
@@ -416,7 +593,7 @@ std::vector<uint32_t> ku_active_tiles(Grid g, const KuShape& k, const std::vecto
         for (int z = int(tz) * k.zc; z < std::min(nnz, int(tz + 1) * k.zc); ++z) {
           bool any = false;
           for (int x = int(tx) * k.TX; x < std::min(nnx, int(tx + 1) * k.TX) && !any; ++x)
-            for (int y = int(ty) * k.TY; y < std::min(nny, int(ty + 1) * k.TY) && !any; ++y)
+            for (int y = int(ty) * k.TY; y < std::min(rows, int(ty + 1) * k.TY) && !any; ++y)
               any = present[size_t(y + int64_t(nny) * (x + int64_t(nnx) * z))] != 0;
           if (any) {
             if (lo < 0) lo = z;
@@ -431,13 +608,47 @@ std::vector<uint32_t> ku_active_tiles(Grid g, const KuShape& k, const std::vecto
   return list;
 }
 
+template <int MODE, typename TC>
+static void launch(cudaStream_t st, const KuArgs& a, dim3 grd) {
+  const int PB = a.sh.TY + 4, PX = a.sh.PX, box = PB * PX, own = a.sh.TY * a.sh.TX;
+  auto up = [](int doubles) { return (doubles + 15) / 16 * 16; };
+  KuMaps m{};
+  KuStage sg{};
+  int at = up(3 * box), used = 4 * box;
+  m.a = field_map(a.in, a.g, 3, PB, PX);
+  m.E = field_map(a.E, a.g, 1, PB, PX);
+  sg.E = at;
+  at += up(box);
+  if (MODE != KU_PLAIN) {
+    m.p = field_map(a.pin, a.g, 3, PB, PX);
+    sg.p = at;
+    at += up(3 * box);
+    m.y = field_map(a.yacc, a.g, 3, a.sh.TY, a.sh.TX);
+    sg.y = at;
+    at += up(3 * own);
+    used += 3 * box + 3 * own;
+  }
+  if (MODE == KU_FUSED) {
+    m.D = field_map(a.D, a.g, 1, PB, PX);
+    sg.D = at;
+    at += up(box);
+    used += box;
+  }
+  sg.len = at;
+  const size_t smem = sizeof(double) * 2 * size_t(at) + sizeof(KuSmem<MODE>);
+  (k_ku<MODE, TC><<<grd, KU_NT, smem, st>>>(a, m, sg, unsigned(8 * used)), topx::count_launch());
+}
 void launch_ku(cudaStream_t st, KuMode mode, const KuArgs& args, int ntiles) {
   const dim3 grd = args.active ? dim3(unsigned(ntiles)) : args.sh.grid;
   if (grd.x == 0) return;
   if (mode == KU_PLAIN)
-    (k_ku<KU_PLAIN><<<grd, KU_NT, sizeof(KuSmem<KU_PLAIN>), st>>>(args), topx::count_launch());
+    launch<KU_PLAIN, double>(st, args, grd);
+  else if (mode == KU_P_UPDATE)
+    launch<KU_P_UPDATE, double>(st, args, grd);
+  else if (args.pre32)
+    launch<KU_FUSED, float>(st, args, grd);
   else
-    (k_ku<KU_P_UPDATE><<<grd, KU_NT, sizeof(KuSmem<KU_P_UPDATE>), st>>>(args), topx::count_launch());
+    launch<KU_FUSED, double>(st, args, grd);
   TOPX_CUDA_OK(cudaGetLastError());
 }
 

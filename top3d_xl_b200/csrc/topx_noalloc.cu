@@ -52,8 +52,8 @@ double* noalloc_scratch(int device) {
 }
 
 // y = K u with u and y compact interleaved DOF vectors in device memory (the reference's DOF
-// order, like apply_K); grid_u and grid_y are caller-provided scratch of 3 * stride doubles.
-void Engine::apply_K_device(const double* d_u, double* d_y, double* grid_u, double* grid_y) {
+// order, like apply_K); grid_u is caller-provided scratch of 3 * stride doubles.
+void Engine::apply_K_device(const double* d_u, double* d_y, double* grid_u) {
   const Grid& g = G[0];
   // The engine stream is non-blocking, so nothing orders it after work the caller still has
   // queued on the legacy default stream (a gpuArray kernel, an asynchronous copy into u):
@@ -64,8 +64,7 @@ void Engine::apply_K_device(const double* d_u, double* d_y, double* grid_u, doub
   // the scratch keeps the previous call's contents: grid nodes outside the domain must read 0
   TOPX_CUDA_OK(cudaMemsetAsync(grid_u, 0, sizeof(double) * size_t(g.stride) * 3, st));
   launch_compact_to_grid_nodes<double>(st, d_u, grid_u, g, nodMapBack0.p, Nn);
-  ku(KU_PLAIN, grid_u, nullptr, nullptr, grid_y, nullptr, nullptr);
-  launch_grid_to_compact_nodes<double>(st, grid_y, d_y, g, nodMapBack0.p, Nn);
+  ku(KU_PLAIN, grid_u, nullptr, nullptr, d_y, nullptr, nullptr, nodMapFwd0.p);
   TOPX_CUDA_OK(cudaStreamSynchronize(st));
 }
 

@@ -43,7 +43,7 @@ __global__ void k_filter_e2n(Grid g, const T* __restrict__ srcE, T* __restrict__
     for (int a = 0; a < 8; ++a) {
       const int ey = gy - hex_ly(a), ex = gx - hex_lx(a), ez = gz - hex_lz(a);
       if (ey < 0 || ey >= g.ny || ex < 0 || ex >= g.nx || ez < 0 || ez >= g.nz) continue;
-      s = s + srcE[ey + int64_t(g.ny) * (ex + int64_t(g.nx) * ez)] * T(0.125);
+      s = s + srcE[ey + int64_t(nny) * (ex + int64_t(nnx) * ez)] * T(0.125);
     }
     node[n] = s;
   }
@@ -67,7 +67,7 @@ __global__ void k_filter_diag(Grid g, const uint8_t* __restrict__ solid, const F
     for (int a = 0; a < 8; ++a) {
       const int ey = gy - hex_ly(a), ex = gx - hex_lx(a), ez = gz - hex_lz(a);
       if (ey < 0 || ey >= g.ny || ex < 0 || ex >= g.nx || ez < 0 || ez >= g.nz) continue;
-      if (solid[ey + int64_t(g.ny) * (ex + int64_t(g.nx) * ez)]) s += kf.v[a * 9];
+      if (solid[ey + int64_t(nny) * (ex + int64_t(nnx) * ez)]) s += kf.v[a * 9];
     }
     dp[n] = s > 0.0 ? T(1.0 / s) : T(0);
   }
@@ -128,7 +128,7 @@ __global__ void __launch_bounds__(FNT) k_filter_ku(Grid g, int zc, const FilterK
       const int ey = y0 - 1 + sy, ex = x0 - 1 + sx;
       T v = T(0);
       if (ez >= 0 && ez < g.nz && ey >= 0 && ey < g.ny && ex >= 0 && ex < g.nx)
-        v = solid[ey + int64_t(g.ny) * (ex + int64_t(g.nx) * ez)] ? T(1) : T(0);
+        v = solid[ey + int64_t(nny) * (ex + int64_t(nnx) * ez)] ? T(1) : T(0);
       ss[slot][sx][sy] = v;
     }
   };
@@ -324,12 +324,11 @@ __global__ void k_filter_n2e(Grid g, const T* __restrict__ node, const int32_t* 
                              double* __restrict__ out) {
   const int nny = g.ny + 1, nnx = g.nx + 1;
   for (int64_t e = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; e < Ne; e += int64_t(gridDim.x) * blockDim.x) {
-    const int64_t id = emb0[e];
-    const int ey = int(id % g.ny), ex = int((id / g.ny) % g.nx), ez = int(id / (int64_t(g.ny) * g.nx));
+    const int64_t id = emb0[e];  // the index of its lowest node
     double s = 0.0;
 #pragma unroll
     for (int a = 0; a < 8; ++a)
-      s += double(node[(ey + hex_ly(a)) + int64_t(nny) * ((ex + hex_lx(a)) + int64_t(nnx) * (ez + hex_lz(a)))]);
+      s += double(node[id + hex_ly(a) + int64_t(nny) * (hex_lx(a) + int64_t(nnx) * hex_lz(a))]);
     out[e] = s * (1.0 / 8);
   }
 }
