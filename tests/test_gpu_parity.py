@@ -326,6 +326,10 @@ def test_pcg_step_edges(shape, precision):
     sol.assemble(E)
     uo, itso, _ = O.pcg(sol.ku, sol.vcycle, m.F[:, 0], m.S.tol, m.S.maxIT)
     f = m.F[:, 0]
+    # the oracle against itself with rounding noise in its V-cycle (a 3 x 3 x 3 model amplifies it to 3e-7)
+    rng = np.random.default_rng(5)
+    un, _, _ = O.pcg(sol.ku, lambda v: sol.vcycle(v) * (1 + 1e-15 * rng.standard_normal(v.shape)), f, m.S.tol, m.S.maxIT)
+    env = abs(f @ un - f @ uo) / abs(f @ uo)
     with Context(precision) as ctx:
         ctx.load_voxels(vox)
         ctx.set_moduli(E)
@@ -335,4 +339,4 @@ def test_pcg_step_edges(shape, precision):
         u, its = ctx.pcg()
     assert abs(its - itso) <= 1
     if its == itso:
-        assert abs(f @ u - f @ uo) / abs(f @ uo) < (1e-8 if precision == "fp64" else 1e-6)
+        assert abs(f @ u - f @ uo) / abs(f @ uo) < max(1e-8 if precision == "fp64" else 1e-6, 10 * env)
