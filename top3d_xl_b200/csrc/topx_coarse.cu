@@ -23,6 +23,7 @@ constexpr int GL2_ELEMS = 16, GL2_THREADS = 192;
 
 __global__ void __launch_bounds__(GL2_THREADS) k_galerkin_l2(Grid gf, Grid gc, const double* __restrict__ Ef,
                                                              const double* __restrict__ Tm, double* __restrict__ Ks) {
+  pdl_wait();
   __shared__ double sE[GL2_ELEMS][64];
   const int64_t nce = gc.nelems();
   const int64_t j0 = int64_t(blockIdx.x) * GL2_ELEMS;
@@ -79,7 +80,7 @@ __global__ void __launch_bounds__(GL2_THREADS) k_galerkin_l2(Grid gf, Grid gc, c
 
 void launch_galerkin_l2(cudaStream_t st, Grid gf, Grid gc, const double* Efine, const double* Tm, double* Ks) {
   const int64_t nb = (gc.nelems() + GL2_ELEMS - 1) / GL2_ELEMS;
-  (k_galerkin_l2<<<unsigned(nb), GL2_THREADS, 0, st>>>(gf, gc, Efine, Tm, Ks), topx::count_launch());
+  launch_pdl(st, k_galerkin_l2, unsigned(nb), GL2_THREADS, 0, gf, gc, Efine, Tm, Ks);
   TOPX_CUDA_OK(cudaGetLastError());
 }
 
@@ -93,6 +94,7 @@ __global__ void __launch_bounds__(GL2_THREADS) k_galerkin_l2_flagged(Grid gf, Gr
                                                                      const double* __restrict__ fl_F,
                                                                      const double* __restrict__ Tall,
                                                                      double* __restrict__ Ks) {
+  pdl_wait();
   __shared__ double sE[64];
   __shared__ int sT[64];
   const int f = blockIdx.x;
@@ -115,7 +117,7 @@ __global__ void __launch_bounds__(GL2_THREADS) k_galerkin_l2_flagged(Grid gf, Gr
 void launch_galerkin_l2_flagged(cudaStream_t st, Grid gf, Grid gc, const double* Efine, int nflag, const int32_t* fl_elem,
                                 const int32_t* fl_tsel, const double* fl_F, const double* Tall, double* Ks) {
   if (nflag <= 0) return;
-  (k_galerkin_l2_flagged<<<nflag, GL2_THREADS, 0, st>>>(gf, gc, Efine, fl_elem, fl_tsel, fl_F, Tall, Ks), topx::count_launch());
+  launch_pdl(st, k_galerkin_l2_flagged, nflag, GL2_THREADS, 0, gf, gc, Efine, fl_elem, fl_tsel, fl_F, Tall, Ks);
   TOPX_CUDA_OK(cudaGetLastError());
 }
 
@@ -132,6 +134,7 @@ constexpr int GS2_PER_THREAD = 8 * 576 / GS2_THREADS;  // 24 outputs of the firs
 __global__ void __launch_bounds__(GS2_THREADS) k_galerkin_span2(Grid gc, const double* __restrict__ Ksf,
                                                                 const uint8_t* __restrict__ cpresent,
                                                                 const double* __restrict__ W8, double* __restrict__ Ks) {
+  pdl_wait();
   __shared__ double sK[8 * 576];  // the 8 children's operators, then T_c = K_c (W_c (x) I) in place
   __shared__ double sW[8 * 64];   // W_c[a'][b] at c * 64 + 8 a' + b
   const int64_t J = blockIdx.x;
@@ -179,7 +182,7 @@ __global__ void __launch_bounds__(GS2_THREADS) k_galerkin_span2(Grid gc, const d
 
 void launch_galerkin_span2(cudaStream_t st, Grid gc, const double* Ksf, const uint8_t* cpresent, const double* W8,
                            double* Ks) {
-  (k_galerkin_span2<<<unsigned(gc.nelems()), GS2_THREADS, 0, st>>>(gc, Ksf, cpresent, W8, Ks), topx::count_launch());
+  launch_pdl(st, k_galerkin_span2, unsigned(gc.nelems()), GS2_THREADS, 0, gc, Ksf, cpresent, W8, Ks);
   TOPX_CUDA_OK(cudaGetLastError());
 }
 
@@ -188,6 +191,7 @@ void launch_galerkin_span2(cudaStream_t st, Grid gc, const double* Ksf, const ui
 template <typename T>
 __global__ void k_diag_coarse(Grid g, const double* __restrict__ Ks, const uint8_t* __restrict__ present,
                               T* __restrict__ d) {
+  pdl_wait();
   const int64_t N = g.nnodes();
   const int nny = g.ny + 1, nnx = g.nx + 1;
   for (int64_t n = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; n < N; n += int64_t(gridDim.x) * blockDim.x) {
@@ -208,7 +212,7 @@ __global__ void k_diag_coarse(Grid g, const double* __restrict__ Ks, const uint8
 
 template <typename T>
 void launch_diag_coarse(cudaStream_t st, Grid g, const double* Ks, const uint8_t* present, T* d) {
-  (k_diag_coarse<T><<<grid1d(g.nnodes(), 256), 256, 0, st>>>(g, Ks, present, d), topx::count_launch());
+  launch_pdl(st, k_diag_coarse<T>, grid1d(g.nnodes(), 256), 256, 0, g, Ks, present, d);
   TOPX_CUDA_OK(cudaGetLastError());
 }
 

@@ -24,6 +24,15 @@ inline std::atomic<long long>& launch_counter() {
 }
 inline void count_launch() { launch_counter().fetch_add(1, std::memory_order_relaxed); }
 
+// Programmatic dependent launch.  Every kernel of the library begins with pdl_wait(): it returns when the
+// launches before it in the stream are complete and their writes visible.  What stands before it may touch nothing that
+// another kernel writes.  Reductions call pdl_trigger() when a CTA's part is done, other kernels end with it: once
+// every CTA is there the next launch begins, and its start overlaps this one's tail.  (Triggering at the
+// start instead let the next launch's CTAs crowd the SMs that ran dry first: 6 % slower at 128x256x128.)
+// A kernel launched without the attribute passes through both.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // Device-resident scalars of one PCG solve (TOP3D_XL.m:600-639).  Written by
 // the last block of each reduction kernel, read by every later kernel, so a
 // whole PCG iteration runs without a host round trip.
@@ -111,6 +120,7 @@ __device__ __forceinline__ double block_max(double v) {
 template <int NS>
 __device__ __forceinline__ bool reduce_publish(double (&v)[NS], RedScratch rs, double (&out)[NS],
                                                unsigned stride = kMaxRedBlocks) {
+  pdl_trigger();
   block_sum<NS>(v);
   const int tid = threadIdx.x + blockDim.x * (threadIdx.y + blockDim.y * threadIdx.z);
   const int nth = blockDim.x * blockDim.y * blockDim.z;

@@ -29,6 +29,7 @@ template <typename T>
 __global__ void k_diag_l1(Grid g, const double* __restrict__ E, const uint8_t* __restrict__ fixbits,
                           const double* __restrict__ cfix, const uint8_t* __restrict__ present, T* __restrict__ d,
                           double* __restrict__ d0) {
+  pdl_wait();
   const int64_t N = g.nnodes();
   const int nny = g.ny + 1, nnx = g.nx + 1;
   for (int64_t n = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; n < N; n += int64_t(gridDim.x) * blockDim.x) {
@@ -54,7 +55,7 @@ __global__ void k_diag_l1(Grid g, const double* __restrict__ E, const uint8_t* _
 template <typename T>
 void launch_diag_l1(cudaStream_t st, Grid g, const double* E, const uint8_t* fixbits, const double* cfix,
                     const uint8_t* present, T* d, double* d0) {
-  (k_diag_l1<T><<<grid1d(g.nnodes(), 256), 256, 0, st>>>(g, E, fixbits, cfix, present, d, d0), topx::count_launch());
+  launch_pdl(st, k_diag_l1<T>, grid1d(g.nnodes(), 256), 256, 0, g, E, fixbits, cfix, present, d, d0);
   TOPX_CUDA_OK(cudaGetLastError());
 }
 
@@ -98,6 +99,7 @@ __device__ __forceinline__ void pcg_stop_test(PcgScalars* sc, double lam, double
 // r'z = omega2 r'D r + (P'r)'xc.
 template <int MODE, typename TC>
 __global__ void __launch_bounds__(256) k_residual(const __grid_constant__ ResidualArgs a, int lines, int cy, FastDiv dcy) {
+  pdl_wait();
   if (MODE == RES_UPDATE && a.sc->done) return;
   const int lane = threadIdx.x & 31;
   const int64_t S = a.g.stride, nlines = int64_t(a.g.nx + 1) * (a.g.nz + 1), ts = nlines * cy;
@@ -194,7 +196,7 @@ void launch_residual(cudaStream_t st, ResidualMode mode, const ResidualArgs& arg
   const int lines = residual_lines(nlines, cy);
   const unsigned nb = unsigned((nlines + 8 * lines - 1) / (8 * lines));
   const FastDiv dcy{uint32_t(cy)};
-  auto go = [&](auto kernel) { (kernel<<<nb, 256, 0, st>>>(args, lines, cy, dcy), topx::count_launch()); };
+  auto go = [&](auto kernel) { launch_pdl(st, kernel, nb, 256, 0, args, lines, cy, dcy); };
   if (mode == RES_KEEP)
     go(k_residual<RES_KEEP, double>);
   else if (mode == RES_INIT && args.pre32)
@@ -211,6 +213,7 @@ void launch_residual(cudaStream_t st, ResidualMode mode, const ResidualArgs& arg
 // The 'Standard' V-cycle's own residual start and update (it restricts another vector)
 __global__ void k_residual_init(Grid g, const double* __restrict__ b, const double* __restrict__ Ay,
                                 double* __restrict__ r, PcgScalars* sc, RedScratch rs, double tol, int maxIT) {
+  pdl_wait();
   const int64_t N = g.nnodes(), S = g.stride;
   double bb = 0.0;
   for (int64_t n = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; n < N; n += int64_t(gridDim.x) * blockDim.x) {
@@ -227,12 +230,13 @@ __global__ void k_residual_init(Grid g, const double* __restrict__ b, const doub
 
 void launch_residual_init(cudaStream_t st, Grid g, const double* b, const double* Ay, double* r, PcgScalars* sc,
                           RedScratch rs, double tol, int maxIT) {
-  (k_residual_init<<<grid1d(g.nnodes(), 256), 256, 0, st>>>(g, b, Ay, r, sc, rs, tol, maxIT), topx::count_launch());
+  launch_pdl(st, k_residual_init, grid1d(g.nnodes(), 256), 256, 0, g, b, Ay, r, sc, rs, tol, maxIT);
   TOPX_CUDA_OK(cudaGetLastError());
 }
 
 __global__ void k_pcg_update(Grid g, double* __restrict__ r, const double* __restrict__ q, PcgScalars* sc,
                              RedScratch rs, const uint32_t* __restrict__ act) {
+  pdl_wait();
   if (sc->done) return;
   const double lam = sc->x1 / sc->pq;
   const int64_t S = g.stride;  // a multiple of 32, so node pairs are aligned
@@ -256,7 +260,7 @@ __global__ void k_pcg_update(Grid g, double* __restrict__ r, const double* __res
 }
 void launch_pcg_update(cudaStream_t st, Grid g, double* r, const double* q, PcgScalars* sc, RedScratch rs,
                        const uint32_t* act) {
-  (k_pcg_update<<<grid1d(g.nnodes(), 256), 256, 0, st>>>(g, r, q, sc, rs, act), topx::count_launch());
+  launch_pdl(st, k_pcg_update, grid1d(g.nnodes(), 256), 256, 0, g, r, q, sc, rs, act);
   TOPX_CUDA_OK(cudaGetLastError());
 }
 
@@ -264,6 +268,7 @@ void launch_pcg_update(cudaStream_t st, Grid g, double* r, const double* q, PcgS
 // leave it to the next K*u)
 __global__ void k_pcg_flush(Grid g, double* __restrict__ y, const double* __restrict__ p, const PcgScalars* sc,
                             const uint32_t* __restrict__ act) {
+  pdl_wait();
   const double lam = sc->lam;
   const int64_t S = g.stride;
   const int64_t npair = (g.nnodes() + 1) / 2;
@@ -283,7 +288,7 @@ __global__ void k_pcg_flush(Grid g, double* __restrict__ y, const double* __rest
 
 void launch_pcg_flush(cudaStream_t st, Grid g, double* y, const double* p, const PcgScalars* sc,
                       const uint32_t* act) {
-  (k_pcg_flush<<<grid1d(g.nnodes(), 256), 256, 0, st>>>(g, y, p, sc, act), topx::count_launch());
+  launch_pdl(st, k_pcg_flush, grid1d(g.nnodes(), 256), 256, 0, g, y, p, sc, act);
   TOPX_CUDA_OK(cudaGetLastError());
 }
 
@@ -299,6 +304,7 @@ __global__ void __launch_bounds__(32 * (2 * KU_SPAN - 1)) k_restrict_xz(const do
                                                                        T* __restrict__ out, double* __restrict__ out64,
                                                                        int64_t ostr, int ony, int onx, FastDiv dy,
                                                                        const PcgScalars* sc) {
+  pdl_wait();
   if (sc && sc->done) return;
   constexpr int W = 2 * KU_SPAN - 1;
   __shared__ double sx[W][3][32];
@@ -339,9 +345,8 @@ void launch_restrict_xz(cudaStream_t st, const double* tmp, Grid gf, T* out, dou
                         const PcgScalars* sc) {
   const int cy = gc.nny(), cx = gc.nnx();
   const dim3 nb(unsigned((cy * cx + 31) / 32), unsigned(gc.nnz()));
-  (k_restrict_xz<T><<<nb, dim3(32, 2 * KU_SPAN - 1), 0, st>>>(tmp, gf.nnx(), gf.nnz(), out, out64, gc.stride, cy, cx,
-                                                              FastDiv{uint32_t(cy)}, sc),
-   topx::count_launch());
+  launch_pdl(st, k_restrict_xz<T>, nb, dim3(32, 2 * KU_SPAN - 1), 0, tmp, gf.nnx(), gf.nnz(), out, out64, gc.stride,
+             cy, cx, FastDiv{uint32_t(cy)}, sc);
   TOPX_CUDA_OK(cudaGetLastError());
 }
 template void launch_restrict_xz<double>(cudaStream_t, const double*, Grid, double*, double*, Grid, const PcgScalars*);
@@ -351,6 +356,7 @@ template <typename T, int S, int AXIS>
 __global__ void k_restrict_axis(const T* __restrict__ in, int64_t istr, int iny, int inx, int inz,
                                 T* __restrict__ out, int64_t ostr, int ony, int onx, int onz, FastDiv fdy,
                                 FastDiv fdx, const PcgScalars* sc) {
+  pdl_wait();
   if (sc && sc->done) return;
   const uint32_t N = uint32_t(ony) * onx * onz;
   for (uint32_t n = blockIdx.x * blockDim.x + threadIdx.x; n < N; n += gridDim.x * blockDim.x) {
@@ -392,6 +398,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) k_restrict_coop(const T* __restrict__ in, int64_t istr, int iny, int inx,
                                                       int inz, T* __restrict__ out, int64_t ostr, int ony, int onx,
                                                       int onz, FastDiv fdy, FastDiv fdx, const PcgScalars* sc) {
+  pdl_wait();
   if (sc && sc->done) return;
   constexpr int W = 3, L = 16, NODES = 256 / L;
   __shared__ T sy[NODES][W * W][3];  // y sums of the node's (dx, dz) columns
@@ -460,17 +467,15 @@ void launch_restrict(cudaStream_t st, const T* in, Grid gf, T* tmp1, T* tmp2, T*
   if (gf.nnodes() >= (int64_t(1) << 32)) throw std::runtime_error("grid too large for 32-bit node indices");
   const FastDiv dcy{uint32_t(cy)}, dfx{uint32_t(fx)}, dcx{uint32_t(cx)};
   if (gf.nnodes() <= kRestrictOneLaunch) {
-    (k_restrict_coop<T><<<grid1d(gc.nnodes() * 16, 256), 256, 0, st>>>(in, gf.stride, fy, fx, fz, out, gc.stride, cy, cx,
-                                                                       cz, dcy, dcx, sc),
-     topx::count_launch());
+    launch_pdl(st, k_restrict_coop<T>, grid1d(gc.nnodes() * 16, 256), 256, 0, in, gf.stride, fy, fx, fz, out,
+               gc.stride, cy, cx, cz, dcy, dcx, sc);
   } else {
-    (k_restrict_axis<T, 2, 0><<<grid1d(s1, 256), 256, 0, st>>>(in, gf.stride, fy, fx, fz, tmp1, s1, cy, fx, fz, dcy, dfx, sc),
-     topx::count_launch());
-    (k_restrict_axis<T, 2, 1><<<grid1d(s2, 256), 256, 0, st>>>(tmp1, s1, cy, fx, fz, tmp2, s2, cy, cx, fz, dcy, dcx, sc),
-     topx::count_launch());
-    (k_restrict_axis<T, 2, 2><<<grid1d(gc.nnodes(), 256), 256, 0, st>>>(tmp2, s2, cy, cx, fz, out, gc.stride, cy, cx, cz,
-                                                                         dcy, dcx, sc),
-     topx::count_launch());
+    launch_pdl(st, k_restrict_axis<T, 2, 0>, grid1d(s1, 256), 256, 0, in, gf.stride, fy, fx, fz, tmp1, s1, cy, fx, fz,
+               dcy, dfx, sc);
+    launch_pdl(st, k_restrict_axis<T, 2, 1>, grid1d(s2, 256), 256, 0, tmp1, s1, cy, fx, fz, tmp2, s2, cy, cx, fz, dcy,
+               dcx, sc);
+    launch_pdl(st, k_restrict_axis<T, 2, 2>, grid1d(gc.nnodes(), 256), 256, 0, tmp2, s2, cy, cx, fz, out, gc.stride,
+               cy, cx, cz, dcy, dcx, sc);
   }
   TOPX_CUDA_OK(cudaGetLastError());
 }
@@ -491,6 +496,7 @@ __global__ void __launch_bounds__(256) k_prolong_smooth(const TX* __restrict__ x
                                                         Grid gf, FastDiv dny, FastDiv dnx, T omega,
                                                         const double* __restrict__ rc, PcgScalars* sc, RedScratch rs,
                                                         int init, double omega2, const uint32_t* __restrict__ act) {
+  pdl_wait();
   if (sc && sc->done) return;
   const uint32_t fny = uint32_t(gf.nny()), fnx = uint32_t(gf.nnx());
   const uint32_t nn = uint32_t(gf.nnodes());  // < 2^32 (checked at launch)
@@ -559,8 +565,8 @@ void launch_prolong_smooth(cudaStream_t st, int span, const TX* xc, Grid gc, con
   const unsigned nb = grid1d(gf.nnodes(), 256, 148 * 8);
   const FastDiv dny{uint32_t(gf.nny())}, dnx{uint32_t(gf.nnx())};
   auto go = [&](auto kernel) {
-    (kernel<<<nb, 256, 0, st>>>(xc, gc, r, d, present, x, gf, dny, dnx, T(omega), rc, sc, rs, init ? 1 : 0, 2.0 * omega, act),
-     topx::count_launch());
+    launch_pdl(st, kernel, nb, 256, 0, xc, gc, r, d, present, x, gf, dny, dnx, T(omega), rc, sc, rs, init ? 1 : 0,
+               2.0 * omega, act);
   };
   if (span == 4)
     go(k_prolong_smooth<TX, T, TD, 4, false>);
@@ -579,8 +585,8 @@ void launch_prolong_add(cudaStream_t st, int span, const TX* xc, Grid gc, const 
   if (gf.nnodes() >= (int64_t(1) << 32)) throw std::runtime_error("grid too large for 32-bit node indices");
   const FastDiv dny{uint32_t(gf.nny())}, dnx{uint32_t(gf.nnx())};
   auto go = [&](auto kernel) {
-    (kernel<<<nb, 256, 0, st>>>(xc, gc, r, d, present, x, gf, dny, dnx, T(omega), nullptr, sc, none, 0, 0.0, nullptr),
-     topx::count_launch());
+    launch_pdl(st, kernel, nb, 256, 0, xc, gc, r, d, present, x, gf, dny, dnx, T(omega), nullptr, sc, none, 0, 0.0,
+               nullptr);
   };
   if (span == 4)
     go(k_prolong_smooth<TX, T, TD, 4, false, false>);
@@ -599,6 +605,7 @@ void launch_prolong_add(cudaStream_t st, int span, const TX* xc, Grid gc, const 
 template <typename TR, typename T, typename TD>
 __global__ void k_jacobi_pre(Grid g, const TR* __restrict__ r, const TD* __restrict__ dinv,
                              const uint8_t* __restrict__ present, T* __restrict__ x, T omega, const PcgScalars* sc) {
+  pdl_wait();
   if (sc->done) return;
   const int64_t N = g.nnodes();
   for (int64_t n = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; n < N; n += int64_t(gridDim.x) * blockDim.x) {
@@ -611,14 +618,14 @@ __global__ void k_jacobi_pre(Grid g, const TR* __restrict__ r, const TD* __restr
 template <typename TR, typename T, typename TD>
 void launch_jacobi_pre(cudaStream_t st, Grid g, const TR* r, const TD* d, const uint8_t* present, T* x, double omega,
                        const PcgScalars* sc) {
-  (k_jacobi_pre<TR, T, TD><<<grid1d(g.nnodes(), 256), 256, 0, st>>>(g, r, d, present, x, T(omega), sc),
-   topx::count_launch());
+  launch_pdl(st, k_jacobi_pre<TR, T, TD>, grid1d(g.nnodes(), 256), 256, 0, g, r, d, present, x, T(omega), sc);
   TOPX_CUDA_OK(cudaGetLastError());
 }
 
 // q = r - q: the residual after pre-smoothing, restricted next (TX:761-762)
 template <typename TR, typename T>
 __global__ void k_residual_inplace(Grid g, const TR* __restrict__ r, T* __restrict__ q, const PcgScalars* sc) {
+  pdl_wait();
   if (sc->done) return;
   const int64_t N = g.nnodes();
   for (int64_t n = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; n < N; n += int64_t(gridDim.x) * blockDim.x) {
@@ -628,7 +635,7 @@ __global__ void k_residual_inplace(Grid g, const TR* __restrict__ r, T* __restri
 }
 template <typename TR, typename T>
 void launch_residual_inplace(cudaStream_t st, Grid g, const TR* r, T* q, const PcgScalars* sc) {
-  (k_residual_inplace<TR, T><<<grid1d(g.nnodes(), 256), 256, 0, st>>>(g, r, q, sc), topx::count_launch());
+  launch_pdl(st, k_residual_inplace<TR, T>, grid1d(g.nnodes(), 256), 256, 0, g, r, q, sc);
   TOPX_CUDA_OK(cudaGetLastError());
 }
 
@@ -639,6 +646,7 @@ __global__ void __launch_bounds__(256) k_jacobi_correct(Grid g, const TR* __rest
                                                         const TD* __restrict__ dinv,
                                                         const uint8_t* __restrict__ present, T* __restrict__ x,
                                                         T omega, PcgScalars* sc, RedScratch rs, int init) {
+  pdl_wait();
   if (sc->done) return;
   const int64_t N = g.nnodes();
   double zr = 0.0;
@@ -670,11 +678,11 @@ void launch_jacobi_correct(cudaStream_t st, Grid g, const TR* r, const T* q, con
                            T* x, double omega, bool dot, bool init, PcgScalars* sc, RedScratch rs) {
   const unsigned nb = grid1d(g.nnodes(), 256, 148 * 8);
   if (dot)
-    (k_jacobi_correct<TR, T, TD, true><<<nb, 256, 0, st>>>(g, r, q, d, present, x, T(omega), sc, rs, init ? 1 : 0),
-     topx::count_launch());
+    launch_pdl(st, k_jacobi_correct<TR, T, TD, true>, nb, 256, 0, g, r, q, d, present, x, T(omega), sc, rs,
+               init ? 1 : 0);
   else
-    (k_jacobi_correct<TR, T, TD, false><<<nb, 256, 0, st>>>(g, r, q, d, present, x, T(omega), sc, rs, init ? 1 : 0),
-     topx::count_launch());
+    launch_pdl(st, k_jacobi_correct<TR, T, TD, false>, nb, 256, 0, g, r, q, d, present, x, T(omega), sc, rs,
+               init ? 1 : 0);
   TOPX_CUDA_OK(cudaGetLastError());
 }
 
@@ -688,6 +696,7 @@ __global__ void __launch_bounds__(256) k_ku_coarse(Grid g, const double* __restr
                                                    const uint8_t* __restrict__ epresent,
                                                    const uint8_t* __restrict__ present, const double* __restrict__ u,
                                                    double* __restrict__ y, const PcgScalars* sc) {
+  pdl_wait();
   if (sc->done) return;
   const int64_t N = g.nnodes();
   const int nny = g.ny + 1, nnx = g.nx + 1;
@@ -723,7 +732,7 @@ __global__ void __launch_bounds__(256) k_ku_coarse(Grid g, const double* __restr
 }
 void launch_ku_coarse(cudaStream_t st, Grid g, const double* Ks, const uint8_t* epresent, const uint8_t* present,
                       const double* u, double* y, const PcgScalars* sc) {
-  (k_ku_coarse<<<grid1d(g.nnodes(), 256), 256, 0, st>>>(g, Ks, epresent, present, u, y, sc), topx::count_launch());
+  launch_pdl(st, k_ku_coarse, grid1d(g.nnodes(), 256), 256, 0, g, Ks, epresent, present, u, y, sc);
   TOPX_CUDA_OK(cudaGetLastError());
 }
 
@@ -732,12 +741,13 @@ void launch_ku_coarse(cudaStream_t st, Grid g, const double* Ks, const uint8_t* 
 // ---------------------------------------------------------------------------
 template <typename TA, typename TB>
 __global__ void k_convert(const TA* __restrict__ a, TB* __restrict__ b, int64_t n) {
+  pdl_wait();
   for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x)
     b[i] = TB(a[i]);
 }
 template <typename TA, typename TB>
 void launch_convert(cudaStream_t st, const TA* a, TB* b, int64_t n) {
-  (k_convert<TA, TB><<<grid1d(n, 256), 256, 0, st>>>(a, b, n), topx::count_launch());
+  launch_pdl(st, k_convert<TA, TB>, grid1d(n, 256), 256, 0, a, b, n);
   TOPX_CUDA_OK(cudaGetLastError());
 }
 
@@ -745,6 +755,7 @@ void launch_convert(cudaStream_t st, const TA* a, TB* b, int64_t n) {
 template <typename T>
 __global__ void k_c2g_nodes(const double* __restrict__ src, T* __restrict__ dst, Grid g,
                             const int32_t* __restrict__ nmb0, int64_t nn) {
+  pdl_wait();
   for (int64_t k = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; k < nn; k += int64_t(gridDim.x) * blockDim.x) {
     const int64_t n = nmb0[k];
     for (int c = 0; c < 3; ++c) dst[n + c * g.stride] = T(src[3 * k + c]);
@@ -753,12 +764,13 @@ __global__ void k_c2g_nodes(const double* __restrict__ src, T* __restrict__ dst,
 template <typename T>
 void launch_compact_to_grid_nodes(cudaStream_t st, const double* src, T* dst, Grid g, const int32_t* nodMapBack0,
                                   int64_t numNodes) {
-  (k_c2g_nodes<T><<<grid1d(numNodes, 256), 256, 0, st>>>(src, dst, g, nodMapBack0, numNodes), topx::count_launch());
+  launch_pdl(st, k_c2g_nodes<T>, grid1d(numNodes, 256), 256, 0, src, dst, g, nodMapBack0, numNodes);
   TOPX_CUDA_OK(cudaGetLastError());
 }
 template <typename T>
 __global__ void k_g2c_nodes(const T* __restrict__ src, double* __restrict__ dst, Grid g,
                             const int32_t* __restrict__ nmb0, int64_t nn) {
+  pdl_wait();
   for (int64_t k = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; k < nn; k += int64_t(gridDim.x) * blockDim.x) {
     const int64_t n = nmb0[k];
     for (int c = 0; c < 3; ++c) dst[3 * k + c] = double(src[n + c * g.stride]);
@@ -767,7 +779,7 @@ __global__ void k_g2c_nodes(const T* __restrict__ src, double* __restrict__ dst,
 template <typename T>
 void launch_grid_to_compact_nodes(cudaStream_t st, const T* src, double* dst, Grid g, const int32_t* nodMapBack0,
                                   int64_t numNodes) {
-  (k_g2c_nodes<T><<<grid1d(numNodes, 256), 256, 0, st>>>(src, dst, g, nodMapBack0, numNodes), topx::count_launch());
+  launch_pdl(st, k_g2c_nodes<T>, grid1d(numNodes, 256), 256, 0, src, dst, g, nodMapBack0, numNodes);
   TOPX_CUDA_OK(cudaGetLastError());
 }
 
@@ -775,6 +787,7 @@ void launch_grid_to_compact_nodes(cudaStream_t st, const T* src, double* dst, Gr
 __global__ void k_simp_scatter(const double* __restrict__ x, const int32_t* __restrict__ emb0, int64_t Ne,
                                double Emin, double E0, double penal, double* __restrict__ Ed,
                                float* __restrict__ Ef) {
+  pdl_wait();
   for (int64_t e = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; e < Ne; e += int64_t(gridDim.x) * blockDim.x) {
     const double v = Emin + pow(x[e], penal) * (E0 - Emin);
     const int64_t k = emb0[e];
@@ -784,7 +797,7 @@ __global__ void k_simp_scatter(const double* __restrict__ x, const int32_t* __re
 }
 void launch_simp_scatter(cudaStream_t st, const double* xPhys, const int32_t* eleMapBack0, int64_t Ne, double Emin,
                          double E0, double penal, double* Ed, float* Ef) {
-  (k_simp_scatter<<<grid1d(Ne, 256), 256, 0, st>>>(xPhys, eleMapBack0, Ne, Emin, E0, penal, Ed, Ef), topx::count_launch());
+  launch_pdl(st, k_simp_scatter, grid1d(Ne, 256), 256, 0, xPhys, eleMapBack0, Ne, Emin, E0, penal, Ed, Ef);
   TOPX_CUDA_OK(cudaGetLastError());
 }
 
@@ -792,6 +805,7 @@ void launch_simp_scatter(cudaStream_t st, const double* xPhys, const int32_t* el
 // unmodified Ke, one thread per element (compact order), FP64.
 __global__ void k_unit_compliance(Grid g, const double* __restrict__ U, const int32_t* __restrict__ emb0,
                                   int64_t Ne, double w, int acc, double* __restrict__ ce) {
+  pdl_wait();
   const int nny = g.ny + 1, nnx = g.nx + 1;
   for (int64_t e = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; e < Ne; e += int64_t(gridDim.x) * blockDim.x) {
     const int64_t id = emb0[e];  // the index of its lowest node
@@ -816,8 +830,7 @@ __global__ void k_unit_compliance(Grid g, const double* __restrict__ U, const in
 }
 void launch_unit_compliance(cudaStream_t st, Grid g, const double* U, const int32_t* eleMapBack0, int64_t Ne,
                             double weight, bool accumulate, double* ce) {
-  (k_unit_compliance<<<grid1d(Ne, 128), 128, 0, st>>>(g, U, eleMapBack0, Ne, weight, accumulate ? 1 : 0, ce),
-   topx::count_launch());
+  launch_pdl(st, k_unit_compliance, grid1d(Ne, 128), 128, 0, g, U, eleMapBack0, Ne, weight, accumulate ? 1 : 0, ce);
   TOPX_CUDA_OK(cudaGetLastError());
 }
 
@@ -857,13 +870,14 @@ namespace topx {
 // TOP3D_XL.m:94-104 uses repmat(modulus_) rather than SIMP(1).
 __global__ void k_fill_scatter(const int32_t* __restrict__ emb0, int64_t Ne, double val, double* __restrict__ Ed,
                                float* __restrict__ Ef) {
+  pdl_wait();
   for (int64_t e = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; e < Ne; e += int64_t(gridDim.x) * blockDim.x) {
     Ed[emb0[e]] = val;
     if (Ef) Ef[emb0[e]] = float(val);
   }
 }
 void launch_fill_scatter(cudaStream_t st, const int32_t* eleMapBack0, int64_t Ne, double val, double* Ed, float* Ef) {
-  (k_fill_scatter<<<grid1d(Ne, 256), 256, 0, st>>>(eleMapBack0, Ne, val, Ed, Ef), topx::count_launch());
+  launch_pdl(st, k_fill_scatter, grid1d(Ne, 256), 256, 0, eleMapBack0, Ne, val, Ed, Ef);
   TOPX_CUDA_OK(cudaGetLastError());
 }
 

@@ -17,6 +17,23 @@ struct CudaError : std::runtime_error {
                            " (" + expr + ")"),
         code(e) {}
 };
+// Launch of a kernel that begins with pdl_wait(): its start overlaps the end of the launch before it.
+template <typename... P, typename... A>
+void launch_pdl(cudaStream_t st, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, A&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+  if (e != cudaSuccess) throw CudaError(e, "cudaLaunchKernelEx", __FILE__, __LINE__);
+  count_launch();
+}
 // A bounded device wait gave up (its poll limit ran out); the engine has cleared the error word
 // and stays usable.
 struct DeviceWaitError : std::runtime_error {

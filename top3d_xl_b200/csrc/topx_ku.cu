@@ -97,6 +97,10 @@ __device__ __forceinline__ T* at(T* base, uint32_t bytes) {
   return reinterpret_cast<T*>(reinterpret_cast<C*>(base) + bytes);
 }
 
+__device__ __forceinline__ void tma_prefetch(const CUtensorMap* map) {
+  asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory");
+}
+
 // Maps of the arrays that a launch reads through TMA, and the places of their boxes in a stage
 struct KuMaps {
   CUtensorMap a, E, p, y, D;  // u, z or r; (PCG) p_in, y; (fused) the Jacobi diagonal
@@ -264,11 +268,17 @@ __global__ void __launch_bounds__(KU_NT, KU_CTAS)
     if (MODE == KU_FUSED && zp % KU_SPAN == 0) issue_coarse(zp / KU_SPAN + 1);
   };
   if (t == 0) {
+    tma_prefetch(&maps.a);
+    tma_prefetch(&maps.E);
+    if (PCG) tma_prefetch(&maps.p);
+    if (PCG) tma_prefetch(&maps.y);
+    if (MODE == KU_FUSED) tma_prefetch(&maps.D);
     mbar_init(&sm.bar[0]);
     mbar_init(&sm.bar[1]);
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
   __syncthreads();
+  pdl_wait();
   if (MODE == KU_FUSED) {
     for (int Z = 0; Z < 3; ++Z) issue_coarse(Zfirst + Z);
   }
@@ -636,7 +646,7 @@ static void launch(cudaStream_t st, const KuArgs& a, dim3 grd) {
   }
   sg.len = at;
   const size_t smem = sizeof(double) * 2 * size_t(at) + sizeof(KuSmem<MODE>);
-  (k_ku<MODE, TC><<<grd, KU_NT, smem, st>>>(a, m, sg, unsigned(8 * used)), topx::count_launch());
+  launch_pdl(st, k_ku<MODE, TC>, grd, KU_NT, smem, a, m, sg, unsigned(8 * used));
 }
 void launch_ku(cudaStream_t st, KuMode mode, const KuArgs& args, int ntiles) {
   const dim3 grd = args.active ? dim3(unsigned(ntiles)) : args.sh.grid;

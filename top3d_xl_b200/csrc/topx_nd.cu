@@ -65,6 +65,7 @@ __device__ __forceinline__ void nd_stage_transposed(double* s, const double* g, 
 // ---------------------------------------------------------------------------
 __global__ void k_nd_assemble(Grid g, const NDFront* __restrict__ fronts, const NDAsm* __restrict__ asmb, int64_t n,
                               const double* __restrict__ Ks, double* __restrict__ pool) {
+  pdl_wait();
   const int nny = g.ny + 1, nnx = g.nx + 1;
   for (int64_t t = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; t < n; t += int64_t(gridDim.x) * blockDim.x) {
     const NDAsm e = asmb[t];
@@ -93,6 +94,7 @@ __global__ void k_nd_assemble(Grid g, const NDFront* __restrict__ fronts, const 
 }
 
 __global__ void k_nd_pad(const int64_t* __restrict__ at, int64_t n, double* __restrict__ pool) {
+  pdl_wait();
   for (int64_t t = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; t < n; t += int64_t(gridDim.x) * blockDim.x)
     pool[at[t]] = 1.0;
 }
@@ -105,6 +107,7 @@ __global__ void __launch_bounds__(ND_THREADS) k_nd_extend(const NDFront* __restr
                                                           const NDTask* __restrict__ tasks,
                                                           const int32_t* __restrict__ upd_map,
                                                           double* __restrict__ pool) {
+  pdl_wait();
   const NDTask tk = tasks[blockIdx.x];
   const NDFront c = fronts[tk.f];
   const NDFront d = fronts[c.parent];
@@ -157,6 +160,7 @@ __device__ __forceinline__ void nd_pivot_acc(double (&acc)[4][2][2], double* A, 
 __global__ void __launch_bounds__(ND_THREADS) k_nd_pivot(const NDFront* __restrict__ fronts,
                                                          const NDTask* __restrict__ tasks, int npiv,
                                                          double* __restrict__ pool, double* __restrict__ scr) {
+  pdl_wait();
   extern __shared__ __align__(16) double nd_smem[];
   const NDTask tk = tasks[blockIdx.x];
   const NDFront d = fronts[tk.f];
@@ -176,6 +180,7 @@ __global__ void __launch_bounds__(ND_THREADS) k_nd_pivot(const NDFront* __restri
 __global__ void __launch_bounds__(ND_THREADS) k_nd_panel(const NDFront* __restrict__ fronts,
                                                          const NDTask* __restrict__ tasks, int npan, int k,
                                                          double* __restrict__ pool, double* __restrict__ scr) {
+  pdl_wait();
   extern __shared__ __align__(16) double nd_smem[];
   const NDTask tk = tasks[blockIdx.x];
   const NDFront d = fronts[tk.f];
@@ -207,6 +212,7 @@ __global__ void __launch_bounds__(ND_THREADS) k_nd_panel(const NDFront* __restri
 __global__ void __launch_bounds__(ND_THREADS) k_nd_update(const NDFront* __restrict__ fronts,
                                                           const NDTask* __restrict__ tasks, int k,
                                                           double* __restrict__ pool, double* __restrict__ scr) {
+  pdl_wait();
   extern __shared__ __align__(16) double nd_smem[];
   double* bufA = nd_smem;
   double* bufB = nd_smem + GF_BUF;
@@ -514,6 +520,7 @@ __device__ __forceinline__ bool nd_backward_task(const NDSolveArgs<T, TM>& a, co
 // one launch per tree level and direction
 template <typename T, typename TM, bool FWD>
 __global__ void __launch_bounds__(ND_THREADS) k_nd_solve_level(NDSolveArgs<T, TM> a, const PcgScalars* sc) {
+  pdl_wait();
   if (sc && sc->done) return;
   __shared__ NDSolveSmem sm;
   if (FWD)
@@ -532,6 +539,7 @@ __global__ void __launch_bounds__(ND_THREADS) k_nd_solve_level(NDSolveArgs<T, TM
 template <typename T, typename TM>
 __global__ void __launch_bounds__(ND_THREADS) k_nd_solve_flow(NDSolveArgs<T, TM> a, int64_t nfwd, int64_t ntot,
                                                               NDFlow fl, int nfronts, const PcgScalars* sc) {
+  pdl_wait();
   if (sc && sc->done) return;  // the same for every CTA
   __shared__ NDSolveSmem sm;
   for (int64_t t = blockIdx.x; t < ntot; t += gridDim.x) {
@@ -558,6 +566,7 @@ __global__ void __launch_bounds__(ND_THREADS) k_nd_solve_flow(NDSolveArgs<T, TM>
 
 // one CTA waits for a counter that nothing raises
 __global__ void k_coop_wait_selftest(CoopControl* ctl) {
+  pdl_wait();
   if (threadIdx.x == 0) coop_wait_count(&ctl->idle, 1u, ctl);
 }
 
@@ -583,33 +592,31 @@ void prepare_nd_kernels() {
 void NDDevice::factor(cudaStream_t st, const NDPlan& P, Grid g, const double* Ks) const {
   TOPX_CUDA_OK(cudaMemsetAsync(pool, 0, sizeof(double) * size_t(P.ntiles) * ND_TILE, st));
   const int64_t na = int64_t(P.asmb.size()), np = int64_t(P.pad_diag.size());
-  (k_nd_assemble<<<nd_grid(na, 256), 256, 0, st>>>(g, fronts, asmb, na, Ks, pool), topx::count_launch());
-  if (np) (k_nd_pad<<<nd_grid(np, 256), 256, 0, st>>>(pad, np, pool), topx::count_launch());
+  launch_pdl(st, k_nd_assemble, nd_grid(na, 256), 256, 0, g, fronts, asmb, na, Ks, pool);
+  if (np) launch_pdl(st, k_nd_pad, nd_grid(np, 256), 256, 0, pad, np, pool);
   for (int l = int(P.levels.size()) - 1; l >= 0; --l) {
     const NDLevel& L = P.levels[size_t(l)];
     for (int s = 0; s < 2; ++s) {
       const int64_t n = L.ext[s + 1] - L.ext[s];
-      if (n) (k_nd_extend<<<unsigned(n), ND_THREADS, 0, st>>>(fronts, tasks + L.ext[s], upd_map, pool), topx::count_launch());
+      if (n) launch_pdl(st, k_nd_extend, unsigned(n), ND_THREADS, 0, fronts, tasks + L.ext[s], upd_map, pool);
     }
     const int64_t npiv0 = L.piv0[1] - L.piv0[0];
     if (npiv0)
-      (k_nd_pivot<<<unsigned(npiv0), ND_THREADS, ND_SMEM_SWEEP, st>>>(fronts, tasks + L.piv0[0], int(npiv0), pool, scr),
-       topx::count_launch());
+      launch_pdl(st, k_nd_pivot, unsigned(npiv0), ND_THREADS, ND_SMEM_SWEEP, fronts, tasks + L.piv0[0], int(npiv0),
+                 pool, scr);
     for (int k = 0; k < L.maxT1; ++k) {
       const int64_t* s = &L.step[size_t(4) * k];
       const int64_t npan = s[1] - s[0], nfin = s[2] - s[1], nupd = s[3] - s[2];
       if (npan + nfin)
-        (k_nd_panel<<<unsigned(npan + nfin), ND_THREADS, ND_SMEM_SWEEP, st>>>(fronts, tasks + s[0], int(npan), k, pool,
-                                                                             scr),
-         topx::count_launch());
+        launch_pdl(st, k_nd_panel, unsigned(npan + nfin), ND_THREADS, ND_SMEM_SWEEP, fronts, tasks + s[0], int(npan),
+                   k, pool, scr);
       if (nupd)
-        (k_nd_update<<<unsigned(nupd), ND_THREADS, ND_SMEM_SWEEP, st>>>(fronts, tasks + s[2], k, pool, scr),
-         topx::count_launch());
+        launch_pdl(st, k_nd_update, unsigned(nupd), ND_THREADS, ND_SMEM_SWEEP, fronts, tasks + s[2], k, pool, scr);
     }
     const int64_t nfin = L.fin_last[1] - L.fin_last[0];
     if (nfin)
-      (k_nd_pivot<<<unsigned(nfin), ND_THREADS, ND_SMEM_SWEEP, st>>>(fronts, tasks + L.fin_last[0], 0, pool, scr),
-       topx::count_launch());
+      launch_pdl(st, k_nd_pivot, unsigned(nfin), ND_THREADS, ND_SMEM_SWEEP, fronts, tasks + L.fin_last[0], 0, pool,
+                 scr);
   }
   TOPX_CUDA_OK(cudaGetLastError());
 }
@@ -642,13 +649,13 @@ void NDDevice::solve(cudaStream_t st, const NDPlan& P, const TM* tiles, const T*
   for (int l = nlev - 1; l >= 0; --l) {
     const NDLevel& L = P.levels[size_t(l)];
     a.tasks = tasks + L.fwd[0];
-    (k_nd_solve_level<T, TM, true><<<unsigned(L.fwd[1] - L.fwd[0]), ND_THREADS, 0, st>>>(a, sc), topx::count_launch());
+    launch_pdl(st, k_nd_solve_level<T, TM, true>, unsigned(L.fwd[1] - L.fwd[0]), ND_THREADS, 0, a, sc);
   }
   for (int l = 0; l < nlev; ++l) {
     const NDLevel& L = P.levels[size_t(l)];
     a.tasks = tasks + L.bwd[0];
     if (L.bwd[1] > L.bwd[0])
-      (k_nd_solve_level<T, TM, false><<<unsigned(L.bwd[1] - L.bwd[0]), ND_THREADS, 0, st>>>(a, sc), topx::count_launch());
+      launch_pdl(st, k_nd_solve_level<T, TM, false>, unsigned(L.bwd[1] - L.bwd[0]), ND_THREADS, 0, a, sc);
   }
   TOPX_CUDA_OK(cudaGetLastError());
 }
@@ -666,7 +673,7 @@ int nd_solve_coop_ctas() {
 }
 
 void launch_coop_wait_selftest(cudaStream_t st, CoopControl* ctl) {
-  (k_coop_wait_selftest<<<1, 32, 0, st>>>(ctl), topx::count_launch());
+  launch_pdl(st, k_coop_wait_selftest, 1, 32, 0, ctl);
   TOPX_CUDA_OK(cudaGetLastError());
 }
 

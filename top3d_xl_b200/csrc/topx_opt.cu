@@ -32,6 +32,7 @@ template FilterKe<float> filter_ke<float>(const double*);
 template <typename T>
 __global__ void k_filter_e2n(Grid g, const T* __restrict__ srcE, T* __restrict__ node, FastDiv dny, FastDiv dnx,
                              const uint32_t* __restrict__ act) {
+  pdl_wait();
   const uint32_t N = uint32_t(g.nnodes());  // < 2^32 (checked at launch)
   const uint32_t nny = uint32_t(g.ny + 1), nnx = uint32_t(g.nx + 1);
   for (uint32_t n = blockIdx.x * blockDim.x + threadIdx.x; n < N; n += gridDim.x * blockDim.x) {
@@ -52,13 +53,14 @@ template <typename T>
 void launch_filter_e2n(cudaStream_t st, Grid g, const T* srcE, T* node, const uint32_t* act) {
   if (g.nnodes() >= (int64_t(1) << 32)) throw std::runtime_error("grid too large for 32-bit node indices");
   const FastDiv dny{uint32_t(g.ny + 1)}, dnx{uint32_t(g.nx + 1)};
-  (k_filter_e2n<T><<<grid1d(g.nnodes(), 256), 256, 0, st>>>(g, srcE, node, dny, dnx, act), topx::count_launch());
+  launch_pdl(st, k_filter_e2n<T>, grid1d(g.nnodes(), 256), 256, 0, g, srcE, node, dny, dnx, act);
   TOPX_CUDA_OK(cudaGetLastError());
 }
 
 // Jacobi preconditioner 1/diag (TOP3D_XL.m:855-867); 0 on absent nodes
 template <typename T>
 __global__ void k_filter_diag(Grid g, const uint8_t* __restrict__ solid, const FilterKe<double> kf, T* __restrict__ dp) {
+  pdl_wait();
   const int64_t N = g.nnodes();
   const int nny = g.ny + 1, nnx = g.nx + 1;
   for (int64_t n = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; n < N; n += int64_t(gridDim.x) * blockDim.x) {
@@ -74,7 +76,7 @@ __global__ void k_filter_diag(Grid g, const uint8_t* __restrict__ solid, const F
 }
 template <typename T>
 void launch_filter_diag(cudaStream_t st, Grid g, const uint8_t* solid, const FilterKe<double>& kf, T* dp) {
-  (k_filter_diag<T><<<grid1d(g.nnodes(), 256), 256, 0, st>>>(g, solid, kf, dp), topx::count_launch());
+  launch_pdl(st, k_filter_diag<T>, grid1d(g.nnodes(), 256), 256, 0, g, solid, kf, dp);
   TOPX_CUDA_OK(cudaGetLastError());
 }
 
@@ -89,6 +91,7 @@ __global__ void __launch_bounds__(FNT) k_filter_ku(Grid g, int zc, const FilterK
                                                     const T* __restrict__ zin, T* __restrict__ out,
                                                     const uint8_t* __restrict__ solid, PcgScalars* sc, RedScratch rs,
                                                     const uint32_t* __restrict__ active) {
+  pdl_wait();
   if (MODE != KU_PLAIN && sc->done) return;
   __shared__ T su[3][FKX + 2][FKY + 2];
   __shared__ T ss[2][FKX + 1][FKY + 1];
@@ -226,11 +229,9 @@ void launch_filter_ku(cudaStream_t st, KuMode mode, Grid g, const FilterKe<T>& k
   const dim3 grd = tiles.list ? dim3(unsigned(tiles.n)) : f.grd;
   if (grd.x == 0) return;
   if (mode == KU_PLAIN)
-    (k_filter_ku<T, KU_PLAIN><<<grd, blk, 0, st>>>(g, f.zc, kf, in, z, out, solid, sc, rs, tiles.list),
-     topx::count_launch());
+    launch_pdl(st, k_filter_ku<T, KU_PLAIN>, grd, blk, 0, g, f.zc, kf, in, z, out, solid, sc, rs, tiles.list);
   else
-    (k_filter_ku<T, KU_P_UPDATE><<<grd, blk, 0, st>>>(g, f.zc, kf, in, z, out, solid, sc, rs, tiles.list),
-     topx::count_launch());
+    launch_pdl(st, k_filter_ku<T, KU_P_UPDATE>, grd, blk, 0, g, f.zc, kf, in, z, out, solid, sc, rs, tiles.list);
   TOPX_CUDA_OK(cudaGetLastError());
 }
 
@@ -239,6 +240,7 @@ template <typename T>
 __global__ void k_filter_init(Grid g, const T* __restrict__ b, const T* __restrict__ dp, T* __restrict__ r,
                               T* __restrict__ z, T* __restrict__ y, PcgScalars* sc, RedScratch rs, double tol,
                               int maxIT, const uint32_t* __restrict__ act) {
+  pdl_wait();
   const int64_t N = g.nnodes();
   double bb = 0.0, zr = 0.0;
   for (int64_t n = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; n < N; n += int64_t(gridDim.x) * blockDim.x) {
@@ -266,8 +268,7 @@ __global__ void k_filter_init(Grid g, const T* __restrict__ b, const T* __restri
 template <typename T>
 void launch_filter_residual_init(cudaStream_t st, Grid g, const T* b, const T* dp, T* r, T* z, T* y, PcgScalars* sc,
                                  RedScratch rs, double tol, int maxIT, const uint32_t* act) {
-  (k_filter_init<T><<<grid1d(g.nnodes(), 256), 256, 0, st>>>(g, b, dp, r, z, y, sc, rs, tol, maxIT, act),
-   topx::count_launch());
+  launch_pdl(st, k_filter_init<T>, grid1d(g.nnodes(), 256), 256, 0, g, b, dp, r, z, y, sc, rs, tol, maxIT, act);
   TOPX_CUDA_OK(cudaGetLastError());
 }
 
@@ -276,6 +277,7 @@ template <typename T>
 __global__ void k_filter_update(Grid g, T* __restrict__ y, T* __restrict__ p, T* __restrict__ r,
                                 const T* __restrict__ q, const T* __restrict__ dp, T* __restrict__ z, PcgScalars* sc,
                                 RedScratch rs, const uint32_t* __restrict__ act) {
+  pdl_wait();
   if (sc->done) return;
   const bool first = sc->first;
   const T beta = T(sc->beta);
@@ -314,7 +316,7 @@ __global__ void k_filter_update(Grid g, T* __restrict__ y, T* __restrict__ p, T*
 template <typename T>
 void launch_filter_update(cudaStream_t st, Grid g, T* y, T* p, T* r, const T* q, const T* dp, T* z, PcgScalars* sc,
                           RedScratch rs, const uint32_t* act) {
-  (k_filter_update<T><<<grid1d(g.nnodes(), 256), 256, 0, st>>>(g, y, p, r, q, dp, z, sc, rs, act), topx::count_launch());
+  launch_pdl(st, k_filter_update<T>, grid1d(g.nnodes(), 256), 256, 0, g, y, p, r, q, dp, z, sc, rs, act);
   TOPX_CUDA_OK(cudaGetLastError());
 }
 
@@ -322,6 +324,7 @@ void launch_filter_update(cudaStream_t st, Grid g, T* y, T* p, T* r, const T* q,
 template <typename T>
 __global__ void k_filter_n2e(Grid g, const T* __restrict__ node, const int32_t* __restrict__ emb0, int64_t Ne,
                              double* __restrict__ out) {
+  pdl_wait();
   const int nny = g.ny + 1, nnx = g.nx + 1;
   for (int64_t e = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; e < Ne; e += int64_t(gridDim.x) * blockDim.x) {
     const int64_t id = emb0[e];  // the index of its lowest node
@@ -334,19 +337,20 @@ __global__ void k_filter_n2e(Grid g, const T* __restrict__ node, const int32_t* 
 }
 template <typename T>
 void launch_filter_n2e(cudaStream_t st, Grid g, const T* node, const int32_t* eleMapBack0, int64_t Ne, double* out) {
-  (k_filter_n2e<T><<<grid1d(Ne, 256), 256, 0, st>>>(g, node, eleMapBack0, Ne, out), topx::count_launch());
+  launch_pdl(st, k_filter_n2e<T>, grid1d(Ne, 256), 256, 0, g, node, eleMapBack0, Ne, out);
   TOPX_CUDA_OK(cudaGetLastError());
 }
 
 template <typename T>
 __global__ void k_scatter_elems(const double* __restrict__ src, const int32_t* __restrict__ emb0, int64_t Ne,
                                 T* __restrict__ dst) {
+  pdl_wait();
   for (int64_t e = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; e < Ne; e += int64_t(gridDim.x) * blockDim.x)
     dst[emb0[e]] = T(src[e]);
 }
 template <typename T>
 void launch_scatter_elems_t(cudaStream_t st, const double* src, const int32_t* eleMapBack0, int64_t Ne, T* dstE) {
-  (k_scatter_elems<T><<<grid1d(Ne, 256), 256, 0, st>>>(src, eleMapBack0, Ne, dstE), topx::count_launch());
+  launch_pdl(st, k_scatter_elems<T>, grid1d(Ne, 256), 256, 0, src, eleMapBack0, Ne, dstE);
   TOPX_CUDA_OK(cudaGetLastError());
 }
 
@@ -356,6 +360,7 @@ void launch_scatter_elems_t(cudaStream_t st, const double* src, const int32_t* e
 __global__ void k_objective(int64_t Ne, const double* __restrict__ ce, const double* __restrict__ xPhys, double cSolid,
                             double Emin, double E0, double penal, double* __restrict__ dc, ObjState* os,
                             RedScratch rs) {
+  pdl_wait();
   double sc = 0.0, sv = 0.0;
   const double dsimp = penal * (E0 - Emin);
   for (int64_t e = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; e < Ne; e += int64_t(gridDim.x) * blockDim.x) {
@@ -374,12 +379,13 @@ __global__ void k_objective(int64_t Ne, const double* __restrict__ ce, const dou
 }
 void launch_objective(cudaStream_t st, int64_t Ne, const double* ce, const double* xPhys, double cSolid, double Emin,
                       double E0, double penal, double* dc, ObjState* os, RedScratch rs) {
-  (k_objective<<<grid1d(Ne, 256), 256, 0, st>>>(Ne, ce, xPhys, cSolid, Emin, E0, penal, dc, os, rs), topx::count_launch());
+  launch_pdl(st, k_objective, grid1d(Ne, 256), 256, 0, Ne, ce, xPhys, cSolid, Emin, E0, penal, dc, os, rs);
   TOPX_CUDA_OK(cudaGetLastError());
 }
 
 __global__ void k_dot(int64_t n, const double* __restrict__ a, const double* __restrict__ b, double* out,
                       RedScratch rs) {
+  pdl_wait();
   double s = 0.0;
   for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x)
     s += b ? a[i] * b[i] : a[i];
@@ -387,12 +393,13 @@ __global__ void k_dot(int64_t n, const double* __restrict__ a, const double* __r
   if (reduce_publish<1>(v, rs, tot) && threadIdx.x == 0) *out = tot[0];
 }
 void launch_sum(cudaStream_t st, int64_t n, const double* a, const double* b, double* out, RedScratch rs) {
-  (k_dot<<<grid1d(n, 256), 256, 0, st>>>(n, a, b, out, rs), topx::count_launch());
+  launch_pdl(st, k_dot, grid1d(n, 256), 256, 0, n, a, b, out, rs);
   TOPX_CUDA_OK(cudaGetLastError());
 }
 
 __global__ void k_ewise(int op, int64_t n, const double* __restrict__ a, const double* __restrict__ b,
                         double* __restrict__ out, double s) {
+  pdl_wait();
   for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x) {
     double v;
     switch (op) {
@@ -409,7 +416,7 @@ __global__ void k_ewise(int op, int64_t n, const double* __restrict__ a, const d
   }
 }
 void launch_ewise(cudaStream_t st, int op, int64_t n, const double* a, const double* b, double* out, double s) {
-  (k_ewise<<<grid1d(n, 256), 256, 0, st>>>(op, n, a, b, out, s), topx::count_launch());
+  launch_pdl(st, k_ewise, grid1d(n, 256), 256, 0, op, n, a, b, out, s);
   TOPX_CUDA_OK(cudaGetLastError());
 }
 
@@ -428,11 +435,12 @@ __device__ __forceinline__ double oc_xnew(double x, double w, double r, double m
 
 __global__ void k_oc_prep(int64_t Ne, const double* __restrict__ x, const double* __restrict__ dc,
                           double* __restrict__ w) {
+  pdl_wait();
   for (int64_t e = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; e < Ne; e += int64_t(gridDim.x) * blockDim.x)
     w[e] = x[e] * sqrt(-dc[e]);
 }
 void launch_oc_prep(cudaStream_t st, int64_t Ne, const double* x, const double* dc, double* w) {
-  (k_oc_prep<<<grid1d(Ne, 256), 256, 0, st>>>(Ne, x, dc, w), topx::count_launch());
+  launch_pdl(st, k_oc_prep, grid1d(Ne, 256), 256, 0, Ne, x, dc, w);
   TOPX_CUDA_OK(cudaGetLastError());
 }
 
@@ -454,6 +462,7 @@ constexpr int kOcNodes = (1 << kOcStepsPerLaunch) - 1;
 __global__ void __launch_bounds__(256) k_oc_bisect(int64_t Ne, const double* __restrict__ x,
                                                    const double* __restrict__ w, const uint8_t* __restrict__ passive,
                                                    OcState* os, RedScratch rs, double move) {
+  pdl_wait();
   if (os->converged) return;
   // thread j < kOcNodes forms node j's 1/sqrt(lmid): its interval follows the path from the root
   __shared__ double sr[kOcNodes];
@@ -526,7 +535,7 @@ void launch_oc_bisect(cudaStream_t st, int64_t Ne, const double* x, const double
                       OcState* os, RedScratch rs, double move) {
   const unsigned nb = grid1d(Ne, 256);
   static_assert(size_t(kOcNodes) * 148 * 16 <= size_t(kMaxRedBlocks) * kMaxRedSlots, "reduction slots");
-  (k_oc_bisect<<<nb, 256, 0, st>>>(Ne, x, w, passive, os, rs, move), topx::count_launch());
+  launch_pdl(st, k_oc_bisect, nb, 256, 0, Ne, x, w, passive, os, rs, move);
   TOPX_CUDA_OK(cudaGetLastError());
 }
 
@@ -534,6 +543,7 @@ void launch_oc_bisect(cudaStream_t st, int64_t Ne, const double* x, const double
 __global__ void k_oc_final(int64_t Ne, double* __restrict__ x, const double* __restrict__ w,
                            const uint8_t* __restrict__ passive, double* __restrict__ xPhys, OcState* os,
                            RedScratch rs, RedScratch rs2, double move) {
+  pdl_wait();
   const double lmid = os->lmid;
   const double r = 1.0 / sqrt(lmid);
   double ch = 0.0, sh = 0.0;
@@ -553,7 +563,7 @@ __global__ void k_oc_final(int64_t Ne, double* __restrict__ x, const double* __r
 }
 void launch_oc_final(cudaStream_t st, int64_t Ne, double* x, const double* w, const uint8_t* passive, double* xPhys,
                      OcState* os, RedScratch rs, RedScratch rs2, double move) {
-  (k_oc_final<<<grid1d(Ne, 256), 256, 0, st>>>(Ne, x, w, passive, xPhys, os, rs, rs2, move), topx::count_launch());
+  launch_pdl(st, k_oc_final, grid1d(Ne, 256), 256, 0, Ne, x, w, passive, xPhys, os, rs, rs2, move);
   TOPX_CUDA_OK(cudaGetLastError());
 }
 
@@ -596,6 +606,7 @@ __global__ void k_mma_gensub(int64_t n, int iter, double move, const double* __r
                              double* __restrict__ alpha, double* __restrict__ beta, double* __restrict__ p0,
                              double* __restrict__ q0, double* __restrict__ pij, double* __restrict__ qij,
                              MmaState* ms, RedScratch rs) {
+  pdl_wait();
   double bs = 0.0;
   for (int64_t e = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; e < n; e += int64_t(gridDim.x) * blockDim.x) {
     if (passive && passive[e]) continue;
@@ -658,8 +669,8 @@ void launch_mma_gensub(cudaStream_t st, int64_t n, int iter, double move, const 
                        double* xold1, double* xold2, double* low, double* upp, const double* dfdx, const double* dgdx,
                        double gx, int64_t nact, double* alpha, double* beta, double* p0, double* q0, double* pij,
                        double* qij, MmaState* ms, RedScratch rs) {
-  (k_mma_gensub<<<grid1d(n, 256), 256, 0, st>>>(n, iter, move, xval, passive, xold1, xold2, low, upp, dfdx, dgdx, gx,
-                                                nact, alpha, beta, p0, q0, pij, qij, ms, rs), topx::count_launch());
+  launch_pdl(st, k_mma_gensub, grid1d(n, 256), 256, 0, n, iter, move, xval, passive, xold1, xold2, low, upp, dfdx,
+             dgdx, gx, nact, alpha, beta, p0, q0, pij, qij, ms, rs);
   TOPX_CUDA_OK(cudaGetLastError());
 }
 
@@ -681,6 +692,7 @@ __global__ void k_mma_newton(int64_t n, const uint8_t* __restrict__ passive, con
                              const double* __restrict__ beta, const double* __restrict__ p0,
                              const double* __restrict__ q0, const double* __restrict__ pij,
                              const double* __restrict__ qij, MmaState* ms, RedScratch rs) {
+  pdl_wait();
   if (ms->finished) return;
   const double lam = fmax(ms->lam, 0.0);
   double sg = 0.0, sh = 0.0;
@@ -726,7 +738,7 @@ __global__ void k_mma_newton(int64_t n, const uint8_t* __restrict__ passive, con
 void launch_mma_newton(cudaStream_t st, int64_t n, const uint8_t* passive, const double* low, const double* upp,
                        const double* alpha, const double* beta, const double* p0, const double* q0, const double* pij,
                        const double* qij, MmaState* ms, RedScratch rs) {
-  (k_mma_newton<<<grid1d(n, 256), 256, 0, st>>>(n, passive, low, upp, alpha, beta, p0, q0, pij, qij, ms, rs), topx::count_launch());
+  launch_pdl(st, k_mma_newton, grid1d(n, 256), 256, 0, n, passive, low, upp, alpha, beta, p0, q0, pij, qij, ms, rs);
   TOPX_CUDA_OK(cudaGetLastError());
 }
 
@@ -736,6 +748,7 @@ __global__ void k_mma_residual(int64_t n, const uint8_t* __restrict__ passive, c
                                const double* __restrict__ beta, const double* __restrict__ p0,
                                const double* __restrict__ q0, const double* __restrict__ pij,
                                const double* __restrict__ qij, double* __restrict__ x, MmaState* ms, RedScratch rs) {
+  pdl_wait();
   if (ms->finished) return;
   const double lam = fmax(ms->lam, 0.0);
   double sp = 0.0, sq = 0.0;
@@ -772,13 +785,15 @@ __global__ void k_mma_residual(int64_t n, const uint8_t* __restrict__ passive, c
 void launch_mma_residual(cudaStream_t st, int64_t n, const uint8_t* passive, const double* low, const double* upp,
                          const double* alpha, const double* beta, const double* p0, const double* q0,
                          const double* pij, const double* qij, double* x, MmaState* ms, RedScratch rs) {
-  (k_mma_residual<<<grid1d(n, 256), 256, 0, st>>>(n, passive, low, upp, alpha, beta, p0, q0, pij, qij, x, ms, rs), topx::count_launch());
+  launch_pdl(st, k_mma_residual, grid1d(n, 256), 256, 0, n, passive, low, upp, alpha, beta, p0, q0, pij, qij, x, ms,
+             rs);
   TOPX_CUDA_OK(cudaGetLastError());
 }
 
 // x = xmma on active elements, 1 on passive ones; change = max |xmma - xval| (xval kept in xold1)
 __global__ void k_mma_finish(int64_t n, const uint8_t* __restrict__ passive, const double* __restrict__ xmma,
                              const double* __restrict__ xold1, double* __restrict__ x, MmaState* ms, RedScratch rs) {
+  pdl_wait();
   double ch = 0.0;
   for (int64_t e = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; e < n; e += int64_t(gridDim.x) * blockDim.x) {
     if (passive && passive[e]) {
@@ -794,7 +809,7 @@ __global__ void k_mma_finish(int64_t n, const uint8_t* __restrict__ passive, con
 
 void launch_mma_finish(cudaStream_t st, int64_t n, const uint8_t* passive, const double* xmma, const double* xold1,
                        double* x, MmaState* ms, RedScratch rs) {
-  (k_mma_finish<<<grid1d(n, 256), 256, 0, st>>>(n, passive, xmma, xold1, x, ms, rs), topx::count_launch());
+  launch_pdl(st, k_mma_finish, grid1d(n, 256), 256, 0, n, passive, xmma, xold1, x, ms, rs);
   TOPX_CUDA_OK(cudaGetLastError());
 }
 
@@ -803,6 +818,7 @@ void launch_mma_finish(cudaStream_t st, int64_t n, const uint8_t* passive, const
 // ---------------------------------------------------------------------------
 __global__ void k_pnorm(int64_t Ne, const double* __restrict__ xhat, double Ve0, double pP, double* out,
                         RedScratch rs) {
+  pdl_wait();
   double s = 0.0;
   const double vm = pow(Ve0, pP);
   for (int64_t e = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; e < Ne; e += int64_t(gridDim.x) * blockDim.x)
@@ -812,13 +828,14 @@ __global__ void k_pnorm(int64_t Ne, const double* __restrict__ xhat, double Ve0,
 }
 void launch_pnorm_terms(cudaStream_t st, int64_t Ne, const double* xhat, double Ve0, int pPIO, double* out_sum,
                         RedScratch rs) {
-  (k_pnorm<<<grid1d(Ne, 256), 256, 0, st>>>(Ne, xhat, Ve0, double(pPIO), out_sum, rs), topx::count_launch());
+  launch_pdl(st, k_pnorm, grid1d(Ne, 256), 256, 0, Ne, xhat, Ve0, double(pPIO), out_sum, rs);
   TOPX_CUDA_OK(cudaGetLastError());
 }
 
 __global__ void k_local_sens(int64_t Ne, const double* __restrict__ xhat, const double* __restrict__ xTilde,
                              const double* __restrict__ dc, double Ve0, double pP, double pn, double bt, double eta,
                              double* __restrict__ dfdx_pde, double* __restrict__ dx, double* __restrict__ dcdx) {
+  pdl_wait();
   const double f = pow(pn, 1.0 / pP - 1.0);
   const double vm = pow(Ve0, pP);
   const double den = tanh(bt * eta) + tanh(bt * (1 - eta));
@@ -833,13 +850,14 @@ __global__ void k_local_sens(int64_t Ne, const double* __restrict__ xhat, const 
 void launch_local_sens(cudaStream_t st, int64_t Ne, const double* xhat, const double* xTilde, const double* dc,
                        double Ve0, int pPIO, double pn, double betaPIO, double etaPIO, double* dfdx_pde, double* dx,
                        double* dcdx) {
-  (k_local_sens<<<grid1d(Ne, 256), 256, 0, st>>>(Ne, xhat, xTilde, dc, Ve0, double(pPIO), pn, betaPIO, etaPIO,
-                                                dfdx_pde, dx, dcdx), topx::count_launch());
+  launch_pdl(st, k_local_sens, grid1d(Ne, 256), 256, 0, Ne, xhat, xTilde, dc, Ve0, double(pPIO), pn, betaPIO, etaPIO,
+             dfdx_pde, dx, dcdx);
   TOPX_CUDA_OK(cudaGetLastError());
 }
 
 __global__ void k_heaviside(int64_t Ne, const double* __restrict__ xTilde, const uint8_t* __restrict__ passive,
                             double bt, double eta, double* __restrict__ xPhys, double* sharpsum, RedScratch rs) {
+  pdl_wait();
   const double a = tanh(bt * eta), den = tanh(bt * eta) + tanh(bt * (1 - eta));
   double s = 0.0;
   for (int64_t e = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; e < Ne; e += int64_t(gridDim.x) * blockDim.x) {
@@ -853,7 +871,7 @@ __global__ void k_heaviside(int64_t Ne, const double* __restrict__ xTilde, const
 }
 void launch_heaviside(cudaStream_t st, int64_t Ne, const double* xTilde, const uint8_t* passive, double betaPIO,
                       double etaPIO, double* xPhys, double* sharpsum, RedScratch rs) {
-  (k_heaviside<<<grid1d(Ne, 256), 256, 0, st>>>(Ne, xTilde, passive, betaPIO, etaPIO, xPhys, sharpsum, rs), topx::count_launch());
+  launch_pdl(st, k_heaviside, grid1d(Ne, 256), 256, 0, Ne, xTilde, passive, betaPIO, etaPIO, xPhys, sharpsum, rs);
   TOPX_CUDA_OK(cudaGetLastError());
 }
 
