@@ -329,7 +329,7 @@ Engine::Engine(Model& model, int precision, int device, bool coarse_coop) : M(mo
   TOPX_CUDA_OK(cudaMallocHost(&h_ctl, sizeof(CoopControl)));
   h_ctl->err = 0;
   // ---- optimiser state -------------------------------------------------------
-  for (DevBuf<double>* b : {&x, &xPhys, &dc, &ce, &tmpA, &tmpB, &xTilde, &xhat, &dfdx, &dxv, &volMax})
+  for (DevBuf<double>* b : {&x, &xPhys, &dc, &ce, &tmpA, &tmpB, &xTilde, &xhat, &dfdx, &dxv})
     b->alloc(size_t(Ne));
   int64_t npas = 0;
   for (auto e : M.passiveElements) npas += (e >= 1 && e <= Ne) ? 1 : 0;
@@ -425,8 +425,17 @@ void Engine::check_coop_waits() {
 }
 
 void Engine::copy_sync(void* dst, const void* src, size_t bytes, cudaMemcpyKind kind) const {
-  TOPX_CUDA_OK(cudaMemcpyAsync(dst, src, bytes, kind, st));
-  TOPX_CUDA_OK(cudaStreamSynchronize(st));
+  if (kind == cudaMemcpyHostToDevice)
+    host_to_device(dst, src, bytes, st);
+  else
+    device_to_host(dst, src, bytes, st);
+}
+
+// The device side of a host vector over the compact DOFs, kept for the next call (an engine that only runs
+// designs never makes it).
+double* Engine::host_vector() {
+  if (!hostVec.p) hostVec.alloc(size_t(Nn) * 3, false);
+  return hostVec.p;
 }
 
 // The persistent coarse solve's dependency waits and the K*u's waits for its copies set an error word instead
@@ -463,29 +472,17 @@ void Engine::selftest_wait(int which) {
 // ---------------------------------------------------------------------------
 // design state
 // ---------------------------------------------------------------------------
-void Engine::set_xphys(const double* h) {
-  TOPX_CUDA_OK(cudaStreamSynchronize(st));
-  copy_sync(xPhys.p, h, sizeof(double) * Ne, cudaMemcpyHostToDevice);
+void Engine::set_xphys(const double* h) { copy_sync(xPhys.p, h, sizeof(double) * Ne, cudaMemcpyHostToDevice); }
+void Engine::get_xphys(double* h) const { copy_sync(h, xPhys.p, sizeof(double) * Ne, cudaMemcpyDeviceToHost); }
+void Engine::get_U(int lc, double* h) {
+  double* v = host_vector();
+  launch_grid_to_compact_nodes<double>(st, U[lc].p, v, G[0], nodMapBack0.p, Nn);
+  copy_sync(h, v, sizeof(double) * Nn * 3, cudaMemcpyDeviceToHost);
 }
-void Engine::get_xphys(double* h) const {
-  TOPX_CUDA_OK(cudaStreamSynchronize(st));
-  copy_sync(h, xPhys.p, sizeof(double) * Ne, cudaMemcpyDeviceToHost);
-}
-void Engine::get_U(int lc, double* h) const {
-  TOPX_CUDA_OK(cudaStreamSynchronize(st));
-  DevBuf<double> tmp;
-  tmp.alloc(size_t(Nn) * 3);
-  launch_grid_to_compact_nodes<double>(st, U[lc].p, tmp.p, G[0], nodMapBack0.p, Nn);
-  TOPX_CUDA_OK(cudaStreamSynchronize(st));
-  copy_sync(h, tmp.p, sizeof(double) * Nn * 3, cudaMemcpyDeviceToHost);
-}
-void Engine::set_U(int lc, const double* h) {
-  TOPX_CUDA_OK(cudaStreamSynchronize(st));
-  DevBuf<double> tmp;
-  tmp.upload(h, size_t(Nn) * 3);
-  TOPX_CUDA_OK(cudaMemsetAsync(U[lc].p, 0, U[lc].bytes(), st));
-  launch_compact_to_grid_nodes<double>(st, tmp.p, U[lc].p, G[0], nodMapBack0.p, Nn);
-  TOPX_CUDA_OK(cudaStreamSynchronize(st));
+void Engine::set_U(int lc, const double* h) {  // absent nodes hold zero and stay so
+  double* v = host_vector();
+  copy_sync(v, h, sizeof(double) * Nn * 3, cudaMemcpyHostToDevice);
+  launch_compact_to_grid_nodes<double>(st, v, U[lc].p, G[0], nodMapBack0.p, Nn);
 }
 
 void Engine::update_moduli(const double* d_xPhys, bool solid) {
@@ -830,34 +827,28 @@ int Engine::filter(int slot, const double* d_src, double* d_out) {
 // test entry points
 // ---------------------------------------------------------------------------
 void Engine::apply_K(const double* h_u, double* h_y) {
-  TOPX_CUDA_OK(cudaStreamSynchronize(st));
-  DevBuf<double> cu, du;
-  cu.upload(h_u, size_t(Nn) * 3);
-  du.alloc(size_t(G[0].stride) * 3);
-  launch_compact_to_grid_nodes<double>(st, cu.p, du.p, G[0], nodMapBack0.p, Nn);
-  ku(KU_PLAIN, du.p, nullptr, nullptr, cu.p, nullptr, nullptr, nodMapFwd0.p);
-  TOPX_CUDA_OK(cudaStreamSynchronize(st));
-  copy_sync(h_y, cu.p, sizeof(double) * Nn * 3, cudaMemcpyDeviceToHost);
+  double* v = host_vector();
+  copy_sync(v, h_u, sizeof(double) * Nn * 3, cudaMemcpyHostToDevice);
+  // z is free between solves, and zero off the domain
+  launch_compact_to_grid_nodes<double>(st, v, kw.z.p, G[0], nodMapBack0.p, Nn);
+  ku(KU_PLAIN, kw.z.p, nullptr, nullptr, v, nullptr, nullptr, nodMapFwd0.p);
+  copy_sync(h_y, v, sizeof(double) * Nn * 3, cudaMemcpyDeviceToHost);
 }
 
 void Engine::apply_vcycle(const double* h_r, double* h_z) {
-  TOPX_CUDA_OK(cudaStreamSynchronize(st));
-  DevBuf<double> cu;
-  cu.upload(h_r, size_t(Nn) * 3);
-  PcgScalars z{};
-  z.done = 0;
-  copy_sync(scE.p, &z, sizeof(z), cudaMemcpyHostToDevice);
-  TOPX_CUDA_OK(cudaMemsetAsync(kw.r.p, 0, kw.r.bytes(), st));
-  launch_compact_to_grid_nodes<double>(st, cu.p, kw.r.p, G[0], nodMapBack0.p, Nn);
+  double* v = host_vector();
+  copy_sync(v, h_r, sizeof(double) * Nn * 3, cudaMemcpyHostToDevice);
+  TOPX_CUDA_OK(cudaMemsetAsync(scE.p, 0, sizeof(PcgScalars), st));
+  launch_compact_to_grid_nodes<double>(st, v, kw.r.p, G[0], nodMapBack0.p, Nn);
   if (standard())
     vcycle_standard(true, scE.p);
   else if (!pre32())
     vcycle_t<double>(v64, scE.p);
   else
     vcycle_t<float>(v32, scE.p);
-  launch_grid_to_compact_nodes<double>(st, kw.z.p, cu.p, G[0], nodMapBack0.p, Nn);
+  launch_grid_to_compact_nodes<double>(st, kw.z.p, v, G[0], nodMapBack0.p, Nn);
+  copy_sync(h_z, v, sizeof(double) * Nn * 3, cudaMemcpyDeviceToHost);
   check_coop_waits();
-  copy_sync(h_z, cu.p, sizeof(double) * Nn * 3, cudaMemcpyDeviceToHost);
 }
 
 void Engine::timer_start() { TOPX_CUDA_OK(cudaEventRecord(tev[0], st)); }
@@ -943,10 +934,8 @@ void Engine::sec_harvest() {
 }
 
 void Engine::set_moduli_host(const double* h_E) {
-  TOPX_CUDA_OK(cudaStreamSynchronize(st));
   copy_sync(tmpA.p, h_E, sizeof(double) * Ne, cudaMemcpyHostToDevice);
   launch_scatter_elems_t<double>(st, tmpA.p, eleMapBack0.p, Ne, E64.p);
-  TOPX_CUDA_OK(cudaStreamSynchronize(st));
 }
 
 int Engine::pcg_host(int lc, double* h_u) {
@@ -958,10 +947,8 @@ int Engine::pcg_host(int lc, double* h_u) {
 
 int Engine::filter_host(double rmin, const double* h_src, double* h_out) {
   setup_filter(0, rmin);
-  TOPX_CUDA_OK(cudaStreamSynchronize(st));
   copy_sync(tmpA.p, h_src, sizeof(double) * Ne, cudaMemcpyHostToDevice);
   const int its = filter(0, tmpA.p, tmpB.p);
-  TOPX_CUDA_OK(cudaStreamSynchronize(st));
   copy_sync(h_out, tmpB.p, sizeof(double) * Ne, cudaMemcpyDeviceToHost);
   return its;
 }
@@ -969,7 +956,6 @@ int Engine::filter_host(double rmin, const double* h_src, double* h_out) {
 void Engine::compliance_host(const double* h_U, double* h_ce) {
   for (size_t lc = 0; lc < U.size(); ++lc) set_U(int(lc), h_U + lc * size_t(Nn) * 3);
   compliance(ce.p);
-  TOPX_CUDA_OK(cudaStreamSynchronize(st));
   copy_sync(h_ce, ce.p, sizeof(double) * Ne, cudaMemcpyDeviceToHost);
 }
 
@@ -1014,8 +1000,7 @@ void Engine::begin(int consType, double V0, int nLoop, double rMin, double rHat)
   betaPIO_ = 1.0;
   setup_filter(0, rMin);
   if (consType == 1) setup_filter(1, rHat);
-  std::vector<double> h(size_t(Ne), V0);
-  for (DevBuf<double>* b : {&x, &xPhys, &xTilde, &volMax}) copy_sync(b->p, h.data(), sizeof(double) * Ne, cudaMemcpyHostToDevice);
+  for (DevBuf<double>* b : {&x, &xPhys, &xTilde}) launch_fill(st, Ne, V0, b->p);
   for (auto& u : U) TOPX_CUDA_OK(cudaMemsetAsync(u.p, 0, u.bytes(), st));
   // compliance of the fully solid domain (TOP3D_XL.m:94-104)
   update_moduli(nullptr, true);

@@ -13,6 +13,7 @@
 #include <string>
 #include <vector>
 
+#include "topx_hostcopy.hpp"
 #include "topx_kernels.cuh"
 #include "topx_mesh.hpp"
 #include "topx_nd_dev.hpp"
@@ -127,7 +128,7 @@ class Engine {
   // ---- design state -----------------------------------------------------
   void set_xphys(const double* h_xPhys);  // host, compact order
   void get_xphys(double* h_xPhys) const;
-  void get_U(int lc, double* h_U) const;  // interleaved compact DOFs
+  void get_U(int lc, double* h_U);  // interleaved compact DOFs
   void set_U(int lc, const double* h_U);
 
   // ---- building blocks (device-resident) -----------------------------------
@@ -274,9 +275,12 @@ class Engine {
   PcgScalars* h_sc = nullptr;  // pinned
   CoopControl* h_ctl = nullptr;  // pinned
   // optimiser state (compact, FP64)
-  DevBuf<double> x, xPhys, dc, ce, tmpA, tmpB, xTilde, xhat, dfdx, dxv, volMax;
-  DevBuf<double> xold1, xold2, low, upp, alpha, beta, p0, q0, pij, qij, xmma, xmin, xmax;
+  DevBuf<double> x, xPhys, dc, ce, tmpA, tmpB, xTilde, xhat, dfdx, dxv;
+  DevBuf<double> xold1, xold2, low, upp, alpha, beta, p0, q0, pij, qij, xmma;
   DevBuf<uint8_t> passive;
+  DevBuf<double> hostVec;
+  double* host_vector();
+  HostCopyHold hostCopies;
   std::array<double, 2> filterR{{0, 0}};
   std::array<FilterKe<double>, 2> filterKe64{};  // filter element matrix per slot
   std::array<FilterKe<float>, 2> filterKe32{};

@@ -383,6 +383,16 @@ void launch_objective(cudaStream_t st, int64_t Ne, const double* ce, const doubl
   TOPX_CUDA_OK(cudaGetLastError());
 }
 
+__global__ void k_fill(int64_t n, double value, double* __restrict__ out) {
+  pdl_wait();
+  for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x)
+    out[i] = value;
+}
+void launch_fill(cudaStream_t st, int64_t n, double value, double* out) {
+  launch_pdl(st, k_fill, grid1d(n, 256), 256, 0, n, value, out);
+  TOPX_CUDA_OK(cudaGetLastError());
+}
+
 __global__ void k_dot(int64_t n, const double* __restrict__ a, const double* __restrict__ b, double* out,
                       RedScratch rs) {
   pdl_wait();

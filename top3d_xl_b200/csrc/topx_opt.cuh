@@ -55,6 +55,7 @@ void launch_scatter_elems_t(cudaStream_t st, const double* src, const int32_t* e
 // --- objective / OC --------------------------------------------------------
 void launch_objective(cudaStream_t st, int64_t Ne, const double* ce, const double* xPhys, double cSolid, double Emin,
                       double E0, double penal, double* dc, ObjState* os, RedScratch rs);
+void launch_fill(cudaStream_t st, int64_t n, double value, double* out);
 void launch_sum(cudaStream_t st, int64_t n, const double* a, const double* b, double* out, RedScratch rs);
 void launch_ewise(cudaStream_t st, int op, int64_t n, const double* a, const double* b, double* out, double s);
 // OC bisection (TOP3D_XL.m:145-156): w = x sqrt(-dc) once, then bisection steps on lmid,
