@@ -340,3 +340,30 @@ def test_pcg_step_edges(shape, precision):
     assert abs(its - itso) <= 1
     if its == itso:
         assert abs(f @ u - f @ uo) / abs(f @ uo) < max(1e-8 if precision == "fp64" else 1e-6, 10 * env)
+
+
+@pytest.mark.parametrize("shape", [(3, 3, 3), (9, 41, 7), (31, 33, 17), (63, 16, 40), (130, 9, 11)])
+@pytest.mark.parametrize("holes", [False, True])
+@pytest.mark.parametrize("precision", ["fp64", "mixed32"])
+def test_filter_tile_edges(shape, holes, precision):
+    # the filter's tiles (odd extents, short chunks, the domain's tile list), in FP64 and with its CG in FP32;
+    # FP64: the bar of test_filter.  FP32: the CG stops at 1e-4 of its right-hand side, and its last step may fall
+    # one iteration apart
+    from top3d_xl_b200 import Context
+    vox = np.ones(shape, bool)
+    if holes:
+        vox[:, 1:-1, :] = np.random.default_rng(3).random((shape[0], shape[1] - 2, shape[2])) < 0.7
+    m = O.build_model(vox)
+    src = np.random.default_rng(6).uniform(0, 1, m.levels[0].numElements)
+    with Context(precision) as ctx:
+        ctx.load_voxels(vox)
+        for rmin in (np.sqrt(3), 6.0):
+            out, its = ctx.filter(rmin, src)
+            flt = O.PDEFilter(m, rmin, m.S)
+            ref = flt(src)
+            if precision == "fp64":
+                assert its == flt.last_its
+                assert _rel(out, ref) < 1e-10
+            else:
+                assert abs(its - flt.last_its) <= 1
+                assert _rel(out, ref) < 1e-3

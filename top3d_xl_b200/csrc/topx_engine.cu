@@ -22,6 +22,7 @@ Engine::Engine(Model& model, int precision, int device, bool coarse_coop) : M(mo
   // graph captures; every host-side copy below waits for this stream first
   TOPX_CUDA_OK(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
   prepare_ku_kernels();
+  prepare_filter_kernels();
   prepare_nd_kernels();
   nl = M.numLevels;
   if (nl >= 3 && int(M.levels.size()) == nl && M.levels[1].span != KU_SPAN)
@@ -57,10 +58,18 @@ Engine::Engine(Model& model, int precision, int device, bool coarse_coop) : M(mo
     for (auto k : L.nodMapBack) pn[l ? k - 1 : pad_node(k - 1)] = 1;
     for (auto k : L.eleMapBack) pe[l ? k - 1 : pad_elem(k - 1)] = 1;
     present[l].upload(pn.data(), pn.size());
-    if (l == 0)
-      solid1.upload(pe.data(), pe.size());
-    else
+    if (l == 0) {  // per node its number of solid elements, and whether the element at it is solid
+      std::vector<uint8_t> f(pn.size(), 0);
+      const int64_t sy = G[0].nny(), sx = G[0].nnx();
+      for (size_t e = 0; e < pe.size(); ++e)
+        if (pe[e]) {
+          f[e] |= 128u;
+          for (int a = 0; a < 8; ++a) f[e + hex_ly(a) + sy * (hex_lx(a) + sx * hex_lz(a))] += 1;
+        }
+      filterFlags.upload(f.data(), f.size());
+    } else {
       epresent[l].upload(pe.data(), pe.size());
+    }
   }
   std::vector<int32_t> emb(Ne), nmb(Nn);
   for (int64_t e = 0; e < Ne; ++e) emb[e] = int32_t(pad_elem(l1.eleMapBack[e] - 1));
@@ -207,16 +216,16 @@ Engine::Engine(Model& model, int precision, int device, bool coarse_coop) : M(mo
     kush = ku_shape(G[0], nodeRows);
     std::vector<uint32_t> zr;
     const std::vector<uint32_t> act = ku_active_tiles(G[0], nodeRows, kush, pn, &zr);
-    const std::vector<uint8_t> all(pn.size(), 1);
     const size_t full = size_t(kush.grid.x) * kush.grid.y * kush.grid.z;
     if (!act.empty() && act.size() < full * 9 / 10) {
       kuTiles.upload(act.data(), act.size());
       kuZr.upload(zr.data(), zr.size());
     }
-    const std::vector<uint32_t> fact = filter_active_tiles(G[0], pn);
-    if (!fact.empty() && fact.size() < filter_active_tiles(G[0], all).size() * 9 / 10) {
+    fsh = filter_shape(G[0], nodeRows, flt32() ? 4 : 8);
+    const std::vector<uint32_t> fact = filter_active_tiles(G[0], nodeRows, fsh, pn, zr);
+    if (!fact.empty() && fact.size() < size_t(fsh.grid.x) * fsh.grid.y * fsh.grid.z * 9 / 10) {
       filterTiles.upload(fact.data(), fact.size());
-      fut = FilterTiles{filterTiles.p, int(fact.size())};
+      filterZr.upload(zr.data(), zr.size());
     }
     // elementwise level-1 passes skip the 32-node chunks without a present node
     const size_t nchunk = (pn.size() + 31) / 32;
@@ -403,11 +412,8 @@ void Engine::alloc_vwork(VWork<TC>& v) {
 
 template <typename TF>
 void Engine::alloc_fwork(FWork<TF>& f) {
-  const size_t N1 = size_t(G[0].nnodes());
-  for (DevBuf<TF>* b : {&f.fr, &f.fz, &f.fp, &f.fq, &f.fy, &f.fb}) b->alloc(N1);
-  f.fsrc.alloc(N1);
-  f.fdp[0].alloc(N1);
-  f.fdp[1].alloc(N1);
+  const size_t S1 = size_t(G[0].stride);
+  for (DevBuf<TF>* b : {&f.fr, &f.fp, &f.fp2, &f.fq, &f.fy, &f.fsrc}) b->alloc(S1);
 }
 
 void Engine::read_scalars(PcgScalars& h, const PcgScalars* d) const {
@@ -768,10 +774,6 @@ void Engine::setup_filter(int slot, double rmin) {
   filterKe64[slot] = filter_ke<double>(KF.data());
   filterKe32[slot] = filter_ke<float>(KF.data());
   filterR[slot] = rmin;
-  if (!flt32())
-    launch_filter_diag<double>(st, G[0], solid1.p, filterKe64[slot], f64.fdp[slot].p);
-  else
-    launch_filter_diag<float>(st, G[0], solid1.p, filterKe64[slot], f32.fdp[slot].p);
 }
 
 template <>
@@ -785,25 +787,41 @@ const FilterKe<float>& Engine::filter_ke_of<float>(int slot) const {
 
 template <typename T>
 int Engine::filter_t(FWork<T>& w, int slot, const double* d_src, double* d_out) {
-  const Grid& g = G[0];
-  PcgScalars* sc = scF.p;
+  FilterArgs<T> a{};
+  a.g = G[0];
+  a.sh = fsh;
+  a.ke = filter_ke_of<T>(slot);
+  a.r = w.fr.p;
+  a.y = w.fy.p;
+  a.q = w.fq.p;
+  a.pin = w.fp.p;
+  a.pout = w.fp2.p;
+  a.flags = filterFlags.p;
+  a.sc = scF.p;
+  a.rs = rs1;
+  a.active = filterTiles.p;
+  a.zr = filterZr.p;
+  a.ntiles = int(filterTiles.n);
+  a.act = act1;
+  a.err = &coopCtl.p->err;
+  a.tol = M.S.tol / 10;
+  a.maxIT = M.S.maxIT;
   launch_scatter_elems_t<T>(st, d_src, eleMapBack0.p, Ne, w.fsrc.p);
-  launch_filter_e2n<T>(st, g, w.fsrc.p, w.fb.p, act1);
-  launch_filter_residual_init<T>(st, g, w.fb.p, w.fdp[slot].p, w.fr.p, w.fz.p, w.fy.p, sc, rs1, M.S.tol / 10,
-                                 M.S.maxIT, act1);
-  const int CH = 8;
+  launch_filter_start<T>(st, a, w.fsrc.p);
+  const int CH = 8;  // even: every chunk starts from fp
   PcgScalars h{};
   int launched = 0;
   // the filter matrix is captured by value: the graph key carries the radius it was built for
   char key[64];
   std::snprintf(key, sizeof(key), "filter_chunk:%d:%.17g", slot, filterR[slot]);
-  const FilterKe<T>& kf = filter_ke_of<T>(slot);
   while (launched < M.S.maxIT) {
     const int n = std::min(CH, M.S.maxIT - launched);
     auto body = [&]() {
+      FilterArgs<T> b = a;
       for (int c = 0; c < n; ++c) {
-        launch_filter_ku<T>(st, KU_P_UPDATE, g, kf, w.fp.p, w.fz.p, nullptr, w.fq.p, solid1.p, sc, rs1, fut);
-        launch_filter_update<T>(st, g, w.fy.p, w.fp.p, w.fr.p, w.fq.p, w.fdp[slot].p, w.fz.p, sc, rs1, act1);
+        launch_filter_ku<T>(st, b);
+        launch_filter_update<T>(st, b);
+        std::swap(b.pin, b.pout);
       }
     };
     if (n == CH)
@@ -811,10 +829,10 @@ int Engine::filter_t(FWork<T>& w, int slot, const double* d_src, double* d_out) 
     else
       body();
     launched += n;
-    read_scalars(h, sc);
+    read_scalars(h, scF.p);
     if (h.done) break;
   }
-  launch_filter_n2e<T>(st, g, w.fy.p, eleMapBack0.p, Ne, d_out);
+  launch_filter_n2e<T>(st, a, eleMapBack0.p, Ne, d_out);
   return h.its;
 }
 

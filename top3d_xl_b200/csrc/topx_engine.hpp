@@ -116,8 +116,7 @@ struct VWork {
 // PDE-filter workspace (scalar node fields) in precision TF.
 template <typename TF>
 struct FWork {
-  DevBuf<TF> fr, fz, fp, fq, fy, fb, fsrc;
-  std::array<DevBuf<TF>, 2> fdp;
+  DevBuf<TF> fr, fp, fp2, fq, fy, fsrc;  // the direction alternates between fp and fp2
 };
 
 class Engine {
@@ -212,7 +211,7 @@ class Engine {
   void read_scalars(PcgScalars& h, const PcgScalars* d) const;
 
   // level-1 static data
-  DevBuf<uint8_t> fixbits, solid1;
+  DevBuf<uint8_t> fixbits, filterFlags;
   std::vector<DevBuf<uint8_t>> present, epresent;  // per level
   DevBuf<int32_t> eleMapBack0, nodMapBack0, nodMapFwd0;  // fwd: compact id of a grid node, or -1
   int nodeRows = 0;   // node rows along y without the padding ones
@@ -233,8 +232,8 @@ class Engine {
   // (compact: out takes the compact DOF order instead of the grid's)
   void ku(KuMode mode, const double* in, const double* pin, double* pout, double* out, PcgScalars* sc, double* y,
           const int32_t* compact = nullptr);
-  DevBuf<uint32_t> filterTiles;  // the same for the filter's K*u (its own z-chunks)
-  FilterTiles fut;
+  DevBuf<uint32_t> filterTiles, filterZr;  // the same for the filter's operator
+  FilterShape fsh{};
   DevBuf<uint32_t> act1Mask;     // level-1 chunk mask (chunk_active) of an irregular domain
   const uint32_t* act1 = nullptr;  // null: every chunk holds a present node
   // coarsest level: nested-dissection plan, its device copy and the factor tiles

@@ -35,10 +35,9 @@
 #include <type_traits>
 #include <vector>
 
-#include <cuda.h>
-
 #include "topx_ke_classes.h"
 #include "topx_kernels.cuh"
+#include "topx_tma.cuh"
 
 namespace topx {
 
@@ -58,48 +57,6 @@ __device__ __forceinline__ void cp_async_el(void* smem, const void* gmem, bool p
   asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"(s), "l"(gmem), "n"(BYTES), "r"(n) : "memory");
 }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
-
-// One barrier per stage counts the bytes of its TMA copies.
-__device__ __forceinline__ unsigned smem_addr(const void* p) { return static_cast<unsigned>(__cvta_generic_to_shared(p)); }
-__device__ __forceinline__ void mbar_init(uint64_t* b) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(b)) : "memory");
-}
-__device__ __forceinline__ void mbar_expect(uint64_t* b, unsigned bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(b)), "r"(bytes) : "memory");
-}
-// waits for the phase of the given parity; bounded (about a second in all), false when it gave up
-__device__ __forceinline__ bool mbar_wait(uint64_t* b, unsigned parity) {
-  for (unsigned it = 0; it < (1u << 20); ++it) {
-    unsigned ok;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
-        : "=r"(ok)
-        : "r"(smem_addr(b)), "r"(parity)
-        : "memory");
-    if (ok) return true;
-  }
-  return false;
-}
-// box of a 4-dimensional map (y, x, z, component) at (y, x, z, 0): entries outside the array read as zero.  y is
-// even: a copy starts on a 16-byte boundary.
-__device__ __forceinline__ void tma_load(void* dst, const CUtensorMap* map, int y, int x, int z, uint64_t* bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.4d.shared::cta.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];" ::"r"(
-          smem_addr(dst)),
-      "l"(map), "r"(y), "r"(x), "r"(z), "r"(0), "r"(smem_addr(bar))
-      : "memory");
-}
-
-// an array element at a 32-bit byte offset from a uniform base
-template <typename T>
-__device__ __forceinline__ T* at(T* base, uint32_t bytes) {
-  using C = typename std::conditional<std::is_const<T>::value, const char, char>::type;
-  return reinterpret_cast<T*>(reinterpret_cast<C*>(base) + bytes);
-}
-
-__device__ __forceinline__ void tma_prefetch(const CUtensorMap* map) {
-  asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory");
-}
 
 // Maps of the arrays that a launch reads through TMA, and the places of their boxes in a stage
 struct KuMaps {
@@ -463,41 +420,6 @@ void ku_smem_attr() {
   TOPX_CUDA_OK(cudaFuncSetAttribute(k_ku<MODE, TC>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024 / KU_CTAS));
 }
 
-// cuTensorMapEncodeTiled through the runtime (the library does not link the driver)
-using EncodeTiled = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
-                                 const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                 CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-EncodeTiled encode_tiled() {
-  static const EncodeTiled fn = [] {
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult q = cudaDriverEntryPointSymbolNotFound;
-    TOPX_CUDA_OK(cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &q));
-    if (!p || q != cudaDriverEntryPointSuccess) throw std::runtime_error("cuTensorMapEncodeTiled is not available");
-    return reinterpret_cast<EncodeTiled>(p);
-  }();
-  return fn;
-}
-
-// map of ncomp node fields of the grid, boxes of by x bx nodes of one plane
-CUtensorMap field_map(const double* p, const Grid& g, int ncomp, int by, int bx) {
-  CUtensorMap m;
-  const cuuint64_t dim[4] = {cuuint64_t(g.nny()), cuuint64_t(g.nnx()), cuuint64_t(g.nnz()), cuuint64_t(ncomp)};
-  const cuuint64_t stride[3] = {8 * dim[0], 8 * dim[0] * dim[1], 8 * cuuint64_t(g.stride)};
-  const cuuint32_t box[4] = {cuuint32_t(by), cuuint32_t(bx), 1, cuuint32_t(ncomp)}, one[4] = {1, 1, 1, 1};
-  if (encode_tiled()(&m, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 4, const_cast<double*>(p), dim, stride, box, one,
-                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-    throw std::runtime_error("cuTensorMapEncodeTiled failed");
-  return m;
-}
-
-int ku_num_sms() {
-  int dev = 0, n = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-    return 148;
-  return n > 0 ? n : 148;
-}
-
 }  // namespace
 
 void prepare_ku_kernels() {
@@ -564,7 +486,7 @@ KuModes ku_modes(const double* Ke576) {
 KuShape ku_shape(Grid g, int rows) {
   const int nny = rows, nnx = g.nnx(), nnz = g.nnz();
   if (g.nnodes() >= (int64_t(1) << 29)) throw std::runtime_error("grid too large for 32-bit byte offsets");
-  const double slots = double(KU_CTAS) * ku_num_sms();
+  const double slots = double(KU_CTAS) * num_sms();
   KuShape best{};
   double bestCost = -1;
   for (int nty = 1; nty <= nny; ++nty) {

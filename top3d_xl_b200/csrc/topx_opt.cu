@@ -1,5 +1,4 @@
-// Optimiser-side kernels of the TOP3D_XL B200 path: the PDE (Helmholtz)
-// density filter (TOP3D_XL.m:816-917), objective/sensitivities
+// Optimiser-side kernels of the TOP3D_XL B200 path: objective/sensitivities
 // (TOP3D_XL.m:124-130), OC bisection (TOP3D_XL.m:145-163), MMA subproblem and
 // dual interior-point steps (TOP3D_XL.m:1804-2049) and the Heaviside chain of
 // the LOCAL driver (TOP3D_XL.m:333-382).
@@ -15,330 +14,6 @@ static inline unsigned grid1d(int64_t n, int threads, int cap = 148 * 16) {
   if (b < 1) b = 1;
   if (b > cap) b = cap;
   return unsigned(b);
-}
-
-// The filter kernel matrix travels as a launch parameter (no process-wide constant memory),
-// so engines with different filter radii can run side by side.
-template <typename T>
-FilterKe<T> filter_ke(const double* KF64) {
-  FilterKe<T> k;
-  for (int i = 0; i < 64; ++i) k.v[i] = T(KF64[i]);
-  return k;
-}
-template FilterKe<double> filter_ke<double>(const double*);
-template FilterKe<float> filter_ke<float>(const double*);
-
-// element -> node: node = sum over its hexes (local-node order) of src_e*(1/8)  (TOP3D_XL.m:880-886)
-template <typename T>
-__global__ void k_filter_e2n(Grid g, const T* __restrict__ srcE, T* __restrict__ node, FastDiv dny, FastDiv dnx,
-                             const uint32_t* __restrict__ act) {
-  pdl_wait();
-  const uint32_t N = uint32_t(g.nnodes());  // < 2^32 (checked at launch)
-  const uint32_t nny = uint32_t(g.ny + 1), nnx = uint32_t(g.nx + 1);
-  for (uint32_t n = blockIdx.x * blockDim.x + threadIdx.x; n < N; n += gridDim.x * blockDim.x) {
-    if (!chunk_active(act, n)) continue;  // no solid element around these nodes: zero
-    const uint32_t q = dny.div(n), qz = dnx.div(q);
-    const int gy = int(n - q * nny), gx = int(q - qz * nnx), gz = int(qz);
-    T s = T(0);
-#pragma unroll
-    for (int a = 0; a < 8; ++a) {
-      const int ey = gy - hex_ly(a), ex = gx - hex_lx(a), ez = gz - hex_lz(a);
-      if (ey < 0 || ey >= g.ny || ex < 0 || ex >= g.nx || ez < 0 || ez >= g.nz) continue;
-      s = s + srcE[ey + int64_t(nny) * (ex + int64_t(nnx) * ez)] * T(0.125);
-    }
-    node[n] = s;
-  }
-}
-template <typename T>
-void launch_filter_e2n(cudaStream_t st, Grid g, const T* srcE, T* node, const uint32_t* act) {
-  if (g.nnodes() >= (int64_t(1) << 32)) throw std::runtime_error("grid too large for 32-bit node indices");
-  const FastDiv dny{uint32_t(g.ny + 1)}, dnx{uint32_t(g.nx + 1)};
-  launch_pdl(st, k_filter_e2n<T>, grid1d(g.nnodes(), 256), 256, 0, g, srcE, node, dny, dnx, act);
-  TOPX_CUDA_OK(cudaGetLastError());
-}
-
-// Jacobi preconditioner 1/diag (TOP3D_XL.m:855-867); 0 on absent nodes
-template <typename T>
-__global__ void k_filter_diag(Grid g, const uint8_t* __restrict__ solid, const FilterKe<double> kf, T* __restrict__ dp) {
-  pdl_wait();
-  const int64_t N = g.nnodes();
-  const int nny = g.ny + 1, nnx = g.nx + 1;
-  for (int64_t n = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; n < N; n += int64_t(gridDim.x) * blockDim.x) {
-    const int gy = int(n % nny), gx = int((n / nny) % nnx), gz = int(n / (int64_t(nny) * nnx));
-    double s = 0.0;
-    for (int a = 0; a < 8; ++a) {
-      const int ey = gy - hex_ly(a), ex = gx - hex_lx(a), ez = gz - hex_lz(a);
-      if (ey < 0 || ey >= g.ny || ex < 0 || ex >= g.nx || ez < 0 || ez >= g.nz) continue;
-      if (solid[ey + int64_t(nny) * (ex + int64_t(nnx) * ez)]) s += kf.v[a * 9];
-    }
-    dp[n] = s > 0.0 ? T(1.0 / s) : T(0);
-  }
-}
-template <typename T>
-void launch_filter_diag(cudaStream_t st, Grid g, const uint8_t* solid, const FilterKe<double>& kf, T* dp) {
-  launch_pdl(st, k_filter_diag<T>, grid1d(g.nnodes(), 256), 256, 0, g, solid, kf, dp);
-  TOPX_CUDA_OK(cudaGetLastError());
-}
-
-// Filter operator y = sum_e KF u_e over solid hexes (MatTimesVec_matrixFree_B, TOP3D_XL.m:904-917),
-// node-centric: a CTA of 32x8 nodes marches FKZ node planes along z with a ring of three node
-// planes and two planes of solid flags in shared memory; fused PCG direction update and p'q.
-// The z-chunk zc is picked per grid so that small grids still give every SM a few CTAs.
-constexpr int FKY = 32, FKX = 8, FNT = FKY * FKX;
-
-template <typename T, int MODE>
-__global__ void __launch_bounds__(FNT) k_filter_ku(Grid g, int zc, const FilterKe<T> kf, const T* __restrict__ in,
-                                                    const T* __restrict__ zin, T* __restrict__ out,
-                                                    const uint8_t* __restrict__ solid, PcgScalars* sc, RedScratch rs,
-                                                    const uint32_t* __restrict__ active) {
-  pdl_wait();
-  if (MODE != KU_PLAIN && sc->done) return;
-  __shared__ T su[3][FKX + 2][FKY + 2];
-  __shared__ T ss[2][FKX + 1][FKY + 1];
-  const int nny = g.ny + 1, nnx = g.nx + 1, nnz = g.nz + 1;
-  // the CTA's tile: blockIdx, or entry blockIdx.x of the list of tiles that own a node of the
-  // domain (y-tile | x-tile << 10 | z-chunk << 20)
-  int tyi = blockIdx.x, txi = blockIdx.y, tzi = blockIdx.z;
-  if (active) {
-    const uint32_t t = active[blockIdx.x];
-    tyi = int(t & 1023u);
-    txi = int((t >> 10) & 1023u);
-    tzi = int(t >> 20);
-  }
-  const int y0 = tyi * FKY, x0 = txi * FKX, zc0 = tzi * zc;
-  const int ty = threadIdx.x, tx = threadIdx.y;
-  const int tid = ty + FKY * tx;
-  const bool first = (MODE != KU_PLAIN) && sc->first;
-  const T beta = (MODE != KU_PLAIN) ? T(sc->beta) : T(0);
-  auto load_nodes = [&](int zp, int slot) {
-    for (int i = tid; i < (FKX + 2) * (FKY + 2); i += FNT) {
-      const int sy = i % (FKY + 2), sx = i / (FKY + 2);
-      const int gy = y0 - 1 + sy, gx = x0 - 1 + sx;
-      T v = T(0);
-      if (zp >= 0 && zp < nnz && gy >= 0 && gy < nny && gx >= 0 && gx < nnx) {
-        const int64_t n = gy + int64_t(nny) * (gx + int64_t(nnx) * zp);
-        if (MODE == KU_PLAIN)
-          v = in[n];
-        else
-          v = first ? zin[n] : zin[n] + beta * in[n];
-      }
-      su[slot][sx][sy] = v;
-    }
-  };
-  auto load_solid = [&](int ez, int slot) {
-    for (int i = tid; i < (FKX + 1) * (FKY + 1); i += FNT) {
-      const int sy = i % (FKY + 1), sx = i / (FKY + 1);
-      const int ey = y0 - 1 + sy, ex = x0 - 1 + sx;
-      T v = T(0);
-      if (ez >= 0 && ez < g.nz && ey >= 0 && ey < g.ny && ex >= 0 && ex < g.nx)
-        v = solid[ey + int64_t(nny) * (ex + int64_t(nnx) * ez)] ? T(1) : T(0);
-      ss[slot][sx][sy] = v;
-    }
-  };
-  load_nodes(zc0 - 1, 0);
-  load_nodes(zc0, 1);
-  load_solid(zc0 - 1, 0);
-  const int gy = y0 + ty, gx = x0 + tx;
-  const bool own = gy < nny && gx < nnx;
-  double dot = 0.0;
-  for (int k = 0; k < zc; ++k) {
-    const int z = zc0 + k;
-    if (z >= nnz) break;
-    load_nodes(z + 1, (k + 2) % 3);
-    load_solid(z, (k + 1) % 2);
-    __syncthreads();
-    if (own) {
-      const T(*const pl[3])[FKY + 2] = {su[k % 3], su[(k + 1) % 3], su[(k + 2) % 3]};
-      const T(*const el[2])[FKY + 1] = {ss[k % 2], ss[(k + 1) % 2]};
-      T acc[8];
-#pragma unroll
-      for (int e = 0; e < 8; ++e) acc[e] = T(0);
-#pragma unroll
-      for (int dz = -1; dz <= 1; ++dz)
-#pragma unroll
-        for (int dx = -1; dx <= 1; ++dx)
-#pragma unroll
-          for (int dy = -1; dy <= 1; ++dy) {
-            const T u = pl[dz + 1][tx + 1 + dx][ty + 1 + dy];
-#pragma unroll
-            for (int e = 0; e < 8; ++e) {
-              const int oy = (e & 1) ? 0 : -1, ox = (e & 2) ? 0 : -1, oz = (e & 4) ? 0 : -1;
-              const int ly = dy - oy, lx = dx - ox, lz = dz - oz;
-              if (ly < 0 || ly > 1 || lx < 0 || lx > 1 || lz < 0 || lz > 1) continue;
-              const int a = hex_local(-oy, -ox, -oz), b = hex_local(ly, lx, lz);
-              acc[e] = fma(kf.v[a * 8 + b], u, acc[e]);
-            }
-          }
-      T y = T(0);
-#pragma unroll
-      for (int a = 0; a < 8; ++a) {
-        const int oy = -hex_ly(a), ox = -hex_lx(a), oz = -hex_lz(a);
-        const int e = (oy + 1) + 2 * (ox + 1) + 4 * (oz + 1);
-        y = fma(el[oz + 1][tx + 1 + ox][ty + 1 + oy], acc[e], y);
-      }
-      const int64_t n = gy + int64_t(nny) * (gx + int64_t(nnx) * z);
-      out[n] = y;
-      if (MODE != KU_PLAIN) dot += double(pl[1][tx + 1][ty + 1]) * double(y);
-    }
-    __syncthreads();
-  }
-  if (MODE != KU_PLAIN) {
-    double v[1] = {dot}, tot[1];
-    if (reduce_publish<1>(v, rs, tot) && tid == 0) sc->pq = tot[0];
-  }
-}
-
-// tiles of 32 x 8 nodes, each a z-chunk of zc planes (aim at four CTAs per SM)
-struct FilterGeometry {
-  dim3 grd;
-  int zc;
-};
-static FilterGeometry filter_geometry(Grid g) {
-  const int tiles = ((g.nny() + FKY - 1) / FKY) * ((g.nnx() + FKX - 1) / FKX);
-  const int chunks = (148 * 4 + tiles - 1) / tiles;
-  FilterGeometry f;
-  f.zc = std::max(2, std::min(16, (g.nnz() + chunks - 1) / chunks));
-  f.grd = dim3((g.nny() + FKY - 1) / FKY, (g.nnx() + FKX - 1) / FKX, (g.nnz() + f.zc - 1) / f.zc);
-  return f;
-}
-
-std::vector<uint32_t> filter_active_tiles(Grid g, const std::vector<uint8_t>& present) {
-  const FilterGeometry f = filter_geometry(g);
-  const int nny = g.nny(), nnx = g.nnx(), nnz = g.nnz();
-  if (f.grd.x > 1024 || f.grd.y > 1024 || f.grd.z > 4095) return {};
-  std::vector<uint32_t> list;
-  for (unsigned tz = 0; tz < f.grd.z; ++tz)
-    for (unsigned tx = 0; tx < f.grd.y; ++tx)
-      for (unsigned ty = 0; ty < f.grd.x; ++ty) {
-        bool any = false;
-        for (int z = int(tz) * f.zc; z < std::min(nnz, int(tz + 1) * f.zc) && !any; ++z)
-          for (int x = int(tx) * FKX; x < std::min(nnx, int(tx + 1) * FKX) && !any; ++x)
-            for (int y = int(ty) * FKY; y < std::min(nny, int(ty + 1) * FKY) && !any; ++y)
-              any = present[size_t(y + int64_t(nny) * (x + int64_t(nnx) * z))] != 0;
-        if (any) list.push_back(ty | (tx << 10) | (tz << 20));
-      }
-  return list;
-}
-
-template <typename T>
-void launch_filter_ku(cudaStream_t st, KuMode mode, Grid g, const FilterKe<T>& kf, const T* in, const T* z, T* pout, T* out,
-                      const uint8_t* solid, PcgScalars* sc, RedScratch rs, FilterTiles tiles) {
-  (void)pout;
-  const FilterGeometry f = filter_geometry(g);
-  dim3 blk(FKY, FKX, 1);
-  const dim3 grd = tiles.list ? dim3(unsigned(tiles.n)) : f.grd;
-  if (grd.x == 0) return;
-  if (mode == KU_PLAIN)
-    launch_pdl(st, k_filter_ku<T, KU_PLAIN>, grd, blk, 0, g, f.zc, kf, in, z, out, solid, sc, rs, tiles.list);
-  else
-    launch_pdl(st, k_filter_ku<T, KU_P_UPDATE>, grd, blk, 0, g, f.zc, kf, in, z, out, solid, sc, rs, tiles.list);
-  TOPX_CUDA_OK(cudaGetLastError());
-}
-
-// r = b (y0 = 0), z = dp.*r, p = z, x1 = z'r, normB = ||b||
-template <typename T>
-__global__ void k_filter_init(Grid g, const T* __restrict__ b, const T* __restrict__ dp, T* __restrict__ r,
-                              T* __restrict__ z, T* __restrict__ y, PcgScalars* sc, RedScratch rs, double tol,
-                              int maxIT, const uint32_t* __restrict__ act) {
-  pdl_wait();
-  const int64_t N = g.nnodes();
-  double bb = 0.0, zr = 0.0;
-  for (int64_t n = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; n < N; n += int64_t(gridDim.x) * blockDim.x) {
-    if (!chunk_active(act, n)) continue;  // zero there and stays so
-    const T bv = b[n];
-    const T zv = dp[n] * bv;
-    r[n] = bv;
-    z[n] = zv;
-    y[n] = T(0);
-    bb += double(bv) * double(bv);
-    zr += double(zv) * double(bv);
-  }
-  double v[2] = {bb, zr}, tot[2];
-  if (reduce_publish<2>(v, rs, tot) && threadIdx.x == 0) {
-    sc->normB = sqrt(tot[0]);
-    sc->x1 = tot[1];
-    sc->tol = tol;
-    sc->maxIT = maxIT;
-    sc->its = 0;
-    sc->done = 0;
-    sc->first = 1;
-    sc->beta = 0.0;
-  }
-}
-template <typename T>
-void launch_filter_residual_init(cudaStream_t st, Grid g, const T* b, const T* dp, T* r, T* z, T* y, PcgScalars* sc,
-                                 RedScratch rs, double tol, int maxIT, const uint32_t* act) {
-  launch_pdl(st, k_filter_init<T>, grid1d(g.nnodes(), 256), 256, 0, g, b, dp, r, z, y, sc, rs, tol, maxIT, act);
-  TOPX_CUDA_OK(cudaGetLastError());
-}
-
-// p = z (+ beta p); y += lam p; r -= lam q; stop test; z = dp.*r; beta = z'r / x1
-template <typename T>
-__global__ void k_filter_update(Grid g, T* __restrict__ y, T* __restrict__ p, T* __restrict__ r,
-                                const T* __restrict__ q, const T* __restrict__ dp, T* __restrict__ z, PcgScalars* sc,
-                                RedScratch rs, const uint32_t* __restrict__ act) {
-  pdl_wait();
-  if (sc->done) return;
-  const bool first = sc->first;
-  const T beta = T(sc->beta);
-  const double lam = sc->x1 / sc->pq;
-  const T lamT = T(lam);
-  const int64_t N = g.nnodes();
-  double rr = 0.0, zr = 0.0;
-  for (int64_t n = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; n < N; n += int64_t(gridDim.x) * blockDim.x) {
-    if (!chunk_active(act, n)) continue;  // zero there and stays so
-    const T pv = first ? z[n] : z[n] + beta * p[n];
-    p[n] = pv;
-    y[n] = y[n] + lamT * pv;
-    const T rv = r[n] - lamT * q[n];
-    r[n] = rv;
-    const T zv = dp[n] * rv;
-    z[n] = zv;
-    rr += double(rv) * double(rv);
-    zr += double(zv) * double(rv);
-  }
-  double v[2] = {rr, zr}, tot[2];
-  if (reduce_publish<2>(v, rs, tot) && threadIdx.x == 0) {
-    sc->rr = tot[0];
-    sc->resnorm = sqrt(tot[0]) / sc->normB;
-    sc->its += 1;
-    sc->first = 0;
-    if (sc->resnorm < sc->tol) {
-      sc->done = 1;
-    } else if (sc->its >= sc->maxIT) {
-      sc->done = 2;
-    } else {
-      sc->beta = tot[1] / sc->x1;
-      sc->x1 = tot[1];
-    }
-  }
-}
-template <typename T>
-void launch_filter_update(cudaStream_t st, Grid g, T* y, T* p, T* r, const T* q, const T* dp, T* z, PcgScalars* sc,
-                          RedScratch rs, const uint32_t* act) {
-  launch_pdl(st, k_filter_update<T>, grid1d(g.nnodes(), 256), 256, 0, g, y, p, r, q, dp, z, sc, rs, act);
-  TOPX_CUDA_OK(cudaGetLastError());
-}
-
-// node -> element mean (TOP3D_XL.m:894-901), compact element order
-template <typename T>
-__global__ void k_filter_n2e(Grid g, const T* __restrict__ node, const int32_t* __restrict__ emb0, int64_t Ne,
-                             double* __restrict__ out) {
-  pdl_wait();
-  const int nny = g.ny + 1, nnx = g.nx + 1;
-  for (int64_t e = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; e < Ne; e += int64_t(gridDim.x) * blockDim.x) {
-    const int64_t id = emb0[e];  // the index of its lowest node
-    double s = 0.0;
-#pragma unroll
-    for (int a = 0; a < 8; ++a)
-      s += double(node[id + hex_ly(a) + int64_t(nny) * (hex_lx(a) + int64_t(nnx) * hex_lz(a))]);
-    out[e] = s * (1.0 / 8);
-  }
-}
-template <typename T>
-void launch_filter_n2e(cudaStream_t st, Grid g, const T* node, const int32_t* eleMapBack0, int64_t Ne, double* out) {
-  launch_pdl(st, k_filter_n2e<T>, grid1d(Ne, 256), 256, 0, g, node, eleMapBack0, Ne, out);
-  TOPX_CUDA_OK(cudaGetLastError());
 }
 
 template <typename T>
@@ -577,24 +252,6 @@ void launch_oc_final(cudaStream_t st, int64_t Ne, double* x, const double* w, co
   TOPX_CUDA_OK(cudaGetLastError());
 }
 
-template void launch_filter_e2n<double>(cudaStream_t, Grid, const double*, double*, const uint32_t*);
-template void launch_filter_e2n<float>(cudaStream_t, Grid, const float*, float*, const uint32_t*);
-template void launch_filter_diag<double>(cudaStream_t, Grid, const uint8_t*, const FilterKe<double>&, double*);
-template void launch_filter_diag<float>(cudaStream_t, Grid, const uint8_t*, const FilterKe<double>&, float*);
-template void launch_filter_ku<double>(cudaStream_t, KuMode, Grid, const FilterKe<double>&, const double*, const double*, double*, double*,
-                                       const uint8_t*, PcgScalars*, RedScratch, FilterTiles);
-template void launch_filter_ku<float>(cudaStream_t, KuMode, Grid, const FilterKe<float>&, const float*, const float*, float*, float*,
-                                      const uint8_t*, PcgScalars*, RedScratch, FilterTiles);
-template void launch_filter_residual_init<double>(cudaStream_t, Grid, const double*, const double*, double*, double*,
-                                                  double*, PcgScalars*, RedScratch, double, int, const uint32_t*);
-template void launch_filter_residual_init<float>(cudaStream_t, Grid, const float*, const float*, float*, float*,
-                                                 float*, PcgScalars*, RedScratch, double, int, const uint32_t*);
-template void launch_filter_update<double>(cudaStream_t, Grid, double*, double*, double*, const double*,
-                                           const double*, double*, PcgScalars*, RedScratch, const uint32_t*);
-template void launch_filter_update<float>(cudaStream_t, Grid, float*, float*, float*, const float*, const float*,
-                                          float*, PcgScalars*, RedScratch, const uint32_t*);
-template void launch_filter_n2e<double>(cudaStream_t, Grid, const double*, const int32_t*, int64_t, double*);
-template void launch_filter_n2e<float>(cudaStream_t, Grid, const float*, const int32_t*, int64_t, double*);
 template void launch_scatter_elems_t<double>(cudaStream_t, const double*, const int32_t*, int64_t, double*);
 template void launch_scatter_elems_t<float>(cudaStream_t, const double*, const int32_t*, int64_t, float*);
 

@@ -20,35 +20,55 @@ struct OcState {
 enum EwOp { EW_COPY = 0, EW_MUL = 1, EW_DIV_MAXX = 2 };
 
 // --- PDE filter ------------------------------------------------------------
-// 8x8 element matrix of the Helmholtz filter (TOP3D_XL.m:845-853), passed by value to kernels
+// The Helmholtz filter's element matrix (TOP3D_XL.m:845-853) in the basis of sums and differences along the
+// axes is diagonal, by the number of differences; dp: inverse diagonal of a node with 0..8 solid elements
 template <typename T>
 struct FilterKe {
-  T v[64];
+  T h[4];
+  T dp[9];
 };
 template <typename T>
 FilterKe<T> filter_ke(const double* KF64);
-template <typename T>
-void launch_filter_e2n(cudaStream_t st, Grid g, const T* srcE, T* node, const uint32_t* act = nullptr);
-template <typename T>
-void launch_filter_diag(cudaStream_t st, Grid g, const uint8_t* solid, const FilterKe<double>& kf, T* dp);
-// tiles of the filter operator's launch that own a node of the domain (a null list launches all)
-struct FilterTiles {
-  const uint32_t* list = nullptr;
-  int n = 0;
+// Tiles of the filter operator's launch: TY x TX nodes written by PY x PX threads, zc planes per CTA
+struct FilterShape {
+  int PY, PX, TY, TX, zc;
+  dim3 grid;
 };
+FilterShape filter_shape(Grid g, int rows, int bytes);  // bytes: of the filter's type
+// tiles that own a node of the domain, and per tile its planes that hold a present node (lo | hi << 16)
+std::vector<uint32_t> filter_active_tiles(Grid g, int rows, const FilterShape& f, const std::vector<uint8_t>& present,
+                                          std::vector<uint32_t>& zranges);
 template <typename T>
-void launch_filter_ku(cudaStream_t st, KuMode mode, Grid g, const FilterKe<T>& kf, const T* in, const T* z, T* pout,
-                      T* out, const uint8_t* solid, PcgScalars* sc, RedScratch rs, FilterTiles tiles = FilterTiles{});
-// tiles of the filter's K*u launch that own a node of the domain (a null list launches them all)
-std::vector<uint32_t> filter_active_tiles(Grid g, const std::vector<uint8_t>& present);
+struct FilterArgs {
+  Grid g;
+  FilterShape sh;
+  FilterKe<T> ke;
+  T *r, *y, *q;
+  T *pin, *pout;         // the previous direction, and the buffer that takes the new one
+  const uint8_t* flags;  // per node its number of solid elements, | 128 when the element above it (lowest corner) is solid
+  PcgScalars* sc;
+  RedScratch rs;
+  const uint32_t* active;  // filter_active_tiles, or null
+  const uint32_t* zr;
+  int ntiles;
+  const uint32_t* act;  // chunk mask (chunk_active), or null
+  int* err;             // takes kCoopErrCopy
+  double tol;
+  int maxIT;
+};
+// r = node sums of the element source (on the grid, at the elements' lowest nodes), and the CG's scalars
 template <typename T>
-void launch_filter_residual_init(cudaStream_t st, Grid g, const T* b, const T* dp, T* r, T* z, T* y, PcgScalars* sc,
-                                 RedScratch rs, double tol, int maxIT, const uint32_t* act = nullptr);
+void launch_filter_start(cudaStream_t st, const FilterArgs<T>& a, const T* srcE);
+// p = D r (+ beta p), q = A p, p'q; the previous step's y += lam p
 template <typename T>
-void launch_filter_update(cudaStream_t st, Grid g, T* y, T* p, T* r, const T* q, const T* dp, T* z, PcgScalars* sc,
-                          RedScratch rs, const uint32_t* act = nullptr);
+void launch_filter_ku(cudaStream_t st, const FilterArgs<T>& a);
+// r -= lam q, the stop test and beta from r'r and r'D r
 template <typename T>
-void launch_filter_n2e(cudaStream_t st, Grid g, const T* node, const int32_t* eleMapBack0, int64_t Ne, double* out);
+void launch_filter_update(cudaStream_t st, const FilterArgs<T>& a);
+// element means of y + lam p, p the last direction (in pin when the number of steps is even, else in pout)
+template <typename T>
+void launch_filter_n2e(cudaStream_t st, const FilterArgs<T>& a, const int32_t* eleMapBack0, int64_t Ne, double* out);
+void prepare_filter_kernels();
 template <typename T>
 void launch_scatter_elems_t(cudaStream_t st, const double* src, const int32_t* eleMapBack0, int64_t Ne, T* dstE);
 
