@@ -44,10 +44,13 @@ struct PcgScalars {
   double resnorm;  // ||r|| / ||b||
   double beta;     // x2 / x1
   double rdr;      // r' D r of the level-1 Jacobi diagonal D
+  double zr[2];    // z'r before step its, at its & 1 (the fused step; x1 is the 'Standard' V-cycle's)
   double lam;      // x1 / pq of the last update: its step y += lam p is applied by the next K*u
                    // (or, after the last iteration, by launch_pcg_flush)
   double tol;
   int its;
+  int its_next;    // its + 1, left by the residual pass for the kernel that takes its sums (no CTA may change a
+                   // word that another one of its launch still has to read)
   int maxIT;
   int done;  // 0 running, 1 converged, 2 hit maxIT
   int first;
@@ -157,6 +160,40 @@ __device__ __forceinline__ bool reduce_publish(double (&v)[NS], RedScratch rs, d
 #pragma unroll
   for (int s = 0; s < NS; ++s) out[s] = tot[s];
   return true;
+}
+
+// A reduction whose sum the next kernel forms: every CTA leaves its part in part[CTA], and every CTA of the consumer
+// adds them up, in one fixed order, while its own copies are on the way.  That spares the producer's tail (a fence, a
+// ticket, and the last CTA's pass over the parts: about 2 us) and is used for up to kMostParts CTAs; n = 0 says that the
+// producer published the sum itself.
+struct Parts {
+  double* part;
+  int n;
+};
+constexpr int kMostParts = 512;
+
+// the sum of the parts, in every thread of the CTA
+__device__ __forceinline__ double parts_sum(const Parts& p) {
+  const int tid = threadIdx.x + blockDim.x * (threadIdx.y + blockDim.y * threadIdx.z);
+  const int nth = blockDim.x * blockDim.y * blockDim.z;
+  double v[1] = {0.0};
+  for (int i = tid; i < p.n; i += nth) v[0] += __ldcg(p.part + i);
+  block_sum<1>(v);
+  __shared__ double total;
+  if (tid == 0) total = v[0];
+  __syncthreads();
+  return total;
+}
+// this CTA's part (called by all its threads)
+template <int NS>
+__device__ __forceinline__ void parts_leave(double (&v)[NS], double* const (&part)[NS]) {
+  pdl_trigger();
+  block_sum<NS>(v);
+  if (threadIdx.x + threadIdx.y + threadIdx.z == 0) {
+    const unsigned bid = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
+#pragma unroll
+    for (int s = 0; s < NS; ++s) part[s][bid] = v[s];
+  }
 }
 
 // Max-reduction analogue of reduce_publish (one slot).

@@ -327,6 +327,16 @@ Engine::Engine(Model& model, int precision, int device, bool coarse_coop) : M(mo
   red2.alloc(size_t(kMaxRedBlocks) * kMaxRedSlots);
   tickets.alloc(8);
   rs1 = RedScratch{red1.p, tickets.p};
+  {
+    partBuf.alloc(4 * kMostParts);
+    auto take = [&](int64_t n, int k) { return Parts{partBuf.p + k * kMostParts, n <= kMostParts ? int(n) : 0}; };
+    const int64_t tiles = kuTiles.p ? int64_t(kuTiles.n) : int64_t(kush.grid.x) * kush.grid.y * kush.grid.z;
+    const int64_t res = residual_blocks(G[0], G[1]);
+    parts.pq = take(tiles, 0);
+    parts.rr = take(res, 1);
+    parts.rd = take(res, 2);
+    parts.dot = take(prolong_blocks(G[1]), 3);
+  }
   rs2 = RedScratch{red2.p, tickets.p + 1};
   scE.alloc(1);
   scF.alloc(1);
@@ -556,15 +566,16 @@ void Engine::residual(ResidualMode mode, double* r, const double* b, PcgScalars*
   a.act = act1;
   a.sc = sc;
   a.rs = rs1;
+  a.parts = parts;
   a.tol = tol;
   a.maxIT = maxIT;
   launch_residual(st, mode, a, G[1]);
 }
 
 template <typename TC>
-void Engine::coarse_correction(VWork<TC>& v, bool dot, bool init, PcgScalars* sc) {
+void Engine::coarse_correction(VWork<TC>& v, bool dot, bool init, PcgScalars* sc, double tol, int maxIT) {
   sec_begin(SEC_RESTRICT);
-  launch_restrict_xz<TC>(st, kw.ty.p, G[0], v.rl[1].p, v.rc64.p, G[1], sc);
+  launch_restrict_xz<TC>(st, kw.ty.p, G[0], v.rl[1].p, v.rc64.p, G[1], sc, dot ? &parts : nullptr, init, tol, maxIT);
   for (int l = 2; l < nl; ++l)
     launch_restrict<TC>(st, v.rl[l - 1].p, G[l - 1], v.tmp1.p, v.tmp2.p, v.rl[l].p, G[l], sc);
   sec_end();
@@ -578,7 +589,7 @@ void Engine::coarse_correction(VWork<TC>& v, bool dot, bool init, PcgScalars* sc
   for (int l = nl - 2; l >= 1; --l)
     launch_prolong_smooth<TC, TC, TC>(st, M.levels[l + 1].span, v.xl[l + 1].p, G[l + 1], v.rl[l].p, v.dl[l].p,
                                       present[l].p, v.xl[l].p, G[l], M.S.weightFactorJacobi,
-                                      dot && l == 1 ? v.rc() : nullptr, init, sc, rs1);
+                                      dot && l == 1 ? v.rc() : nullptr, parts.dot, sc, rs1);
   sec_end();
 }
 
@@ -587,10 +598,10 @@ void Engine::vcycle_t(VWork<TC>& v, PcgScalars* sc) {
   sec_begin(SEC_RESTRICT);
   residual(RES_KEEP, kw.r.p, nullptr, sc, 0.0, 0);
   sec_end();
-  coarse_correction<TC>(v, false, false, sc);
+  coarse_correction<TC>(v, false, false, sc, 0.0, 0);
   sec_begin(SEC_PROLONG);
   launch_prolong_smooth<TC, double, TC>(st, M.levels[1].span, v.xl[1].p, G[1], kw.r.p, v.d1.p, present[0].p,
-                                        kw.z.p, G[0], M.S.weightFactorJacobi, nullptr, false, sc, rs1, act1);
+                                        kw.z.p, G[0], M.S.weightFactorJacobi, nullptr, Parts{}, sc, rs1, act1);
   sec_end();
 }
 
@@ -635,13 +646,13 @@ void Engine::vcycle_standard(bool init, PcgScalars* sc) {
   sec_end();
 }
 
-void Engine::precondition(bool init, PcgScalars* sc) {
+void Engine::precondition(bool init, PcgScalars* sc, double tol, int maxIT) {
   if (standard())
     vcycle_standard(init, sc);
   else if (!pre32())
-    coarse_correction<double>(v64, true, init, sc);
+    coarse_correction<double>(v64, true, init, sc, tol, maxIT);
   else
-    coarse_correction<float>(v32, true, init, sc);
+    coarse_correction<float>(v32, true, init, sc, tol, maxIT);
 }
 
 void Engine::ku(KuMode mode, const double* in, const double* pin, double* pout, double* out, PcgScalars* sc,
@@ -665,6 +676,7 @@ void Engine::ku(KuMode mode, const double* in, const double* pin, double* pout, 
   a.icfix = icfix64.p;
   a.sc = sc;
   a.rs = rs1;
+  a.parts = parts;
   a.err = &coopCtl.p->err;
   a.active = kuTiles.p;
   a.zr = kuZr.p;
@@ -690,7 +702,7 @@ int Engine::pcg(const double* b, double* y, bool warm, double tol, int maxIT) {
       launch_residual_init(st, g, b, kw.q.p, kw.r.p, sc, rs1, tol, maxIT);
     else
       residual(RES_INIT, kw.r.p, b, sc, tol, maxIT);
-    precondition(true, sc);
+    precondition(true, sc, tol, maxIT);
   });
   auto step_ku = [&](double* pin, double* pnew) {
     if (standard())
@@ -717,7 +729,7 @@ int Engine::pcg(const double* b, double* y, bool warm, double tol, int maxIT) {
           double* pnew = (c & 1) ? kw.p.p : kw.p2.p;
           step_ku(pin, pnew);
           step_residual();
-          precondition(false, sc);
+          precondition(false, sc, tol, maxIT);
         }
       });
       launched += CH;
@@ -734,7 +746,7 @@ int Engine::pcg(const double* b, double* y, bool warm, double tol, int maxIT) {
       sec_begin(SEC_UPDATE);
       step_residual();
       sec_end();
-      precondition(false, sc);
+      precondition(false, sc, tol, maxIT);
     }
     read_scalars(h, sc);
     if (prof_) {

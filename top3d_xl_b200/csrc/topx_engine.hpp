@@ -193,12 +193,14 @@ class Engine {
   void alloc_fwork(FWork<TF>& f);
   // xl[1] from the level-1 residual whose y pass is in kw.ty; dot: completes z'r in sc
   template <typename TC>
-  void coarse_correction(VWork<TC>& v, bool dot, bool init, PcgScalars* sc);
+  void coarse_correction(VWork<TC>& v, bool dot, bool init, PcgScalars* sc, double tol, int maxIT);
   template <typename TC>
   void vcycle_t(VWork<TC>& v, PcgScalars* sc);
   void vcycle_standard(bool init, PcgScalars* sc);
   bool standard() const { return !pre32() && M.S.typeVcycle == 1; }
-  void precondition(bool init, PcgScalars* sc);  // inside the PCG
+  void precondition(bool init, PcgScalars* sc, double tol, int maxIT);  // inside the PCG
+  PcgParts parts{};  // the fused step's sums (Parts)
+  DevBuf<double> partBuf;
   void residual(ResidualMode mode, double* r, const double* b, PcgScalars* sc, double tol, int maxIT);
   int pcg(const double* b, double* y, bool warm, double tol, int maxIT);
   template <typename TF>

@@ -78,15 +78,14 @@ __device__ __forceinline__ void pcg_start(PcgScalars* sc, double bb, double tol,
   sc->first = 1;
   sc->beta = 0.0;
 }
-__device__ __forceinline__ void pcg_stop_test(PcgScalars* sc, double lam, double rr) {
-  sc->lam = lam;
+// after step number its
+__device__ __forceinline__ void pcg_stop_test(PcgScalars* sc, double rr, int its) {
   sc->rr = rr;
   sc->resnorm = sqrt(rr) / sc->normB;
-  sc->its += 1;
   sc->first = 0;
   if (sc->resnorm < sc->tol)
     sc->done = 1;
-  else if (sc->its >= sc->maxIT)
+  else if (its >= sc->maxIT)
     sc->done = 2;
 }
 
@@ -107,7 +106,12 @@ __global__ void __launch_bounds__(256) k_residual(const __grid_constant__ Residu
   const double* __restrict__ const src = MODE == RES_INIT ? a.b : a.r;
   const double* __restrict__ const q = a.q;
   const double* __restrict__ const D = a.D;
-  const double lam = MODE == RES_UPDATE ? a.sc->x1 / a.sc->pq : 0.0;
+  double lam = 0.0;
+  int its = 0;
+  if (MODE == RES_UPDATE) {
+    its = a.sc->its;
+    lam = a.sc->zr[its & 1] / (a.parts.pq.n ? parts_sum(a.parts.pq) : a.sc->pq);
+  }
   double s0 = 0.0, rd = 0.0;  // b'b or r'r, and r'D r
   const int64_t line0 = (int64_t(blockIdx.x) * 8 + (threadIdx.x >> 5)) * lines;
   const int cells = line0 < nlines ? int(min(int64_t(lines), nlines - line0)) * cy : 0;
@@ -162,14 +166,23 @@ __global__ void __launch_bounds__(256) k_residual(const __grid_constant__ Residu
       if (i < cells) a.tmp[cell + c * ts] = begins ? own : own + prev;
     }
   }
-  if (MODE != RES_KEEP) {
+  if (MODE == RES_UPDATE && blockIdx.x == 0 && threadIdx.x == 0) {
+    a.sc->lam = lam;
+    a.sc->its_next = its + 1;
+  }
+  if (MODE != RES_KEEP && a.parts.rr.n) {  // the x and z passes' kernel sums them
+    double t[2] = {s0, rd};
+    parts_leave<2>(t, {a.parts.rr.part, a.parts.rd.part});
+  } else if (MODE != RES_KEEP) {
     double t[2] = {s0, rd}, tot[2];
     if (reduce_publish<2>(t, a.rs, tot) && threadIdx.x == 0) {
       a.sc->rdr = tot[1];
       if (MODE == RES_INIT)
         pcg_start(a.sc, tot[0], a.tol, a.maxIT);
-      else
-        pcg_stop_test(a.sc, lam, tot[0]);
+      else {
+        a.sc->its = its + 1;
+        pcg_stop_test(a.sc, tot[0], its + 1);
+      }
     }
   }
 }
@@ -189,12 +202,17 @@ static int residual_lines(int64_t nlines, int cy) {
   }
   return best;
 }
+int residual_blocks(Grid g, Grid gc) {
+  const int64_t nlines = int64_t(g.nnx()) * g.nnz();
+  const int lines = residual_lines(nlines, gc.nny());
+  return int((nlines + 8 * lines - 1) / (8 * lines));
+}
 void launch_residual(cudaStream_t st, ResidualMode mode, const ResidualArgs& args, Grid gc) {
   const int cy = gc.nny();
   if (args.g.nny() != 4 * cy) throw std::runtime_error("level-1 rows do not hold four nodes per coarse node");
   const int64_t nlines = int64_t(args.g.nnx()) * args.g.nnz();
   const int lines = residual_lines(nlines, cy);
-  const unsigned nb = unsigned((nlines + 8 * lines - 1) / (8 * lines));
+  const unsigned nb = unsigned(residual_blocks(args.g, gc));
   const FastDiv dcy{uint32_t(cy)};
   auto go = [&](auto kernel) { launch_pdl(st, kernel, nb, 256, 0, args, lines, cy, dcy); };
   if (mode == RES_KEEP)
@@ -256,7 +274,11 @@ __global__ void k_pcg_update(Grid g, double* __restrict__ r, const double* __res
     }
   }
   double v[1] = {rr}, tot[1];
-  if (reduce_publish<1>(v, rs, tot) && threadIdx.x == 0) pcg_stop_test(sc, lam, tot[0]);
+  if (reduce_publish<1>(v, rs, tot) && threadIdx.x == 0) {
+    sc->lam = lam;
+    sc->its += 1;
+    pcg_stop_test(sc, tot[0], sc->its);
+  }
 }
 void launch_pcg_update(cudaStream_t st, Grid g, double* r, const double* q, PcgScalars* sc, RedScratch rs,
                        const uint32_t* act) {
@@ -303,9 +325,27 @@ template <typename T>
 __global__ void __launch_bounds__(32 * (2 * KU_SPAN - 1)) k_restrict_xz(const double* __restrict__ tmp, int inx, int inz,
                                                                        T* __restrict__ out, double* __restrict__ out64,
                                                                        int64_t ostr, int ony, int onx, FastDiv dy,
-                                                                       const PcgScalars* sc) {
+                                                                       PcgScalars* sc, PcgParts parts, int init,
+                                                                       double tol, int maxIT) {
   pdl_wait();
-  if (sc && sc->done) return;
+  if (sc && !init && sc->done) return;
+  if (parts.rr.n) {  // the residual pass's sums: every CTA takes the same decision, the first one writes it down
+    const bool first = blockIdx.x + blockIdx.y + threadIdx.x + threadIdx.y == 0;
+    const double rr = parts_sum(parts.rr);
+    if (blockIdx.x + blockIdx.y == 0) {
+      const double rd = parts_sum(parts.rd);
+      if (first) sc->rdr = rd;
+      if (first && init) pcg_start(sc, rr, tol, maxIT);
+    }
+    if (!init) {
+      const int its = sc->its_next;
+      if (first) {
+        sc->its = its;
+        pcg_stop_test(sc, rr, its);
+      }
+      if (sqrt(rr) / sc->normB < sc->tol || its >= sc->maxIT) return;
+    }
+  }
   constexpr int W = 2 * KU_SPAN - 1;
   __shared__ double sx[W][3][32];
   const int lane = threadIdx.x, dz = threadIdx.y, oz = blockIdx.y;
@@ -341,16 +381,18 @@ __global__ void __launch_bounds__(32 * (2 * KU_SPAN - 1)) k_restrict_xz(const do
   }
 }
 template <typename T>
-void launch_restrict_xz(cudaStream_t st, const double* tmp, Grid gf, T* out, double* out64, Grid gc,
-                        const PcgScalars* sc) {
+void launch_restrict_xz(cudaStream_t st, const double* tmp, Grid gf, T* out, double* out64, Grid gc, PcgScalars* sc,
+                        const PcgParts* parts, bool init, double tol, int maxIT) {
   const int cy = gc.nny(), cx = gc.nnx();
   const dim3 nb(unsigned((cy * cx + 31) / 32), unsigned(gc.nnz()));
-  launch_pdl(st, k_restrict_xz<T>, nb, dim3(32, 2 * KU_SPAN - 1), 0, tmp, gf.nnx(), gf.nnz(), out, out64, gc.stride,
-             cy, cx, FastDiv{uint32_t(cy)}, sc);
+  launch_pdl(st, k_restrict_xz<T>, nb, dim3(32, 2 * KU_SPAN - 1), 0, tmp, gf.nnx(), gf.nnz(), out, out64, gc.stride, cy, cx,
+             FastDiv{uint32_t(cy)}, sc, parts ? *parts : PcgParts{}, init ? 1 : 0, tol, maxIT);
   TOPX_CUDA_OK(cudaGetLastError());
 }
-template void launch_restrict_xz<double>(cudaStream_t, const double*, Grid, double*, double*, Grid, const PcgScalars*);
-template void launch_restrict_xz<float>(cudaStream_t, const double*, Grid, float*, double*, Grid, const PcgScalars*);
+template void launch_restrict_xz<double>(cudaStream_t, const double*, Grid, double*, double*, Grid, PcgScalars*,
+                                         const PcgParts*, bool, double, int);
+template void launch_restrict_xz<float>(cudaStream_t, const double*, Grid, float*, double*, Grid, PcgScalars*,
+                                        const PcgParts*, bool, double, int);
 
 template <typename T, int S, int AXIS>
 __global__ void k_restrict_axis(const T* __restrict__ in, int64_t istr, int iny, int inx, int inz,
@@ -495,7 +537,7 @@ __global__ void __launch_bounds__(256) k_prolong_smooth(const TX* __restrict__ x
                                                         const uint8_t* __restrict__ present, T* __restrict__ x,
                                                         Grid gf, FastDiv dny, FastDiv dnx, T omega,
                                                         const double* __restrict__ rc, PcgScalars* sc, RedScratch rs,
-                                                        int init, double omega2, const uint32_t* __restrict__ act) {
+                                                        Parts dot, double omega2, const uint32_t* __restrict__ act) {
   pdl_wait();
   if (sc && sc->done) return;
   const uint32_t fny = uint32_t(gf.nny()), fnx = uint32_t(gf.nnx());
@@ -547,25 +589,31 @@ __global__ void __launch_bounds__(256) k_prolong_smooth(const TX* __restrict__ x
 #pragma unroll
     for (int c = 0; c < 3; ++c) x[n + c * gf.stride] = v[c];
   }
-  if (DOT) {
+  if (DOT && dot.n) {  // the next K*u sums them
+    double vv[1] = {zr};
+    parts_leave<1>(vv, {dot.part});
+  } else if (DOT) {
     double vv[1] = {zr}, tot[1];
     if (reduce_publish<1>(vv, rs, tot) && threadIdx.x == 0) {
+      const int its = sc->its;
       const double x2 = fma(omega2, sc->rdr, tot[0]);
-      if (!init) sc->beta = x2 / sc->x1;
-      sc->x1 = x2;
+      if (its > 0) sc->beta = x2 / sc->zr[(its - 1) & 1];
+      sc->zr[its & 1] = x2;
     }
   }
 }
 
+int prolong_blocks(Grid gf) { return int(grid1d(gf.nnodes(), 256, 148 * 8)); }
+
 template <typename TX, typename T, typename TD>
 void launch_prolong_smooth(cudaStream_t st, int span, const TX* xc, Grid gc, const T* r, const TD* d,
-                           const uint8_t* present, T* x, Grid gf, double omega, const double* rc, bool init,
+                           const uint8_t* present, T* x, Grid gf, double omega, const double* rc, Parts dot,
                            PcgScalars* sc, RedScratch rs, const uint32_t* act) {
   if (gf.nnodes() >= (int64_t(1) << 32)) throw std::runtime_error("grid too large for 32-bit node indices");
-  const unsigned nb = grid1d(gf.nnodes(), 256, 148 * 8);
+  const unsigned nb = unsigned(prolong_blocks(gf));
   const FastDiv dny{uint32_t(gf.nny())}, dnx{uint32_t(gf.nnx())};
   auto go = [&](auto kernel) {
-    launch_pdl(st, kernel, nb, 256, 0, xc, gc, r, d, present, x, gf, dny, dnx, T(omega), rc, sc, rs, init ? 1 : 0,
+    launch_pdl(st, kernel, nb, 256, 0, xc, gc, r, d, present, x, gf, dny, dnx, T(omega), rc, sc, rs, dot,
                2.0 * omega, act);
   };
   if (span == 4)
@@ -585,8 +633,8 @@ void launch_prolong_add(cudaStream_t st, int span, const TX* xc, Grid gc, const 
   if (gf.nnodes() >= (int64_t(1) << 32)) throw std::runtime_error("grid too large for 32-bit node indices");
   const FastDiv dny{uint32_t(gf.nny())}, dnx{uint32_t(gf.nnx())};
   auto go = [&](auto kernel) {
-    launch_pdl(st, kernel, nb, 256, 0, xc, gc, r, d, present, x, gf, dny, dnx, T(omega), nullptr, sc, none, 0, 0.0,
-               nullptr);
+    launch_pdl(st, kernel, nb, 256, 0, xc, gc, r, d, present, x, gf, dny, dnx, T(omega), nullptr, sc, none,
+               Parts{}, 0.0, nullptr);
   };
   if (span == 4)
     go(k_prolong_smooth<TX, T, TD, 4, false, false>);
@@ -840,7 +888,7 @@ void launch_unit_compliance(cudaStream_t st, Grid g, const double* U, const int3
                                   const uint8_t*, T*, double*);                                                    \
   template void launch_restrict<T>(cudaStream_t, const T*, Grid, T*, T*, T*, Grid, const PcgScalars*);           \
   template void launch_prolong_smooth<T, T, T>(cudaStream_t, int, const T*, Grid, const T*, const T*,            \
-                                               const uint8_t*, T*, Grid, double, const double*, bool,            \
+                                               const uint8_t*, T*, Grid, double, const double*, Parts,           \
                                                PcgScalars*, RedScratch, const uint32_t*);
 TOPX_INST(double)
 TOPX_INST(float)
@@ -848,7 +896,7 @@ template void launch_compact_to_grid_nodes<double>(cudaStream_t, const double*, 
 template void launch_grid_to_compact_nodes<double>(cudaStream_t, const double*, double*, Grid, const int32_t*, int64_t);
 template void launch_prolong_smooth<float, double, float>(cudaStream_t, int, const float*, Grid, const double*,
                                                           const float*, const uint8_t*, double*, Grid, double,
-                                                          const double*, bool, PcgScalars*, RedScratch, const uint32_t*);
+                                                          const double*, Parts, PcgScalars*, RedScratch, const uint32_t*);
 template void launch_prolong_add<double, double, double>(cudaStream_t, int, const double*, Grid, const double*,
                                                         const double*, const uint8_t*, double*, Grid, double,
                                                         PcgScalars*);

@@ -58,6 +58,14 @@ struct Grid {
 // KU_P_UPDATE with z given, KU_FUSED with z = omega2 (r D) + P xc formed from the residual r
 enum KuMode { KU_PLAIN = 0, KU_P_UPDATE = 2, KU_FUSED = 3 };
 
+// The sums of a fused PCG step that the next kernel forms (Parts): p'q of K*u, r'r (or b'b) and r'D r of the residual
+// pass, and the level-2 part of z'r
+struct PcgParts {
+  Parts pq, rr, rd, dot;
+};
+int residual_blocks(Grid g, Grid gc);
+int prolong_blocks(Grid gf);
+
 // element matrices in constant memory
 void upload_ke(const double* Ke576);
 
@@ -92,6 +100,7 @@ struct KuArgs {
   const double *cfix, *icfix;  // a fixed DOF's diagonal, and its inverse (fused)
   PcgScalars* sc;
   RedScratch rs;
+  PcgParts parts;  // fused
   const uint32_t* active;  // the tiles that own a node of the domain (ku_active_tiles), or null for all
   const uint32_t* zr;      // per listed tile, the planes [lo, hi) of its z-chunk that hold a present node (lo | hi << 16)
   double* yacc;
@@ -131,6 +140,7 @@ struct ResidualArgs {
   const uint32_t* act;
   PcgScalars* sc;
   RedScratch rs;
+  PcgParts parts;
   double tol;
   int maxIT;
 };
@@ -138,18 +148,19 @@ void launch_residual(cudaStream_t st, ResidualMode mode, const ResidualArgs& arg
 // --- transfers -----------------------------------------------------------
 // the x and z passes of the level-1 restriction: tmp -> out, and out64 when given
 template <typename T>
-void launch_restrict_xz(cudaStream_t st, const double* tmp, Grid gf, T* out, double* out64, Grid gc,
-                        const PcgScalars* sc);
+// inside the PCG (parts) it also takes the residual pass's sums, which the stop test needs (init: the solve's start)
+void launch_restrict_xz(cudaStream_t st, const double* tmp, Grid gf, T* out, double* out64, Grid gc, PcgScalars* sc,
+                        const PcgParts* parts = nullptr, bool init = false, double tol = 0.0, int maxIT = 0);
 // restriction between coarse levels (span 2)
 template <typename T>
 void launch_restrict(cudaStream_t st, const T* in, Grid gf, T* tmp1, T* tmp2, T* out, Grid gc, const PcgScalars* sc);
 constexpr int64_t kRestrictOneLaunch = int64_t(1) << 21;  // nodes of the fine grid up to which tmp1 and tmp2 are not used
 // x = omega*(r/d) + P(xc) + (omega*r)/d on present fine nodes.  rc (level 2 inside the PCG): the restricted
-// residual in FP64; z'r = omega2 sc->rdr + rc'x goes into sc (init: x1 = z'r; else beta = z'r/x1, x1 = z'r)
+// residual in FP64; rc'x goes into dot, or z'r = omega2 sc->rdr + rc'x and beta into sc
 template <typename TX, typename T, typename TD>
 // act: the fine grid's chunk mask (chunk_active), or null
 void launch_prolong_smooth(cudaStream_t st, int span, const TX* xc, Grid gc, const T* r, const TD* d,
-                           const uint8_t* present, T* x, Grid gf, double omega, const double* rc, bool init,
+                           const uint8_t* present, T* x, Grid gf, double omega, const double* rc, Parts dot,
                            PcgScalars* sc, RedScratch rs, const uint32_t* act = nullptr);
 // 'Standard' V-cycle (TX:758-763, 772-777): x = omega*(r/d) + P(xc) without the smoothing term;
 // x = omega*(r/d); q = r - q; x += omega*(r - q)/d (with dot: z.r into sc as above); coarse-level

@@ -245,14 +245,21 @@ __global__ void __launch_bounds__(KU_NT, KU_CTAS)
     return inb && zp >= 0 && zp < nnz ? unsigned(a.flags[(n0 + np * uint32_t(zp)) / 8u]) : 0u;
   };
   unsigned f = flags_at(zc0 - 1), fo = 0;  // of the plane, and of the one below
-  const bool first = PCG && a.sc->first;
-  const double beta = PCG ? a.sc->beta : 0.0, lam = PCG ? a.sc->lam : 0.0;
+  const bool first = PCG && (MODE == KU_FUSED ? a.sc->its == 0 : a.sc->first != 0);
+  const double lam = PCG ? a.sc->lam : 0.0;
+  double beta = PCG ? a.sc->beta : 0.0;
   bool ok = true;  // no wait gave up
   if (PCG && a.sc->done) {  // the same for the whole launch
     cp_async_wait_all();
     ok = mbar_wait(&sm.bar[0], 0) && mbar_wait(&sm.bar[1], 0);
     if (!ok && t == 0) atomicCAS(a.err, 0, kCoopErrCopy);
     return;
+  }
+  if (MODE == KU_FUSED && a.parts.dot.n) {  // z'r, whose level-2 part the prolongation left in parts
+    const int its = a.sc->its;
+    const double zr = fma(a.omega2, a.sc->rdr, parts_sum(a.parts.dot));
+    if (its > 0) beta = zr / a.sc->zr[(its - 1) & 1];
+    if (blockIdx.x + blockIdx.y + blockIdx.z == 0 && t == 0) a.sc->zr[its & 1] = zr;
   }
   // xc interpolated to the node's (y, x) on level-2 plane Z (fused)
   auto coarse = [&](int Z) {
@@ -409,7 +416,10 @@ __global__ void __launch_bounds__(KU_NT, KU_CTAS)
   }
   cp_async_wait_all();
   if (!ok) atomicCAS(a.err, 0, kCoopErrCopy);
-  if (PCG) {
+  if (MODE == KU_FUSED && a.parts.pq.n) {  // the residual pass sums them
+    double r[1] = {dot};
+    parts_leave<1>(r, {a.parts.pq.part});
+  } else if (PCG) {
     double r[1] = {dot}, tot[1];
     if (reduce_publish<1>(r, a.rs, tot) && t == 0) a.sc->pq = tot[0];
   }
