@@ -367,3 +367,28 @@ def test_filter_tile_edges(shape, holes, precision):
             else:
                 assert abs(its - flt.last_its) <= 1
                 assert _rel(out, ref) < 1e-3
+
+
+@pytest.mark.parametrize("shape", [(32, 64, 40), (40, 64, 40), (8, 8, 200), (31, 40, 17)])
+@pytest.mark.parametrize("holes", [False, True])
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_small_coarse_levels(shape, holes, precision):
+    # the levels below the first as one cluster launch (one front of at most 320 nodes: 32 x 64 x 40 has 270) and as
+    # separate launches (40 x 64 x 40 has 324): both against the oracle's V-cycle, with test_vcycle's bars
+    from top3d_xl_b200 import Context
+    vox = np.ones(shape, bool)
+    if holes:
+        vox[:, 1:-1, :] = np.random.default_rng(3).random((shape[0], shape[1] - 2, shape[2])) < 0.7
+    m = O.build_model(vox)
+    x = np.random.default_rng(1).uniform(0.3, 1.0, m.levels[0].numElements)
+    S = m.S
+    E = S.modulusMin + x ** S.SIMPpenalty * (S.modulus - S.modulusMin)
+    sol = O.Solver(m)
+    sol.assemble(E)
+    with Context(precision) as ctx:
+        ctx.load_voxels(vox)
+        ctx.set_moduli(E)
+        ctx.assemble()
+        for seed in (3, 4):
+            r = np.random.default_rng(seed).standard_normal(m.levels[0].numDOFs)
+            assert _rel(ctx.vcycle(r), sol.vcycle(r)) < (1e-10 if precision == "fp64" else 1e-5)

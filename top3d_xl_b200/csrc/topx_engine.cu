@@ -335,7 +335,8 @@ Engine::Engine(Model& model, int precision, int device, bool coarse_coop) : M(mo
     parts.pq = take(tiles, 0);
     parts.rr = take(res, 1);
     parts.rd = take(res, 2);
-    parts.dot = take(prolong_blocks(G[1]), 3);
+    smallCoarse = small_coarse(nd, nl, G[1]);
+    parts.dot = take(smallCoarse ? kSmallCoarseCtas : prolong_blocks(G[1]), 3);
   }
   rs2 = RedScratch{red2.p, tickets.p + 1};
   scE.alloc(1);
@@ -574,6 +575,34 @@ void Engine::residual(ResidualMode mode, double* r, const double* b, PcgScalars*
 
 template <typename TC>
 void Engine::coarse_correction(VWork<TC>& v, bool dot, bool init, PcgScalars* sc, double tol, int maxIT) {
+  if (smallCoarse) {
+    sec_begin(SEC_COARSE_SOLVE);
+    SmallCoarse<TC> a{};
+    a.tmp = kw.ty.p;
+    a.g0 = G[0];
+    a.g1 = G[1];
+    a.g2 = G[2];
+    a.r1 = v.rl[1].p;
+    a.r2 = v.rl[2].p;
+    a.x2 = v.xl[2].p;
+    a.x1 = v.xl[1].p;
+    a.r1_64 = v.rc64.p;
+    a.d1 = v.dl[1].p;
+    a.present1 = present[1].p;
+    a.front = nd.fronts[0];
+    a.tiles = std::is_same<TC, double>::value ? (const TC*)ndPool.p : (const TC*)ndPool32.p;
+    a.sep_dof = ndSep.p;
+    a.sc = sc;
+    if (dot) a.parts = parts;
+    a.dot = dot;
+    a.init = init;
+    a.tol = tol;
+    a.omega = M.S.weightFactorJacobi;
+    a.maxIT = maxIT;
+    launch_small_coarse<TC>(st, a);
+    sec_end();
+    return;
+  }
   sec_begin(SEC_RESTRICT);
   launch_restrict_xz<TC>(st, kw.ty.p, G[0], v.rl[1].p, v.rc64.p, G[1], sc, dot ? &parts : nullptr, init, tol, maxIT);
   for (int l = 2; l < nl; ++l)

@@ -197,6 +197,7 @@ class Engine {
   template <typename TC>
   void vcycle_t(VWork<TC>& v, PcgScalars* sc);
   void vcycle_standard(bool init, PcgScalars* sc);
+  bool smallCoarse = false;  // the coarse part of the V-cycle runs as one launch
   bool standard() const { return !pre32() && M.S.typeVcycle == 1; }
   void precondition(bool init, PcgScalars* sc, double tol, int maxIT);  // inside the PCG
   PcgParts parts{};  // the fused step's sums (Parts)

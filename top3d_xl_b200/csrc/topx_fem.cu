@@ -4,6 +4,7 @@
 #include <stdexcept>
 
 #include "topx_kernels.cuh"
+#include "topx_pcg.cuh"
 
 namespace topx {
 
@@ -69,26 +70,6 @@ __device__ __forceinline__ void load4(const double* p, double (&v)[4]) {
   v[2] = b.x;
   v[3] = b.y;
 }
-__device__ __forceinline__ void pcg_start(PcgScalars* sc, double bb, double tol, int maxIT) {
-  sc->normB = sqrt(bb);
-  sc->tol = tol;
-  sc->maxIT = maxIT;
-  sc->its = 0;
-  sc->done = 0;
-  sc->first = 1;
-  sc->beta = 0.0;
-}
-// after step number its
-__device__ __forceinline__ void pcg_stop_test(PcgScalars* sc, double rr, int its) {
-  sc->rr = rr;
-  sc->resnorm = sqrt(rr) / sc->normB;
-  sc->first = 0;
-  if (sc->resnorm < sc->tol)
-    sc->done = 1;
-  else if (its >= sc->maxIT)
-    sc->done = 2;
-}
-
 // The first V-cycle of a solve and every iteration run one pass over the level-1 residual: the update
 // r -= lambda q (or r = b - q), the sums r'r and r'D r, and the y pass of the restriction from the new
 // values.  A lane takes four nodes along y (32 bytes of every field, and a coarse node's own cell: rows hold a
@@ -329,23 +310,7 @@ __global__ void __launch_bounds__(32 * (2 * KU_SPAN - 1)) k_restrict_xz(const do
                                                                        double tol, int maxIT) {
   pdl_wait();
   if (sc && !init && sc->done) return;
-  if (parts.rr.n) {  // the residual pass's sums: every CTA takes the same decision, the first one writes it down
-    const bool first = blockIdx.x + blockIdx.y + threadIdx.x + threadIdx.y == 0;
-    const double rr = parts_sum(parts.rr);
-    if (blockIdx.x + blockIdx.y == 0) {
-      const double rd = parts_sum(parts.rd);
-      if (first) sc->rdr = rd;
-      if (first && init) pcg_start(sc, rr, tol, maxIT);
-    }
-    if (!init) {
-      const int its = sc->its_next;
-      if (first) {
-        sc->its = its;
-        pcg_stop_test(sc, rr, its);
-      }
-      if (sqrt(rr) / sc->normB < sc->tol || its >= sc->maxIT) return;
-    }
-  }
+  if (pcg_decide(sc, parts, init != 0, tol, maxIT)) return;
   constexpr int W = 2 * KU_SPAN - 1;
   __shared__ double sx[W][3][32];
   const int lane = threadIdx.x, dz = threadIdx.y, oz = blockIdx.y;

@@ -18,21 +18,31 @@ struct CudaError : std::runtime_error {
         code(e) {}
 };
 // Launch of a kernel that begins with pdl_wait(): its start overlaps the end of the launch before it.
+// cluster: CTAs of a cluster along x.
 template <typename... P, typename... A>
-void launch_pdl(cudaStream_t st, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, A&&... args) {
+void launch_clusters(cudaStream_t st, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, unsigned cluster,
+                     A&&... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = cluster;
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = cluster > 1 ? 2 : 1;
   const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
   if (e != cudaSuccess) throw CudaError(e, "cudaLaunchKernelEx", __FILE__, __LINE__);
   count_launch();
+}
+template <typename... P, typename... A>
+void launch_pdl(cudaStream_t st, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, A&&... args) {
+  launch_clusters(st, kernel, grid, block, smem, 1u, args...);
 }
 // A bounded device wait gave up (its poll limit ran out); the engine has cleared the error word
 // and stays usable.

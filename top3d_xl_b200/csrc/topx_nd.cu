@@ -21,6 +21,7 @@
 #include "topx_kernels.cuh"
 #include "topx_nd.hpp"
 #include "topx_nd_dev.hpp"
+#include "topx_pcg.cuh"
 #include "topx_tile64.cuh"
 
 namespace topx {
@@ -564,6 +565,142 @@ __global__ void __launch_bounds__(ND_THREADS) k_nd_solve_flow(NDSolveArgs<T, TM>
   }
 }
 
+// ---------------------------------------------------------------------------
+// small grids: the V-cycle below level 1 as one cluster
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ void cluster_sync() {  // writes before it are visible to the cluster after it
+  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+constexpr int SC_THREADS = 512, SC_WARPS = SC_THREADS / 32;
+constexpr int SC_TILES = 15;  // 3 * kNdOneFrontNodes DOFs
+static_assert(SC_TILES * ND_T >= 3 * kNdOneFrontNodes && SC_TILES <= kSmallCoarseCtas, "a tile row per CTA");
+
+// Four launches of 4 to 8 us each took these steps when each has a few hundred outputs.  Sixteen CTAs in a cluster
+// take them with three hardware barriers in between (well under a microsecond each) and no co-residency to ask
+// for, so engines that share the GPU use it as well.  All sums are formed in FP64; values another CTA wrote
+// are read past L1.
+template <typename TC>
+__global__ void __launch_bounds__(SC_THREADS) k_small_coarse(const __grid_constant__ SmallCoarse<TC> a) {
+  pdl_wait();
+  if (a.dot && !a.init && a.sc->done) return;  // the same in every CTA, or about to be (pcg_decide)
+  if (!a.dot && a.sc && a.sc->done) return;
+  if (a.dot && pcg_decide(a.sc, a.parts, a.init, a.tol, a.maxIT)) return;
+  __shared__ double vec[SC_TILES * ND_T];
+  __shared__ double red[2 * SC_TILES][ND_T];
+  const int rank = blockIdx.x, tid = threadIdx.x, gid = rank * SC_THREADS + tid, all = kSmallCoarseCtas * SC_THREADS;
+  const int cy = a.g1.nny(), cx = a.g1.nnx(), n1 = int(a.g1.nnodes());
+  {  // x and z passes: eight lanes per level-2 node, seven of them with a z tap each
+    const int fx = a.g0.nnx(), fz = a.g0.nnz();
+    const int64_t ts = int64_t(cy) * fx * fz;
+    const int sub = tid & 7;
+    for (int m0 = 0; m0 < n1; m0 += all / 8) {
+      const int m = m0 + (gid >> 3);
+      double t[3] = {0.0, 0.0, 0.0};
+      const int oy = m % cy, ox = (m / cy) % cx, oz = m / (cy * cx), iz = KU_SPAN * oz + sub - (KU_SPAN - 1);
+      if (m < n1 && sub < 2 * KU_SPAN - 1 && iz >= 0 && iz < fz) {
+#pragma unroll
+        for (int dx = -(KU_SPAN - 1); dx <= KU_SPAN - 1; ++dx) {
+          const int ix = KU_SPAN * ox + dx;
+          if (ix < 0 || ix >= fx) continue;
+          const double w = double(KU_SPAN - (dx < 0 ? -dx : dx)) / KU_SPAN;
+          const int64_t k = oy + int64_t(cy) * (ix + int64_t(fx) * iz);
+#pragma unroll
+          for (int c = 0; c < 3; ++c) t[c] = fma(w, a.tmp[k + c * ts], t[c]);
+        }
+        const int dz = sub - (KU_SPAN - 1);
+        const double w = double(KU_SPAN - (dz < 0 ? -dz : dz)) / KU_SPAN;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) t[c] *= w;
+      }
+#pragma unroll
+      for (int c = 0; c < 3; ++c)
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) t[c] += __shfl_xor_sync(0xffffffffu, t[c], o);
+      if (m < n1 && sub < 3) {
+        const double v = sub == 0 ? t[0] : sub == 1 ? t[1] : t[2];
+        a.r1[m + sub * a.g1.stride] = TC(v);
+        if (a.r1_64) a.r1_64[m + sub * a.g1.stride] = v;
+      }
+    }
+  }
+  cluster_sync();
+  {  // to the coarsest level: a thread per DOF
+    const int ny = a.g2.nny(), nx = a.g2.nnx(), n2 = int(a.g2.nnodes());
+    for (int i = gid; i < 3 * n2; i += all) {
+      const int c = i / n2, m = i - c * n2, oy = m % ny, ox = (m / ny) % nx, oz = m / (ny * nx);
+      double s = 0.0;
+#pragma unroll
+      for (int d = 0; d < 27; ++d) {
+        const int dy = d % 3 - 1, dx = d / 3 % 3 - 1, dz = d / 9 - 1;
+        const int iy = 2 * oy + dy, ix = 2 * ox + dx, iz = 2 * oz + dz;
+        if (iy < 0 || iy >= cy || ix < 0 || ix >= cx || iz < 0 || iz > a.g1.nz) continue;
+        const double w = (dy ? 0.5 : 1.0) * (dx ? 0.5 : 1.0) * (dz ? 0.5 : 1.0);
+        s = fma(w, double(__ldcg(a.r1 + iy + cy * (ix + cx * iz) + c * a.g1.stride)), s);
+      }
+      a.r2[m + c * a.g2.stride] = TC(s);
+    }
+  }
+  cluster_sync();
+  {  // x = F11^-1 b: CTA r takes tile row r, a warp a half tile at a time
+    const NDFront& d = a.front;
+    const int warp = tid >> 5, lane = tid & 31, h = lane >> 4, c = lane & 15;
+    for (int i = tid; i < d.T1 * ND_T; i += SC_THREADS) {
+      const int32_t g = a.sep_dof[d.pos0 + i];
+      vec[i] = g >= 0 ? double(__ldcg(a.r2 + g)) : 0.0;
+    }
+    if (const int i = rank; i < d.T1) {
+      for (int e = tid; e < 2 * d.T1 * ND_T; e += SC_THREADS) red[e / ND_T][e % ND_T] = 0.0;
+      __syncthreads();
+      for (int u = warp; u < 2 * d.T1; u += SC_WARPS) {
+        const int j = u >> 1, rh = u & 1;
+        if (j <= i)
+          nd_chunk_rows(nd_tile_c(a.tiles, d, i, j), vec + ND_T * j, red[u], rh, h, c);
+        else  // F11^-1 (i, j) = (stored tile (j, i))^T
+          nd_chunk_cols(nd_tile_c(a.tiles, d, j, i), vec + ND_T * j, red[u], rh, h, c);
+      }
+      __syncthreads();
+      if (tid < ND_T) {
+        double s = 0.0;
+        for (int u = 0; u < 2 * d.T1; ++u) s += red[u][tid];
+        const int32_t g = a.sep_dof[d.pos0 + ND_T * i + tid];
+        if (g >= 0) a.x2[g] = TC(s);
+      }
+    }
+  }
+  cluster_sync();
+  // prolongation to level 2 with the Jacobi smoothing (k_prolong_smooth), and its part of z'r
+  double zr = 0.0;
+  const int cny = a.g2.nny(), cnx = a.g2.nnx();
+  for (int m = gid; m < n1; m += all) {
+    const int fy = m % cy, fx = (m / cy) % cx, fz = m / (cy * cx);
+    const bool pres = a.present1[m] != 0;
+    const int Y = fy / 2, X = fx / 2, Z = fz / 2, ty = fy & 1, tx = fx & 1, tz = fz & 1;
+    double pc[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const int oy = hex_ly(k), ox = hex_lx(k), oz = hex_lz(k);
+      if ((oy && ty == 0) || (ox && tx == 0) || (oz && tz == 0)) continue;
+      const double w = (ty ? 0.5 : 1.0) * (tx ? 0.5 : 1.0) * (tz ? 0.5 : 1.0);
+      const int n = (Y + oy) + cny * ((X + ox) + cnx * (Z + oz));
+#pragma unroll
+      for (int c = 0; c < 3; ++c) pc[c] = fma(w, double(__ldcg(a.x2 + n + c * a.g2.stride)), pc[c]);
+    }
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      const int64_t n = m + c * a.g1.stride;
+      const double rv = double(__ldcg(a.r1 + n)), rc = a.r1_64 ? __ldcg(a.r1_64 + n) : rv;
+      const TC x = pres ? TC(fma(2.0 * a.omega * rv, double(a.d1[n]), pc[c])) : TC(0);
+      a.x1[n] = x;
+      zr = fma(double(x), rc, zr);
+    }
+  }
+  if (a.dot) {
+    double v[1] = {zr};
+    parts_leave<1>(v, {a.parts.dot.part});
+  }
+}
+
 // one CTA waits for a counter that nothing raises
 __global__ void k_coop_wait_selftest(CoopControl* ctl) {
   pdl_wait();
@@ -583,6 +720,8 @@ void prepare_nd_kernels() {
   TOPX_CUDA_OK(cudaGetDevice(&dev));
   std::lock_guard<std::mutex> lock(mu);
   if (dev >= 0 && dev < 64 && done[dev]) return;
+  TOPX_CUDA_OK(cudaFuncSetAttribute(k_small_coarse<double>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  TOPX_CUDA_OK(cudaFuncSetAttribute(k_small_coarse<float>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
   TOPX_CUDA_OK(cudaFuncSetAttribute(k_nd_pivot, cudaFuncAttributeMaxDynamicSharedMemorySize, int(ND_SMEM_SWEEP)));
   TOPX_CUDA_OK(cudaFuncSetAttribute(k_nd_panel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(ND_SMEM_SWEEP)));
   TOPX_CUDA_OK(cudaFuncSetAttribute(k_nd_update, cudaFuncAttributeMaxDynamicSharedMemorySize, int(ND_SMEM_SWEEP)));
@@ -659,6 +798,33 @@ void NDDevice::solve(cudaStream_t st, const NDPlan& P, const TM* tiles, const T*
   }
   TOPX_CUDA_OK(cudaGetLastError());
 }
+
+// One front, within the cluster's tile rows; up to 16384 level-2 nodes (four passes of the cluster's threads), beyond
+// which the separate launches' many CTAs win.
+bool small_coarse(const NDPlan& P, int levels, Grid g1) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(kSmallCoarseCtas);
+  cfg.blockDim = dim3(SC_THREADS);
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = kSmallCoarseCtas;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  int n = 0;
+  if (cudaOccupancyMaxActiveClusters(&n, k_small_coarse<double>, &cfg) != cudaSuccess) {
+    cudaGetLastError();
+    n = 0;
+  }
+  return n > 0 && levels == 3 && P.fronts.size() == 1 && P.fronts[0].n2 == 0 && P.fronts[0].T1 >= 1 &&
+         P.fronts[0].T1 <= SC_TILES && g1.nnodes() <= 16384;
+}
+template <typename TC>
+void launch_small_coarse(cudaStream_t st, const SmallCoarse<TC>& a) {
+  launch_clusters(st, k_small_coarse<TC>, kSmallCoarseCtas, SC_THREADS, 0, kSmallCoarseCtas, a);
+}
+template void launch_small_coarse<double>(cudaStream_t, const SmallCoarse<double>&);
+template void launch_small_coarse<float>(cudaStream_t, const SmallCoarse<float>&);
 
 int nd_solve_coop_ctas() {
   int dev = 0, coop = 0, nsm = 0, per = 0, per32 = 0;

@@ -39,6 +39,31 @@ struct NDDevice {
   void solve(cudaStream_t st, const NDPlan& P, const TM* tiles, const T* b, T* x, const PcgScalars* sc) const;
 };
 
+// The coarse part of the V-cycle of a small grid in one launch (small_coarse): the x and z passes of the level-1
+// restriction, the restriction to the coarsest level, its solve with the one front's inverse, and the prolongation
+// to level 2.  TC: the preconditioner's type.
+template <typename TC>
+struct SmallCoarse {
+  const double* tmp;    // y pass of the level-1 restriction
+  Grid g0, g1, g2;      // levels 1, 2 and 3 (the coarsest)
+  TC *r1, *r2, *x2, *x1;
+  double* r1_64;        // FP64 copy of r1 (null when TC is double)
+  const TC* d1;
+  const uint8_t* present1;
+  NDFront front;
+  const TC* tiles;
+  const int32_t* sep_dof;
+  PcgScalars* sc;
+  PcgParts parts;       // inside the PCG (dot), else empty
+  bool dot, init;
+  double tol, omega;
+  int maxIT;
+};
+constexpr int kSmallCoarseCtas = 16;  // one cluster, a tile row of the front each
+bool small_coarse(const NDPlan& P, int levels, Grid g1);
+template <typename TC>
+void launch_small_coarse(cudaStream_t st, const SmallCoarse<TC>& a);
+
 // kernel attributes (once per device; outside stream capture)
 void prepare_nd_kernels();
 // CTAs of the persistent solve on the current device (all resident), or 0 when the device has
