@@ -392,3 +392,27 @@ def test_small_coarse_levels(shape, holes, precision):
         for seed in (3, 4):
             r = np.random.default_rng(seed).standard_normal(m.levels[0].numDOFs)
             assert _rel(ctx.vcycle(r), sol.vcycle(r)) < (1e-10 if precision == "fp64" else 1e-5)
+
+
+@pytest.mark.parametrize("shape", [(52, 56, 52), (52, 52, 60)])
+@pytest.mark.parametrize("holes", [False, True])
+def test_galerkin_group_sizes(shape, holes):
+    # 13 x 14 x 13 = 2366 level-2 elements go two to a block, 13 x 13 x 15 = 2535 sixteen (the last block is short);
+    # with holes some groups are void, and both have elements with BC-modified templates; test_vcycle's bar
+    from top3d_xl_b200 import Context
+    vox = np.ones(shape, bool)
+    if holes:
+        vox[:, 1:-1, :] = np.random.default_rng(5).random((shape[0], shape[1] - 2, shape[2])) < 0.8
+        vox[8:40, 8:44, 12:20] = False
+    m = O.build_model(vox)
+    x = np.random.default_rng(1).uniform(0.3, 1.0, m.levels[0].numElements)
+    S = m.S
+    E = S.modulusMin + x ** S.SIMPpenalty * (S.modulus - S.modulusMin)
+    sol = O.Solver(m)
+    sol.assemble(E)
+    with Context("fp64") as ctx:
+        ctx.load_voxels(vox)
+        ctx.set_moduli(E)
+        ctx.assemble()
+        r = np.random.default_rng(3).standard_normal(m.levels[0].numDOFs)
+        assert _rel(ctx.vcycle(r), sol.vcycle(r)) < 1e-10

@@ -198,14 +198,10 @@ Engine::Engine(Model& model, int precision, int device, bool coarse_coop) : M(mo
       fl_elem.upload(fe.data(), fe.size());
       fl_tsel.upload(ts.data(), ts.size());
       fl_F.upload(ff.data(), ff.size());
+      std::vector<uint8_t> fl(size_t(G[1].nelems()), 0);
+      for (int32_t e : fe) fl[size_t(e)] = 1;
+      flagged.upload(fl.data(), fl.size());
     }
-    // span-2 child prolongators P_c = W_c (x) I_3: their node weights
-    const std::vector<double> P2 = child_prolongators(2);
-    std::vector<double> w8(8 * 64);
-    for (int c = 0; c < 8; ++c)
-      for (int a = 0; a < 8; ++a)
-        for (int b = 0; b < 8; ++b) w8[size_t(c) * 64 + 8 * a + b] = P2[size_t(c) * 576 + (3 * a) * 24 + 3 * b];
-    W8.upload(w8.data(), w8.size());
   }
   Ks.resize(nl);
   for (int l = 1; l < nl; ++l) Ks[l].alloc(size_t(G[l].nelems()) * 576);
@@ -526,11 +522,10 @@ void Engine::assemble_launches() {
     launch_diag_l1<float>(st, G[0], E64.p, fixbits.p, cfix64.p, present[0].p, v32.d1.p, d0.p);
   sec_end();
   sec_begin(SEC_GALERKIN2);
-  launch_galerkin_l2(st, G[0], G[1], E64.p, Tall.p, Ks[1].p);
-  launch_galerkin_l2_flagged(st, G[0], G[1], E64.p, nflag, fl_elem.p, fl_tsel.p, fl_F.p, Tall.p, Ks[1].p);
+  launch_galerkin_l2(st, G[0], G[1], E64.p, Tall.p, nflag, fl_elem.p, fl_tsel.p, fl_F.p, flagged.p, Ks[1].p);
   sec_end();
   sec_begin(SEC_GALERKIN3);
-  for (int l = 2; l < nl; ++l) launch_galerkin_span2(st, G[l], Ks[l - 1].p, epresent[l].p, W8.p, Ks[l].p);
+  for (int l = 2; l < nl; ++l) launch_galerkin_span2(st, G[l], Ks[l - 1].p, epresent[l].p, Ks[l].p);
   sec_end();
   sec_begin(SEC_DIAG);
   for (int l = 1; l < nl - 1; ++l) {
