@@ -172,8 +172,8 @@ __device__ __forceinline__ void nd_finalize_task(const NDFront& d, NDTask tk, do
 __device__ __forceinline__ void nd_pivot_acc(double (&acc)[4][2][2], double* A, double* scr, const NDFront& d,
                                              double* smem) {
   double* Pinv = scr + int64_t(d.scr0) * ND_TILE;
-  gf_pivot(acc, nullptr, 0, 0, ND_T, Pinv, *reinterpret_cast<GFPivotSmem*>(smem));
-  gf_for_outputs(acc, [&](int r, int c, double v) { A[r * ND_T + c] = v; });
+  gf_pivot(acc, Pinv, *reinterpret_cast<GFPivotSmem*>(smem));
+  gf_store_acc(A, acc);
 }
 
 // Blocks [0, npiv): pivot of step 0 of front f (tile (0, 0) <- its inverse, also into scratch

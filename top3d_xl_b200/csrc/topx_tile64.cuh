@@ -117,35 +117,63 @@ struct GFPivotSmem {
   double rowS[2][8][72];   // pivot row block (old values), double-buffered by step
   double colT[2][8][72];   // pivot column block, transposed: colT[t][row]
   double rowR[2][8][72];   // R = -Pinv rowS per warp row (wr)
-  double pinv[8][8];
+  double pinv[2][8][8];    // inverse of the pivot block, double-buffered by step
 };
 static_assert(sizeof(GFPivotSmem) <= GF_BUF * sizeof(double), "pivot workspace exceeds a staging buffer");
 
-// 1/v: hardware reciprocal approximation refined by two Newton-Raphson steps
-// x <- x + x (1 - v x) (each doubles the correct bits), off the long IEEE division.
+// 1/v: the hardware approximation x (it keeps 20 bits), then with e = 1 - v x the series x (1 + e + e^2), whose
+// remainder e^3 is below 2^-56: three dependent operations, off the long IEEE division.
 __device__ __forceinline__ double gf_recip(double v) {
   double x;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(x) : "d"(v));
-  double e = fma(-v, x, 1.0);
-  x = fma(x, e, x);
-  e = fma(-v, x, 1.0);
-  return fma(x, e, x);
+  const double e = fma(-v, x, 1.0);
+  return fma(x, fma(e, e, e), x);
 }
-// PIV: the 64 x 64 diagonal tile (identity beyond kb) inverted by blocked Gauss-Jordan exchange
-// on 8-wide pivot blocks, held in registers in the FP64 tensor-core accumulator layout of
-// gf_product (warp (wr, wc) = rows 32 wr.., columns 16 wc..).  Per block S:
+
+// Pivot t of the 8 x 8 pivot block's Gauss-Jordan inversion in one warp: lane (g, q) holds P[g][2q], P[g][2q+1].
+__device__ __forceinline__ void gf_pivot_step(int t, double& p0, double& p1) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
+  // pivot value in lane 4t + t/2, pivot row at my columns in lane 4t + q, my row's pivot
+  // column in lane 4g + t/2
+  const double pt = __shfl_sync(0xffffffffu, (t & 1) ? p1 : p0, 4 * t + (t >> 1));
+  const double rt0 = __shfl_sync(0xffffffffu, p0, 4 * t + q);
+  const double rt1 = __shfl_sync(0xffffffffu, p1, 4 * t + q);
+  const double ct = __shfl_sync(0xffffffffu, (t & 1) ? p1 : p0, 4 * g + (t >> 1));
+  const double d = gf_recip(pt);
+  const double cd = ct * d;
+  if (g == t) {
+    p0 = (2 * q == t) ? d : -d * rt0;
+    p1 = (2 * q + 1 == t) ? d : -d * rt1;
+  } else {
+    p0 = (2 * q == t) ? cd : fma(-cd, rt0, p0);
+    p1 = (2 * q + 1 == t) ? cd : fma(-cd, rt1, p1);
+  }
+}
+
+// PIV: the 64 x 64 tile in acc inverted by blocked Gauss-Jordan exchange on 8-wide pivot blocks,
+// held in registers in the FP64 tensor-core accumulator layout of gf_product (warp (wr, wc) =
+// rows 32 wr.., columns 16 wc..).  Per block S, with P^-1 = A[S, S]^-1 at hand:
 //   the owners publish row block A[S, :] and column block A[:, S] to shared memory;
-//   warp 0 inverts P = A[S, S] (one pivot per step, operands by shuffles);
 //   every warp forms R = -P^-1 A[S, cols] for its columns and then, on the tensor cores,
-//   A[i, j] += A[i, S] R_j,  A[i, S] = A[i, S] P^-1,  A[S, j] = R_j,  A[S, S] = P^-1.
-// acc: the tile (identity beyond kb) on entry, P^-1 on return (also stored to Pinv, and to the
-// tile's place in M unless M is null).
-__device__ __forceinline__ void gf_pivot(double (&acc)[4][2][2], double* __restrict__ M, int m, int k0, int kb,
-                                         double* __restrict__ Pinv, GFPivotSmem& sm) {
+//   A[i, j] += A[i, S] R_j,  A[i, S] = A[i, S] P^-1,  A[S, j] = R_j,  A[S, S] = P^-1;
+//   the warp that holds the next pivot block updates it first and inverts it while the others form their products.
+// The chain of the 64 pivots bounds it.  With the inversion by warp 0 before the products, two barriers a block and one
+// more dependent operation in a reciprocal, the factorisation of 50 x 100 x 50 elements took 482 us, now 445;
+// 64 x 128 x 64: 489, now 469; 128 x 256 x 128: 2510, now 2323.  (Pivot steps between the products wait for the FP64
+// unit that those keep busy: 2 us a tile slower than pivot steps before them; so are products with the pivot row formed
+// beside the reciprocal, by the operations they add.)
+// acc: the tile on entry, its inverse on return (also stored to Pinv).
+__device__ __forceinline__ void gf_pivot(double (&acc)[4][2][2], double* __restrict__ Pinv, GFPivotSmem& sm) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
   const int wr = warp >> 2, wc = warp & 3, rb = wr * 32, cb = wc * 16;
-  const int nsteps = (kb + 7) >> 3;
-  for (int s = 0; s < nsteps; ++s) {
+  double p0 = acc[0][0][0], p1 = acc[0][0][1];
+  if (warp == 0) {
+#pragma unroll
+    for (int t = 0; t < 8; ++t) gf_pivot_step(t, p0, p1);
+    *reinterpret_cast<double2*>(&sm.pinv[0][g][2 * q]) = make_double2(p0, p1);
+  }
+#pragma unroll 1
+  for (int s = 0; s < 8; ++s) {
     const int buf = s & 1;
     const int sfr = s & 3, swr = s >> 2, sfc = s & 1, swc = s >> 1;
     // publish the pivot row block (warps of row half swr, fragment row sfr) and column block
@@ -168,29 +196,7 @@ __device__ __forceinline__ void gf_pivot(double (&acc)[4][2][2], double* __restr
           }
     }
     __syncthreads();
-    if (warp == 0) {  // 8 x 8 pivot block inverse, one pivot per step: lane holds P[g][2q], P[g][2q+1]
-      double p0 = sm.rowS[buf][g][8 * s + 2 * q], p1 = sm.rowS[buf][g][8 * s + 2 * q + 1];
-#pragma unroll
-      for (int t = 0; t < 8; ++t) {
-        // pivot value in lane 4t + t/2, pivot row at my columns in lane 4t + q, my row's pivot
-        // column in lane 4g + t/2
-        const double pt = __shfl_sync(0xffffffffu, (t & 1) ? p1 : p0, 4 * t + (t >> 1));
-        const double rt0 = __shfl_sync(0xffffffffu, p0, 4 * t + q);
-        const double rt1 = __shfl_sync(0xffffffffu, p1, 4 * t + q);
-        const double ct = __shfl_sync(0xffffffffu, (t & 1) ? p1 : p0, 4 * g + (t >> 1));
-        const double d = gf_recip(pt);
-        const double cd = ct * d;
-        if (g == t) {
-          p0 = (2 * q == t) ? d : -d * rt0;
-          p1 = (2 * q + 1 == t) ? d : -d * rt1;
-        } else {
-          p0 = (2 * q == t) ? cd : fma(-cd, rt0, p0);
-          p1 = (2 * q + 1 == t) ? cd : fma(-cd, rt1, p1);
-        }
-      }
-      *reinterpret_cast<double2*>(&sm.pinv[g][2 * q]) = make_double2(p0, p1);
-    }
-    __syncthreads();
+    const double(*pinv)[8] = sm.pinv[buf];
     // R = -Pinv rowS for this warp's 16 columns (D layout: R[g][cb + 8 fc + 2q + h])
     double R[2][2];
 #pragma unroll
@@ -198,12 +204,31 @@ __device__ __forceinline__ void gf_pivot(double (&acc)[4][2][2], double* __restr
       R[fc][0] = R[fc][1] = 0.0;
 #pragma unroll
       for (int k4 = 0; k4 < 2; ++k4)
-        gf_dmma(R[fc][0], R[fc][1], sm.pinv[g][4 * k4 + q], sm.rowS[buf][4 * k4 + q][cb + 8 * fc + g]);
+        gf_dmma(R[fc][0], R[fc][1], pinv[g][4 * k4 + q], sm.rowS[buf][4 * k4 + q][cb + 8 * fc + g]);
       R[fc][0] = -R[fc][0];
       R[fc][1] = -R[fc][1];
       *reinterpret_cast<double2*>(&sm.rowR[wr][g][cb + 8 * fc + 2 * q]) = make_double2(R[fc][0], R[fc][1]);
     }
     __syncwarp();
+    // the next pivot block, in the warp that holds it: A + C R as for every fragment below
+    const int n = s + 1, nfr = n & 3, nfc = n & 1;
+    const bool ahead = n < 8 && wr == n >> 2 && wc == n >> 1;
+    if (ahead) {
+#pragma unroll
+      for (int fr = 0; fr < 4; ++fr)
+#pragma unroll
+        for (int fc = 0; fc < 2; ++fc)
+          if (fr == nfr && fc == nfc) {
+            p0 = acc[fr][fc][0];
+            p1 = acc[fr][fc][1];
+          }
+#pragma unroll
+      for (int k4 = 0; k4 < 2; ++k4)
+        gf_dmma(p0, p1, sm.colT[buf][4 * k4 + q][rb + 8 * nfr + g], sm.rowR[wr][4 * k4 + q][cb + 8 * nfc + g]);
+#pragma unroll
+      for (int t = 0; t < 8; ++t) gf_pivot_step(t, p0, p1);
+      *reinterpret_cast<double2*>(&sm.pinv[buf ^ 1][g][2 * q]) = make_double2(p0, p1);
+    }
     // one tensor-core product for every fragment (no branches, so the products interleave):
     // column block S takes C P^-1 (B = P^-1, from zero), all others A + C R; the pivot row
     // block then takes R and the pivot block P^-1
@@ -215,7 +240,7 @@ __device__ __forceinline__ void gf_pivot(double (&acc)[4][2][2], double* __restr
 #pragma unroll
       for (int fc = 0; fc < 2; ++fc) {
         const bool inCol = (wc == swc && fc == sfc);
-        const double* bsrc = inCol ? &sm.pinv[q][g] : &sm.rowR[wr][q][cb + 8 * fc + g];
+        const double* bsrc = inCol ? &pinv[q][g] : &sm.rowR[wr][q][cb + 8 * fc + g];
         const int bstep = inCol ? 4 * 8 : 4 * 72;  // 4 rows down in pinv or rowR
         acc[fr][fc][0] = inCol ? 0.0 : acc[fr][fc][0];
         acc[fr][fc][1] = inCol ? 0.0 : acc[fr][fc][1];
@@ -230,21 +255,17 @@ __device__ __forceinline__ void gf_pivot(double (&acc)[4][2][2], double* __restr
 #pragma unroll
           for (int fc = 0; fc < 2; ++fc) {
             const bool inCol = (wc == swc && fc == sfc);
-            acc[fr][fc][0] = inCol ? sm.pinv[g][2 * q] : R[fc][0];
-            acc[fr][fc][1] = inCol ? sm.pinv[g][2 * q + 1] : R[fc][1];
+            acc[fr][fc][0] = inCol ? pinv[g][2 * q] : R[fc][0];
+            acc[fr][fc][1] = inCol ? pinv[g][2 * q + 1] : R[fc][1];
           }
     }
   }
-  // outputs: Pinv into the ring and the tile of M
 #pragma unroll
   for (int fr = 0; fr < 4; ++fr)
 #pragma unroll
     for (int fc = 0; fc < 2; ++fc) {
       const int r = rb + 8 * fr + g, c = cb + 8 * fc + 2 * q;
       *reinterpret_cast<double2*>(Pinv + r * 64 + c) = make_double2(acc[fr][fc][0], acc[fr][fc][1]);
-#pragma unroll
-      for (int h = 0; h < 2; ++h)
-        if (M && r < kb && c + h < kb) M[int64_t(k0 + r) * m + k0 + c + h] = acc[fr][fc][h];
     }
 }
 
