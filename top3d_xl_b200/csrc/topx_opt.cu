@@ -137,6 +137,10 @@ void launch_oc_prep(cudaStream_t st, int64_t Ne, const double* x, const double* 
 // included, that D launches of a one-step kernel take.  Every node's midpoint and sum are
 // formed as the one-step kernel forms them (same expressions, same per-thread order, same
 // block-order reduction), so l1, l2, lmid and the step count come out bit-identical.
+// Bound by the launch and the reduction, whose 15 sums cost a block as much as a dozen elements do: two blocks an SM,
+// more elements a thread (four of its loads in flight).  The bisection and the final pass, us, with a thread per element
+// and three steps a launch, three steps, four, five (its sums spill): 50 x 100 x 50 elements 258, 185, 179, 306;
+// 64 x 128 x 64: 419, 223, 213, 398; 96 x 192 x 96: 550, 355, 369, 710.
 // In the per-element clamp, max(0, max(x - move, min(1, min(x + move, t)))) is regrouped as
 // max(lo, min(hi, t)) with lo = max(0, x - move), hi = min(1, x + move) formed once per element,
 // and the two outer selections are written as comparisons (a NaN t, from a positive dc, selects
@@ -144,7 +148,7 @@ void launch_oc_prep(cudaStream_t st, int64_t Ne, const double* x, const double* 
 // the sign of a zero term of the sum).
 constexpr int kOcNodes = (1 << kOcStepsPerLaunch) - 1;
 
-__global__ void __launch_bounds__(256) k_oc_bisect(int64_t Ne, const double* __restrict__ x,
+__global__ void __launch_bounds__(256, 2) k_oc_bisect(int64_t Ne, const double* __restrict__ x,
                                                    const double* __restrict__ w, const uint8_t* __restrict__ passive,
                                                    OcState* os, RedScratch rs, double move) {
   pdl_wait();
@@ -173,19 +177,32 @@ __global__ void __launch_bounds__(256) k_oc_bisect(int64_t Ne, const double* __r
   double s[kOcNodes];
 #pragma unroll
   for (int j = 0; j < kOcNodes; ++j) s[j] = 0.0;
-  for (int64_t e = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; e < Ne; e += int64_t(gridDim.x) * blockDim.x) {
-    const double xv = x[e];
-    if (passive && passive[e]) {
+  constexpr int BATCH = 4;
+  const int64_t stride = int64_t(gridDim.x) * blockDim.x;
+  for (int64_t e0 = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; e0 < Ne; e0 += BATCH * stride) {
+    double xv[BATCH], wv[BATCH];
+    bool pas[BATCH];
 #pragma unroll
-      for (int j = 0; j < kOcNodes; ++j) s[j] += 1.0 - xv;
-    } else {
-      const double wv = w[e];
-      const double lo = fmax(0.0, xv - move), hi = fmin(1.0, xv + move);
+    for (int b = 0; b < BATCH; ++b) {
+      const int64_t e = e0 + b * stride;
+      xv[b] = e < Ne ? x[e] : 0.0;
+      wv[b] = e < Ne ? w[e] : 0.0;
+      pas[b] = passive && e < Ne && passive[e];
+    }
 #pragma unroll
-      for (int j = 0; j < kOcNodes; ++j) {
-        const double t = wv * r[j];
-        const double u = t < hi ? t : hi;
-        s[j] += (u > lo ? u : lo) - xv;
+    for (int b = 0; b < BATCH; ++b) {
+      if (e0 + b * stride >= Ne) break;
+      if (pas[b]) {
+#pragma unroll
+        for (int j = 0; j < kOcNodes; ++j) s[j] += 1.0 - xv[b];
+      } else {
+        const double lo = fmax(0.0, xv[b] - move), hi = fmin(1.0, xv[b] + move);
+#pragma unroll
+        for (int j = 0; j < kOcNodes; ++j) {
+          const double t = wv[b] * r[j];
+          const double u = t < hi ? t : hi;
+          s[j] += (u > lo ? u : lo) - xv[b];
+        }
       }
     }
   }
@@ -218,8 +235,8 @@ __global__ void __launch_bounds__(256) k_oc_bisect(int64_t Ne, const double* __r
 }
 void launch_oc_bisect(cudaStream_t st, int64_t Ne, const double* x, const double* w, const uint8_t* passive,
                       OcState* os, RedScratch rs, double move) {
-  const unsigned nb = grid1d(Ne, 256);
-  static_assert(size_t(kOcNodes) * 148 * 16 <= size_t(kMaxRedBlocks) * kMaxRedSlots, "reduction slots");
+  const unsigned nb = grid1d(Ne, 256, 2 * 148);
+  static_assert(size_t(kOcNodes) * 148 * 2 <= size_t(kMaxRedBlocks) * kMaxRedSlots, "reduction slots");
   launch_pdl(st, k_oc_bisect, nb, 256, 0, Ne, x, w, passive, os, rs, move);
   TOPX_CUDA_OK(cudaGetLastError());
 }

@@ -80,7 +80,7 @@ void launch_sum(cudaStream_t st, int64_t n, const double* a, const double* b, do
 void launch_ewise(cudaStream_t st, int op, int64_t n, const double* a, const double* b, double* out, double s);
 // OC bisection (TOP3D_XL.m:145-156): w = x sqrt(-dc) once, then bisection steps on lmid,
 // kOcStepsPerLaunch of them per launch of launch_oc_bisect
-constexpr int kOcStepsPerLaunch = 3;
+constexpr int kOcStepsPerLaunch = 4;
 void launch_oc_prep(cudaStream_t st, int64_t Ne, const double* x, const double* dc, double* w);
 void launch_oc_bisect(cudaStream_t st, int64_t Ne, const double* x, const double* w, const uint8_t* passive,
                       OcState* os, RedScratch rs, double move);
