@@ -1189,10 +1189,8 @@ void Engine::step_local(IterRecord& rec, const ObjState& os) {
                     alpha.p, beta.p, p0.p, q0.p, pij.p, qij.p, mmaS.p, rs1);
   MmaState ms{};
   for (int chunk = 0; chunk < 64; ++chunk) {
-    for (int k = 0; k < 16; ++k) {
-      launch_mma_newton(st, Ne, pas, low.p, upp.p, alpha.p, beta.p, p0.p, q0.p, pij.p, qij.p, mmaS.p, rs1);
-      launch_mma_residual(st, Ne, pas, low.p, upp.p, alpha.p, beta.p, p0.p, q0.p, pij.p, qij.p, xmma.p, mmaS.p, rs1);
-    }
+    for (int k = chunk == 0 ? -1 : 0; k < 16; ++k)
+      launch_mma_step(st, Ne, pas, low.p, upp.p, alpha.p, beta.p, p0.p, q0.p, pij.p, qij.p, xmma.p, mmaS.p, rs1);
     TOPX_CUDA_OK(cudaMemcpyAsync(&ms, mmaS.p, sizeof(ms), cudaMemcpyDeviceToHost, st));
     TOPX_CUDA_OK(cudaStreamSynchronize(st));
     if (ms.finished) break;

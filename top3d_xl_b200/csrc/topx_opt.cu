@@ -346,6 +346,7 @@ __global__ void k_mma_gensub(int64_t n, int iter, double move, const double* __r
     ms->inner = 0;
     ms->total = 0;
     ms->finished = 0;
+    ms->stepped = 0;
   }
 }
 
@@ -369,35 +370,62 @@ __device__ __forceinline__ void mma_x(double lam, double lo, double up, double a
   if (xcl - be > 0) xcl = be;
 }
 
-// one Newton step of the dual interior point method (XYZofLAMBDA, DualGrad,
-// DualHess, DualLineSearch: TOP3D_XL.m:1930-2031)
-__global__ void k_mma_newton(int64_t n, const uint8_t* __restrict__ passive, const double* __restrict__ low,
-                             const double* __restrict__ upp, const double* __restrict__ alpha,
-                             const double* __restrict__ beta, const double* __restrict__ p0,
-                             const double* __restrict__ q0, const double* __restrict__ pij,
-                             const double* __restrict__ qij, MmaState* ms, RedScratch rs) {
+// One pass of the dual interior point method at the multiplier lam: x(lam) and the dual residual of the Newton step that
+// led to lam, with the epsilon schedule (XYZofLAMBDA, DualResidual: TOP3D_XL.m:1967-1984, 2033-2049; not on the first
+// pass, which follows no step), and, unless that ends the solve, the next Newton step (DualGrad, DualHess,
+// DualLineSearch: TOP3D_XL.m:1930-2031).  Bound by reading the eight arrays; residual and Newton step need the same x,
+// so that a step reads them once (128 x 256 x 128 elements, two loops of 11 steps each: 43.18 ms with a pass each, now 42.44).
+__global__ void k_mma_step(int64_t n, const uint8_t* __restrict__ passive, const double* __restrict__ low,
+                           const double* __restrict__ upp, const double* __restrict__ alpha,
+                           const double* __restrict__ beta, const double* __restrict__ p0,
+                           const double* __restrict__ q0, const double* __restrict__ pij,
+                           const double* __restrict__ qij, double* __restrict__ x, MmaState* ms, RedScratch rs) {
   pdl_wait();
   if (ms->finished) return;
   const double lam = fmax(ms->lam, 0.0);
-  double sg = 0.0, sh = 0.0;
+  double sg = 0.0, sh = 0.0, sp = 0.0, sq = 0.0;
   for (int64_t e = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; e < n; e += int64_t(gridDim.x) * blockDim.x) {
     if (passive && passive[e]) continue;
-    const double lo = low[e], up = upp[e];
+    const double lo = low[e], up = upp[e], al = alpha[e], be = beta[e], pe = pij[e], qe = qij[e];
     double xc, xu, pj, qj;
-    mma_x(lam, lo, up, alpha[e], beta[e], p0[e], q0[e], pij[e], qij[e], xc, xu, pj, qj);
+    mma_x(lam, lo, up, al, be, p0[e], q0[e], pe, qe, xc, xu, pj, qj);
+    x[e] = xc;
     const double ux = up - xc, xl = xc - lo;
-    sg += pij[e] / ux + qij[e] / xl;
-    const double PQ = pij[e] / (ux * ux) - qij[e] / (xl * xl);
+    const double pu = pe / ux, ql = qe / xl;
+    sp += pu;
+    sq += ql;
+    sg += pu + ql;
+    const double PQ = pe / (ux * ux) - qe / (xl * xl);
     double df2 = -1.0 / (2.0 * pj / (ux * ux * ux) + 2.0 * qj / (xl * xl * xl));
-    if (xu - alpha[e] < 0) df2 = 0.0;
-    if (xu - beta[e] > 0) df2 = 0.0;
+    if (xu - al < 0) df2 = 0.0;
+    if (xu - be > 0) df2 = 0.0;
     sh += PQ * df2 * PQ;
   }
-  double v[2] = {sg, sh}, tot[2];
-  if (reduce_publish<2>(v, rs, tot) && threadIdx.x == 0) {
-    double L = lam, mu = ms->mu;
-    const double epsi = ms->epsi;
-    const double y = fmax(L - kMmaC, 0.0);
+  double v[4] = {sg, sh, sp, sq}, tot[4];
+  if (reduce_publish<4>(v, rs, tot) && threadIdx.x == 0) {
+    const double L = lam, y = fmax(L - kMmaC, 0.0);
+    double mu = ms->mu, epsi = ms->epsi;
+    ms->lam = L;
+    if (ms->stepped) {
+      double r1 = -ms->b - 0.0 - y + mu;
+      r1 = r1 + tot[2] + tot[3];
+      const double r2 = mu * L - epsi;
+      double err = 0.0;
+      if (err < fabs(r1)) err = fabs(r1);
+      if (err < fabs(r2)) err = fabs(r2);
+      ms->err = err;
+      ms->inner += 1;
+      ms->total += 1;
+      if (!(err > 0.9 * epsi && ms->inner < 100)) {
+        epsi *= 0.1;
+        ms->epsi = epsi;
+        ms->inner = 0;
+        if (!(epsi > ms->tol)) {
+          ms->finished = 1;
+          return;
+        }
+      }
+    }
     double grad = -ms->b - 0.0 - y + tot[0];
     grad = -1.0 * grad - epsi / L;
     double H = tot[1];
@@ -416,61 +444,14 @@ __global__ void k_mma_newton(int64_t n, const uint8_t* __restrict__ passive, con
     ms->mu = mu + theta * s2;
     ms->grad = grad;
     ms->hess = H;
+    ms->stepped = 1;
   }
 }
 
-void launch_mma_newton(cudaStream_t st, int64_t n, const uint8_t* passive, const double* low, const double* upp,
-                       const double* alpha, const double* beta, const double* p0, const double* q0, const double* pij,
-                       const double* qij, MmaState* ms, RedScratch rs) {
-  launch_pdl(st, k_mma_newton, grid1d(n, 256), 256, 0, n, passive, low, upp, alpha, beta, p0, q0, pij, qij, ms, rs);
-  TOPX_CUDA_OK(cudaGetLastError());
-}
-
-// XYZofLAMBDA + DualResidual (TOP3D_XL.m:1967-1984, 2033-2049) and the epsilon schedule
-__global__ void k_mma_residual(int64_t n, const uint8_t* __restrict__ passive, const double* __restrict__ low,
-                               const double* __restrict__ upp, const double* __restrict__ alpha,
-                               const double* __restrict__ beta, const double* __restrict__ p0,
-                               const double* __restrict__ q0, const double* __restrict__ pij,
-                               const double* __restrict__ qij, double* __restrict__ x, MmaState* ms, RedScratch rs) {
-  pdl_wait();
-  if (ms->finished) return;
-  const double lam = fmax(ms->lam, 0.0);
-  double sp = 0.0, sq = 0.0;
-  for (int64_t e = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; e < n; e += int64_t(gridDim.x) * blockDim.x) {
-    if (passive && passive[e]) continue;
-    const double lo = low[e], up = upp[e];
-    double xc, xu, pj, qj;
-    mma_x(lam, lo, up, alpha[e], beta[e], p0[e], q0[e], pij[e], qij[e], xc, xu, pj, qj);
-    x[e] = xc;
-    sp += pij[e] / (up - xc);
-    sq += qij[e] / (xc - lo);
-  }
-  double v[2] = {sp, sq}, tot[2];
-  if (reduce_publish<2>(v, rs, tot) && threadIdx.x == 0) {
-    ms->lam = lam;
-    const double y = fmax(lam - kMmaC, 0.0);
-    double r1 = -ms->b - 0.0 - y + ms->mu;
-    r1 = r1 + tot[0] + tot[1];
-    const double r2 = ms->mu * lam - ms->epsi;
-    double err = 0.0;
-    if (err < fabs(r1)) err = fabs(r1);
-    if (err < fabs(r2)) err = fabs(r2);
-    ms->err = err;
-    ms->inner += 1;
-    ms->total += 1;
-    if (!(err > 0.9 * ms->epsi && ms->inner < 100)) {
-      ms->epsi *= 0.1;
-      ms->inner = 0;
-      if (!(ms->epsi > ms->tol)) ms->finished = 1;
-    }
-  }
-}
-
-void launch_mma_residual(cudaStream_t st, int64_t n, const uint8_t* passive, const double* low, const double* upp,
-                         const double* alpha, const double* beta, const double* p0, const double* q0,
-                         const double* pij, const double* qij, double* x, MmaState* ms, RedScratch rs) {
-  launch_pdl(st, k_mma_residual, grid1d(n, 256), 256, 0, n, passive, low, upp, alpha, beta, p0, q0, pij, qij, x, ms,
-             rs);
+void launch_mma_step(cudaStream_t st, int64_t n, const uint8_t* passive, const double* low, const double* upp,
+                     const double* alpha, const double* beta, const double* p0, const double* q0, const double* pij,
+                     const double* qij, double* x, MmaState* ms, RedScratch rs) {
+  launch_pdl(st, k_mma_step, grid1d(n, 256), 256, 0, n, passive, low, upp, alpha, beta, p0, q0, pij, qij, x, ms, rs);
   TOPX_CUDA_OK(cudaGetLastError());
 }
 

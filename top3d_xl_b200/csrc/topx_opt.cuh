@@ -96,17 +96,15 @@ struct MmaState {
   int inner;      // Newton steps at the current epsilon
   int total;      // Newton steps overall
   int finished;
+  int stepped;    // a Newton step led to lam
 };
 void launch_mma_gensub(cudaStream_t st, int64_t n, int iter, double move, const double* xval, const uint8_t* passive,
                        double* xold1, double* xold2, double* low, double* upp, const double* dfdx, const double* dgdx,
                        double gx, int64_t nact, double* alpha, double* beta, double* p0, double* q0, double* pij,
                        double* qij, MmaState* ms, RedScratch rs);
-void launch_mma_newton(cudaStream_t st, int64_t n, const uint8_t* passive, const double* low, const double* upp,
-                       const double* alpha, const double* beta, const double* p0, const double* q0, const double* pij,
-                       const double* qij, MmaState* ms, RedScratch rs);
-void launch_mma_residual(cudaStream_t st, int64_t n, const uint8_t* passive, const double* low, const double* upp,
-                         const double* alpha, const double* beta, const double* p0, const double* q0,
-                         const double* pij, const double* qij, double* x, MmaState* ms, RedScratch rs);
+void launch_mma_step(cudaStream_t st, int64_t n, const uint8_t* passive, const double* low, const double* upp,
+                     const double* alpha, const double* beta, const double* p0, const double* q0, const double* pij,
+                     const double* qij, double* x, MmaState* ms, RedScratch rs);
 void launch_mma_finish(cudaStream_t st, int64_t n, const uint8_t* passive, const double* xmma, const double* xold1,
                        double* x, MmaState* ms, RedScratch rs);
 // LOCAL driver elementwise chain (TOP3D_XL.m:333-382)
