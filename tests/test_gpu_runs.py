@@ -154,3 +154,18 @@ def test_config3_large_cuboid_global_2_iterations():
     g = np.load(os.path.join(GOLD, "config3_global_2.npz"))
     cs, hist, x = _run(np.ones((128, 256, 128), bool), "GLOBAL", 0.12, 50, np.sqrt(3), 0.0, 2)
     _check(g, cs, hist, x)
+
+
+@pytest.mark.parametrize("shape", [(8, 6, 5), (16, 16, 17), (32, 32, 32), (32, 32, 33), (40, 60, 64)])
+def test_oc_bisection_sizes(shape):
+    # up to 32768 elements the bisection is one cluster launch (one to eight elements a thread, the last ones short),
+    # beyond it launches of several blocks; the volume that it leaves shows any lost element.  Bars of the runs above.
+    import sys
+    sys.path.insert(0, os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
+    from oracle import top3dxl_oracle as O
+    vox = np.ones(shape, bool)
+    h = O.run_global(vox, 0.3, 50, np.sqrt(3), max_loops=1)
+    cs, hist, x = _run(vox, "GLOBAL", 0.3, 50, np.sqrt(3), 0.0, 1)
+    assert abs(cs - h["cSolid"]) / h["cSolid"] < 1e-9
+    assert abs(hist[0]["change"] - h["change"][0]) < 1e-6
+    assert np.max(np.abs(x - h["xPhys"])) < 1e-6

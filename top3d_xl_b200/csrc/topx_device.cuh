@@ -196,6 +196,17 @@ __device__ __forceinline__ void parts_leave(double (&v)[NS], double* const (&par
   }
 }
 
+// Barrier of a cluster: writes before it are visible to the cluster after it.
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// *p = v in the shared memory of CTA `rank` of the cluster (p: the address in this CTA's)
+__device__ __forceinline__ void cluster_store(double* p, unsigned rank, double v) {
+  unsigned a;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(unsigned(__cvta_generic_to_shared(p))), "r"(rank));
+  asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory");
+}
+
 // Max-reduction analogue of reduce_publish (one slot).
 __device__ __forceinline__ bool reduce_publish_max(double v, RedScratch rs, double& out) {
   v = block_max(v);

@@ -23,6 +23,7 @@ Engine::Engine(Model& model, int precision, int device, bool coarse_coop) : M(mo
   TOPX_CUDA_OK(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
   prepare_ku_kernels();
   prepare_filter_kernels();
+  prepare_oc_kernels();
   prepare_nd_kernels();
   nl = M.numLevels;
   if (nl >= 3 && int(M.levels.size()) == nl && M.levels[1].span != KU_SPAN)
@@ -1114,10 +1115,12 @@ bool Engine::step(IterRecord& rec) {
     sec_begin(SEC_OC);
     const uint8_t* pas = passive.p;
     launch_oc_prep(st, Ne, x.p, dc.p, tmpA.p);  // tmpA is free once the filter has run
-    // at most 258 steps: 60 in the first round trip (the interval test usually passes after
+    // at most kOcMostSteps: 60 in the first round trip (the interval test usually passes after
     // 50-60 steps from (0, 1e9)), then 16 per round trip
     static_assert(60 % kOcStepsPerLaunch == 0 && 16 % kOcStepsPerLaunch == 0, "steps per round trip");
-    for (int launched = 0; launched * kOcStepsPerLaunch < 256;) {
+    const bool one = Ne <= kOcClusterElems;
+    if (one) launch_oc_cluster(st, Ne, x.p, tmpA.p, pas, ocS.p, 0.2);
+    for (int launched = 0; !one && launched * kOcStepsPerLaunch < kOcMostSteps;) {
       const int n = (launched == 0 ? 60 : 16) / kOcStepsPerLaunch;
       for (int k = 0; k < n; ++k) launch_oc_bisect(st, Ne, x.p, tmpA.p, pas, ocS.p, rs1, 0.2);
       launched += n;

@@ -588,10 +588,6 @@ __global__ void __launch_bounds__(ND_THREADS) k_nd_solve_flow(NDSolveArgs<T, TM>
 // ---------------------------------------------------------------------------
 // small grids: the V-cycle below level 1 as one cluster
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ void cluster_sync() {  // writes before it are visible to the cluster after it
-  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-
 constexpr int SC_THREADS = 512, SC_WARPS = SC_THREADS / 32;
 constexpr int SC_TILES = 15;  // 3 * kNdOneFrontNodes DOFs
 static_assert(SC_TILES * ND_T >= 3 * kNdOneFrontNodes && SC_TILES <= kSmallCoarseCtas, "a tile row per CTA");

@@ -148,28 +148,47 @@ void launch_oc_prep(cudaStream_t st, int64_t Ne, const double* x, const double* 
 // the sign of a zero term of the sum).
 constexpr int kOcNodes = (1 << kOcStepsPerLaunch) - 1;
 
+// 1/sqrt(lmid) of node j: its interval follows the path from the root
+__device__ __forceinline__ double oc_node(int j, double a, double b) {
+  int depth = 0;
+  while ((j + 1) >> (depth + 1)) ++depth;  // node j sits at depth floor(log2(j + 1))
+  for (int d = depth - 1; d >= 0; --d) {   // the branch taken at each level, root first
+    const int node = ((j + 1) >> (d + 1)) - 1;
+    const double lmid = 0.5 * (b + a);
+    if (j + 1 - ((node + 1) << (d + 1)) < (1 << d))  // lower half: l2 = lmid
+      b = lmid;
+    else
+      a = lmid;
+  }
+  return 1.0 / sqrt(0.5 * (b + a));
+}
+
+// the decisions of kOcStepsPerLaunch steps on the nodes' sums; true once the interval test fails
+__device__ __forceinline__ bool oc_walk(double fval, const double* tot, double& l1, double& l2, double& lmid,
+                                        int& steps) {
+  int j = 0;
+  for (int d = 0; d < kOcStepsPerLaunch; ++d) {
+    lmid = 0.5 * (l2 + l1);
+    if (fval + tot[j] > 0) {
+      l1 = lmid;
+      j = 2 * j + 2;
+    } else {
+      l2 = lmid;
+      j = 2 * j + 1;
+    }
+    steps += 1;
+    if (!((l2 - l1) / (l1 + l2) > 1e-6)) return true;
+  }
+  return false;
+}
+
 __global__ void __launch_bounds__(256, 2) k_oc_bisect(int64_t Ne, const double* __restrict__ x,
                                                    const double* __restrict__ w, const uint8_t* __restrict__ passive,
                                                    OcState* os, RedScratch rs, double move) {
   pdl_wait();
   if (os->converged) return;
-  // thread j < kOcNodes forms node j's 1/sqrt(lmid): its interval follows the path from the root
   __shared__ double sr[kOcNodes];
-  if (threadIdx.x < kOcNodes) {
-    const int j = threadIdx.x;
-    int depth = 0;
-    while ((j + 1) >> (depth + 1)) ++depth;  // node j sits at depth floor(log2(j + 1))
-    double a = os->l1, b = os->l2;
-    for (int d = depth - 1; d >= 0; --d) {  // the branch taken at each level, root first
-      const int node = ((j + 1) >> (d + 1)) - 1;
-      const double lmid = 0.5 * (b + a);
-      if (j + 1 - ((node + 1) << (d + 1)) < (1 << d))  // lower half: l2 = lmid
-        b = lmid;
-      else
-        a = lmid;
-    }
-    sr[j] = 1.0 / sqrt(0.5 * (b + a));
-  }
+  if (threadIdx.x < kOcNodes) sr[threadIdx.x] = oc_node(threadIdx.x, os->l1, os->l2);
   __syncthreads();
   double r[kOcNodes];
 #pragma unroll
@@ -209,23 +228,8 @@ __global__ void __launch_bounds__(256, 2) k_oc_bisect(int64_t Ne, const double* 
   double tot[kOcNodes];
   if (reduce_publish<kOcNodes>(s, rs, tot, gridDim.x) && threadIdx.x == 0) {
     double l1 = os->l1, l2 = os->l2, lmid = os->lmid;
-    int steps = os->steps, conv = 0, j = 0;
-    for (int d = 0; d < kOcStepsPerLaunch; ++d) {
-      lmid = 0.5 * (l2 + l1);
-      const double gt = os->fval + tot[j];
-      if (gt > 0) {
-        l1 = lmid;
-        j = 2 * j + 2;
-      } else {
-        l2 = lmid;
-        j = 2 * j + 1;
-      }
-      steps += 1;
-      if (!((l2 - l1) / (l1 + l2) > 1e-6)) {
-        conv = 1;
-        break;
-      }
-    }
+    int steps = os->steps;
+    const bool conv = oc_walk(os->fval, tot, l1, l2, lmid, steps);
     os->l1 = l1;
     os->l2 = l2;
     os->lmid = lmid;
@@ -238,6 +242,100 @@ void launch_oc_bisect(cudaStream_t st, int64_t Ne, const double* x, const double
   const unsigned nb = grid1d(Ne, 256, 2 * 148);
   static_assert(size_t(kOcNodes) * 148 * 2 <= size_t(kMaxRedBlocks) * kMaxRedSlots, "reduction slots");
   launch_pdl(st, k_oc_bisect, nb, 256, 0, Ne, x, w, passive, os, rs, move);
+  TOPX_CUDA_OK(cudaGetLastError());
+}
+
+// The whole bisection in one launch for a small design: a cluster of eight CTAs keeps x and w in shared memory, and the
+// CTAs leave their sums of the 15 nodes in one another's, so that a round of four steps costs a cluster barrier instead
+// of a launch and its reduction's tail.  Every CTA adds the eight parts in the same order and takes the same decisions.
+// The bisection and the final pass, us, as launches and as a cluster: 16 x 32 x 16 elements 124, 80; 25 x 50 x 25: 127,
+// 119; 32 x 32 x 32: 128, 116; from there on its eight SMs' arithmetic takes longer than the launches.
+constexpr unsigned OCC_CTAS = 8, OCC_THREADS = 512;
+constexpr int OCC_ELEMS = 8;
+static_assert(kOcClusterElems == int64_t(OCC_CTAS) * OCC_THREADS * OCC_ELEMS, "elements of a cluster");
+
+__global__ void __launch_bounds__(OCC_THREADS) k_oc_cluster(int Ne, const double* __restrict__ x,
+                                                            const double* __restrict__ w,
+                                                            const uint8_t* __restrict__ passive, OcState* os,
+                                                            double move) {
+  pdl_wait();
+  __shared__ double part[2][OCC_CTAS][kOcNodes];  // by round parity: a CTA ahead writes the other
+  __shared__ double sr[kOcNodes], tot[kOcNodes];
+  const int tid = threadIdx.x;
+  extern __shared__ double2 occ_xw[];  // x and w of the CTA's elements; a thread reads its own only
+  const int nb = (Ne + int(OCC_CTAS * OCC_THREADS) - 1) / int(OCC_CTAS * OCC_THREADS);  // elements a thread
+  unsigned pas = 0;
+  for (int b = 0; b < nb; ++b) {
+    const int e = (b * int(OCC_CTAS) + int(blockIdx.x)) * int(OCC_THREADS) + tid;
+    // beyond the last element x = w = 0 adds zero to every sum
+    occ_xw[b * int(OCC_THREADS) + tid] = e < Ne ? make_double2(x[e], w[e]) : make_double2(0.0, 0.0);
+    if (passive && e < Ne && passive[e]) pas |= 1u << b;
+  }
+  double l1 = os->l1, l2 = os->l2, lmid = os->lmid;
+  const double fval = os->fval;
+  int steps = os->steps;
+  bool conv = os->converged != 0;
+  cluster_sync();  // every CTA runs: its shared memory may be written
+  for (int round = 0; !conv && round < kOcMostSteps / kOcStepsPerLaunch; ++round) {
+    if (tid < kOcNodes) sr[tid] = oc_node(tid, l1, l2);
+    __syncthreads();
+    double r[kOcNodes], s[kOcNodes];
+#pragma unroll
+    for (int j = 0; j < kOcNodes; ++j) {
+      r[j] = sr[j];
+      s[j] = 0.0;
+    }
+#pragma unroll 1
+    for (int b = 0; b < nb; ++b) {
+      const double2 xw = occ_xw[b * int(OCC_THREADS) + tid];
+      if (pas >> b & 1u) {
+#pragma unroll
+        for (int j = 0; j < kOcNodes; ++j) s[j] += 1.0 - xw.x;
+      } else {
+        const double lo = fmax(0.0, xw.x - move), hi = fmin(1.0, xw.x + move);
+#pragma unroll
+        for (int j = 0; j < kOcNodes; ++j) {
+          const double t = xw.y * r[j];
+          const double u = t < hi ? t : hi;
+          s[j] += (u > lo ? u : lo) - xw.x;
+        }
+      }
+    }
+    block_sum<kOcNodes>(s);
+    double* const mine = part[round & 1][blockIdx.x];
+    if (tid < 32) {  // the sums are in every lane of warp 0: lane p tells CTA p
+      if (tid < int(OCC_CTAS))
+#pragma unroll
+        for (int j = 0; j < kOcNodes; ++j) cluster_store(mine + j, unsigned(tid), s[j]);
+    }
+    cluster_sync();
+    if (tid < kOcNodes) {
+      double t = 0.0;
+#pragma unroll
+      for (unsigned p = 0; p < OCC_CTAS; ++p) t += part[round & 1][p][tid];
+      tot[tid] = t;
+    }
+    __syncthreads();
+    conv = oc_walk(fval, tot, l1, l2, lmid, steps);
+  }
+  if (blockIdx.x == 0 && tid == 0) {
+    os->l1 = l1;
+    os->l2 = l2;
+    os->lmid = lmid;
+    os->steps = steps;
+    os->converged = conv;
+  }
+}
+void prepare_oc_kernels() {
+  TOPX_CUDA_OK(cudaFuncSetAttribute(k_oc_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    int(OCC_ELEMS * OCC_THREADS * sizeof(double2))));
+}
+void launch_oc_cluster(cudaStream_t st, int64_t Ne, const double* x, const double* w, const uint8_t* passive,
+                       OcState* os, double move) {
+  // x and w of the elements that a CTA has
+  const int64_t nb = (Ne + OCC_CTAS * OCC_THREADS - 1) / (OCC_CTAS * OCC_THREADS);
+  launch_clusters(st, k_oc_cluster, OCC_CTAS, OCC_THREADS, size_t(nb) * OCC_THREADS * sizeof(double2), OCC_CTAS, int(Ne),
+                  x, w, passive, os, move);
   TOPX_CUDA_OK(cudaGetLastError());
 }
 

@@ -81,9 +81,15 @@ void launch_ewise(cudaStream_t st, int op, int64_t n, const double* a, const dou
 // OC bisection (TOP3D_XL.m:145-156): w = x sqrt(-dc) once, then bisection steps on lmid,
 // kOcStepsPerLaunch of them per launch of launch_oc_bisect
 constexpr int kOcStepsPerLaunch = 4;
+constexpr int kOcMostSteps = 268;  // the first 60, then 16 at a time
 void launch_oc_prep(cudaStream_t st, int64_t Ne, const double* x, const double* dc, double* w);
 void launch_oc_bisect(cudaStream_t st, int64_t Ne, const double* x, const double* w, const uint8_t* passive,
                       OcState* os, RedScratch rs, double move);
+// all steps in one launch, for up to kOcClusterElems elements
+constexpr int64_t kOcClusterElems = 32768;
+void prepare_oc_kernels();
+void launch_oc_cluster(cudaStream_t st, int64_t Ne, const double* x, const double* w, const uint8_t* passive,
+                       OcState* os, double move);
 void launch_oc_final(cudaStream_t st, int64_t Ne, double* x, const double* w, const uint8_t* passive, double* xPhys,
                      OcState* os, RedScratch rs, RedScratch rs2, double move);
 
