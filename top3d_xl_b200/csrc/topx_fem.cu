@@ -764,6 +764,21 @@ void launch_convert(cudaStream_t st, const TA* a, TB* b, int64_t n) {
   TOPX_CUDA_OK(cudaGetLastError());
 }
 
+// interleaved compact DOF vector (3k+c) -> SoA dense grid field with unknown contents: every entry is written, zero
+// where the domain has no node (node_id: compact id of a grid node or -1), so that the field needs no zeroing first.
+__global__ void k_fill_grid_nodes(const double* __restrict__ src, double* __restrict__ dst, int64_t nnodes,
+                                  int64_t stride, const int32_t* __restrict__ node_id) {
+  pdl_wait();
+  for (int64_t n = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; n < stride; n += int64_t(gridDim.x) * blockDim.x) {
+    const int64_t k = n < nnodes ? node_id[n] : -1;
+    for (int c = 0; c < 3; ++c) dst[n + c * stride] = k >= 0 ? src[3 * k + c] : 0.0;
+  }
+}
+void launch_fill_grid_nodes(cudaStream_t st, const double* src, double* dst, Grid g, const int32_t* node_id) {
+  launch_pdl(st, k_fill_grid_nodes, grid1d(g.stride, 256), 256, 0, src, dst, g.nnodes(), g.stride, node_id);
+  TOPX_CUDA_OK(cudaGetLastError());
+}
+
 // interleaved compact DOF vector (3k+c) -> SoA dense grid field
 template <typename T>
 __global__ void k_c2g_nodes(const double* __restrict__ src, T* __restrict__ dst, Grid g,

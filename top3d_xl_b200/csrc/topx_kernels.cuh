@@ -194,6 +194,7 @@ void launch_convert(cudaStream_t st, const TA* a, TB* b, int64_t n);
 template <typename T>
 void launch_compact_to_grid_nodes(cudaStream_t st, const double* src, T* dst, Grid g, const int32_t* nodMapBack0,
                                   int64_t numNodes);
+void launch_fill_grid_nodes(cudaStream_t st, const double* src, double* dst, Grid g, const int32_t* node_id);
 template <typename T>
 void launch_grid_to_compact_nodes(cudaStream_t st, const T* src, double* dst, Grid g, const int32_t* nodMapBack0,
                                   int64_t numNodes);

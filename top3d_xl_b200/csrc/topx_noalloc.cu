@@ -4,12 +4,14 @@
 // Some callers cannot allow that: a host whose device memory is all handed out by its own
 // pool or allocator (MATLAB's gpuArray manager, a framework's caching allocator capped to a
 // fraction of the GPU), or a real-time loop that must not call cudaMalloc/cudaFree, which
-// synchronise the device.  For them this file keeps the two grid-layout vectors that the
-// operator needs as scratch in one fixed, file-scope device array instead of allocating them.
+// synchronise the device.  For them this file keeps the grid-layout vector that the operator
+// needs as scratch in one fixed, file-scope device array instead of allocating it; the result
+// goes straight to the caller's vector.
 //
-// Limit: the array holds kNoAllocScratchBytes = 32 MiB = 4,194,304 doubles, and the two vectors
-// need 2 * 3 * stride of them, so the level-1 grid may have at most 699,040 nodes after padding
-// (stride: grid nodes rounded up to 32), e.g. an 87x87x87-element cuboid (88^3 nodes).
+// Limit: the array holds kNoAllocScratchBytes = 32 MiB = 4,194,304 doubles.  The call serves level-1
+// grids of up to 699,040 nodes, e.g. an 87x87x87-element cuboid (88^3 nodes): two vectors of
+// 3 * stride doubles (stride: the domain's padded grid nodes rounded up to 32) fit the array, and
+// so does the one that is needed with the rows rounded up to 4 nodes as the kernels store them.
 // Every GPU on which the library's module is loaded holds the array until the process exits.
 #include <cuda_runtime.h>
 
@@ -62,8 +64,7 @@ void Engine::apply_K_device(const double* d_u, double* d_y, double* grid_u) {
   TOPX_CUDA_OK(cudaEventRecord(ev_legacy, cudaStreamLegacy));
   TOPX_CUDA_OK(cudaStreamWaitEvent(st, ev_legacy, 0));
   // the scratch keeps the previous call's contents: grid nodes outside the domain must read 0
-  TOPX_CUDA_OK(cudaMemsetAsync(grid_u, 0, sizeof(double) * size_t(g.stride) * 3, st));
-  launch_compact_to_grid_nodes<double>(st, d_u, grid_u, g, nodMapBack0.p, Nn);
+  launch_fill_grid_nodes(st, d_u, grid_u, g, nodMapFwd0.p);
   ku(KU_PLAIN, grid_u, nullptr, nullptr, d_y, nullptr, nullptr, nodMapFwd0.p);
   TOPX_CUDA_OK(cudaStreamSynchronize(st));
 }
