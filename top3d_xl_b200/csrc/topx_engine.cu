@@ -1115,14 +1115,14 @@ bool Engine::step(IterRecord& rec) {
     sec_begin(SEC_OC);
     const uint8_t* pas = passive.p;
     launch_oc_prep(st, Ne, x.p, dc.p, tmpA.p);  // tmpA is free once the filter has run
-    // at most kOcMostSteps: 60 in the first round trip (the interval test usually passes after
-    // 50-60 steps from (0, 1e9)), then 16 per round trip
-    static_assert(60 % kOcStepsPerLaunch == 0 && 16 % kOcStepsPerLaunch == 0, "steps per round trip");
+    // at most about kOcMostSteps: 60 in the first round trip (the interval test usually passes after
+    // 50-60 steps from (0, 1e9)), then five launches per round trip
     const bool one = Ne <= kOcClusterElems;
     if (one) launch_oc_cluster(st, Ne, x.p, tmpA.p, pas, ocS.p, 0.2);
-    for (int launched = 0; !one && launched * kOcStepsPerLaunch < kOcMostSteps;) {
-      const int n = (launched == 0 ? 60 : 16) / kOcStepsPerLaunch;
-      for (int k = 0; k < n; ++k) launch_oc_bisect(st, Ne, x.p, tmpA.p, pas, ocS.p, rs1, 0.2);
+    const int steps = oc_steps_per_launch(Ne);
+    for (int launched = 0; !one && launched * steps < kOcMostSteps;) {
+      const int n = launched == 0 ? 60 / steps : 5;
+      for (int k = 0; k < n; ++k) launch_oc_bisect(st, Ne, x.p, tmpA.p, pas, ocS.p, rs1, 0.2, steps);
       launched += n;
       TOPX_CUDA_OK(cudaMemcpyAsync(&oc, ocS.p, sizeof(oc), cudaMemcpyDeviceToHost, st));
       TOPX_CUDA_OK(cudaStreamSynchronize(st));

@@ -107,7 +107,7 @@ void launch_ewise(cudaStream_t st, int op, int64_t n, const double* a, const dou
 
 // ---------------------------------------------------------------------------
 // OC update with Lagrange-multiplier bisection (TOP3D_XL.m:145-156).  Each
-// launch evaluates kOcStepsPerLaunch bisection steps as one grid reduction; once
+// launch evaluates three or four bisection steps as one grid reduction; once
 // the interval test fails the remaining launches return at once.
 // ---------------------------------------------------------------------------
 // x sqrt(-dc / lmid) evaluated as w * r with w = x sqrt(-dc) formed once per OC iteration
@@ -129,7 +129,7 @@ void launch_oc_prep(cudaStream_t st, int64_t Ne, const double* x, const double* 
   TOPX_CUDA_OK(cudaGetLastError());
 }
 
-// kOcStepsPerLaunch bisection steps per launch.  The multipliers the next D = kOcStepsPerLaunch
+// D bisection steps per launch.  The multipliers the next D
 // steps can try form a binary tree below the current interval (l1, l2): node 0 is its midpoint,
 // child 2j+1 the midpoint of node j's lower half (the step found the volume too low, l2 = lmid),
 // child 2j+2 of its upper half (l1 = lmid).  One pass over x and w sums the volume change of all
@@ -137,16 +137,17 @@ void launch_oc_prep(cudaStream_t st, int64_t Ne, const double* x, const double* 
 // included, that D launches of a one-step kernel take.  Every node's midpoint and sum are
 // formed as the one-step kernel forms them (same expressions, same per-thread order, same
 // block-order reduction), so l1, l2, lmid and the step count come out bit-identical.
-// Bound by the launch and the reduction, whose 15 sums cost a block as much as a dozen elements do: two blocks an SM,
-// more elements a thread (four of its loads in flight).  The bisection and the final pass, us, with a thread per element
-// and three steps a launch, three steps, four, five (its sums spill): 50 x 100 x 50 elements 258, 185, 179, 306;
-// 64 x 128 x 64: 419, 223, 213, 398; 96 x 192 x 96: 550, 355, 369, 710.
+// Up to 2^20 elements bound by the launch and the reduction, whose 15 sums cost a block as much as a dozen elements do:
+// four steps a launch, two blocks an SM, more elements a thread (four of its loads in flight).  Beyond, the nodes' FP64
+// operations bound it: three steps.  The bisection and the final pass, us, with a thread per element and three
+// steps a launch, three steps, four, five (its sums spill): 50 x 100 x 50 elements 258, 185, 179, 306;
+// 64 x 128 x 64: 419, 223, 213, 398; 96 x 192 x 96: 550, 355, 369, 710; 128 x 256 x 128: 755, 586, 752.
 // In the per-element clamp, max(0, max(x - move, min(1, min(x + move, t)))) is regrouped as
 // max(lo, min(hi, t)) with lo = max(0, x - move), hi = min(1, x + move) formed once per element,
 // and the two outer selections are written as comparisons (a NaN t, from a positive dc, selects
 // hi as fmin does): min and max select one operand exactly, so neither changes a value (up to
 // the sign of a zero term of the sum).
-constexpr int kOcNodes = (1 << kOcStepsPerLaunch) - 1;
+constexpr int oc_nodes(int steps) { return (1 << steps) - 1; }
 
 // 1/sqrt(lmid) of node j: its interval follows the path from the root
 __device__ __forceinline__ double oc_node(int j, double a, double b) {
@@ -163,11 +164,12 @@ __device__ __forceinline__ double oc_node(int j, double a, double b) {
   return 1.0 / sqrt(0.5 * (b + a));
 }
 
-// the decisions of kOcStepsPerLaunch steps on the nodes' sums; true once the interval test fails
+// the decisions of D steps on the nodes' sums; true once the interval test fails
+template <int D>
 __device__ __forceinline__ bool oc_walk(double fval, const double* tot, double& l1, double& l2, double& lmid,
                                         int& steps) {
   int j = 0;
-  for (int d = 0; d < kOcStepsPerLaunch; ++d) {
+  for (int d = 0; d < D; ++d) {
     lmid = 0.5 * (l2 + l1);
     if (fval + tot[j] > 0) {
       l1 = lmid;
@@ -182,9 +184,11 @@ __device__ __forceinline__ bool oc_walk(double fval, const double* tot, double& 
   return false;
 }
 
+template <int D>
 __global__ void __launch_bounds__(256, 2) k_oc_bisect(int64_t Ne, const double* __restrict__ x,
                                                    const double* __restrict__ w, const uint8_t* __restrict__ passive,
                                                    OcState* os, RedScratch rs, double move) {
+  constexpr int kOcNodes = oc_nodes(D);
   pdl_wait();
   if (os->converged) return;
   __shared__ double sr[kOcNodes];
@@ -229,7 +233,7 @@ __global__ void __launch_bounds__(256, 2) k_oc_bisect(int64_t Ne, const double* 
   if (reduce_publish<kOcNodes>(s, rs, tot, gridDim.x) && threadIdx.x == 0) {
     double l1 = os->l1, l2 = os->l2, lmid = os->lmid;
     int steps = os->steps;
-    const bool conv = oc_walk(os->fval, tot, l1, l2, lmid, steps);
+    const bool conv = oc_walk<D>(os->fval, tot, l1, l2, lmid, steps);
     os->l1 = l1;
     os->l2 = l2;
     os->lmid = lmid;
@@ -238,10 +242,10 @@ __global__ void __launch_bounds__(256, 2) k_oc_bisect(int64_t Ne, const double* 
   }
 }
 void launch_oc_bisect(cudaStream_t st, int64_t Ne, const double* x, const double* w, const uint8_t* passive,
-                      OcState* os, RedScratch rs, double move) {
+                      OcState* os, RedScratch rs, double move, int steps) {
   const unsigned nb = grid1d(Ne, 256, 2 * 148);
-  static_assert(size_t(kOcNodes) * 148 * 2 <= size_t(kMaxRedBlocks) * kMaxRedSlots, "reduction slots");
-  launch_pdl(st, k_oc_bisect, nb, 256, 0, Ne, x, w, passive, os, rs, move);
+  static_assert(size_t(oc_nodes(4)) * 148 * 2 <= size_t(kMaxRedBlocks) * kMaxRedSlots, "reduction slots");
+  launch_pdl(st, steps == 4 ? k_oc_bisect<4> : k_oc_bisect<3>, nb, 256, 0, Ne, x, w, passive, os, rs, move);
   TOPX_CUDA_OK(cudaGetLastError());
 }
 
@@ -251,13 +255,14 @@ void launch_oc_bisect(cudaStream_t st, int64_t Ne, const double* x, const double
 // The bisection and the final pass, us, as launches and as a cluster: 16 x 32 x 16 elements 124, 80; 25 x 50 x 25: 127,
 // 119; 32 x 32 x 32: 128, 116; from there on its eight SMs' arithmetic takes longer than the launches.
 constexpr unsigned OCC_CTAS = 8, OCC_THREADS = 512;
-constexpr int OCC_ELEMS = 8;
+constexpr int OCC_ELEMS = 8, OCC_STEPS = 4;
 static_assert(kOcClusterElems == int64_t(OCC_CTAS) * OCC_THREADS * OCC_ELEMS, "elements of a cluster");
 
 __global__ void __launch_bounds__(OCC_THREADS) k_oc_cluster(int Ne, const double* __restrict__ x,
                                                             const double* __restrict__ w,
                                                             const uint8_t* __restrict__ passive, OcState* os,
                                                             double move) {
+  constexpr int kOcNodes = oc_nodes(OCC_STEPS);
   pdl_wait();
   __shared__ double part[2][OCC_CTAS][kOcNodes];  // by round parity: a CTA ahead writes the other
   __shared__ double sr[kOcNodes], tot[kOcNodes];
@@ -276,7 +281,7 @@ __global__ void __launch_bounds__(OCC_THREADS) k_oc_cluster(int Ne, const double
   int steps = os->steps;
   bool conv = os->converged != 0;
   cluster_sync();  // every CTA runs: its shared memory may be written
-  for (int round = 0; !conv && round < kOcMostSteps / kOcStepsPerLaunch; ++round) {
+  for (int round = 0; !conv && round < kOcMostSteps / OCC_STEPS; ++round) {
     if (tid < kOcNodes) sr[tid] = oc_node(tid, l1, l2);
     __syncthreads();
     double r[kOcNodes], s[kOcNodes];
@@ -316,7 +321,7 @@ __global__ void __launch_bounds__(OCC_THREADS) k_oc_cluster(int Ne, const double
       tot[tid] = t;
     }
     __syncthreads();
-    conv = oc_walk(fval, tot, l1, l2, lmid, steps);
+    conv = oc_walk<OCC_STEPS>(fval, tot, l1, l2, lmid, steps);
   }
   if (blockIdx.x == 0 && tid == 0) {
     os->l1 = l1;

@@ -79,12 +79,12 @@ void launch_fill(cudaStream_t st, int64_t n, double value, double* out);
 void launch_sum(cudaStream_t st, int64_t n, const double* a, const double* b, double* out, RedScratch rs);
 void launch_ewise(cudaStream_t st, int op, int64_t n, const double* a, const double* b, double* out, double s);
 // OC bisection (TOP3D_XL.m:145-156): w = x sqrt(-dc) once, then bisection steps on lmid,
-// kOcStepsPerLaunch of them per launch of launch_oc_bisect
-constexpr int kOcStepsPerLaunch = 4;
-constexpr int kOcMostSteps = 268;  // the first 60, then 16 at a time
+// `steps` (4 or 3) of them per launch of launch_oc_bisect
+inline int oc_steps_per_launch(int64_t Ne) { return Ne <= (int64_t(1) << 20) ? 4 : 3; }
+constexpr int kOcMostSteps = 268;
 void launch_oc_prep(cudaStream_t st, int64_t Ne, const double* x, const double* dc, double* w);
 void launch_oc_bisect(cudaStream_t st, int64_t Ne, const double* x, const double* w, const uint8_t* passive,
-                      OcState* os, RedScratch rs, double move);
+                      OcState* os, RedScratch rs, double move, int steps);
 // all steps in one launch, for up to kOcClusterElems elements
 constexpr int64_t kOcClusterElems = 32768;
 void prepare_oc_kernels();
