@@ -67,11 +67,10 @@ def load_workload(ctx, wl):
     else:
         ctx.load_voxels(src)
 METRIC = "OC iterations/s (GLOBAL, FP64; mixed precision beside it)"
-# DRAM bytes (read + write) per grid node of one K*u launch in PCG mode (tile kernel + last-row
-# kernel), from an ncu capture of the 128x256x128 cuboid: dram__bytes_read.sum +
-# dram__bytes_write.sum of the tile kernel (637.2 MB) and the last-row kernel (52.9 MB) over
-# 4,276,737 nodes; the traffic of a launch scales with its node count.
-KU_TRAFFIC_PER_NODE = 690.1e6 / 4276737
+# DRAM bytes (read + write) per grid node of one K*u launch in PCG mode, from an ncu capture of the
+# 128x256x128 cuboid: dram__bytes_read.sum + dram__bytes_write.sum (674 MB) over 4,276,737
+# nodes; the traffic of a launch scales with its node count.
+KU_TRAFFIC_PER_NODE = 674e6 / 4276737
 # Nominal FP64 rate of a B200 on CUDA cores: 148 SMs x 64 FMA/clk x 2 flop x 1.965 GHz.
 FP64_NOMINAL_TFLOPS = 148 * 64 * 2 * 1.965e9 / 1e12
 
@@ -509,16 +508,16 @@ def main(argv=None):
     n = min(len(cm), len(cd))
     relerrs = np.abs(cm[:n] - cd[:n]) / np.abs(cd[:n])
     relerr = float(np.max(relerrs))
-    # roofline of the dominant kernel: level-1 K*u in PCG mode (FP64 in both arms; the tile
-    # kernel and its last-row kernel).  Per launch it reads p_old and z and writes q and the new
-    # direction p, and reads and writes the solution y for the previous iteration's step (3
-    # doubles per node each), reads the moduli (1 double per element) and the free-DOF bits (1
-    # byte per node): 145 B/node + 8 B/element; per node 8 hexes x 3 rows x 24 DOFs + 24
-    # scalings = 600 FMA.
+    # roofline of the dominant kernel: level-1 K*u in PCG mode (FP64 in both arms), which forms the
+    # search direction from the residual and the level-2 correction.  Per launch it reads the
+    # residual, p_old and the inverse diagonal, writes q and the new direction p, and reads and
+    # writes the solution y for the previous iteration's step (3 doubles per node each, the inverse
+    # diagonal 1), reads the moduli (1 double per element) and a byte of flags per node: 153 B/node
+    # + 8 B/element.  In sums and differences a node takes about 160 FP64 operations.
     prof = fp64["prof"]
     nn = fp64["nnodes"]
-    alg_bytes = 145 * nn + 8 * fp64["ne"]
-    flop = 2 * 600 * nn
+    alg_bytes = 153 * nn + 8 * fp64["ne"]
+    flop = 160 * nn
     ku_ms = prof["ku_ms"] / max(1, prof["ku_launches"])
     achieved = alg_bytes / (ku_ms * 1e-3) / 1e9
     tflops = flop / (ku_ms * 1e-3) / 1e12
@@ -547,7 +546,7 @@ def main(argv=None):
             "sections_ms_per_step": {k: round(v[0] / prof["steps"], 3) for k, v in prof["sections"].items()},
             "section_groups_per_step": {k: round(v[1] / prof["steps"], 1) for k, v in prof["sections"].items()},
             "gpu_launches": fp64["launches"],
-            "roofline": {"kernel": "k_ku_l1<double, KU_P_UPDATE> (level-1 K*u, PCG mode)", "bound": "hbm",
+            "roofline": {"kernel": "k_ku<KU_FUSED, double> (level-1 K*u, PCG mode)", "bound": "hbm",
                          "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                          "peak_kind": kind, "algorithmic_bytes_per_launch": alg_bytes,
                          "ms_per_launch": ku_ms, "traffic": KU_TRAFFIC_PER_NODE * nn if KU_TRAFFIC_PER_NODE else None,

@@ -267,8 +267,8 @@ void launch_pcg_update(cudaStream_t st, Grid g, double* r, const double* q, PcgS
   TOPX_CUDA_OK(cudaGetLastError());
 }
 
-// y += sc->lam * p over every node: the solution step of the last PCG iteration (PGIVEN updates
-// leave it to the next K*u)
+// y += sc->lam * p over every node: the solution step of the last PCG iteration (an earlier one's is
+// applied by the next K*u)
 __global__ void k_pcg_flush(Grid g, double* __restrict__ y, const double* __restrict__ p, const PcgScalars* sc,
                             const uint32_t* __restrict__ act) {
   pdl_wait();
