@@ -416,3 +416,24 @@ def test_galerkin_group_sizes(shape, holes):
         ctx.assemble()
         r = np.random.default_rng(3).standard_normal(m.levels[0].numDOFs)
         assert _rel(ctx.vcycle(r), sol.vcycle(r)) < 1e-10
+
+
+@pytest.mark.parametrize("shape", [(16, 32, 16), (30, 41, 40), (56, 100, 56)])
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_pcg_end_is_one_decision(shape, precision):
+    # the kernel that takes the residual pass's sums also ends the solve: all its CTAs and warps have to act alike
+    # (one cluster launch, or the restriction of larger grids), with the launches of the chunk that follow
+    # doing nothing.  Every sum has a fixed order, so repeated solves are equal bit for bit.
+    from top3d_xl_b200 import Context
+    vox = np.ones(shape, bool)
+    E = np.random.default_rng(1).uniform(0.05, 1.0, vox.size)
+    with Context(precision) as ctx:
+        ctx.load_voxels(vox)
+        ctx.set_moduli(E)
+        ctx.assemble()
+        u0, its0 = ctx.pcg()
+        assert 0 < its0 < 800
+        for _ in range(12):
+            u, its = ctx.pcg()
+            assert its == its0
+            assert np.array_equal(u, u0)

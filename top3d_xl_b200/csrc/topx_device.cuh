@@ -53,6 +53,7 @@ struct PcgScalars {
                    // word that another one of its launch still has to read)
   int maxIT;
   int done;  // 0 running, 1 converged, 2 hit maxIT
+  int ended;  // done before the last residual pass, for the kernel that takes its sums and writes done
   int first;
 };
 

@@ -80,7 +80,11 @@ __device__ __forceinline__ void load4(const double* p, double (&v)[4]) {
 template <int MODE, typename TC>
 __global__ void __launch_bounds__(256) k_residual(const __grid_constant__ ResidualArgs a, int lines, int cy, FastDiv dcy) {
   pdl_wait();
-  if (MODE == RES_UPDATE && a.sc->done) return;
+  if (MODE == RES_UPDATE) {
+    const int done = a.sc->done;
+    if (a.parts.rr.n && blockIdx.x == 0 && threadIdx.x == 0) a.sc->ended = done;  // (pcg_ended)
+    if (done) return;
+  }
   const int lane = threadIdx.x & 31;
   const int64_t S = a.g.stride, nlines = int64_t(a.g.nx + 1) * (a.g.nz + 1), ts = nlines * cy;
   double* __restrict__ const r = a.r;
@@ -309,7 +313,7 @@ __global__ void __launch_bounds__(32 * (2 * KU_SPAN - 1)) k_restrict_xz(const do
                                                                        PcgScalars* sc, PcgParts parts, int init,
                                                                        double tol, int maxIT) {
   pdl_wait();
-  if (sc && !init && sc->done) return;
+  if (sc && !init && pcg_ended(sc, parts)) return;
   if (pcg_decide(sc, parts, init != 0, tol, maxIT)) return;
   constexpr int W = 2 * KU_SPAN - 1;
   __shared__ double sx[W][3][32];

@@ -599,8 +599,7 @@ static_assert(SC_TILES * ND_T >= 3 * kNdOneFrontNodes && SC_TILES <= kSmallCoars
 template <typename TC>
 __global__ void __launch_bounds__(SC_THREADS) k_small_coarse(const __grid_constant__ SmallCoarse<TC> a) {
   pdl_wait();
-  if (a.dot && !a.init && a.sc->done) return;  // the same in every CTA, or about to be (pcg_decide)
-  if (!a.dot && a.sc && a.sc->done) return;
+  if (a.sc && !(a.dot && a.init) && pcg_ended(a.sc, a.parts)) return;  // the same for the whole launch
   if (a.dot && pcg_decide(a.sc, a.parts, a.init, a.tol, a.maxIT)) return;
   __shared__ double vec[SC_TILES * ND_T];
   __shared__ double red[2 * SC_TILES][ND_T];

@@ -25,6 +25,12 @@ __device__ __forceinline__ void pcg_stop_test(PcgScalars* sc, double rr, int its
   else if (its >= sc->maxIT)
     sc->done = 2;
 }
+// The solve had ended before the residual pass whose result this kernel takes.  With parts.rr given, pcg_decide writes
+// done in this launch, so that its CTAs (and the warps of one) could read different values of it: ended is the residual
+// pass's copy.  No word that a launch of the PCG reads is written by another CTA of that launch.
+__device__ __forceinline__ bool pcg_ended(const PcgScalars* sc, const PcgParts& parts) {
+  return (parts.rr.n ? sc->ended : sc->done) != 0;
+}
 // parts.rr given: sums the residual pass's r'r (b'b) and r'D r.  Every CTA takes the same decision, the first one writes
 // it down.  True: the solve has ended.
 __device__ __forceinline__ bool pcg_decide(PcgScalars* sc, const PcgParts& parts, bool init, double tol, int maxIT) {
