@@ -215,12 +215,17 @@ topx_status topx_set_density(topx_ctx* ctx, const double* xPhys, size_t ne);
 topx_status topx_get_displacement(topx_ctx* ctx, int lc, double* out, size_t ndof);
 
 /* ---- failure handling (no reference counterpart) ----------------------------- */
-/* Test of the give-up path of the one bounded wait in the library's kernels: in the persistent
-   coarsest-level solve (contexts with topx_params.coarse_coop = 1) a task waits for the tasks of
-   the fronts it reads.  which must be 0: one CTA waits for a counter that nothing raises, so its
-   wait exhausts its poll limit (about a second) and sets the solve's error word.  Returns
-   TOPX_ERR_TIMEOUT with a message naming the wait, as a real give-up inside a solve would; the
-   context stays usable. */
+/* Test of the give-up paths of the two bounded waits in the library's kernels.
+   which = 0: in the persistent coarsest-level solve (contexts with topx_params.coarse_coop = 1) a
+   task waits for the tasks of the fronts it reads.  One CTA waits for a counter that nothing
+   raises, so its wait exhausts its poll limit (about a second) and sets the solve's error word.
+   Returns TOPX_ERR_TIMEOUT with a message naming the wait, as a real give-up inside a solve would.
+   which = 2: K*u and the filter wait for their copies into shared memory.  One CTA waits for a
+   barrier that no copy completes (about a second, and once more for each stage's copies) and sets
+   the copies' error word.  Returns TOPX_OK; the next call on the context that runs K*u, the filter,
+   the V-cycle or the PCG finds the word as it would after a give-up of its own, and returns
+   TOPX_ERR_TIMEOUT.
+   Other values: TOPX_ERR_ARG.  The context stays usable. */
 topx_status topx_selftest_wait(topx_ctx* ctx, int which);
 
 /* ---- measurement (no reference counterpart) --------------------------------- */

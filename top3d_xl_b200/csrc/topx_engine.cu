@@ -345,6 +345,8 @@ Engine::Engine(Model& model, int precision, int device, bool coarse_coop) : M(mo
   TOPX_CUDA_OK(cudaMallocHost(&h_sc, sizeof(PcgScalars)));
   TOPX_CUDA_OK(cudaMallocHost(&h_ctl, sizeof(CoopControl)));
   h_ctl->err = 0;
+  TOPX_CUDA_OK(cudaMallocHost(&h_copyErr, sizeof(int)));
+  *h_copyErr = 0;
   // ---- optimiser state -------------------------------------------------------
   for (DevBuf<double>* b : {&x, &xPhys, &dc, &ce, &tmpA, &tmpB, &xTilde, &xhat, &dfdx, &dxv})
     b->alloc(size_t(Ne));
@@ -395,6 +397,7 @@ Engine::~Engine() {
   if (ev_legacy) cudaEventDestroy(ev_legacy);
   if (h_sc) cudaFreeHost(h_sc);
   if (h_ctl) cudaFreeHost(h_ctl);
+  if (h_copyErr) cudaFreeHost(h_copyErr);
   if (st) cudaStreamDestroy(st);
 }
 
@@ -452,29 +455,39 @@ double* Engine::host_vector() {
   return hostVec.p;
 }
 
-// The persistent coarse solve's dependency waits and the K*u's waits for its copies set an error word instead
-// of spinning on (they are bounded); the word was copied into pinned memory before the caller's stream sync.  A word
-// that is set is cleared (so the engine stays usable) and reported.
+// The persistent coarse solve's dependency waits, and the K*u's and the filter's waits for their copies, set an error word
+// instead of spinning on (they are bounded).  The first one was copied into pinned memory before the caller's stream
+// sync, the second one is there.  A word that is set is cleared (so the engine stays usable) and reported: by every
+// call that launches such a kernel, after its last sync.
 void Engine::check_device_waits() const {
-  if (h_ctl->err) {
-    const int err = h_ctl->err;
+  const int copies = *static_cast<volatile int*>(h_copyErr);
+  if (h_ctl->err || copies) {
+    const int err = h_ctl->err ? h_ctl->err : copies;
     h_ctl->err = 0;
+    *h_copyErr = 0;
     // a launch that gave up may leave chunk tickets and dependency counts behind
     TOPX_CUDA_OK(cudaMemsetAsync(coopCtl.p, 0, sizeof(CoopControl), st));
     TOPX_CUDA_OK(cudaMemsetAsync(ndCnt.p, 0, sizeof(unsigned) * ndCnt.n, st));
     if (ndDone.p) TOPX_CUDA_OK(cudaMemsetAsync(ndDone.p, 0, sizeof(unsigned) * ndDone.n, st));
     TOPX_CUDA_OK(cudaStreamSynchronize(st));
     throw DeviceWaitError(err == kCoopErrWait ? "coarse solve: a dependency wait gave up (persistent launch not co-resident)"
-                          : err == kCoopErrCopy ? "K*u: a wait for copies into shared memory gave up"
+                          : err == kCoopErrCopy ? "K*u or filter: a wait for copies into shared memory gave up"
                                                 : "unknown wait error");
   }
 }
 
 // Drives the persistent coarse solve's bounded dependency wait to its poll limit: one CTA waits
 // for a counter that nothing raises.  The wait gives up within about a second and the check below
-// throws DeviceWaitError after clearing the words.
+// throws DeviceWaitError after clearing the words.  2: the same for the K*u's wait for copies, whose word is left for the
+// next call that has to look at it.
 void Engine::selftest_wait(int which) {
-  if (which != 0) throw std::invalid_argument("selftest_wait: which must be 0 (the coarse solve's dependency wait)");
+  if (which == 2) {
+    launch_copy_wait_selftest(st, h_copyErr);
+    TOPX_CUDA_OK(cudaStreamSynchronize(st));
+    return;
+  }
+  if (which != 0)
+    throw std::invalid_argument("selftest_wait: which must be 0 (the coarse solve's dependency wait) or 2 (the K*u's wait for copies)");
   if (!coopCtas)
     throw std::invalid_argument("selftest_wait: this context runs the coarse solve without a persistent launch");
   TOPX_CUDA_OK(cudaStreamSynchronize(st));
@@ -702,7 +715,7 @@ void Engine::ku(KuMode mode, const double* in, const double* pin, double* pout, 
   a.sc = sc;
   a.rs = rs1;
   a.parts = parts;
-  a.err = &coopCtl.p->err;
+  a.err = h_copyErr;
   a.active = kuTiles.p;
   a.zr = kuZr.p;
   a.yacc = y;
@@ -840,7 +853,7 @@ int Engine::filter_t(FWork<T>& w, int slot, const double* d_src, double* d_out) 
   a.zr = filterZr.p;
   a.ntiles = int(filterTiles.n);
   a.act = act1;
-  a.err = &coopCtl.p->err;
+  a.err = h_copyErr;
   a.tol = M.S.tol / 10;
   a.maxIT = M.S.maxIT;
   launch_scatter_elems_t<T>(st, d_src, eleMapBack0.p, Ne, w.fsrc.p);
@@ -888,6 +901,7 @@ void Engine::apply_K(const double* h_u, double* h_y) {
   launch_compact_to_grid_nodes<double>(st, v, kw.z.p, G[0], nodMapBack0.p, Nn);
   ku(KU_PLAIN, kw.z.p, nullptr, nullptr, v, nullptr, nullptr, nodMapFwd0.p);
   copy_sync(h_y, v, sizeof(double) * Nn * 3, cudaMemcpyDeviceToHost);
+  check_device_waits();
 }
 
 void Engine::apply_vcycle(const double* h_r, double* h_z) {

@@ -277,6 +277,7 @@ class Engine {
   DevBuf<double> dscal;
   PcgScalars* h_sc = nullptr;  // pinned
   CoopControl* h_ctl = nullptr;  // pinned
+  int* h_copyErr = nullptr;      // pinned; kernels write it (report_copy_wait)
   // optimiser state (compact, FP64)
   DevBuf<double> x, xPhys, dc, ce, tmpA, tmpB, xTilde, xhat, dfdx, dxv;
   DevBuf<double> xold1, xold2, low, upp, alpha, beta, p0, q0, pij, qij, xmma;

@@ -86,8 +86,9 @@ __global__ void __launch_bounds__(FK_NT, FK_CTAS)
   const bool own = inb && ly >= 1 && ly <= a.sh.TY && lx >= 1 && lx <= a.sh.TX;
   const int o = in_tile ? lx * (a.sh.TY + 2 * HB) + ly + HB - 1 : 0, oy = own ? (lx - 1) * a.sh.TY + ly - 1 : 0;
   const int64_t n0 = inb ? gy + int64_t(nny) * gx : 0, np = int64_t(nny) * nnx;
+  bool ok = true;  // no wait of this thread gave up
   auto issue = [&](int zp, int s) {
-    if (t == 0) {
+    if (t == 0 && ok) {
       T* d = stages + s * len;
       mbar_expect(&sm.bar[s], bytes);
       tma_load(d, &maps.r, y0 - HB, x0 - 1, zp, &sm.bar[s]);
@@ -113,10 +114,9 @@ __global__ void __launch_bounds__(FK_NT, FK_CTAS)
   unsigned f = flags_at(zc0 - 1);
   const int its = a.sc->its;  // steps done: none (p = z), one (y starts), more
   const T beta = T(a.sc->beta), lam = T(a.sc->lam);
-  bool ok = true;
   if (a.sc->done) {  // the same for the whole launch
-    ok = mbar_wait(&sm.bar[0], 0) && mbar_wait(&sm.bar[1], 0);
-    if (!ok && t == 0) atomicCAS(a.err, 0, kCoopErrCopy);
+    ok = plane_wait(sm.bar, 0, 1, t == 0) && plane_wait(sm.bar, 1, 1, t == 0);
+    if (!ok) report_copy_wait(a.err);
     return;
   }
   double dot = 0.0;
@@ -129,7 +129,7 @@ __global__ void __launch_bounds__(FK_NT, FK_CTAS)
     const int s = (zp - zc0 + 1) & 1;
     const T* st = stages + s * len;
     const int64_t n = n0 + np * zp;
-    if (ok) ok = mbar_wait(&sm.bar[s], unsigned(zp - zc0 + 1) >> 1 & 1u);
+    if (ok) ok = plane_wait(sm.bar, zp - zc0 + 1, zend - zc0 + 1, t == 0);
     T v = a.ke.dp[f & 15u] * st[o];  // D r; 0 off the domain
     const T po = st[box + o];
     if (its > 0) v = v + beta * po;
@@ -170,7 +170,7 @@ __global__ void __launch_bounds__(FK_NT, FK_CTAS)
     solid = (f & 128u) != 0u;
     f = fn;
   }
-  if (!ok) atomicCAS(a.err, 0, kCoopErrCopy);
+  if (!ok) report_copy_wait(a.err);
   double r[1] = {dot}, tot[1];
   if (reduce_publish<1>(r, a.rs, tot) && t == 0) a.sc->pq = tot[0];
 }

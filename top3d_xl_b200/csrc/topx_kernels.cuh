@@ -115,7 +115,7 @@ struct KuArgs {
   const uint32_t* zr;      // per listed tile, the planes [lo, hi) of its z-chunk that hold a present node (lo | hi << 16)
   double* yacc;
   const int32_t* compact;  // KU_PLAIN: out in compact DOF order through this map, or null
-  int* err;                // takes kCoopErrCopy
+  int* err;                // takes kCoopErrCopy (report_copy_wait)
 };
 // tiles of the launch that own a node of the domain; zranges (optional): the z-range entry of each
 std::vector<uint32_t> ku_active_tiles(Grid g, int rows, const KuShape& k, const std::vector<uint8_t>& present,
@@ -225,10 +225,12 @@ struct CoopControl {
   int err;         // 0, or kCoopErrWait once a wait gave up
   int pad;
 };
-constexpr int kCoopErrCopy = 2;  // a wait for asynchronous copies into shared memory gave up
 constexpr int kCoopErrWait = 1;  // a wait for another CTA's tasks (dataflow solve) gave up
+constexpr int kCoopErrCopy = 2;  // a wait for asynchronous copies into shared memory (K*u, filter) gave up; has its own word
 // Self-test of the dataflow solve's bounded dependency wait: one CTA waits for a counter that
 // nothing raises, gives up within about a second and sets ctl->err to kCoopErrWait.
 void launch_coop_wait_selftest(cudaStream_t st, CoopControl* ctl);
+// The same for the K*u's wait for copies: one CTA waits for a barrier that no copy completes.
+void launch_copy_wait_selftest(cudaStream_t st, int* err);
 
 }  // namespace topx

@@ -208,9 +208,10 @@ __global__ void __launch_bounds__(KU_NT, KU_CTAS)
       cp_async_el<int(sizeof(TC))>(dst, xc + (ok ? int64_t(e) + int64_t(a.gc.ny + 1) * (a.gc.nx + 1) * Z : 0), ok);
     }
   };
+  bool ok = true;  // no wait of this thread gave up
   // one thread issues the copies of plane zp and of the layer below it
   auto issue = [&](int zp, int s) {
-    if (t == 0) {
+    if (t == 0 && ok) {
       double* d = ku_stages + s * sg.len;
       mbar_expect(&sm.bar[s], bytes);
       tma_load(d, &maps.a, y0 - 2, x0 - 1, zp, &sm.bar[s]);
@@ -248,11 +249,10 @@ __global__ void __launch_bounds__(KU_NT, KU_CTAS)
   const bool first = PCG && (MODE == KU_FUSED ? a.sc->its == 0 : a.sc->first != 0);
   const double lam = PCG ? a.sc->lam : 0.0;
   double beta = PCG ? a.sc->beta : 0.0;
-  bool ok = true;  // no wait gave up
   if (PCG && a.sc->done) {  // the same for the whole launch
     cp_async_wait_all();
-    ok = mbar_wait(&sm.bar[0], 0) && mbar_wait(&sm.bar[1], 0);
-    if (!ok && t == 0) atomicCAS(a.err, 0, kCoopErrCopy);
+    ok = plane_wait(sm.bar, 0, 1, t == 0) && plane_wait(sm.bar, 1, 1, t == 0);
+    if (!ok) report_copy_wait(a.err);
     return;
   }
   if (MODE == KU_FUSED && a.parts.dot.n) {  // z'r, whose level-2 part the prolongation left in parts
@@ -284,7 +284,7 @@ __global__ void __launch_bounds__(KU_NT, KU_CTAS)
     const uint32_t n = n0 + np * uint32_t(zp);
     const bool mine = own && zp >= zc0 && zp < zend;
     const double* st = ku_stages + s * sg.len;
-    if (ok) ok = mbar_wait(&sm.bar[s], unsigned(zp - zc0 + 1) >> 1 & 1u);
+    if (ok) ok = plane_wait(sm.bar, zp - zc0 + 1, zend - zc0 + 1, t == 0);
     if (MODE == KU_FUSED) cp_async_wait_all();  // level-2 planes, a plane ahead of their use
     const double E = st[sg.E + o];
     double v[3], y[3];
@@ -415,7 +415,7 @@ __global__ void __launch_bounds__(KU_NT, KU_CTAS)
       }
   }
   cp_async_wait_all();
-  if (!ok) atomicCAS(a.err, 0, kCoopErrCopy);
+  if (!ok) report_copy_wait(a.err);
   if (MODE == KU_FUSED && a.parts.pq.n) {  // the residual pass sums them
     double r[1] = {dot};
     parts_leave<1>(r, {a.parts.pq.part});
@@ -431,6 +431,23 @@ void ku_smem_attr() {
 }
 
 }  // namespace
+
+// the give-up path of the operator's waits: two barriers that no copy completes
+__global__ void k_copy_wait_selftest(int* err) {
+  pdl_wait();
+  __shared__ uint64_t bar[2];
+  if (threadIdx.x == 0) {
+    mbar_init(&bar[0]);
+    mbar_init(&bar[1]);
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
+  __syncthreads();
+  if (!plane_wait(bar, 0, 1, threadIdx.x == 0)) report_copy_wait(err);
+}
+void launch_copy_wait_selftest(cudaStream_t st, int* err) {
+  launch_pdl(st, k_copy_wait_selftest, 1, 32, 0, err);
+  TOPX_CUDA_OK(cudaGetLastError());
+}
 
 void prepare_ku_kernels() {
   ku_smem_attr<KU_PLAIN, double>();

@@ -67,6 +67,7 @@ void Engine::apply_K_device(const double* d_u, double* d_y, double* grid_u) {
   launch_fill_grid_nodes(st, d_u, grid_u, g, nodMapFwd0.p);
   ku(KU_PLAIN, grid_u, nullptr, nullptr, d_y, nullptr, nullptr, nodMapFwd0.p);
   TOPX_CUDA_OK(cudaStreamSynchronize(st));
+  check_device_waits();
 }
 
 }  // namespace topx

@@ -52,7 +52,7 @@ struct FilterArgs {
   const uint32_t* zr;
   int ntiles;
   const uint32_t* act;  // chunk mask (chunk_active), or null
-  int* err;             // takes kCoopErrCopy
+  int* err;             // takes kCoopErrCopy (report_copy_wait)
   double tol;
   int maxIT;
 };

@@ -26,19 +26,38 @@ __device__ __forceinline__ void mbar_init(uint64_t* b) {
 __device__ __forceinline__ void mbar_expect(uint64_t* b, unsigned bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(b)), "r"(bytes) : "memory");
 }
-// waits for the phase of the given parity; bounded (about a second in all), false when it gave up
+__device__ __forceinline__ bool mbar_try(uint64_t* b, unsigned parity) {
+  unsigned ok;
+  asm volatile(
+      "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
+      : "=r"(ok)
+      : "r"(smem_addr(b)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+// waits for the phase of the given parity; false when it gave up, after about a second of the SM's clock
+constexpr long long kWaitCycles = 1ll << 31;
 __device__ __forceinline__ bool mbar_wait(uint64_t* b, unsigned parity) {
-  for (unsigned it = 0; it < (1u << 20); ++it) {
-    unsigned ok;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
-        : "=r"(ok)
-        : "r"(smem_addr(b)), "r"(parity)
-        : "memory");
-    if (ok) return true;
+  if (mbar_try(b, parity)) return true;
+  const long long t0 = clock64();
+  do {
+    if (mbar_try(b, parity)) return true;
+  } while (clock64() - t0 < kWaitCycles);
+  return false;
+}
+// A CTA's planes k = 0 .. last pass through two stages, each with its barrier, copied up to one plane ahead of the plane
+// that is waited for.  False when the wait for plane k gave up: the thread that issues the copies has then waited
+// once more for those in flight, and must issue no more, so that none lands after the CTA has ended.
+__device__ __forceinline__ bool plane_wait(uint64_t* bar, int k, int last, bool issues) {
+  if (mbar_wait(bar + (k & 1), unsigned(k) >> 1 & 1u)) return true;
+  if (issues) {
+    mbar_wait(bar + (k & 1), unsigned(k) >> 1 & 1u);
+    if (k < last) mbar_wait(bar + (~k & 1), unsigned(k + 1) >> 1 & 1u);
   }
   return false;
 }
+// err: the engine's word for give-ups, in page-locked host memory (a host call that has synchronised reads it without a copy)
+__device__ __forceinline__ void report_copy_wait(int* err) { *static_cast<volatile int*>(err) = kCoopErrCopy; }
 // box of a 4-dimensional map (y, x, z, component) at (y, x, z, 0): entries outside the array read as zero.  y is
 // even: a copy starts on a 16-byte boundary.
 __device__ __forceinline__ void tma_load(void* dst, const CUtensorMap* map, int y, int x, int z, uint64_t* bar) {
