@@ -437,3 +437,35 @@ def test_pcg_end_is_one_decision(shape, precision):
             u, its = ctx.pcg()
             assert its == its0
             assert np.array_equal(u, u0)
+
+
+@pytest.mark.parametrize("bad", ["start", "moduli"])
+def test_solve_after_a_nan_solve(bad):
+    # a solve that ends in NaN (a NaN in its start vector or moduli) leaves nothing behind, off the domain either: the next
+    # solve on the context is the one that a fresh context computes
+    from top3d_xl_b200 import Context
+    vox = np.ones((20, 36, 24), bool)
+    vox[6:14, 10:24, 5:18] = False
+    vox[:, 28:, 12:] = False
+    E = np.random.default_rng(1).uniform(0.05, 1.0, int(vox.sum()))
+    with Context("fp64", maxIT=200) as ctx:
+        ctx.load_voxels(vox)
+        ctx.set_moduli(E)
+        ctx.assemble()
+        u0, its0 = ctx.pcg()
+        assert its0 < 200 and np.isfinite(u0).all()
+        y0, f0 = ctx.ku(u0), ctx.filter(2.5, E)[0]
+        if bad == "start":
+            ctx.pcg(np.full(ctx.numDOFs, np.nan))
+        else:
+            ctx.set_moduli(np.full(E.size, np.nan))
+            ctx.assemble()
+            ctx.pcg()
+            ctx.set_moduli(E)
+            ctx.assemble()
+        ctx.ku(np.full(ctx.numDOFs, np.nan))
+        ctx.filter(2.5, np.full(E.size, np.nan))
+        u, its = ctx.pcg()
+        assert its == its0
+        assert np.array_equal(u, u0)
+        assert np.array_equal(ctx.ku(u0), y0) and np.array_equal(ctx.filter(2.5, E)[0], f0)

@@ -506,10 +506,11 @@ void Engine::get_U(int lc, double* h) {
   launch_grid_to_compact_nodes<double>(st, U[lc].p, v, G[0], nodMapBack0.p, Nn);
   copy_sync(h, v, sizeof(double) * Nn * 3, cudaMemcpyDeviceToHost);
 }
-void Engine::set_U(int lc, const double* h) {  // absent nodes hold zero and stay so
+void Engine::set_U(int lc, const double* h) {
   double* v = host_vector();
   copy_sync(v, h, sizeof(double) * Nn * 3, cudaMemcpyHostToDevice);
-  launch_compact_to_grid_nodes<double>(st, v, U[lc].p, G[0], nodMapBack0.p, Nn);
+  // absent nodes too: a solve that ended in NaN (lam) has left y + lam p = NaN there
+  launch_fill_grid_nodes(st, v, U[lc].p, G[0], nodMapFwd0.p);
 }
 
 void Engine::update_moduli(const double* d_xPhys, bool solid) {
