@@ -229,8 +229,10 @@ __global__ void __launch_bounds__(ND_THREADS) k_nd_panel(const NDFront* __restri
 }
 
 // A[i][j] += A[i][k] R_j for a stored tile (i >= j); the CTA of tile (k+1, k+1) then inverts it,
-// the pivot of step k+1
-__global__ void __launch_bounds__(ND_THREADS) k_nd_update(const NDFront* __restrict__ fronts,
+// the pivot of step k+1.  Two CTAs an SM, not the three that shared memory allows: that CTA's chain of pivots is the
+// launch's last, and beside two others it gets less of the FP64 unit (128 x 256 x 128 elements: 2450 us with three, 2312
+// with two; 50 x 100 x 50: 475, 448).
+__global__ void __launch_bounds__(ND_THREADS, 2) k_nd_update(const NDFront* __restrict__ fronts,
                                                           const NDTask* __restrict__ tasks, int k,
                                                           double* __restrict__ pool, double* __restrict__ scr) {
   pdl_wait();

@@ -5,6 +5,8 @@
 
 #include <cstdint>
 
+#include "topx_recip.h"
+
 namespace topx {
 
 constexpr int GF_T = 64;  // tile width
@@ -121,13 +123,11 @@ struct GFPivotSmem {
 };
 static_assert(sizeof(GFPivotSmem) <= GF_BUF * sizeof(double), "pivot workspace exceeds a staging buffer");
 
-// 1/v: the hardware approximation x (it keeps 20 bits), then with e = 1 - v x the series x (1 + e + e^2), whose
-// remainder e^3 is below 2^-56: three dependent operations, off the long IEEE division.
+// 1/v from the hardware approximation (it keeps 20 bits) in three dependent operations, off the long IEEE division.
 __device__ __forceinline__ double gf_recip(double v) {
   double x;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(x) : "d"(v));
-  const double e = fma(-v, x, 1.0);
-  return fma(x, fma(e, e, e), x);
+  return recip_series(v, x);
 }
 
 // Pivot t of the 8 x 8 pivot block's Gauss-Jordan inversion in one warp: lane (g, q) holds P[g][2q], P[g][2q+1].
@@ -157,9 +157,9 @@ __device__ __forceinline__ void gf_pivot_step(int t, double& p0, double& p1) {
 //   every warp forms R = -P^-1 A[S, cols] for its columns and then, on the tensor cores,
 //   A[i, j] += A[i, S] R_j,  A[i, S] = A[i, S] P^-1,  A[S, j] = R_j,  A[S, S] = P^-1;
 //   the warp that holds the next pivot block updates it first and inverts it while the others form their products.
-// The chain of the 64 pivots bounds it.  With the inversion by warp 0 before the products, two barriers a block and one
-// more dependent operation in a reciprocal, the factorisation of 50 x 100 x 50 elements took 482 us, now 445;
-// 64 x 128 x 64: 489, now 469; 128 x 256 x 128: 2510, now 2323.  (Pivot steps between the products wait for the FP64
+// The chain of the 64 pivots bounds it.  With the inversion by warp 0 before the products and two barriers a block, the
+// factorisation of 50 x 100 x 50 elements took 482 us, now 448;
+// 64 x 128 x 64: 489, now 477; 128 x 256 x 128: 2510, now 2312 (one box; boxes differ by 2 %).  (Pivot steps between the products wait for the FP64
 // unit that those keep busy: 2 us a tile slower than pivot steps before them; so are products with the pivot row formed
 // beside the reciprocal, by the operations they add.)
 // acc: the tile on entry, its inverse on return (also stored to Pinv).
