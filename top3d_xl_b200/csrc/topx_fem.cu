@@ -768,6 +768,27 @@ void launch_convert(cudaStream_t st, const TA* a, TB* b, int64_t n) {
   TOPX_CUDA_OK(cudaGetLastError());
 }
 
+__global__ void k_index_nodes(const int32_t* __restrict__ nmb0, int64_t nn, int32_t* __restrict__ node_id) {
+  pdl_wait();
+  for (int64_t k = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; k < nn; k += int64_t(gridDim.x) * blockDim.x)
+    node_id[nmb0[k]] = int32_t(k);
+}
+void launch_index_nodes(cudaStream_t st, const int32_t* nodMapBack0, int64_t numNodes, int32_t* node_id, int64_t n) {
+  TOPX_CUDA_OK(cudaMemsetAsync(node_id, 0xff, sizeof(int32_t) * size_t(n), st));
+  launch_pdl(st, k_index_nodes, grid1d(numNodes, 256), 256, 0, nodMapBack0, numNodes, node_id);
+  TOPX_CUDA_OK(cudaGetLastError());
+}
+
+__global__ void k_invert(int64_t n, const double* __restrict__ a, double* __restrict__ out) {
+  pdl_wait();
+  for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x)
+    out[i] = a[i] != 0.0 ? 1.0 / a[i] : 0.0;
+}
+void launch_invert(cudaStream_t st, int64_t n, const double* a, double* out) {
+  launch_pdl(st, k_invert, grid1d(n, 256), 256, 0, n, a, out);
+  TOPX_CUDA_OK(cudaGetLastError());
+}
+
 // interleaved compact DOF vector (3k+c) -> SoA dense grid field with unknown contents: every entry is written, zero
 // where the domain has no node (node_id: compact id of a grid node or -1), so that the field needs no zeroing first.
 __global__ void k_fill_grid_nodes(const double* __restrict__ src, double* __restrict__ dst, int64_t nnodes,

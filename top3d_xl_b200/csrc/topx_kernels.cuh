@@ -194,6 +194,10 @@ void launch_convert(cudaStream_t st, const TA* a, TB* b, int64_t n);
 template <typename T>
 void launch_compact_to_grid_nodes(cudaStream_t st, const double* src, T* dst, Grid g, const int32_t* nodMapBack0,
                                   int64_t numNodes);
+// node_id: compact id of a grid node (n of them), or -1
+void launch_index_nodes(cudaStream_t st, const int32_t* nodMapBack0, int64_t numNodes, int32_t* node_id, int64_t n);
+// out = 1 / a, 0 where a is
+void launch_invert(cudaStream_t st, int64_t n, const double* a, double* out);
 void launch_fill_grid_nodes(cudaStream_t st, const double* src, double* dst, Grid g, const int32_t* node_id);
 template <typename T>
 void launch_grid_to_compact_nodes(cudaStream_t st, const T* src, double* dst, Grid g, const int32_t* nodMapBack0,
