@@ -469,3 +469,18 @@ def test_solve_after_a_nan_solve(bad):
         assert its == its0
         assert np.array_equal(u, u0)
         assert np.array_equal(ctx.ku(u0), y0) and np.array_equal(ctx.filter(2.5, E)[0], f0)
+
+
+def test_host_copies_before_and_with_the_slots():
+    # long copies from and to pageable memory: the first 64 MB go through the runtime, later ones through page-locked
+    # slots in chunks of 1 MB (the last one short); both carry every byte, and a new context starts over
+    from top3d_xl_b200 import Context
+    shape = (64, 96, 72)  # 3.4 MB of densities
+    rng = np.random.default_rng(9)
+    for _ in range(2):
+        with Context("fp64") as ctx:
+            ctx.load_voxels(np.ones(shape, bool))
+            for k in range(14):  # 6.8 MB each
+                x = rng.uniform(0.0, 1.0, ctx.numElements)
+                ctx.set_density(x)
+                assert np.array_equal(ctx.density(), x), k

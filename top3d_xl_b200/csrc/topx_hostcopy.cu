@@ -16,11 +16,16 @@ namespace {
 constexpr int kCopyThreads = 4;
 constexpr size_t kChunk = size_t(1) << 20;
 constexpr size_t kStagedFrom = size_t(3) << 20;  // below, starting the threads costs what they save
+// Making and giving back the slots takes 4 to 9 ms, and a staged copy saves about 0.07 ms a MB (100 MB to the device 9.5 ms
+// through the runtime, 2.5 staged; back 6.3, 3.1): they pay from about 100 MB on.  Made after 64 MB of long copies, they
+// cost a program that makes one context after another, each with a few copies, nothing.
+constexpr size_t kSlotsFrom = size_t(64) << 20;
 
 struct Slots {
   std::mutex busy;  // held by the copy that uses the slots
   std::mutex mu;    // guards the rest
   int holders = 0;
+  size_t moved = 0;  // bytes of long copies through the runtime since the first holder came
   char* mem = nullptr;
 } g_slots;
 
@@ -33,10 +38,15 @@ bool page_locked(const void* h) {
   return a.type != cudaMemoryTypeUnregistered;
 }
 
-char* slots_memory() {
+// the slots, or null while a copy of `bytes` goes through the runtime
+char* slots_memory(size_t bytes) {
   std::lock_guard<std::mutex> lock(g_slots.mu);
-  if (!g_slots.mem && g_slots.holders > 0 &&
-      cudaHostAlloc(reinterpret_cast<void**>(&g_slots.mem), kCopyThreads * 2 * kChunk, cudaHostAllocPortable) != cudaSuccess) {
+  if (g_slots.mem || g_slots.holders == 0) return g_slots.mem;
+  if (g_slots.moved < kSlotsFrom) {
+    g_slots.moved += bytes;
+    return nullptr;
+  }
+  if (cudaHostAlloc(reinterpret_cast<void**>(&g_slots.mem), kCopyThreads * 2 * kChunk, cudaHostAllocPortable) != cudaSuccess) {
     cudaGetLastError();
     g_slots.mem = nullptr;
   }
@@ -78,7 +88,7 @@ cudaError_t share(int w, int device, char* slots, char* d, char* h, size_t bytes
 void copy(char* d, char* h, size_t bytes, bool to_device, cudaStream_t st) {
   if (bytes >= kStagedFrom && !page_locked(h)) {
     std::unique_lock<std::mutex> lock(g_slots.busy, std::try_to_lock);
-    char* mem = lock.owns_lock() ? slots_memory() : nullptr;
+    char* mem = lock.owns_lock() ? slots_memory(bytes) : nullptr;
     if (mem) {
       int device = 0;
       TOPX_CUDA_OK(cudaGetDevice(&device));
@@ -117,10 +127,10 @@ HostCopyHold::HostCopyHold() {
 }
 HostCopyHold::~HostCopyHold() {
   std::lock_guard<std::mutex> lock(g_slots.mu);
-  if (--g_slots.holders == 0 && g_slots.mem) {
-    cudaFreeHost(g_slots.mem);
-    g_slots.mem = nullptr;
-  }
+  if (--g_slots.holders > 0) return;
+  if (g_slots.mem) cudaFreeHost(g_slots.mem);
+  g_slots.mem = nullptr;
+  g_slots.moved = 0;
 }
 
 }  // namespace topx

@@ -15,8 +15,9 @@ namespace topx {
 void host_to_device(void* d, const void* h, size_t bytes, cudaStream_t st);
 void device_to_host(void* h, const void* d, size_t bytes, cudaStream_t st);
 
-// The page-locked slots (kCopyThreads x 2 x 1 MB) are shared by the process: made at the first long copy, used by one
-// copy at a time (another thread's copy meanwhile goes through the runtime), given back when the last holder is gone.
+// The page-locked slots (kCopyThreads x 2 x 1 MB) are shared by the process: made once long copies have moved 64 MB (those
+// before go through the runtime), used by one copy at a time (another thread's copy meanwhile goes through the
+// runtime), given back when the last holder is gone.
 class HostCopyHold {
  public:
   HostCopyHold();
