@@ -484,3 +484,76 @@ def test_host_copies_before_and_with_the_slots():
                 x = rng.uniform(0.0, 1.0, ctx.numElements)
                 ctx.set_density(x)
                 assert np.array_equal(ctx.density(), x), k
+
+
+@pytest.mark.parametrize("shape", [(56, 48, 56), (52, 56, 52)])
+def test_galerkin_blocks_on_both_sides_of_the_line(shape):
+    # extents are padded to multiples of 8, level 2 has 14 x 12 x 14 = 2352 elements, just below the line at 2368 (two to a
+    # block), or 14 x 14 x 14 = 2744, above it (sixteen to a block, the last one short); groups that are void, and
+    # elements with BC-modified templates, in both; test_vcycle's bar
+    from top3d_xl_b200 import Context
+    vox = np.ones(shape, bool)
+    vox[:, 20:40, 12:24] = False  # 14 x 5 level-2 elements in a row of the numbering, three times
+    vox[8:30, 4:18, 30:41] = False
+    m = O.build_model(vox)
+    L2 = m.levels[1]
+    n2 = L2.resX * L2.resY * L2.resZ
+    assert n2 == {48: 2352, 56: 2744}[shape[1]] and (n2 < 148 * 16) == (shape[1] == 48)
+    assert n2 < 148 * 16 or n2 % 16 != 0
+    x = np.random.default_rng(1).uniform(0.3, 1.0, m.levels[0].numElements)
+    S = m.S
+    E = S.modulusMin + x ** S.SIMPpenalty * (S.modulus - S.modulusMin)
+    sol = O.Solver(m)
+    sol.assemble(E)
+    with Context("fp64") as ctx:
+        ctx.load_voxels(vox)
+        ctx.set_moduli(E)
+        ctx.assemble()
+        for seed in (3, 4):
+            r = np.random.default_rng(seed).standard_normal(m.levels[0].numDOFs)
+            assert _rel(ctx.vcycle(r), sol.vcycle(r)) < 1e-10
+
+
+@pytest.mark.parametrize("shape,zlo,zhi", [((31, 48, 63), 10, 49), ((31, 31, 100), 13, 91)])
+@pytest.mark.parametrize("precision", ["fp64", "mixed32"])
+def test_tile_lists_with_gaps(shape, zlo, zhi, precision):
+    # a void larger than a tile along y, x and z, which begins and ends inside z-chunks: the launches of K*u, of the fused
+    # PCG step and of the filter take lists with gaps inside the domain, and planes [lo, hi) of a chunk that begin after
+    # or end before the chunk's own (for the first shape 48 of 264 K*u tiles are left out, 4 begin late and 16 end early).
+    # Bars: test_ku_tile_edges', test_vcycle's and test_filter_tile_edges'; the solve goes to 1e-8, so that its compliance
+    # is within 1e-8 of the oracle's (its error is of the order of the residual's square), with counts within a twentieth
+    # (a tenth with the preconditioner in FP32)
+    from top3d_xl_b200 import Context
+    vox = np.ones(shape, bool)
+    vox[3:, shape[1] // 5:shape[1] - 5, zlo:zhi] = False
+    m = O.build_model(vox)
+    x = np.random.default_rng(1).uniform(0.3, 1.0, m.levels[0].numElements)
+    S = m.S
+    E = S.modulusMin + x ** S.SIMPpenalty * (S.modulus - S.modulusMin)
+    sol = O.Solver(m)
+    sol.assemble(E)
+    f = m.F[:, 0]
+    uo, itso, _ = O.pcg(sol.ku, sol.vcycle, f, 1e-8, 800)
+    u = np.random.default_rng(2).standard_normal(m.levels[0].numDOFs)
+    src = np.random.default_rng(6).uniform(0, 1, m.levels[0].numElements)
+    with Context(precision, tol=1e-8) as ctx:
+        ctx.load_voxels(vox)
+        ctx.set_moduli(E)
+        assert _rel(ctx.ku(u), sol.ku(u)) < 1e-13
+        ctx.assemble()
+        assert _rel(ctx.vcycle(u), sol.vcycle(u)) < (1e-10 if precision == "fp64" else 1e-5)
+        ug, its = ctx.pcg()
+        assert itso < 800 and abs(its - itso) <= max(1, itso // (20 if precision == "fp64" else 10))
+        assert abs(f @ ug - f @ uo) / abs(f @ uo) < 1e-8
+    with Context(precision) as ctx:
+        ctx.load_voxels(vox)
+        for rmin in (np.sqrt(3), 6.0):
+            out, its = ctx.filter(rmin, src)
+            flt = O.PDEFilter(m, rmin, m.S)
+            ref = flt(src)
+            if precision == "fp64":
+                assert its == flt.last_its
+                assert _rel(out, ref) < 1e-10
+            else:
+                assert abs(its - flt.last_its) <= 1
+                assert _rel(out, ref) < 1e-3
