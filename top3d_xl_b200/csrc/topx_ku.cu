@@ -150,7 +150,8 @@ __device__ __forceinline__ void ku_layer(const KuModes& K, double E, double (&W0
 // value per node: the diagonal entries of its free DOFs are equal) and the level-2 correction xc, so no
 // pass over the level-1 grid writes or reads z.  TC: the preconditioner's type.
 // Both store p, reduce p'q into sc->pq and apply the previous iteration's solution step y += lam p_in.
-template <int MODE, typename TC>
+// OFF: the type of a node's byte offset.
+template <int MODE, typename TC, typename OFF>
 __global__ void __launch_bounds__(KU_NT, KU_CTAS)
     k_ku(const __grid_constant__ KuArgs a, const __grid_constant__ KuMaps maps, const KuStage sg, const unsigned bytes) {
   constexpr bool PCG = MODE != KU_PLAIN;
@@ -178,8 +179,8 @@ __global__ void __launch_bounds__(KU_NT, KU_CTAS)
   const bool in_tile = lx < a.sh.PX;
   const bool inb = in_tile && gy >= 0 && gy < nny && gx >= 0 && gx < nnx;
   const bool own = inb && ly >= 1 && ly <= a.sh.TY && lx >= 1 && lx <= a.sh.TX;
-  // byte offsets of the node on plane 0 and of a plane (an array has less than 4 GB: checked at launch)
-  const uint32_t n0 = inb ? 8u * uint32_t(gy + nny * gx) : 0u, np = 8u * uint32_t(nny) * uint32_t(nnx);
+  // byte offsets of the node on plane 0 and of a plane
+  const OFF n0 = inb ? 8u * OFF(gy + nny * gx) : 0u, np = 8u * OFF(nny) * OFF(nnx);
   // the node's place in a box of TY + 4 rows from y0 - 2, and (own nodes) in y's box of the tile itself
   const int PB = a.sh.TY + 4, bx = PB * a.sh.PX, o = in_tile ? lx * PB + ly + 1 : 0;
   const int oy = own ? (lx - 1) * a.sh.TY + ly - 1 : 0, by = a.sh.TY * a.sh.TX;
@@ -243,7 +244,7 @@ __global__ void __launch_bounds__(KU_NT, KU_CTAS)
   issue(zc0 - 1, 0);
   issue(zc0, 1);
   auto flags_at = [&](int zp) -> unsigned {
-    return inb && zp >= 0 && zp < nnz ? unsigned(a.flags[(n0 + np * uint32_t(zp)) / 8u]) : 0u;
+    return inb && zp >= 0 && zp < nnz ? unsigned(a.flags[(n0 + np * OFF(zp)) / 8u]) : 0u;
   };
   unsigned f = flags_at(zc0 - 1), fo = 0;  // of the plane, and of the one below
   const bool first = PCG && (MODE == KU_FUSED ? a.sc->its == 0 : a.sc->first != 0);
@@ -281,7 +282,7 @@ __global__ void __launch_bounds__(KU_NT, KU_CTAS)
   // Plane zp in slot s, and the element layer below it (between the faces Wp and W): plane zp - 1 is then
   // complete.  G holds its forces in face modes, Bn takes the layer's part of plane zp's.
   auto step = [&](int zp, int s, double (&Wp)[3][4], double (&W)[3][4], double (&G)[3][4], double (&Bn)[3][4]) {
-    const uint32_t n = n0 + np * uint32_t(zp);
+    const OFF n = n0 + np * OFF(zp);
     const bool mine = own && zp >= zc0 && zp < zend;
     const double* st = ku_stages + s * sg.len;
     if (ok) ok = plane_wait(sm.bar, zp - zc0 + 1, zend - zc0 + 1, t == 0);
@@ -358,7 +359,7 @@ __global__ void __launch_bounds__(KU_NT, KU_CTAS)
         }
         __syncthreads();
         if (own) {
-          const uint32_t m = n - np;
+          const OFF m = n - np;
           double p[3];
 #pragma unroll
           for (int c = 0; c < 3; ++c) {
@@ -425,9 +426,14 @@ __global__ void __launch_bounds__(KU_NT, KU_CTAS)
   }
 }
 
+// Grids below this many nodes have fields of less than 4 GB, whose offsets fit 32 bits and cost no instruction;
+// beyond, the same kernel with 64-bit offsets.
+constexpr int64_t kOffset32Nodes = int64_t(1) << 29;
+
 template <int MODE, typename TC>
 void ku_smem_attr() {
-  TOPX_CUDA_OK(cudaFuncSetAttribute(k_ku<MODE, TC>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024 / KU_CTAS));
+  for (auto kernel : {k_ku<MODE, TC, uint32_t>, k_ku<MODE, TC, uint64_t>})
+    TOPX_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024 / KU_CTAS));
 }
 
 }  // namespace
@@ -512,7 +518,6 @@ KuModes ku_modes(const double* Ke576) {
 // chunks at the sizes above found at most 5 % more.
 KuShape ku_shape(Grid g, int rows) {
   const int nny = rows, nnx = g.nnx(), nnz = g.nnz();
-  if (g.nnodes() >= (int64_t(1) << 29)) throw std::runtime_error("grid too large for 32-bit byte offsets");
   const double slots = double(KU_CTAS) * num_sms();
   KuShape best{};
   double bestCost = -1;
@@ -595,7 +600,8 @@ static void launch(cudaStream_t st, const KuArgs& a, dim3 grd) {
   }
   sg.len = at;
   const size_t smem = sizeof(double) * 2 * size_t(at) + sizeof(KuSmem<MODE>);
-  launch_pdl(st, k_ku<MODE, TC>, grd, KU_NT, smem, a, m, sg, unsigned(8 * used));
+  launch_pdl(st, a.g.nnodes() < kOffset32Nodes ? k_ku<MODE, TC, uint32_t> : k_ku<MODE, TC, uint64_t>, grd, KU_NT, smem, a, m,
+             sg, unsigned(8 * used));
 }
 void launch_ku(cudaStream_t st, KuMode mode, const KuArgs& args, int ntiles) {
   const dim3 grd = args.active ? dim3(unsigned(ntiles)) : args.sh.grid;

@@ -7,9 +7,9 @@
 
 namespace topx {
 
-// an array element at a 32-bit byte offset from a uniform base
-template <typename T>
-__device__ __forceinline__ T* at(T* base, uint32_t bytes) {
+// an array element at a byte offset (32 bits: no address arithmetic) from a uniform base
+template <typename T, typename OFF>
+__device__ __forceinline__ T* at(T* base, OFF bytes) {
   using C = typename std::conditional<std::is_const<T>::value, const char, char>::type;
   return reinterpret_cast<T*>(reinterpret_cast<C*>(base) + bytes);
 }
