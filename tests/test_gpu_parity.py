@@ -440,21 +440,23 @@ def test_pcg_end_is_one_decision(shape, precision):
 
 
 @pytest.mark.parametrize("bad", ["start", "moduli"])
-def test_solve_after_a_nan_solve(bad):
+@pytest.mark.parametrize("shape,cycle", [((20, 36, 24), "Adapted"), ((50, 100, 50), "Adapted")])
+def test_solve_after_a_nan_solve(shape, cycle, bad):
     # a solve that ends in NaN (a NaN in its start vector or moduli) leaves nothing behind, off the domain either: the next
     # solve on the context is the one that a fresh context computes
     from top3d_xl_b200 import Context
-    vox = np.ones((20, 36, 24), bool)
-    vox[6:14, 10:24, 5:18] = False
-    vox[:, 28:, 12:] = False
+    ny, nx, nz = shape
+    vox = np.ones(shape, bool)
+    vox[ny // 4:3 * ny // 4, nx // 4:2 * nx // 3, nz // 4:3 * nz // 4] = False
+    vox[:, 4 * nx // 5:, nz // 2:] = False
     E = np.random.default_rng(1).uniform(0.05, 1.0, int(vox.sum()))
-    with Context("fp64", maxIT=200) as ctx:
+    with Context("fp64", maxIT=200, typeVcycle=cycle) as ctx:
         ctx.load_voxels(vox)
         ctx.set_moduli(E)
         ctx.assemble()
         u0, its0 = ctx.pcg()
         assert its0 < 200 and np.isfinite(u0).all()
-        y0, f0 = ctx.ku(u0), ctx.filter(2.5, E)[0]
+        y0, f0, z0 = ctx.ku(u0), ctx.filter(2.5, E)[0], ctx.vcycle(u0)
         if bad == "start":
             ctx.pcg(np.full(ctx.numDOFs, np.nan))
         else:
@@ -465,6 +467,7 @@ def test_solve_after_a_nan_solve(bad):
             ctx.assemble()
         ctx.ku(np.full(ctx.numDOFs, np.nan))
         ctx.filter(2.5, np.full(E.size, np.nan))
+        assert np.array_equal(ctx.vcycle(u0), z0)
         u, its = ctx.pcg()
         assert its == its0
         assert np.array_equal(u, u0)

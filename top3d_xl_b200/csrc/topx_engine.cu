@@ -927,7 +927,7 @@ void Engine::apply_vcycle(const double* h_r, double* h_z) {
   double* v = host_vector();
   copy_sync(v, h_r, sizeof(double) * Nn * 3, cudaMemcpyHostToDevice);
   TOPX_CUDA_OK(cudaMemsetAsync(scE.p, 0, sizeof(PcgScalars), st));
-  launch_compact_to_grid_nodes<double>(st, v, kw.r.p, G[0], nodMapBack0.p, Nn);
+  launch_fill_grid_nodes(st, v, kw.r.p, G[0], nodMapFwd0.p);  // absent nodes too, as in set_U
   if (standard())
     vcycle_standard(true, scE.p);
   else if (!pre32())
