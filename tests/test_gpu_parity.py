@@ -440,7 +440,7 @@ def test_pcg_end_is_one_decision(shape, precision):
 
 
 @pytest.mark.parametrize("bad", ["start", "moduli"])
-@pytest.mark.parametrize("shape,cycle", [((20, 36, 24), "Adapted"), ((50, 100, 50), "Adapted")])
+@pytest.mark.parametrize("shape,cycle", [((20, 36, 24), "Adapted"), ((50, 100, 50), "Adapted"), ((50, 100, 50), "Standard")])
 def test_solve_after_a_nan_solve(shape, cycle, bad):
     # a solve that ends in NaN (a NaN in its start vector or moduli) leaves nothing behind, off the domain either: the next
     # solve on the context is the one that a fresh context computes

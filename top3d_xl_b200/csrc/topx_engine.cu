@@ -674,13 +674,13 @@ void Engine::vcycle_standard(bool init, PcgScalars* sc) {
   sec_begin(SEC_RESTRICT);
   launch_jacobi_pre<double, double, double>(st, G[0], kw.r.p, v.d1.p, present[0].p, kw.z.p, om, sc);
   ku(KU_PLAIN, kw.z.p, nullptr, nullptr, kw.q.p, sc, nullptr);
-  launch_residual_inplace<double, double>(st, G[0], kw.r.p, kw.q.p, sc);
+  launch_residual_inplace<double, double>(st, G[0], kw.r.p, present[0].p, kw.q.p, sc);
   residual(RES_KEEP, kw.q.p, nullptr, sc, 0.0, 0);
   launch_restrict_xz<double>(st, kw.ty.p, G[0], v.rl[1].p, nullptr, G[1], sc);
   for (int l = 1; l < nl - 1; ++l) {
     launch_jacobi_pre<double, double, double>(st, G[l], v.rl[l].p, v.dl[l].p, present[l].p, v.xl[l].p, om, sc);
     launch_ku_coarse(st, G[l], Ks[l].p, epresent[l].p, present[l].p, v.xl[l].p, vq[l].p, sc);
-    launch_residual_inplace<double, double>(st, G[l], v.rl[l].p, vq[l].p, sc);
+    launch_residual_inplace<double, double>(st, G[l], v.rl[l].p, present[l].p, vq[l].p, sc);
     launch_restrict<double>(st, vq[l].p, G[l], v.tmp1.p, v.tmp2.p, v.rl[l + 1].p, G[l + 1], sc);
   }
   sec_end();

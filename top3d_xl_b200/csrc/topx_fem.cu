@@ -639,20 +639,23 @@ void launch_jacobi_pre(cudaStream_t st, Grid g, const TR* r, const TD* d, const 
   TOPX_CUDA_OK(cudaGetLastError());
 }
 
-// q = r - q: the residual after pre-smoothing, restricted next (TX:761-762)
+// q = r - q: the residual after pre-smoothing, restricted next (TX:761-762).  Zero on absent nodes: where the K*u's tiles
+// leave some out, q keeps what stands there, a NaN of an earlier solve too.
 template <typename TR, typename T>
-__global__ void k_residual_inplace(Grid g, const TR* __restrict__ r, T* __restrict__ q, const PcgScalars* sc) {
+__global__ void k_residual_inplace(Grid g, const TR* __restrict__ r, const uint8_t* __restrict__ present,
+                                   T* __restrict__ q, const PcgScalars* sc) {
   pdl_wait();
   if (sc->done) return;
   const int64_t N = g.nnodes();
   for (int64_t n = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; n < N; n += int64_t(gridDim.x) * blockDim.x) {
+    const bool pres = present[n] != 0;
 #pragma unroll
-    for (int c = 0; c < 3; ++c) q[n + c * g.stride] = T(r[n + c * g.stride]) - q[n + c * g.stride];
+    for (int c = 0; c < 3; ++c) q[n + c * g.stride] = pres ? T(r[n + c * g.stride]) - q[n + c * g.stride] : T(0);
   }
 }
 template <typename TR, typename T>
-void launch_residual_inplace(cudaStream_t st, Grid g, const TR* r, T* q, const PcgScalars* sc) {
-  launch_pdl(st, k_residual_inplace<TR, T>, grid1d(g.nnodes(), 256), 256, 0, g, r, q, sc);
+void launch_residual_inplace(cudaStream_t st, Grid g, const TR* r, const uint8_t* present, T* q, const PcgScalars* sc) {
+  launch_pdl(st, k_residual_inplace<TR, T>, grid1d(g.nnodes(), 256), 256, 0, g, r, present, q, sc);
   TOPX_CUDA_OK(cudaGetLastError());
 }
 
@@ -907,7 +910,8 @@ template void launch_prolong_add<double, double, double>(cudaStream_t, int, cons
                                                         PcgScalars*);
 template void launch_jacobi_pre<double, double, double>(cudaStream_t, Grid, const double*, const double*,
                                                         const uint8_t*, double*, double, const PcgScalars*);
-template void launch_residual_inplace<double, double>(cudaStream_t, Grid, const double*, double*, const PcgScalars*);
+template void launch_residual_inplace<double, double>(cudaStream_t, Grid, const double*, const uint8_t*, double*,
+                                                      const PcgScalars*);
 template void launch_jacobi_correct<double, double, double>(cudaStream_t, Grid, const double*, const double*,
                                                             const double*, const uint8_t*, double*, double, bool,
                                                             bool, PcgScalars*, RedScratch);

@@ -182,7 +182,7 @@ template <typename TR, typename T, typename TD>
 void launch_jacobi_pre(cudaStream_t st, Grid g, const TR* r, const TD* d, const uint8_t* present, T* x, double omega,
                        const PcgScalars* sc);
 template <typename TR, typename T>
-void launch_residual_inplace(cudaStream_t st, Grid g, const TR* r, T* q, const PcgScalars* sc);
+void launch_residual_inplace(cudaStream_t st, Grid g, const TR* r, const uint8_t* present, T* q, const PcgScalars* sc);
 template <typename TR, typename T, typename TD>
 void launch_jacobi_correct(cudaStream_t st, Grid g, const TR* r, const T* q, const TD* d, const uint8_t* present,
                            T* x, double omega, bool dot, bool init, PcgScalars* sc, RedScratch rs);
