@@ -163,8 +163,9 @@ topx_status topx_set_moduli(topx_ctx* ctx, const double* E, size_t n);
 topx_status topx_ku(topx_ctx* ctx, const double* u, double* y, size_t ndof);
 /* No counterpart in the reference.  y = K(E) u exactly like topx_ku, but u and y are device
    pointers (ndof doubles each, on the context's GPU) and the call allocates no device memory:
-   topx_ku allocates temporary device buffers on every call, which callers whose device memory
-   is owned by another allocator (MATLAB gpuArray, a framework's caching pool) or whose loop may
+   topx_ku, like the other calls with host vectors, allocates a device vector of ndof doubles the
+   first time and keeps it until the context is destroyed, which callers whose device memory is
+   owned by another allocator (MATLAB gpuArray, a framework's caching pool) or whose loop may
    not call cudaMalloc/cudaFree cannot accept.  Its scratch is one fixed 32 MiB static device
    array, enough for level-1 grids of up to 699,040 padded nodes; larger models get
    TOPX_ERR_ARG.  The context's device state must exist already (e.g. after topx_set_moduli).

@@ -1,6 +1,7 @@
 // Allocation-free level-1 operator application (topx_ku_noalloc in include/topx.h).
 //
-// topx_ku copies its host vectors through device buffers that it allocates on every call.
+// topx_ku copies its host vectors through a device vector that it allocates on its first call and keeps until the
+// context is destroyed (24 bytes per node).
 // Some callers cannot allow that: a host whose device memory is all handed out by its own
 // pool or allocator (MATLAB's gpuArray manager, a framework's caching allocator capped to a
 // fraction of the GPU), or a real-time loop that must not call cudaMalloc/cudaFree, which
